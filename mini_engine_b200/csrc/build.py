@@ -31,6 +31,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fPIC
 LIBRARIES = {
     "elementwise": "elementwise.cu",
     "gemm_simt": "gemm_simt.cu",
+    "gemm_split": "gemm_split.cu",
     "attention_generic": "attention_generic.cu",
     "attention_biased": "attention_biased.cu",
     "latent_attention": "latent_attention.cu",

@@ -438,6 +438,20 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
     _check(code, "gemm_simt")
 
 
+def split_gemm_supports(weight: torch.Tensor) -> bool:
+    """Whether the float32 tensor-core product takes this weight; others take the CUDA-core kernel."""
+    return tensor_core.split_supports(weight)
+
+
+def SplitPlan(weight: torch.Tensor):
+    return tensor_core.SplitPlan(weight)
+
+
+def gemm_split(plan, x: torch.Tensor, out: torch.Tensor) -> None:
+    """``out[T, N] = x[T, K] @ weight[N, K]^T`` in float32 on the tensor cores."""
+    tensor_core.gemm_split(plan, x, out)
+
+
 def tensor_core_gemm_supports(outs: int, inner: int) -> bool:
     """TMA addresses rows whose pitch is a multiple of 16 bytes: ``inner % 8 == 0`` for
     bfloat16.  Other shapes take the CUDA-core kernel."""

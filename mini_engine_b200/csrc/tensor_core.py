@@ -236,6 +236,107 @@ def gemm_swiglu(
         raise RuntimeError(f"gated tensor-core product failed to launch (code {code})")
 
 
+# ------------------------------------------------------------------------------ float32
+
+SPLIT_TILES = (16, 64)  # tokens per CTA: up to 16 two CTAs share an SM and stream weights, else one
+SPLIT_MIN_K_BLOCKS = 4  # of a segment
+# Shorter reductions stay on CUDA cores: a chain of fmaf over so few terms is as exact as the short chain of the tensor
+# core (relative error at 64: 1.5e-7 against 1.2e-7; at 4: 4e-8 against 7e-8), and nothing is to be gained.
+SPLIT_MIN_INNER = 64
+_split_lib = None
+
+
+def _split_library():
+    global _split_lib
+    if _split_lib is None:
+        lib = load_library("gemm_split")
+        lib.me_make_tensor_map_f32.argtypes = [c_void_p, c_void_p, c_ulonglong, c_ulonglong, c_uint]
+        lib.me_make_tensor_map_f32.restype = c_int
+        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 6 + [c_void_p]
+        lib.me_gemm_split.restype = c_int
+        lib.me_gemm_split_take_error.argtypes = [ctypes.POINTER(c_int)]
+        lib.me_gemm_split_take_error.restype = c_int
+        _split_lib = lib
+    return _split_lib
+
+
+def split_supports(weight: torch.Tensor) -> bool:
+    """TMA wants a 16-byte aligned start and row pitch: ``inner`` a multiple of 4 float32 values.  A property of the weight
+    alone: every step of a model takes the same kernel."""
+    return (
+        weight.dtype == torch.float32 and weight.is_cuda and weight.is_contiguous()
+        and weight.shape[1] % 4 == 0 and weight.shape[1] >= SPLIT_MIN_INNER and weight.data_ptr() % 16 == 0
+    )  # fmt: skip
+
+
+def split_segments(outs: int, inner: int) -> int:
+    """Ranges of k blocks that an output's sum is formed in.  From the weight's shape alone, never from the tokens: a row's
+    bits must not depend on the batch.  About one CTA per SM when a single token tile runs with its segments side by side."""
+    tiles, k_blocks = -(-outs // BLOCK_N), -(-inner // BLOCK_K)
+    wanted = min(8, max(1, 160 // tiles), max(1, k_blocks // SPLIT_MIN_K_BLOCKS))
+    per_segment = -(-k_blocks // wanted)
+    return -(-k_blocks // per_segment)
+
+
+def split_side_by_side(tokens: int, outs: int, segments: int) -> bool:
+    """Whether a tile's segments run in the CTAs of a cluster (few tiles) or one after the other in a CTA; the bits are the
+    same.  Side by side when that takes fewer rounds of resident CTAs, a round being one segment long."""
+    tile = SPLIT_TILES[0] if tokens <= SPLIT_TILES[0] else SPLIT_TILES[1]
+    slots = NUM_SMS * (2 if tile == SPLIT_TILES[0] else 1)
+    ctas = -(-outs // BLOCK_N) * -(-tokens // tile)
+    return -(-ctas * segments // slots) < -(-ctas // slots) * segments
+
+
+class SplitPlan:
+    """A float32 weight for :func:`gemm_split`."""
+
+    def __init__(self, weight: torch.Tensor):
+        if not split_supports(weight):
+            raise RuntimeError(f"the float32 tensor-core product takes a contiguous float32 CUDA weight whose width is a multiple of 4 and at least {SPLIT_MIN_INNER}")
+        self.weight = weight
+        self.rows, self.inner = weight.shape
+        self.segments = split_segments(self.rows, self.inner)
+        self.map = _make_map_f32(weight, BLOCK_N)
+
+
+def _make_map_f32(tensor: torch.Tensor, box_rows: int) -> ctypes.Array:
+    holder = (ctypes.c_ubyte * 128)()
+    rows, inner = tensor.shape
+    code = _split_library().me_make_tensor_map_f32(holder, tensor.data_ptr(), rows, inner, box_rows)
+    if code != 0:
+        raise RuntimeError(f"could not make a TMA descriptor for a {rows} x {inner} float32 matrix (code {code})")
+    return holder
+
+
+_split_activation_maps: dict[tuple[int, int, int, int], ctypes.Array] = {}
+
+
+def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side: bool | None = None) -> None:
+    """``out[T, rows] = x @ weight^T`` in float32 (three bfloat16 pieces of each operand, see gemm_split.cu).
+    ``side_by_side`` pins where a tile's segments run instead of the rule's choice: the kernel tests run both."""
+    tokens = x.shape[0]
+    if x.dtype != torch.float32 or not x.is_contiguous() or x.dim() != 2 or x.shape[1] != plan.inner or x.data_ptr() % 16:
+        raise RuntimeError(f"activation {tuple(x.shape)} {x.dtype} does not fit a float32 weight of width {plan.inner}")
+    if out.dtype != torch.float32 or tuple(out.shape) != (tokens, plan.rows) or not out.is_contiguous():
+        raise RuntimeError(f"output {tuple(out.shape)} does not fit [{tokens}, {plan.rows}] float32")
+    tile = SPLIT_TILES[0] if tokens <= SPLIT_TILES[0] else SPLIT_TILES[1]
+    key = (x.data_ptr(), tokens, plan.inner, tile)
+    held = _split_activation_maps.get(key)
+    if held is None:
+        if len(_split_activation_maps) > 8192:
+            _split_activation_maps.clear()
+        held = _split_activation_maps[key] = _make_map_f32(x, tile)
+    if side_by_side is None:
+        side_by_side = split_side_by_side(tokens, plan.rows, plan.segments)
+    code = _split_library().me_gemm_split(
+        plan.map, held, x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,
+        plan.segments, 1 if side_by_side else 0, _ops_stream(),
+    )  # fmt: skip
+    _count_launch()
+    if code != 0:
+        raise RuntimeError(f"float32 tensor-core product failed to launch (code {code})")
+
+
 GROUP_PAD = 128  # rows of a run of the sorted rows that belongs to one group: the token tile of the grouped product
 
 
@@ -287,10 +388,13 @@ def wait_probe(polls: int = 4096) -> bool:
 def take_error() -> int:
     """The first failure that a tensor-core kernel recorded on the device since the last call
     (a wait that ran into its limit), or 0.  Synchronises the device."""
-    if _lib is None:
-        return 0
-    code = c_int(0)
-    status = _lib.me_gemm_take_error(ctypes.byref(code))
-    if status != 0:
-        raise RuntimeError(f"could not read the kernels' error flag (CUDA error {status})")
-    return code.value
+    first = 0
+    for lib, name in ((_lib, "me_gemm_take_error"), (_split_lib, "me_gemm_split_take_error")):
+        if lib is None:
+            continue
+        code = c_int(0)
+        status = getattr(lib, name)(ctypes.byref(code))
+        if status != 0:
+            raise RuntimeError(f"could not read the kernels' error flag (CUDA error {status})")
+        first = first or code.value
+    return first

@@ -9,9 +9,11 @@ YuvGev00/mini-engine) and pick the kernel:
   2,048-token prompt and a single decoded token; for few tokens the reduction axis is
   split over several CTAs and the result comes back as ``S`` partial sums that the consumer
   adds in a fixed order.
-* float32, and bfloat16 shapes that TMA cannot address: a CUDA-core kernel that adds the
-  products of one output element in ascending ``k`` with one accumulator, so a row's
-  result never depends on which other rows are in the batch.
+* float32 with ``in`` a multiple of 4: the tensor-core kernel on three bfloat16 pieces of each
+  operand (their exact sum), with the sums in an order that depends on the weight's shape alone,
+  so a row's result never depends on which other rows are in the batch.
+* shapes that TMA cannot address: a CUDA-core kernel that adds the products of one output
+  element in ascending ``k`` with one accumulator.
 """
 
 from __future__ import annotations
@@ -56,6 +58,7 @@ class Linear:
             self.out_features, self.in_features
         )
         self.plan = ops.GemmPlan(weight) if self.tensor_core else None
+        self.split_plan = ops.SplitPlan(weight) if ops.split_gemm_supports(weight) else None
 
     def forward(self, x: torch.Tensor, ctx: StepContext, out_name: str, whole: bool = False) -> torch.Tensor:
         """``x [T, in]`` -> ``[S, T, out]`` float32 in the named workspace buffer.  With
@@ -71,6 +74,8 @@ class Linear:
             out = ctx.workspace.partials(out_name, splits, tokens, self.out_features)
         if self.tensor_core:
             ops.gemm_tensor_core(self.plan, x, out, splits)
+        elif self.split_plan is not None:
+            ops.gemm_split(self.split_plan, x, out[0])
         else:
             ops.gemm_simt(x, self.weight, out[0])
         return out

@@ -1,0 +1,91 @@
+"""The float32 product on the tensor cores (three bfloat16 pieces of each operand): against float64, beside the
+CUDA-core kernel's error, and the order of its sums."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+
+def tensor_core():
+    from mini_engine_b200.csrc import tensor_core as module
+
+    return module
+
+
+@pytest.mark.parametrize("outs", [1, 128, 130, 2048, 4096, 6144, 24576, 151936])
+@pytest.mark.parametrize("inner", [64, 260, 1024, 4096, 12288])
+def test_segments_cover_the_reduction(outs, inner):
+    tc = tensor_core()
+    segments = tc.split_segments(outs, inner)
+    blocks = -(-inner // tc.BLOCK_K)
+    per_segment = -(-blocks // segments)
+    assert 1 <= segments <= 8
+    assert (segments - 1) * per_segment < blocks <= segments * per_segment  # none is empty, none is missing
+
+
+# tokens: one, a full and an overfull small tile, a full and an overfull large tile; outs: less than a tile, a ragged
+# second tile; inner: one block, a partial block, several segments of which the last is shorter
+SHAPES = [(1, 5, 64), (16, 128, 100), (17, 130, 68), (64, 200, 2048), (65, 300, 1100), (130, 520, 260), (8, 2048, 2816), (300, 4096, 1000)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,outs,inner", SHAPES)
+def test_split_product(tokens, outs, inner):
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(3)
+    x = torch.randn(tokens, inner, device="cuda") * torch.exp(2 * torch.randn(tokens, 1, device="cuda"))
+    w = torch.randn(outs, inner, device="cuda")
+    plan = tc.SplitPlan(w)
+    simt = torch.empty(tokens, outs, device="cuda")
+    ops.gemm_simt(x, w, simt)
+    want = x.double() @ w.double().T
+
+    def error(y):
+        return float(((y.double() - want) / want.norm(dim=1, keepdim=True)).norm())
+
+    out = torch.full((tokens, outs), float("nan"), device="cuda")
+    tc.gemm_split(plan, x, out, side_by_side=False)
+    assert tc.take_error() == 0
+    # no less exact than the fmaf chain; a quarter more for the few outputs of the small shapes
+    assert error(out) <= 1.25 * error(simt)
+    # the same bits with the segments in a cluster, and for rows of another batch (another token tile)
+    other = torch.full((tokens, outs), float("nan"), device="cuda")
+    tc.gemm_split(plan, x, other, side_by_side=True)
+    assert tc.take_error() == 0
+    assert torch.equal(out, other)
+    for rows in (slice(tokens // 2, tokens // 2 + 1), slice(0, min(tokens, 16)), slice(tokens // 3, tokens)):
+        part = torch.empty(len(range(*rows.indices(tokens))), outs, device="cuda")
+        tc.gemm_split(plan, x[rows].clone(), part)
+        assert torch.equal(part, out[rows])
+
+
+@pytest.mark.gpu
+def test_infinities_and_nan_come_out_as_in_one_chain():
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(4)
+    x, w = torch.randn(40, 256, device="cuda"), torch.randn(130, 256, device="cuda")
+    x[3, 5], x[4, 7], w[9, 5], w[7, 3] = float("inf"), float("nan"), 1.0, -float("inf")
+    x[6] *= 1e38
+    x[8], w[11] = 1e-38, 1e-38
+    out, want = torch.empty(40, 130, device="cuda"), torch.empty(40, 130, device="cuda")
+    tc.gemm_split(tc.SplitPlan(w), x, out)
+    ops.gemm_simt(x, w, want)
+    assert torch.equal(torch.isnan(out), torch.isnan(want))
+    odd = torch.isinf(want)
+    assert odd.any() and torch.equal(out[odd], want[odd]) and not torch.isinf(out[~odd]).any()
+
+
+@pytest.mark.gpu
+def test_weights_that_tma_cannot_address_are_refused_by_the_rule():
+    tc = tensor_core()
+    base = torch.randn(4 * 128 + 1, device="cuda")
+    assert tc.split_supports(base[: 4 * 128].view(4, 128))
+    assert not tc.split_supports(base[1:].view(4, 128))  # starts on 4 bytes
+    assert not tc.split_supports(torch.randn(4, 130, device="cuda"))
+    assert not tc.split_supports(torch.randn(4, 60, device="cuda"))
+    assert not tc.split_supports(torch.randn(4, 128, device="cuda").to(torch.bfloat16))
