@@ -16,7 +16,7 @@
 // head g's warp applies its weights to the values of EVERY KV head c: A[g][c] = sum_j w_g(j) v_c(j).
 // The mixed output of head h is then sum_g talk[h][g] * A[g][kv(h)], which a second small kernel forms.
 // The weights themselves are never stored and one pass over the keys suffices.
-#include "common.cuh"
+#include "mma_sync.cuh"
 
 #include <algorithm>
 
@@ -622,6 +622,349 @@ ME_EXPORT int me_mixed_attention(const void* q, const void* k_pages, const void*
     if (type != ME_BF16) return launch_two_kernels<float, 4>(s, talk, stream);
     if (static_cast<long long>(tokens) * kv_heads >= 1024) return launch_two_kernels<__nv_bfloat16, 2>(s, talk, stream);
     return launch_two_kernels<__nv_bfloat16, 16>(s, talk, stream);
+}
+
+// ------------------------------------------------- mixing on tensor cores (portions of prompts, bfloat16)
+//
+// A block takes eight consecutive tokens of an entry and all heads; a warp one KV head with its GROUP query heads, two heads
+// to the 16 rows of a product, so its keys, values, scores and output stay with it.  The first walk over the key tiles
+// gives every row's maximum and denominator, the second forms the normalised weights, leaves them in shared memory as two
+// bfloat16 terms (their sum is the weight to 17 bits), mixes them there as products [heads x heads] . [heads x
+// (query, key)], each warp its own columns and in place, and applies them to the values.  Nothing but the output is
+// written.  The distance bias is taken per (head, distance), 39 distances a tile of 32 keys, instead of per score.  Products are m16n8k16 with float32 sums.
+//
+// Bound by the instructions a warp issues around its products (exponentials, masks, the split of the weights), with
+// one block to an SM; see the figures at launch_mixed_tiles.  A tile of eight tokens, since the output of four heads and
+// 16 tokens would take every register of a warp.
+constexpr int TILE_Q = 8, TILE_K = 32, TILE_DIM = 128;
+constexpr int BIAS_SPAN = TILE_Q + TILE_K;  // distances within a tile, one spare
+
+template <int KV, int GROUP>
+struct MixTile {
+    static constexpr int HEADS = KV * GROUP;
+    static constexpr int PITCH = TILE_Q * TILE_K + 8;  // weights of a head, 16 bytes of padding: rows fall into different banks
+    static constexpr int TALK_PITCH = HEADS + 8;
+    static constexpr int KV_BYTES = TILE_K * TILE_DIM * 2;
+    static constexpr int SMEM = 2 * KV * KV_BYTES + 2 * HEADS * PITCH * 2 + 2 * HEADS * TALK_PITCH * 2 + HEADS * BIAS_SPAN * 4;
+};
+
+struct MixTileArgs {
+    BiasedArgs a;
+    const float* talk;
+    const int* cu_tokens;  // [entries + 1]
+};
+
+__device__ __forceinline__ void two_terms(float x, float y, uint32_t& high, uint32_t& low) {
+    high = pack_bf16(x, y);
+    low = pack_bf16(x - __uint_as_float(high << 16), y - __uint_as_float(high & 0xffff0000u));
+}
+
+template <int KV, int GROUP>
+__global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTileArgs m) {
+    using C = MixTile<KV, GROUP>;
+    constexpr int HEADS = C::HEADS, ROWS = GROUP / 2;  // ROWS: products of 16 rows per warp
+    static_assert(GROUP % 2 == 0 && (HEADS == 16 || HEADS == 32), "two heads to a product, 16 or 32 heads to mix");
+    const BiasedArgs& a = m.a;
+    extern __shared__ __align__(16) uint8_t mix_tile_shared[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, q = lane >> 2;
+    __nv_bfloat16* keys = reinterpret_cast<__nv_bfloat16*>(mix_tile_shared) + warp * (C::KV_BYTES / 2);
+    __nv_bfloat16* values = keys + KV * (C::KV_BYTES / 2);
+    __nv_bfloat16* weights = reinterpret_cast<__nv_bfloat16*>(mix_tile_shared) + 2 * KV * (C::KV_BYTES / 2);  // [2][HEADS][PITCH]
+    __nv_bfloat16* talk = weights + 2 * HEADS * C::PITCH;                                               // [2][HEADS][TALK_PITCH]
+    float* bias = reinterpret_cast<float*>(talk + 2 * HEADS * C::TALK_PITCH) + warp * GROUP * BIAS_SPAN;
+    constexpr int PLANE = HEADS * C::PITCH, TALK_PLANE = HEADS * C::TALK_PITCH;
+
+    const int entry = blockIdx.y, begin = m.cu_tokens[entry];
+    const int first = static_cast<int>(gridDim.x - 1 - blockIdx.x) * TILE_Q;  // the last tokens see the most keys: they go first
+    const int count = min(m.cu_tokens[entry + 1] - begin - first, TILE_Q);
+    if (count <= 0) return;
+    const int head0 = warp * GROUP;
+    for (int i = threadIdx.x; i < HEADS * HEADS; i += KV * 32) {
+        const float t = m.talk[i];
+        const __nv_bfloat16 high = __float2bfloat16_rn(t);
+        const int at = i / HEADS * C::TALK_PITCH + i % HEADS;
+        talk[at] = high;
+        talk[TALK_PLANE + at] = __float2bfloat16_rn(t - __bfloat162float(high));
+    }
+    const int p0 = a.positions[begin + first], p_last = p0 + count - 1;
+    const int* table = a.block_table + static_cast<size_t>(entry) * a.table_width;
+    const __nv_bfloat16* k_pages = static_cast<const __nv_bfloat16*>(a.k_pages);
+    const __nv_bfloat16* v_pages = static_cast<const __nv_bfloat16*>(a.v_pages);
+
+    uint32_t query[ROWS][TILE_DIM / 16][4];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int k = 0; k < TILE_DIM / 16; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.q) +
+                    (static_cast<size_t>(begin + first + q) * HEADS + head0 + 2 * r + (i & 1)) * TILE_DIM + 16 * k + 8 * (i >> 1) + 2 * quad;
+                query[r][k][i] = q < count ? *reinterpret_cast<const uint32_t*>(src) : 0u;
+            }
+
+    // Tiles: the kept keys behind every window of the block, then from the first window on.
+    const int lowest = max(p0 - a.window + 1, 0);
+    const int kept = min(a.keep_first, lowest);
+    const int kept_tiles = (kept + TILE_K - 1) / TILE_K, tiles = kept_tiles + p_last / TILE_K - lowest / TILE_K + 1;
+    auto tile_start = [&](int i) { return i < kept_tiles ? i * TILE_K : (lowest / TILE_K + i - kept_tiles) * TILE_K; };
+    // This warp's 32 rows of a page array into shared memory (asynchronous); which keys there are.
+    auto fetch = [&](const __nv_bfloat16* pages, __nv_bfloat16* to, int i) -> uint32_t {
+        const int key = tile_start(i) + lane;
+        long long row = -1;
+        if (i < kept_tiles ? key < kept : key >= lowest && key <= p_last) {
+            const int page = table[key / a.page_size];
+            if (page >= 0) row = ((static_cast<long long>(page) * KV + warp) * a.page_size + key % a.page_size) * TILE_DIM;
+        }
+#pragma unroll
+        for (int j = 0; j < TILE_K / 2; ++j) {
+            const int r = 2 * j + (lane >> 4), chunk = lane & 15;
+            const long long from = __shfl_sync(0xffffffffu, row, r);
+            cp_async_16(to + swizzled<TILE_DIM>(r, chunk) * 8, pages + max(from, 0ll) + chunk * 8, from >= 0);
+        }
+        cp_async_commit();
+        return __ballot_sync(0xffffffffu, row >= 0);
+    };
+    // bias[h][x]: distance x - 31 from the tile's first key to the block's first query
+    auto distances = [&](int i) {
+        const int base = p0 - tile_start(i) - (TILE_K - 1);
+        __syncwarp();
+        for (int x = lane; x < GROUP * BIAS_SPAN; x += 32) {
+            const int h = head0 + x / BIAS_SPAN;
+            bias[x] = a.r1 ? a.r1[h] * logf(1.0f + a.r2[h] * static_cast<float>(max(base + x % BIAS_SPAN, 0))) : 0.0f;
+        }
+        __syncwarp();
+    };
+    // Scores of 16 keys of a tile (`half`), -inf where the query does not see the key.
+    auto scores = [&](const __nv_bfloat16* from, int i, int half, uint32_t there, float (&s)[ROWS][2][4]) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[r][n][c] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < TILE_DIM / 16; ++k) {
+            uint32_t b[4];
+            ldmatrix_x4(b, from + swizzled<TILE_DIM>(half * 16 + (lane >> 4) * 8 + (lane & 7), 2 * k + ((lane >> 3) & 1)) * 8);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                mma_bf16(s[r][0], query[r][k], b[0], b[1]);
+                mma_bf16(s[r][1], query[r][k], b[2], b[3]);
+            }
+        }
+        const int start = tile_start(i);
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int place = half * 16 + n * 8 + 2 * quad + e, distance = p0 + q - start - place;
+                const bool seen = (there >> place & 1u) && distance >= 0 && (distance < a.window || start + place < a.keep_first) && q < count;
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float& v = s[r][n][2 * h + e];
+                        v = seen ? v * a.scale - bias[(2 * r + h) * BIAS_SPAN + q + TILE_K - 1 - place] : -INFINITY;
+                    }
+            }
+    };
+
+    // First walk: maximum and denominator of every row (a lane's own columns, then the four lanes of a row).
+    float top[ROWS][2], total[ROWS][2];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) top[r][0] = top[r][1] = -INFINITY, total[r][0] = total[r][1] = 0.0f;
+    uint32_t there = fetch(k_pages, keys, 0);
+    for (int i = 0; i < tiles; ++i) {
+        __nv_bfloat16* held = i & 1 ? values : keys;
+        uint32_t there_next = 0;
+        if (i + 1 < tiles) there_next = fetch(k_pages, i & 1 ? keys : values, i + 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        distances(i);  // and the warp meets: every lane's copies are there
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float s[ROWS][2][4];
+            scores(held, i, half, there, s);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float peak = fmaxf(top[r][h], fmaxf(fmaxf(s[r][0][2 * h], s[r][0][2 * h + 1]), fmaxf(s[r][1][2 * h], s[r][1][2 * h + 1])));
+                    if (peak == -INFINITY) continue;
+                    total[r][h] = total[r][h] * expf(top[r][h] - peak) + ((expf(s[r][0][2 * h] - peak) + expf(s[r][0][2 * h + 1] - peak)) +
+                                                                            (expf(s[r][1][2 * h] - peak) + expf(s[r][1][2 * h + 1] - peak)));
+                    top[r][h] = peak;
+                }
+        }
+        there = there_next;
+        __syncwarp();  // the next copies overwrite this tile
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float peak = fmaxf(top[r][h], __shfl_xor_sync(0xffffffffu, top[r][h], 1));
+            peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, 2));
+            float sum = peak == -INFINITY ? 0.0f : total[r][h] * expf(top[r][h] - peak);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            top[r][h] = peak;
+            total[r][h] = sum > 0.0f ? 1.0f / sum : 0.0f;
+        }
+
+    // Second walk.
+    float out[ROWS][TILE_DIM / 8][4];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int n = 0; n < TILE_DIM / 8; ++n)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) out[r][n][c] = 0.0f;
+    there = fetch(k_pages, keys, 0);
+    fetch(v_pages, values, 0);
+    for (int i = 0; i < tiles; ++i) {
+        cp_async_wait<1>();
+        distances(i);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float s[ROWS][2][4];
+            scores(keys, i, half, there, s);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float w[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float v = s[r][n][2 * h + e];
+                            w[e] = v == -INFINITY ? 0.0f : expf(v - top[r][h]) * total[r][h];
+                        }
+                        uint32_t high, low;
+                        two_terms(w[0], w[1], high, low);
+                        // columns of a head: (8 keys, query, key), so that a query's eight keys are one 16-byte row
+                        __nv_bfloat16* to = weights + (head0 + 2 * r + h) * C::PITCH + ((half * 2 + n) * TILE_Q + q) * 8 + 2 * quad;
+                        *reinterpret_cast<uint32_t*>(to) = high;
+                        *reinterpret_cast<uint32_t*>(to + PLANE) = low;
+                    }
+        }
+        __syncwarp();
+        if (i + 1 < tiles) there = fetch(k_pages, keys, i + 1);
+        else cp_async_commit();
+        __syncthreads();  // every head's weights
+#pragma unroll
+        for (int column = warp; column < TILE_Q * TILE_K / 8; column += KV) {
+            uint32_t high[HEADS / 8], low[HEADS / 8];  // B operands: eight (query, key) columns of all heads
+            {
+                uint32_t b[4];
+                if constexpr (HEADS == 32) {
+                    ldmatrix_x4_trans(b, weights + lane * C::PITCH + column * 8);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) high[j] = b[j];
+                    ldmatrix_x4_trans(b, weights + PLANE + lane * C::PITCH + column * 8);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) low[j] = b[j];
+                } else {
+                    ldmatrix_x4_trans(b, weights + (lane >> 4) * PLANE + (lane & 15) * C::PITCH + column * 8);
+                    high[0] = b[0], high[1] = b[1], low[0] = b[2], low[1] = b[3];
+                }
+            }
+            __syncwarp();  // the columns are read before their mixed weights take their place
+#pragma unroll
+            for (int r = 0; r < HEADS / 16; ++r) {
+                float mixed[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int k = 0; k < HEADS / 16; ++k) {
+                    uint32_t t[4];
+                    const int at = (r * 16 + (lane & 15)) * C::TALK_PITCH + k * 16 + (lane >> 4) * 8;
+                    ldmatrix_x4(t, talk + TALK_PLANE + at);
+                    mma_bf16(mixed, t, high[2 * k], high[2 * k + 1]);
+                    ldmatrix_x4(t, talk + at);
+                    mma_bf16(mixed, t, low[2 * k], low[2 * k + 1]);
+                    mma_bf16(mixed, t, high[2 * k], high[2 * k + 1]);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t top_term, low_term;
+                    two_terms(mixed[2 * h], mixed[2 * h + 1], top_term, low_term);
+                    __nv_bfloat16* to = weights + (r * 16 + q + 8 * h) * C::PITCH + column * 8 + 2 * quad;
+                    *reinterpret_cast<uint32_t*>(to) = top_term;
+                    *reinterpret_cast<uint32_t*>(to + PLANE) = low_term;
+                }
+            }
+        }
+        cp_async_wait<1>();
+        __syncthreads();  // every column's mixed weights; each warp reads its own heads' and overwrites them alone
+#pragma unroll
+        for (int k = 0; k < TILE_K / 16; ++k) {
+            uint32_t w[ROWS][2][4];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int plane = 0; plane < 2; ++plane)
+                    ldmatrix_x4(w[r][plane], weights + plane * PLANE + (head0 + 2 * r + ((lane >> 3) & 1)) * C::PITCH +
+                                                 ((2 * k + (lane >> 4)) * TILE_Q + (lane & 7)) * 8);
+#pragma unroll
+            for (int n = 0; n < TILE_DIM / 16; ++n) {
+                uint32_t b[4];
+                ldmatrix_x4_trans(b, values + swizzled<TILE_DIM>(k * 16 + (lane & 15), 2 * n + (lane >> 4)) * 8);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int plane = 1; plane >= 0; --plane) {
+                        mma_bf16(out[r][2 * n], w[r][plane], b[0], b[1]);
+                        mma_bf16(out[r][2 * n + 1], w[r][plane], b[2], b[3]);
+                    }
+            }
+        }
+        __syncwarp();
+        if (i + 1 < tiles) fetch(v_pages, values, i + 1);
+        else cp_async_commit();
+    }
+    cp_async_wait<0>();
+    if (q >= count) return;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            __nv_bfloat16* to = static_cast<__nv_bfloat16*>(a.out) + (static_cast<size_t>(begin + first + q) * HEADS + head0 + 2 * r + h) * TILE_DIM + 2 * quad;
+#pragma unroll
+            for (int n = 0; n < TILE_DIM / 8; ++n) *reinterpret_cast<uint32_t*>(to + 8 * n) = pack_bf16(out[r][n][2 * h], out[r][n][2 * h + 1]);
+        }
+}
+
+// Against the two kernels above on one prompt of 2,048 tokens (window 1,024, 64 kept): 32 heads of 8 KV heads 7,795 -> 548 us,
+// 16 heads 5,294 -> 308 us; 700 tokens behind 800: 3,448 -> 356 and 2,363 -> 198 us.  Error against float64 the same (1.66e-3,
+// the output's rounding to bfloat16).
+template <int KV, int GROUP>
+static int launch_mixed_tiles(const MixTileArgs& m, int entries, int longest, cudaStream_t stream) {
+    static SharedMemoryOptIn opt_in;
+    if (const int code = opt_in(mixed_attention_tiles_kernel<KV, GROUP>, MixTile<KV, GROUP>::SMEM)) return code;
+    const dim3 grid((longest + TILE_Q - 1) / TILE_Q, entries);
+    return launch_kernel_in_order(mixed_attention_tiles_kernel<KV, GROUP>, grid, KV * 32, MixTile<KV, GROUP>::SMEM, stream, m);
+}
+
+// The same result from tiles of tokens; bfloat16, 128-wide heads, the (kv_heads, group) pairs below.  The tokens of entry e are
+// cu_tokens[e] .. cu_tokens[e + 1], at consecutive positions; none has more than `longest`.
+ME_EXPORT int me_mixed_attention_tiles(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
+                                       const int* cu_tokens, const int* positions, const float* r1, const float* r2,
+                                       const float* talk, void* out, float scale, int entries, int longest, int heads, int kv_heads,
+                                       int dim, int vdim, int page_size, int table_width, int window, int keep_first, cudaStream_t stream) {
+    if (entries <= 0 || longest <= 0) return 0;
+    if (dim != TILE_DIM || vdim != TILE_DIM || kv_heads < 1 || heads % kv_heads || entries > 65535) return ME_ERR_UNSUPPORTED;
+    if (reinterpret_cast<uintptr_t>(k_pages) % 16 || reinterpret_cast<uintptr_t>(v_pages) % 16 || reinterpret_cast<uintptr_t>(q) % 4 || reinterpret_cast<uintptr_t>(out) % 4)
+        return ME_ERR_UNSUPPORTED;
+    if ((r1 == nullptr) != (r2 == nullptr) || window < 1 || keep_first < 0 || talk == nullptr) return ME_ERR_ARGUMENT;
+    MixTileArgs m{{q, k_pages, v_pages, block_table, nullptr, positions, r1, r2, out, scale, 0, heads, kv_heads, dim, vdim,
+                   page_size, table_width, window, keep_first, 0},
+                  talk, cu_tokens};
+    const int group = heads / kv_heads;
+    if (kv_heads == 8 && group == 4) return launch_mixed_tiles<8, 4>(m, entries, longest, stream);
+    if (kv_heads == 8 && group == 2) return launch_mixed_tiles<8, 2>(m, entries, longest, stream);
+    if (kv_heads == 4 && group == 4) return launch_mixed_tiles<4, 4>(m, entries, longest, stream);
+    return ME_ERR_UNSUPPORTED;
 }
 
 // out[t][h][e] = sum_g talk[h][g] * spread[t][g][kv(h)][e], ascending g.

@@ -820,6 +820,44 @@ def mixed_attention(
     _check(code, "mixed_attention")
 
 
+MIXED_TILES = {(8, 4), (8, 2), (4, 4)}  # (KV heads, query heads of each) that the tile kernel is built for
+
+
+def mixed_attention_tiles_supports(dtype: torch.dtype, heads: int, kv_heads: int, head_dim: int, value_dim: int) -> bool:
+    return dtype == torch.bfloat16 and head_dim == value_dim == 128 and heads % kv_heads == 0 and (kv_heads, heads // kv_heads) in MIXED_TILES
+
+
+def mixed_attention_tiles(
+    *, q, k_pages, v_pages, block_table, cu_tokens, longest: int, positions, out, heads: int, kv_heads: int, head_dim: int,
+    value_dim: int, scale: float, window: int, keep_first: int, r1: torch.Tensor | None, r2: torch.Tensor | None, talk: torch.Tensor,
+) -> None:  # fmt: skip
+    """The attention of :func:`mixed_attention` from tiles of eight tokens on tensor cores, for the sizes of
+    :func:`mixed_attention_tiles_supports`.  An entry's tokens (``cu_tokens``: int32, one more than entries) lie at consecutive
+    positions and are at most ``longest``; ``window`` is positive."""
+    for name, tensor in (("q", q), ("out", out), ("k_pages", k_pages), ("v_pages", v_pages)):
+        _need(tensor, torch.bfloat16, name)
+    for name, tensor in (("block_table", block_table), ("cu_tokens", cu_tokens), ("positions", positions)):
+        _need(tensor, torch.int32, name)
+    _need(talk, torch.float32, "talk")
+    for name, vector in (("r1", r1), ("r2", r2)):
+        if vector is not None:
+            _need(vector, torch.float32, name)
+            if vector.shape != (heads,):
+                raise KernelError(f"{name} must have one value per head")
+    if k_pages.shape[1:] != (kv_heads, k_pages.shape[2], head_dim) or v_pages.shape[1:] != (kv_heads, k_pages.shape[2], value_dim):
+        raise KernelError(f"pages {tuple(k_pages.shape)}, {tuple(v_pages.shape)} do not fit the head sizes")
+    entries = cu_tokens.shape[0] - 1
+    if talk.shape != (heads, heads) or block_table.shape[0] < entries or out.numel() < q.shape[0] * heads * value_dim:
+        raise KernelError("talk must be [heads, heads], the block table must have a row per entry, out a value row per token and head")
+    fn = _fn("attention_biased", "me_mixed_attention_tiles", [c_void_p] * 10 + [c_float] + [c_int] * 10 + [c_void_p])
+    code = fn(
+        _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), _ptr(cu_tokens), _ptr(positions), _ptr(r1), _ptr(r2), _ptr(talk),
+        _ptr(out), float(scale), entries, int(longest), heads, kv_heads, head_dim, value_dim, k_pages.shape[2],
+        block_table.shape[1], int(window), int(keep_first), _stream(),
+    )  # fmt: skip
+    _check(code, "mixed_attention_tiles")
+
+
 def branch_sum(branches: list[tuple[torch.Tensor, float]], out: torch.Tensor) -> None:
     """``out [T, width] = sum_b factor_b * sum_s partial_b[s]`` for up to four ``[S, T, width]`` float32
     partial-sum arrays."""

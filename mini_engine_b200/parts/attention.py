@@ -73,6 +73,10 @@ from mini_engine_b200.parts.base import (
 from mini_engine_b200.parts.linear import Linear
 from mini_engine_b200.weights.loader import WeightSpec
 
+# Mixed heads run from tiles of eight tokens on tensor cores when some entry of the step brings this many tokens.  A tile
+# takes as long with one token in it as with eight: below, one block per (token, head) of the two-kernel form is faster.
+MIXING_TILES_MIN_TOKENS = 8
+
 
 @register("mixer", "gqa_attention")
 class GroupedQueryAttention(Mixer):
@@ -174,6 +178,7 @@ class GroupedQueryAttention(Mixer):
             self.talking_heads and window
             and num_heads // kv_heads <= ops.MIXED_ATTENTION_MAX_GROUP and self.value_dim <= ops.MIXED_ATTENTION_MAX_VALUE_DIM
         )  # fmt: skip
+        self.mixing_tiles = False  # set at load, where the dtype is known
         self.scale = float(scale) if scale is not None else head_dim**-0.5
         self.reads_shared_cache = reads_shared_cache
         self.qkv_bias = qkv_bias  # the reference's projections have none (src/mini_engine/model.py:97-100)
@@ -284,6 +289,9 @@ class GroupedQueryAttention(Mixer):
             self.r1, self.r2 = tensors[n["r1"]], tensors[n["r2"]]
         if self.talking_heads:
             self.talk = tensors[n["talk"]]
+            self.mixing_tiles = ops.mixed_attention_tiles_supports(
+                tensors[n["q"]].dtype, self.heads, self.kv_heads, self.head_dim, self.value_dim
+            )
         if self.position is not None:
             self.position.load(tensors)
 
@@ -328,6 +336,14 @@ class GroupedQueryAttention(Mixer):
             # The scratch is sized for the engine's token capacity, so the choice never depends on the batch.
             stride = (self.window or 0) + self.keep_first
             capacity = max(tokens, ctx.workspace.max_tokens)
+            if self.two_kernel_mixing and self.mixing_tiles and ctx.max_query_len >= MIXING_TILES_MIN_TOKENS:
+                ops.mixed_attention_tiles(
+                    q=q, k_pages=cache.k, v_pages=cache.v, block_table=ctx.block_tables[cache.group], cu_tokens=ctx.cu_tokens,
+                    longest=ctx.max_query_len, positions=ctx.positions, out=out, heads=self.heads, kv_heads=self.kv_heads, head_dim=d,
+                    value_dim=self.value_dim, scale=self.scale, window=self.window, keep_first=self.keep_first, r1=self.r1,
+                    r2=self.r2, talk=self.talk,
+                )  # fmt: skip
+                return self.out.forward(out, ctx, "attn.o")
             if self.two_kernel_mixing and capacity * self.heads * stride * 4 <= 2 << 30:
                 scores = ctx.buffer("attn.scores", (tokens, self.heads * stride), torch.float32)
                 stats = ctx.buffer("attn.stats", (tokens, self.heads * 2), torch.float32)

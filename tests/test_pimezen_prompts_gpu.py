@@ -1,0 +1,74 @@
+"""The kernel that long portions of the Pimezen design take in bfloat16: mixed heads from tiles of eight tokens on tensor
+cores, against float64 and beside the kernels that short portions take."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from test_pimezen_gpu import paged, plain_attention
+
+pytestmark = pytest.mark.gpu
+
+
+def tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size):
+    """Requests ``(past, new)`` in one step through both forms; returns (tiles, rows, float64) of all new tokens."""
+    from mini_engine_b200.csrc import ops
+
+    dim, dtype = 128, torch.bfloat16
+    r1, r2, talk = torch.rand(heads) * 2, torch.rand(heads) + 0.1, torch.randn(heads, heads)
+    q_rows, positions, cu, tables, wants, pools = [], [], [0], [], [], []
+    width = max(-(-(past + new) // page_size) for past, new in requests)
+    base = 0
+    for i, (past, new) in enumerate(requests):
+        total = past + new
+        q, k, v = (torch.randn(total, h, dim).to(dtype).float() for h in (heads, kv_heads, kv_heads))
+        count = 2 * (-(-total // page_size)) + 1
+        k_pages, table = paged(k, page_size, count, torch.Generator().manual_seed(i))
+        v_pages, _ = paged(v, page_size, count, torch.Generator().manual_seed(i))
+        row = torch.full((width,), -1, dtype=torch.int32)
+        row[: len(table)] = table + base
+        base += k_pages.shape[0]
+        pools.append((k_pages, v_pages)), tables.append(row), q_rows.append(q[past:])
+        positions += range(past, total)
+        cu.append(cu[-1] + new)
+        wants.append(plain_attention(q, k, v, r1, r2, talk, dim**-0.5, window, keep_first)[past:])
+    cuda = lambda t, dt=None: t.to(device="cuda", dtype=dt or t.dtype).contiguous()  # noqa: E731
+    n, stride = cu[-1], window + keep_first
+    shared = dict(
+        q=cuda(torch.cat(q_rows).view(n, -1), dtype), k_pages=cuda(torch.cat([p[0] for p in pools]), dtype),
+        v_pages=cuda(torch.cat([p[1] for p in pools]), dtype), block_table=cuda(torch.stack(tables)),
+        positions=torch.tensor(positions, dtype=torch.int32, device="cuda"), heads=heads, kv_heads=kv_heads, head_dim=dim,
+        value_dim=dim, scale=dim**-0.5, window=window, keep_first=keep_first, r1=cuda(r1), r2=cuda(r2), talk=cuda(talk),
+    )  # fmt: skip
+    tiles, rows = (torch.full((n, heads * dim), float("nan"), dtype=dtype, device="cuda") for _ in range(2))
+    ops.mixed_attention_tiles(
+        **shared, out=tiles, cu_tokens=torch.tensor(cu, dtype=torch.int32, device="cuda"), longest=max(new for _, new in requests)
+    )
+    entry = torch.cat([torch.full((new,), i, dtype=torch.int32) for i, (_, new) in enumerate(requests)])
+    ops.mixed_attention(
+        **shared, out=rows, entry_of_token=cuda(entry), scores=torch.full((n * heads * stride,), float("nan"), device="cuda"),
+        stats=torch.empty(n * heads * 2, device="cuda"), stride=stride,
+    )  # fmt: skip
+    torch.cuda.synchronize()
+    return tiles.double().cpu(), rows.double().cpu(), torch.cat(wants).reshape(n, -1).double()
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(32, 8), (16, 8), (16, 4)])
+@pytest.mark.parametrize(
+    "requests,window,keep_first,page_size",
+    [
+        ([(0, 9)], 5, 40, 16),  # every key kept, a second tile of one token
+        ([(0, 33), (20, 8), (61, 1)], 20, 6, 16),  # window and kept keys within tiles; portion and decoded token beside a prompt
+        ([(90, 47)], 33, 17, 8),
+        ([(0, 130), (200, 3)], 64, 64, 32),  # kept keys fill two tiles
+        ([(5, 70)], 1, 0, 16),  # a query sees itself alone
+    ],
+)
+def test_mixed_heads_from_tiles(heads, kv_heads, requests, window, keep_first, page_size):
+    torch.manual_seed(heads + window)
+    tiles, rows, want = tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size)
+    scale = want.norm()
+    # both round the output to bfloat16 (relative 2^-9 / sqrt(3) = 1.1e-3 at most); the weights' two terms add nothing to it
+    assert float((tiles - want).norm() / scale) < 2.5e-3
+    assert float((tiles - want).norm()) < 1.02 * float((rows - want).norm())
