@@ -42,6 +42,7 @@ struct PrepArgs {
     float* prepared;          // [tokens][heads][3][dim]
     float q_scale, inv_tau;
     int tokens, heads, dim, rank;
+    int row = 0, v_col = 0, vdim = 0;  // row > 0: prepared[token][head] is `row` floats, q, k, decay and the vdim value sums
 };
 
 constexpr int PREP_TOKENS = 8;
@@ -82,10 +83,20 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(PrepArgs a) {
                 q += row[p * a.split_stride + a.q_col];
                 k += row[p * a.split_stride + a.k_col];
             }
-            float* dst = a.prepared + ((static_cast<size_t>(first + t) * a.heads + head) * 3) * a.dim + d;
+            float* dst = a.prepared + (static_cast<size_t>(first + t) * a.heads + head) * (a.row ? a.row : 3 * a.dim) + d;
             dst[0] = q * a.q_scale;
             dst[a.dim] = k;
             dst[2 * a.dim] = expf(log_sigmoid(z[t] + bias) * a.inv_tau);
+        }
+    }
+    if (!a.row) return;
+    const int values = a.heads * a.vdim;
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < values; i += gridDim.y * blockDim.x) {
+        for (int t = 0; t < count; ++t) {
+            const float* src = a.proj + static_cast<size_t>(first + t) * a.width + a.v_col + i;
+            float v = 0.0f;
+            for (int p = 0; p < a.splits; ++p) v += src[p * a.split_stride];
+            a.prepared[(static_cast<size_t>(first + t) * a.heads + i / a.vdim) * a.row + 3 * a.dim + i % a.vdim] = v;
         }
     }
 }
@@ -107,6 +118,8 @@ struct ScanArgs {
     int heads, dim, vdim;
     int max_count = 0;       // > 0: entries with more tokens than this are left to the chunked kernels
     int silu = 0;            // 1: the value sums pass silu
+    int row = 0;             // floats of a prepared row, 0: 3 * dim
+    int v_head = 0;          // floats between two heads' values in `proj`, 0: vdim
 };
 
 constexpr int SCAN_CHUNK = 16;
@@ -134,6 +147,7 @@ __global__ void __launch_bounds__(32) gla_scan_kernel(ScanArgs a) {
     const int column = blockIdx.z * 32 + lane;
     const bool live = column < a.vdim;
     const int dim = a.dim;
+    const int row = a.row ? a.row : 3 * dim, v_head = a.v_head ? a.v_head : a.vdim;
     const bool vector = dim % 4 == 0;
     for (int i = lane; i < 2 * SCAN_CHUNK * 3 * (DIMP - dim); i += 32)  // channels dim..DIMP are zero for good
         tiles[(i / (DIMP - dim)) * DIMP + dim + i % (DIMP - dim)] = 0.0f;
@@ -158,12 +172,12 @@ __global__ void __launch_bounds__(32) gla_scan_kernel(ScanArgs a) {
                 const int t = i / quads, j = (i % quads) * 4;
                 const int which = j / dim, d = j % dim;
                 copy_async_16(tile + (t * 3 + which) * DIMP + d,
-                              a.prepared + ((static_cast<size_t>(chunk + t) * a.heads + head) * 3) * dim + j);
+                              a.prepared + (static_cast<size_t>(chunk + t) * a.heads + head) * row + j);
             }
         } else {
             for (int i = lane; i < count * 3 * dim; i += 32) {
                 const int t = i / (3 * dim), j = i % (3 * dim);
-                tile[(t * 3 + j / dim) * DIMP + j % dim] = a.prepared[((static_cast<size_t>(chunk + t) * a.heads + head) * 3) * dim + j];
+                tile[(t * 3 + j / dim) * DIMP + j % dim] = a.prepared[(static_cast<size_t>(chunk + t) * a.heads + head) * row + j];
             }
         }
         copy_async_commit();
@@ -174,7 +188,7 @@ __global__ void __launch_bounds__(32) gla_scan_kernel(ScanArgs a) {
         for (int t = 0; t < SCAN_CHUNK; ++t) {
             v[t] = 0.0f;
             if (live && t < count) {
-                const float* src = a.proj + static_cast<size_t>(chunk + t) * a.width + a.v_col + head * a.vdim + column;
+                const float* src = a.proj + static_cast<size_t>(chunk + t) * a.width + a.v_col + head * v_head + column;
                 for (int p = 0; p < a.splits; ++p) v[t] += src[p * a.split_stride];
                 if (a.silu) v[t] = silu_of(v[t]);
             }
@@ -250,25 +264,34 @@ static int launch_scan(const ScanArgs& a, int entries, cudaStream_t stream) {
 }
 
 // Both kernels, one after the other: `prepared` is scratch of tokens * heads * 3 * dim floats, `a2t` the
-// decay's second factor transposed to [rank][heads*dim].
+// decay's second factor transposed to [rank][heads*dim].  With `chunk_min` > 0 the rows of `prepared` hold the vdim value
+// sums as well (what the chunked kernels of state_chunks.cu read) and the scan leaves entries of at least that many tokens alone.
 ME_EXPORT int me_gla_scan(const float* proj, int splits, long long split_stride, int width, int q_col, int k_col,
                           int v_col, int a_col, const float* a2t, const float* a2_bias, const int* cu_tokens,
                           const int* state_slots, const int* fresh, float* state, float* out, float* prepared,
                           float q_scale, float tau, int tokens, int entries, int heads, int dim, int vdim, int rank,
-                          cudaStream_t stream) {
+                          int chunk_min, cudaStream_t stream) {
     if (entries <= 0 || tokens <= 0) return 0;
     if (dim < 1 || vdim < 1 || rank < 1 || heads < 1 || !(tau > 0.0f)) return ME_ERR_ARGUMENT;
     if (static_cast<size_t>(PREP_TOKENS) * rank * sizeof(float) > 48 * 1024) return ME_ERR_UNSUPPORTED;
     PrepArgs p{proj, splits, static_cast<size_t>(split_stride), width, q_col, k_col, a_col, a2t, a2_bias, prepared,
                q_scale, 1.0f / tau, tokens, heads, dim, rank};
-    // Few tokens: the channels of a token block are spread over several blocks as well.
+    if (chunk_min > 0) p.row = 3 * dim + vdim, p.v_col = v_col, p.vdim = vdim;
+    // The channels of a token block are spread over several blocks as well: a thread's chain (its rows of A2, then the
+    // decays of eight tokens) is long, and only many warps to an SM hide it.  2,048 tokens of 32 heads of 128: 254 us with
+    // one block per eight tokens, 176 with 16.
     const int token_blocks = (tokens + PREP_TOKENS - 1) / PREP_TOKENS;
-    const int channel_blocks = token_blocks >= 148 ? 1 : std::min((heads * dim + 255) / 256, 16);
+    const int channel_blocks = std::min((heads * dim + 255) / 256, 16);
     const int code = launch_kernel(gla_prepare_kernel, dim3(token_blocks, channel_blocks), 256,
                                    static_cast<size_t>(PREP_TOKENS) * rank * sizeof(float), stream, p);
     if (code) return code;
     ScanArgs a{proj, splits, static_cast<size_t>(split_stride), width, v_col, prepared, cu_tokens, state_slots,
                fresh, state, out, heads, dim, vdim};
+    if (chunk_min > 0) {
+        a.proj = prepared, a.splits = 1, a.split_stride = 0;
+        a.row = a.v_head = 3 * dim + vdim, a.v_col = 3 * dim, a.width = heads * a.row;
+        a.max_count = chunk_min - 1;
+    }
     if (dim <= 16) return launch_scan<16>(a, entries, stream);
     if (dim <= 32) return launch_scan<32>(a, entries, stream);
     if (dim <= 64) return launch_scan<64>(a, entries, stream);

@@ -881,30 +881,46 @@ def branch_sum(branches: list[tuple[torch.Tensor, float]], out: torch.Tensor) ->
 def gla_scan(
     *, proj: torch.Tensor, columns: dict[str, int], a2t: torch.Tensor, a2_bias: torch.Tensor, ctx, state: torch.Tensor,
     out: torch.Tensor, prepared: torch.Tensor, q_scale: float, tau: float, heads: int, dim: int, vdim: int,
+    chunk_min: int = 0, records: torch.Tensor | None = None,
 ) -> None:  # fmt: skip
     """The recurrence of gated linear attention over the batch's tokens, entry by entry, from and
     into each request's state slot.  ``proj`` is ``[S, T, width]`` float32 partial sums whose
     ``columns`` ``q, k, v, a`` say where each projection starts; ``a2t`` is the decay's second factor
     transposed, ``[rank, heads * dim]``; ``out`` is float32 ``[T, heads, vdim]``; ``prepared`` is float32
-    scratch of ``T * heads * 3 * dim`` values (q, k and decay of every token, made by a first kernel)."""
+    scratch of ``T * heads * 3 * dim`` values (q, k and decay of every token, made by a first kernel).  ``chunk_min`` > 0:
+    entries of at least that many tokens run in chunks of ``STATE_CHUNK`` tokens (:func:`state_chunks_support` says for
+    which sizes), with ``records [chunks, heads * state_record_floats("gated", dim)]`` as scratch for all of their chunks and
+    ``prepared`` of ``T * heads * (3 * dim + vdim)`` values; the other entries walk token by token."""
     _need(proj, torch.float32, "proj"), _need(a2t, torch.float32, "a2t"), _need(a2_bias, torch.float32, "a2_bias")
     _need(state, torch.float32, "state"), _need(out, torch.float32, "out"), _need(prepared, torch.float32, "prepared")
     rank, tokens = a2t.shape[0], proj.shape[1]
     if a2t.shape != (rank, heads * dim) or a2_bias.shape != (heads * dim,) or state.shape[1:] != (heads, dim, vdim):
         raise KernelError("gla_scan: decay weights or state do not fit heads/dim/vdim")
-    if prepared.numel() < tokens * heads * 3 * dim or out.numel() < tokens * heads * vdim:
+    if prepared.numel() < tokens * heads * (3 * dim + (vdim if chunk_min else 0)) or out.numel() < tokens * heads * vdim:
         raise KernelError("gla_scan: scratch or output too small")
+    slot_floats = heads * dim * vdim
+    if chunk_min:
+        _need(records, torch.float32, "records")
+        if not state_chunks_support(dim, vdim, slot_floats) or records.dim() != 2 or records.shape[1] != heads * state_record_floats("gated", dim):
+            raise KernelError("gla_scan: the chunks' records or the head sizes do not fit")
     fn = _fn(
         "linear_attention",
         "me_gla_scan",
-        [c_void_p, c_int, c_longlong] + [c_int] * 5 + [c_void_p] * 8 + [c_float, c_float] + [c_int] * 6 + [c_void_p],
+        [c_void_p, c_int, c_longlong] + [c_int] * 5 + [c_void_p] * 8 + [c_float, c_float] + [c_int] * 7 + [c_void_p],
     )
     code = fn(
         _ptr(proj), proj.shape[0], proj.stride(0), proj.shape[2], columns["q"], columns["k"], columns["v"], columns["a"],
         _ptr(a2t), _ptr(a2_bias), _ptr(ctx.cu_tokens), _ptr(ctx.state_slots), _ptr(ctx.fresh), _ptr(state), _ptr(out),
-        _ptr(prepared), float(q_scale), float(tau), tokens, ctx.num_entries, heads, dim, vdim, rank, _stream(),
+        _ptr(prepared), float(q_scale), float(tau), tokens, ctx.num_entries, heads, dim, vdim, rank, int(chunk_min), _stream(),
     )  # fmt: skip
     _check(code, "gla_scan")
+    if chunk_min:
+        fn = _fn("state_chunks", "me_state_chunks", _STATE_CHUNKS)
+        code = fn(
+            _ptr(prepared), _ptr(None), _ptr(ctx.cu_tokens), _ptr(ctx.state_slots), _ptr(ctx.fresh), _ptr(state), slot_floats,
+            _ptr(out), _ptr(records), _CHUNK_RULES["gated"], ctx.num_entries, heads, dim, vdim, int(chunk_min), records.shape[0], _stream(),
+        )  # fmt: skip
+        _check(code, "state_chunks")
 
 
 FINISH_GATES = {"silu": 0, "sigmoid": 1}
@@ -1289,6 +1305,7 @@ def delta_scan(
 
 
 STATE_RULES = {"removal": 1, "bonus": 2}
+_CHUNK_RULES = {**STATE_RULES, "gated": 3}  # what the chunked kernels know: gated linear attention too
 _RULE_FLOATS = {"removal": (4, 4), "bonus": (3, 2)}  # vectors of a key head's width, numbers per token and head
 
 
@@ -1298,6 +1315,7 @@ def state_rule_floats(rule: str, dim: int, vdim: int) -> tuple[int, int]:
     return vectors * dim + vdim, numbers
 
 
+_STATE_CHUNKS = [c_void_p] * 6 + [c_longlong, c_void_p, c_void_p] + [c_int] * 7 + [c_void_p]
 STATE_CHUNK = 16  # tokens of a chunk of the chunked recurrences
 
 
@@ -1312,7 +1330,7 @@ def state_record_floats(rule: str, dim: int) -> int:
     """Floats of a chunk's record per head."""
     fn = load_library("state_chunks").me_state_chunks_record_floats
     fn.argtypes, fn.restype = [c_int, c_int], c_int
-    return int(fn(STATE_RULES[rule], int(dim)))
+    return int(fn(_CHUNK_RULES[rule], int(dim)))
 
 
 def state_prepare(
@@ -1365,7 +1383,7 @@ def state_walk(
         _need(records, torch.float32, "records")
         if not state_chunks_support(dim, vdim, state.shape[1]) or records.dim() != 2 or records.shape[1] != heads * state_record_floats(rule, dim):
             raise KernelError("state_walk: the chunks' records or the head sizes do not fit")
-        fn = _fn("state_chunks", "me_state_chunks", [c_void_p] * 6 + [c_longlong, c_void_p, c_void_p] + [c_int] * 7 + [c_void_p])
+        fn = _fn("state_chunks", "me_state_chunks", _STATE_CHUNKS)
         code = fn(
             _ptr(rows), _ptr(scalars), _ptr(ctx.cu_tokens), _ptr(ctx.state_slots), _ptr(ctx.fresh), _ptr(state), state.shape[1],
             _ptr(out), _ptr(records), STATE_RULES[rule], ctx.num_entries, heads, dim, vdim, int(chunk_min), records.shape[0], _stream(),

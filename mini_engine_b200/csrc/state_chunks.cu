@@ -27,7 +27,7 @@
 
 #include <algorithm>
 
-enum : int { RULE_REMOVAL = 1, RULE_BONUS = 2 };
+enum : int { RULE_REMOVAL = 1, RULE_BONUS = 2, RULE_GATED = 3 };
 
 constexpr int CHUNK = 16;
 constexpr int COLUMNS = 32;  // value columns of a walking block
@@ -36,6 +36,8 @@ constexpr int WALK_THREADS = 256;  // of a walking block
 constexpr int WALK_WARPS = WALK_THREADS / 32;
 constexpr int STAGES = 3;  // records that a walking block holds: two are on their way
 
+// RULE_GATED is gated linear attention (linear_attention.cu): nothing is removed, o_t = q_t^T S_t, so that r_t = q_t g_t and the
+// diagonal of RK is q . k; its rows are q, k, g and v, without numbers, and its state is [heads][dim][vdim].
 template <int RULE>
 struct Rule;
 // VECTORS and SCALARS: what a prepared row holds (see delta_rule.cu); ROWS: rows of the two products of a chunk.
@@ -43,6 +45,8 @@ template <>
 struct Rule<RULE_REMOVAL> { static constexpr int VECTORS = 4, SCALARS = 4, ROWS = 2 * CHUNK; };
 template <>
 struct Rule<RULE_BONUS> { static constexpr int VECTORS = 3, SCALARS = 2, ROWS = CHUNK; };
+template <>
+struct Rule<RULE_GATED> { static constexpr int VECTORS = 3, SCALARS = 0, ROWS = CHUNK; };
 
 // A chunk's record: the reading matrix transposed, [DIM + CHUNK][ROWS] (the key channels of (A' | R'), then the tokens of (M1 |
 // M2)), the writing matrix [ROWS][DIM] (decayed k, then decayed b) and the decay over the chunk [DIM].
@@ -51,11 +55,11 @@ struct Record { static constexpr int FLOATS = (DIM + CHUNK) * Rule<RULE>::ROWS +
 
 struct ChunkArgs {
     const float* rows;     // [tokens][heads][VECTORS * dim + vdim]
-    const float* scalars;  // [tokens][heads][SCALARS]
+    const float* scalars;  // [tokens][heads][SCALARS], null without any
     const int* cu_tokens;
     const int* state_slots;
     const int* fresh;
-    float* state;  // [slots + 1][slot_floats], a slot starts with [heads][vdim][dim]
+    float* state;  // [slots + 1][slot_floats], a slot starts with [heads][vdim][dim] (RULE_GATED: [heads][dim][vdim])
     size_t slot_floats;
     float* out;      // [tokens][heads][vdim]
     float* records;  // [heads][max_chunks][record floats]: a walking block reads its records one after the other
@@ -94,7 +98,7 @@ __global__ void __launch_bounds__(THREADS) chunk_record_kernel(ChunkArgs a) {
     if (!locate_chunk(a, blockIdx.x, first, count)) return;
     const int row_floats = VECTORS * a.dim + a.vdim;
     const float* rows = a.rows + (static_cast<size_t>(first) * a.heads + head) * row_floats;
-    const float* scalars = a.scalars + (static_cast<size_t>(first) * a.heads + head) * SCALARS;
+    const float* scalars = SCALARS ? a.scalars + (static_cast<size_t>(first) * a.heads + head) * SCALARS : nullptr;
     const size_t row_step = static_cast<size_t>(a.heads) * row_floats;
     // Tokens behind the portion's end: no key, nothing removed, no decay.
     for (int i = threadIdx.x; i < CHUNK * VECTORS * (DIM / 4); i += THREADS) {
@@ -108,7 +112,20 @@ __global__ void __launch_bounds__(THREADS) chunk_record_kernel(ChunkArgs a) {
     __syncthreads();
     const float *r = vectors, *k = vectors + CHUNK * DIM, *g = vectors + 2 * CHUNK * DIM, *b = vectors + 3 * CHUNK * DIM;
     float *ak = pairs, *rk = pairs + CHUNK * CHUNK, *ab = pairs + 2 * CHUNK * CHUNK, *rb = pairs + 3 * CHUNK * CHUNK;
-    if (threadIdx.x < CHUNK) {
+    if constexpr (RULE == RULE_GATED) {  // eight lanes a token
+        const int t = threadIdx.x / 8;
+        float dot = 0.0f;
+#pragma unroll
+        for (int d = threadIdx.x % 8 * 4; d < DIM; d += 32) {
+            float4* mine = reinterpret_cast<float4*>(vectors + t * DIM + d);
+            const float4 q4 = *mine, k4 = *reinterpret_cast<const float4*>(k + t * DIM + d), g4 = *reinterpret_cast<const float4*>(g + t * DIM + d);
+            dot = fmaf(q4.x, k4.x, fmaf(q4.y, k4.y, fmaf(q4.z, k4.z, fmaf(q4.w, k4.w, dot))));
+            *mine = make_float4(q4.x * g4.x, q4.y * g4.y, q4.z * g4.z, q4.w * g4.w);
+        }
+#pragma unroll
+        for (int offset = 1; offset < 8; offset <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, offset);
+        if (threadIdx.x % 8 == 0) rk[t * CHUNK + t] = dot;
+    } else if (threadIdx.x < CHUNK) {
         const int t = threadIdx.x;
         const float* mine = scalars + t * static_cast<size_t>(a.heads) * SCALARS;
         const bool live = t < count;
@@ -271,12 +288,20 @@ __global__ void __launch_bounds__(WALK_THREADS) chunk_walk_kernel(ChunkArgs a) {
     const bool owner = threadIdx.x < 128;
     float4 s[TILES][4];  // [channel] of four columns
     float* state = a.state + static_cast<size_t>(a.state_slots[entry]) * a.slot_floats + (static_cast<size_t>(head) * a.vdim + first_column + 4 * strip) * a.dim;
+    float* channels = a.state + static_cast<size_t>(a.state_slots[entry]) * a.slot_floats + static_cast<size_t>(head) * a.dim * a.vdim + first_column + 4 * strip;
+    const bool live = first_column + 4 * strip < a.vdim;
     auto columns_of = [](float4& row, int c) -> float& { return c == 0 ? row.x : c == 1 ? row.y : c == 2 ? row.z : row.w; };
 #pragma unroll
     for (int tile = 0; tile < TILES; ++tile) {
         const int d = 4 * (quad + 16 * tile);
+        if constexpr (RULE == RULE_GATED) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+            for (int i = 0; i < 4; ++i)
+                s[tile][i] = live && d < a.dim && a.fresh[entry] == 0 ? *reinterpret_cast<const float4*>(channels + static_cast<size_t>(d + i) * a.vdim)
+                                                                     : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int c = 0; c < 4 && RULE != RULE_GATED; ++c) {
             float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (d < a.dim && first_column + 4 * strip + c < a.vdim && a.fresh[entry] == 0) x = *reinterpret_cast<const float4*>(state + static_cast<size_t>(c) * a.dim + d);
             columns_of(s[tile][0], c) = x.x, columns_of(s[tile][1], c) = x.y, columns_of(s[tile][2], c) = x.z, columns_of(s[tile][3], c) = x.w;
@@ -383,8 +408,13 @@ __global__ void __launch_bounds__(WALK_THREADS) chunk_walk_kernel(ChunkArgs a) {
 #pragma unroll
     for (int tile = 0; tile < TILES; ++tile) {
         const int d = 4 * (quad + 16 * tile);
+        if constexpr (RULE == RULE_GATED) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+            for (int i = 0; i < 4; ++i)
+                if (owner && live && d < a.dim) *reinterpret_cast<float4*>(channels + static_cast<size_t>(d + i) * a.vdim) = s[tile][i];
+        }
+#pragma unroll
+        for (int c = 0; c < 4 && RULE != RULE_GATED; ++c) {
             if (owner && d < a.dim && first_column + 4 * strip + c < a.vdim)
                 *reinterpret_cast<float4*>(state + static_cast<size_t>(c) * a.dim + d) =
                     make_float4(columns_of(s[tile][0], c), columns_of(s[tile][1], c), columns_of(s[tile][2], c), columns_of(s[tile][3], c));
@@ -430,11 +460,13 @@ ME_EXPORT int me_state_chunks(const float* rows, const float* scalars, const int
                               float* state, long long slot_floats, float* out, float* records, int rule, int entries, int heads, int dim,
                               int vdim, int min_count, int max_chunks, cudaStream_t stream) {
     if (entries <= 0 || max_chunks <= 0) return 0;
-    if (heads < 1 || min_count < 1 || (rule != RULE_REMOVAL && rule != RULE_BONUS)) return ME_ERR_ARGUMENT;
+    if (heads < 1 || min_count < 1 || (rule != RULE_REMOVAL && rule != RULE_BONUS && rule != RULE_GATED)) return ME_ERR_ARGUMENT;
+    if (rule != RULE_GATED && scalars == nullptr) return ME_ERR_ARGUMENT;
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     if (!me_state_chunks_supports(dim, vdim) || slot_floats % 4 || !aligned(rows) || !aligned(state) || !aligned(out) || !aligned(records))
         return ME_ERR_UNSUPPORTED;
     if (slot_floats < static_cast<long long>(heads) * dim * vdim) return ME_ERR_ARGUMENT;
     ChunkArgs a{rows, scalars, cu_tokens, state_slots, fresh, state, (size_t)slot_floats, out, records, entries, heads, dim, vdim, min_count, max_chunks};
+    if (rule == RULE_GATED) return dispatch_chunks<RULE_GATED>(a, max_chunks, stream);
     return rule == RULE_REMOVAL ? dispatch_chunks<RULE_REMOVAL>(a, max_chunks, stream) : dispatch_chunks<RULE_BONUS>(a, max_chunks, stream);
 }

@@ -44,6 +44,11 @@ from mini_engine_b200.parts.linear import Linear
 from mini_engine_b200.weights.loader import WeightSpec
 
 
+# An entry of at least this many tokens runs in chunks.  Below, the walk is as fast, and decoded tokens and short
+# portions keep the bits of a token-by-token run.
+CHUNKED_MIN_TOKENS = 33
+
+
 @register("mixer", "gated_linear_attention")
 class GatedLinearAttention(Mixer):
     capturable = True
@@ -115,10 +120,21 @@ class GatedLinearAttention(Mixer):
         tokens = h.shape[0]
         proj = self.proj.forward(h, ctx, "gla.proj")
         raw = ctx.buffer("gla.raw", (tokens, self.heads * self.vdim), torch.float32)
-        prepared = ctx.buffer("gla.prepared", (tokens, self.heads * 3 * self.dim), torch.float32)
+        # Long entries run in chunks of tokens side by side.  In float32 every entry walks: a token's bits there do not depend on
+        # how its request was cut.  A step's longest entry is known on the host.
+        chunk_min, records, row = 0, None, 3 * self.dim
+        if (
+            ctx.dtype == torch.bfloat16 and ctx.max_query_len >= CHUNKED_MIN_TOKENS
+            and ops.state_chunks_support(self.dim, self.vdim, self.heads * self.dim * self.vdim)
+        ):  # fmt: skip
+            chunk_min, row = CHUNKED_MIN_TOKENS, 3 * self.dim + self.vdim
+            chunks = tokens // ops.STATE_CHUNK + ctx.num_entries
+            records = ctx.workspace.growing("gla.records", (chunks, self.heads * ops.state_record_floats("gated", self.dim)), torch.float32)
+        prepared = ctx.buffer("gla.prepared", (tokens, self.heads * row), torch.float32)
         ops.gla_scan(
             proj=proj, columns=self.columns, a2t=self.a2t, a2_bias=self.a2_bias, ctx=ctx, state=cache.state, out=raw,
             prepared=prepared, q_scale=self.q_scale, tau=self.tau, heads=self.heads, dim=self.dim, vdim=self.vdim,
+            chunk_min=chunk_min, records=records,
         )  # fmt: skip
         gated = ctx.buffer("gla.out", (tokens, self.heads * self.vdim), ctx.dtype)
         ops.gla_finish(
@@ -126,11 +142,6 @@ class GatedLinearAttention(Mixer):
             heads=self.heads, vdim=self.vdim,
         )  # fmt: skip
         return self.out.forward(gated, ctx, "gla.o")
-
-
-# An entry of at least this many tokens runs in chunks.  Below, the walk is as fast, and decoded tokens and short
-# portions keep the bits of a token-by-token run.
-CHUNKED_MIN_TOKENS = 33
 
 
 @register("mixer", "retention")

@@ -1,5 +1,5 @@
-"""The kernel that long portions of the Pimezen design take in bfloat16: mixed heads from tiles of eight tokens on tensor
-cores, against float64 and beside the kernels that short portions take."""
+"""The kernels that long portions of the Pimezen design take in bfloat16: mixed heads from tiles of eight tokens on tensor
+cores, the gated recurrence in chunks of 16 tokens; each against float64 and beside the kernel that short portions take."""
 
 from __future__ import annotations
 
@@ -72,3 +72,59 @@ def test_mixed_heads_from_tiles(heads, kv_heads, requests, window, keep_first, p
     # both round the output to bfloat16 (relative 2^-9 / sqrt(3) = 1.1e-3 at most); the weights' two terms add nothing to it
     assert float((tiles - want).norm() / scale) < 2.5e-3
     assert float((tiles - want).norm()) < 1.02 * float((rows - want).norm())
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 24), (3, 64, 128), (2, 128, 128), (1, 100, 36)])
+@pytest.mark.parametrize("counts,starts", [([33], [0]), ([48, 5], [7, 0]), ([1, 200, 34], [3, 0, 50])])
+def test_gated_recurrence_in_chunks(heads, dim, vdim, counts, starts):
+    """Entries below and above the chunks' minimum, from zero and from a held state, against the walk token by token and
+    against float64; the states behind them too."""
+    from test_pimezen_gpu import FakeContext
+
+    from mini_engine_b200.csrc import ops
+
+    torch.manual_seed(dim + len(counts))
+    tokens, rank, tau = sum(counts), 4, 6.0
+    widths = {"q": heads * dim, "k": heads * dim, "v": heads * vdim, "g": heads * vdim, "a": rank}
+    columns, width = {}, 0
+    for key, w in widths.items():
+        columns[key], width = width, width + w
+    proj = torch.randn(2, tokens, width)
+    a2, bias = torch.randn(heads * dim, rank) * 0.5, torch.randn(heads * dim)
+    slots, fresh = list(range(len(counts))), [1 if start == 0 else 0 for start in starts]
+    first = torch.randn(len(counts) + 1, heads, dim, vdim)
+    results = []
+    for chunk_min in (0, 33):
+        state, out = first.clone().cuda(), torch.full((tokens, heads * vdim), float("nan"), device="cuda")
+        prepared = torch.full((tokens * heads * (3 * dim + vdim),), float("nan"), device="cuda")
+        chunks = tokens // ops.STATE_CHUNK + len(counts)
+        records = torch.full((chunks, heads * ops.state_record_floats("gated", dim)), float("nan"), device="cuda")
+        ops.gla_scan(
+            proj=proj.cuda(), columns=columns, a2t=a2.t().contiguous().cuda(), a2_bias=bias.cuda(), ctx=FakeContext(counts, slots, fresh),
+            state=state, out=out, prepared=prepared, q_scale=dim**-0.5, tau=tau, heads=heads, dim=dim, vdim=vdim,
+            chunk_min=chunk_min, records=records if chunk_min else None,
+        )  # fmt: skip
+        torch.cuda.synchronize()
+        results.append((out.cpu().double(), state.cpu().double()))
+    summed = proj.double().sum(0)
+    take = lambda key: summed[:, columns[key] : columns[key] + widths[key]]  # noqa: E731
+    q, k, v = take("q").view(tokens, heads, dim) * dim**-0.5, take("k").view(tokens, heads, dim), take("v").view(tokens, heads, vdim)
+    decay = torch.sigmoid(take("a") @ a2.double().T + bias.double()).pow(1 / tau).view(tokens, heads, dim)
+    want, states, t = [], first.clone().double(), 0
+    for slot, (count, start) in enumerate(zip(counts, starts)):
+        s = states[slot] if start else torch.zeros(heads, dim, vdim, dtype=torch.float64)
+        for _ in range(count):
+            s = decay[t].unsqueeze(-1) * s + k[t].unsqueeze(-1) * v[t].unsqueeze(1)
+            want.append((q[t].unsqueeze(1) @ s).reshape(-1))
+            t += 1
+        states[slot] = s
+    want = torch.stack(want)
+    (walk, walk_state), (chunked, chunk_state) = results
+    for got, exact in ((walk, want), (chunked, want), (walk_state, states), (chunk_state, states)):
+        assert float((got - exact).norm() / exact.norm()) < 2e-6  # sums of float32, up to 200 terms a state element
+    # entries below the minimum walk in both
+    begin = 0
+    for count in counts:
+        if count < 33:
+            assert torch.equal(walk[begin : begin + count], chunked[begin : begin + count])
+        begin += count
