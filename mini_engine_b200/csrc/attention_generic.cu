@@ -19,7 +19,7 @@
 // and are combined in ascending order, so the arithmetic of a query depends only on its own
 // position: the same bits come out whether the token arrived in a whole prompt, in a
 // two-token portion or as a decoded token, and whatever else is in the batch.
-#include "common.cuh"
+#include "mma_sync.cuh"
 
 struct AttnArgs {
     const void* q;         // [tokens][heads][head_dim]
@@ -134,6 +134,275 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) paged_attention_generic_kerne
             out[e] = from_float<T>(y);
         }
     }
+}
+
+// ------------------------------------------------------------------ float32, keys shared by many rows
+//
+// The same attention in float32 with every key and value fetched once for a block of R rows, a row being a (token, query
+// head) pair of one entry and KV head: row r of an entry is its token r / group, head r % group of the group.  The
+// arithmetic of a row is the kernel's above, operation by operation (a score is one fmaf chain over the head; maximum and sum of
+// a tile by the same butterflies over its 32 keys; a value element one fmaf chain over the keys), so the bits are the same
+// whichever kernel and whichever R a step takes.  Tiles of 32 keys arrive by asynchronous copies, two buffers; 256 threads form
+// R x 32 scores (a thread 2 rows x 4 keys, or 1 x 2), a warp takes whole rows for the softmax, and a thread keeps one quad
+// of value elements of R * QP / 256 rows.  A tile that some row sees in part marks the weights of unseen keys, and
+// their values are left out (they may be anything); a tile that all rows see whole is not looked at twice.
+// Bound by the multiply-adds at R = 64 (256 FMA of a tile's 32 keys and a head of 128 per row and lane), by the latency of
+// a tile's chains at R = 16; see the figures at launch_rows.
+constexpr int ROW_THREADS = 256;
+constexpr uint32_t UNSEEN = 0x80000000u;  // the weight -0: a key that the row does not see
+
+struct RowArgs {
+    AttnArgs a;
+    const int* cu_tokens;
+};
+
+template <int R, int QP>
+__global__ void __launch_bounds__(ROW_THREADS) paged_attention_rows_kernel(RowArgs m) {
+    constexpr int KEYS = R == 64 ? 4 : 2, KEY_LANES = 32 / KEYS, ROWS = R * KEY_LANES / ROW_THREADS;  // a thread's scores
+    constexpr int HELD = R * QP / ROW_THREADS;                                                      // its rows of values
+    static_assert(ROWS >= 1 && HELD >= 1, "every thread has work");
+    constexpr int SP = 36;  // floats between two rows of weights
+    const AttnArgs& a = m.a;
+    extern __shared__ __align__(16) float row_shared[];
+    __shared__ int key_there[2][32];
+    __shared__ float row_max[R], row_sum[R], row_scale[R];
+    const int d = a.head_dim, dv = a.value_dim, kp = d + 4, vp = dv + 4;
+    const bool shared_rows = a.k_pages == a.v_pages;  // values are the first elements of the key rows
+    float* q = row_shared;                                   // [R][kp]
+    float* keys = q + R * kp;                                // [2][32][kp]
+    float* values = shared_rows ? keys : keys + 2 * 32 * kp; // [2][32][vp]
+    const int v_pitch = shared_rows ? kp : vp;
+    float* weights = shared_rows ? keys + 2 * 32 * kp : values + 2 * 32 * vp;  // [R][SP]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_trigger();
+    pdl_wait();
+    const int entry = blockIdx.z, kv = blockIdx.y, group = a.heads / a.kv_heads;
+    const int begin = m.cu_tokens[entry], rows = (m.cu_tokens[entry + 1] - begin) * group;
+    const int row0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * R;  // the last rows see the most keys: they go first
+    if (row0 >= rows) return;
+    const int live = min(R, rows - row0);
+    const int* table = a.block_table + static_cast<size_t>(entry) * a.table_width;
+    const float *k_pages = static_cast<const float*>(a.k_pages), *v_pages = static_cast<const float*>(a.v_pages);
+    auto position_of = [&](int r) { return a.positions[begin + (row0 + r) / group]; };
+    auto lowest_of = [&](int position) {
+        const int low = a.window > 0 ? max(position - a.window + 1, 0) : 0;
+        return a.chunk > 0 ? max(low, position / a.chunk * a.chunk) : low;
+    };
+    const int first_position = position_of(0), last_position = position_of(live - 1);
+    const int lowest = lowest_of(first_position), highest_low = lowest_of(last_position);
+
+    for (int i = tid; i < R * (d / 4); i += ROW_THREADS) {
+        const int r = i / (d / 4), e = i % (d / 4) * 4;
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < live)
+            x = *reinterpret_cast<const float4*>(static_cast<const float*>(a.q) +
+                                                 (static_cast<size_t>(begin + (row0 + r) / group) * a.heads + kv * group + (row0 + r) % group) * d + e);
+        *reinterpret_cast<float4*>(q + r * kp + e) = x;
+    }
+    for (int r = tid; r < R; r += ROW_THREADS) row_max[r] = -INFINITY, row_sum[r] = 0.0f;
+
+    // Eight threads fetch a key's row and its values.
+    auto fetch = [&](int tile, int buffer) {
+        const int j = tid >> 3, key = tile + j;
+        int page = -1;
+        if (key >= lowest && key <= last_position) page = table[key / a.page_size];
+        const size_t row = page >= 0 ? (static_cast<size_t>(page) * a.kv_heads + kv) * a.page_size + key % a.page_size : 0;
+        float* to = keys + (buffer * 32 + j) * kp;
+        for (int e = (tid & 7) * 4; e < d; e += 32) cp_async_16(to + e, k_pages + row * d + e, page >= 0);
+        if (!shared_rows) {
+            float* v_to = values + (buffer * 32 + j) * vp;
+            for (int e = (tid & 7) * 4; e < dv; e += 32) cp_async_16(v_to + e, v_pages + row * a.value_stride + e, page >= 0);
+        }
+        if ((tid & 7) == 0) key_there[buffer][j] = page >= 0;
+        cp_async_commit();
+    };
+
+    const int quad = tid % QP * 4, held0 = tid / QP * HELD;  // value elements, first row
+    float4 acc[HELD];
+#pragma unroll
+    for (int i = 0; i < HELD; ++i) acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int key_lane = tid % KEY_LANES, score_row = tid / KEY_LANES * ROWS;
+    const bool sigmoid = a.sigmoid_bias != nullptr;
+
+    int buffer = 0;
+    fetch(lowest / 32 * 32, 0);
+    for (int tile = lowest / 32 * 32; tile <= last_position; tile += 32, buffer ^= 1) {
+        if (tile + 32 <= last_position) fetch(tile + 32, buffer ^ 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* k_tile = keys + buffer * 32 * kp;
+        {
+            float dot[ROWS][KEYS];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int k = 0; k < KEYS; ++k) dot[r][k] = 0.0f;
+#pragma unroll 4
+            for (int e = 0; e < d; e += 4) {
+                float4 qq[ROWS], kk[KEYS];
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) qq[r] = *reinterpret_cast<const float4*>(q + (score_row + r) * kp + e);
+#pragma unroll
+                for (int k = 0; k < KEYS; ++k) kk[k] = *reinterpret_cast<const float4*>(k_tile + (key_lane + KEY_LANES * k) * kp + e);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int k = 0; k < KEYS; ++k) {
+                        dot[r][k] = fmaf(qq[r].x, kk[k].x, dot[r][k]);
+                        dot[r][k] = fmaf(qq[r].y, kk[k].y, dot[r][k]);
+                        dot[r][k] = fmaf(qq[r].z, kk[k].z, dot[r][k]);
+                        dot[r][k] = fmaf(qq[r].w, kk[k].w, dot[r][k]);
+                    }
+            }
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int k = 0; k < KEYS; ++k) weights[(score_row + r) * SP + key_lane + KEY_LANES * k] = dot[r][k];
+        }
+        __syncthreads();
+        const bool there = key_there[buffer][lane] != 0;
+        const bool whole = __all_sync(0xffffffffu, there) && tile >= highest_low && tile + 31 <= first_position;
+#pragma unroll 4
+        for (int r = warp; r < R; r += ROW_THREADS / 32) {
+            if (r >= live) break;
+            const int position = position_of(r), head = kv * group + (row0 + r) % group, key = tile + lane;
+            const bool seen = there && key >= lowest_of(position) && key <= position;
+            float score = -INFINITY;
+            if (seen) {
+                score = weights[r * SP + lane] * a.scale;
+                if (a.softcap > 0.0f) score = a.softcap * tanhf(score / a.softcap);
+                if (a.slopes) score -= a.slopes[head] * static_cast<float>(position - key);
+            }
+            float p = __uint_as_float(UNSEEN);
+            if (sigmoid) {
+                if (seen) p = 1.0f / (1.0f + expf(-(score + a.sigmoid_bias[head])));
+            } else {
+                const float old_max = row_max[r], new_max = fmaxf(old_max, warp_max(score));
+                float rescale = 1.0f;
+                if (new_max != -INFINITY) {  // uniform across the warp
+                    rescale = expf(old_max - new_max);
+                    const float weight = seen ? expf(score - new_max) : 0.0f;
+                    const float sum = row_sum[r] * rescale + warp_sum(weight);
+                    if (seen) p = weight;
+                    __syncwarp();
+                    if (lane == 0) row_max[r] = new_max, row_sum[r] = sum;
+                }
+                if (lane == 0) row_scale[r] = rescale;
+            }
+            weights[r * SP + lane] = p;
+        }
+        __syncthreads();
+        if (quad < dv) {
+            if (!sigmoid) {
+#pragma unroll
+                for (int i = 0; i < HELD; ++i) {
+                    const float f = row_scale[held0 + i];
+                    acc[i].x *= f, acc[i].y *= f, acc[i].z *= f, acc[i].w *= f;
+                }
+            }
+            const float* v_tile = values + buffer * 32 * v_pitch + quad;
+#pragma unroll 2
+            for (int j = 0; j < 32; j += 4) {
+                float4 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(v_tile + (j + u) * v_pitch);
+#pragma unroll
+                for (int i = 0; i < HELD; ++i) {
+                    const float4 w4 = *reinterpret_cast<const float4*>(weights + (held0 + i) * SP + j);
+                    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (!whole && __float_as_uint(w[u]) == UNSEEN) continue;
+                        acc[i].x = fmaf(w[u], v[u].x, acc[i].x);
+                        acc[i].y = fmaf(w[u], v[u].y, acc[i].y);
+                        acc[i].z = fmaf(w[u], v[u].z, acc[i].z);
+                        acc[i].w = fmaf(w[u], v[u].w, acc[i].w);
+                    }
+                }
+            }
+        }
+        __syncthreads();  // the next copies overwrite this buffer
+    }
+    cp_async_wait<0>();
+    if (quad >= dv) return;
+#pragma unroll
+    for (int i = 0; i < HELD; ++i) {
+        const int r = held0 + i;
+        if (r >= live) break;
+        const int token = begin + (row0 + r) / group, head = kv * group + (row0 + r) % group;
+        float denom = row_sum[r];
+        if (a.sink) denom += expf((a.sink_values ? a.sink_values[head] : 0.0f) - row_max[r]);  // the silent participant
+        float inv = sigmoid ? 1.0f : 1.0f / denom;
+        const size_t at = static_cast<size_t>(token) * a.heads + head;
+        if (a.gate && a.gate_width == 1) inv *= a.gate[at];
+        float4 y = make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv);
+        if (a.gate && a.gate_width > 1) {
+            const float* g = a.gate + at * a.gate_width + quad;
+            y.x *= g[0], y.y *= g[1], y.z *= g[2], y.w *= g[3];
+        }
+        *reinterpret_cast<float4*>(static_cast<float*>(a.out) + at * dv + quad) = y;
+    }
+}
+
+static size_t rows_shared_bytes(const AttnArgs& a, int rows) {
+    const size_t kp = a.head_dim + 4, vp = a.k_pages == a.v_pages ? 0 : a.value_dim + 4;
+    return (rows * kp + 64 * (kp + vp) + static_cast<size_t>(rows) * 36) * sizeof(float);
+}
+
+// Against one warp per (token, head), a prompt of 512 tokens, 16 heads of 128 in 8 KV heads: 1,361 -> 165 us; 256 tokens, 32
+// heads: 826 -> 143; eight decoded tokens behind 17 to 512: 768 -> 68, over latent rows of 576 with 512 values 768 -> 179 us.
+template <int R, int QP>
+static int launch_rows(const RowArgs& m, int entries, int longest, cudaStream_t stream) {
+    static SharedMemoryOptIn opt_in;
+    if (const int e = opt_in(paged_attention_rows_kernel<R, QP>, 200 * 1024)) return e;
+    const int group = m.a.heads / m.a.kv_heads;
+    const long long blocks = (static_cast<long long>(longest) * group + R - 1) / R;
+    if (blocks > 0x7fffffffll || m.a.kv_heads > 65535 || entries > 65535) return ME_ERR_UNSUPPORTED;
+    return launch_kernel(paged_attention_rows_kernel<R, QP>, dim3(static_cast<unsigned>(blocks), m.a.kv_heads, entries), ROW_THREADS,
+                         rows_shared_bytes(m.a, R), stream, m);
+}
+
+template <int R>
+static int launch_rows_of(const RowArgs& m, int entries, int longest, cudaStream_t stream) {
+    if (m.a.value_dim <= 64) return launch_rows<R, 16>(m, entries, longest, stream);
+    if (m.a.value_dim <= 128) return launch_rows<R, 32>(m, entries, longest, stream);
+    if (m.a.value_dim <= 256) return launch_rows<R, 64>(m, entries, longest, stream);
+    return launch_rows<R, 128>(m, entries, longest, stream);
+}
+
+// Whether the kernel takes these sizes (float32; everything else takes the one above): rows of whole 16-byte pieces, and 16 rows'
+// queries, weights and two tiles in shared memory.
+ME_EXPORT int me_paged_attention_rows_supports(int head_dim, int value_dim, int value_stride, int values_in_keys) {
+    AttnArgs a = {};
+    a.head_dim = head_dim, a.value_dim = value_dim, a.value_stride = value_stride;
+    a.v_pages = values_in_keys ? nullptr : &a;  // compared with k_pages, not read
+    return head_dim >= 4 && head_dim % 4 == 0 && value_dim >= 4 && value_dim % 4 == 0 && value_dim <= 32 * MAX_DIM_PER_LANE &&
+           value_stride % 4 == 0 && rows_shared_bytes(a, 16) <= 200 * 1024;
+}
+
+// The attention of me_paged_attention_generic in float32, with its bits.  The tokens of entry e are cu_tokens[e] ..
+// cu_tokens[e + 1], in ascending position; no entry has more than `longest`.
+ME_EXPORT int me_paged_attention_rows(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
+                                      const int* cu_tokens, const int* positions, void* out, float scale, int entries, int longest,
+                                      int heads, int kv_heads, int head_dim, int page_size, int table_width, int window,
+                                      int value_dim, int sink, const float* gate, int gate_width, int value_stride,
+                                      const float* slopes, const float* sink_values, float softcap, int chunk,
+                                      const float* sigmoid_bias, cudaStream_t stream) {
+    if (entries <= 0 || longest <= 0) return 0;
+    if (gate && gate_width != 1 && gate_width != value_dim) return ME_ERR_ARGUMENT;
+    if (value_stride < value_dim || chunk < 0 || (sigmoid_bias && sink)) return ME_ERR_ARGUMENT;
+    if (heads < 1 || kv_heads < 1 || heads % kv_heads || !me_paged_attention_rows_supports(head_dim, value_dim, value_stride, k_pages == v_pages)) return ME_ERR_UNSUPPORTED;
+    for (const void* p : {q, k_pages, v_pages, static_cast<const void*>(out)})
+        if (reinterpret_cast<uintptr_t>(p) % 16) return ME_ERR_UNSUPPORTED;
+    RowArgs m{{q, k_pages, v_pages, block_table, nullptr, positions, out, scale, 0, heads, kv_heads, head_dim, page_size,
+               table_width, window, value_dim, sink, gate, gate_width, value_stride, slopes, sink_values, softcap, chunk, sigmoid_bias},
+              cu_tokens};
+    // 64 rows share a key where an entry brings that many; else 16, whose tiles take a third of the time.  Two blocks of
+    // 64 rows fit an SM up to heads of 128.
+    const long long rows = static_cast<long long>(longest) * (heads / kv_heads);
+    if (rows > 32 && rows_shared_bytes(m.a, 64) <= 113 * 1024) return launch_rows_of<64>(m, entries, longest, stream);
+    return launch_rows_of<16>(m, entries, longest, stream);
 }
 
 ME_EXPORT int me_paged_attention_generic(const void* q, const void* k_pages, const void* v_pages,

@@ -481,20 +481,8 @@ def gemm_tensor_core_swiglu(plan, x: torch.Tensor, act: torch.Tensor, activation
 # -------------------------------------------------------------------------------- attention
 
 
-def paged_attention_generic(
-    q, k_pages, v_pages, block_table, entry_of_token, positions, out, heads, kv_heads, head_dim, scale, window,
-    value_dim: int | None = None, sink: bool = False, gate: torch.Tensor | None = None,
-    slopes: torch.Tensor | None = None, sink_values: torch.Tensor | None = None, softcap: float = 0.0, chunk: int = 0,
-    sigmoid_bias: torch.Tensor | None = None,
-) -> None:
-    """One warp per (token, head), any head size; ``softcap`` > 0: a scaled score ``s`` becomes ``softcap * tanh(s /
-    softcap)``; ``value_dim``: width of a value head when it differs;
-    ``sink``: one more participant of score zero and no value in the softmax, or of the learned score
-    ``sink_values[h]`` (float32 ``[heads]``); ``gate`` (float32 ``[T, heads]`` or ``[T, heads * value_dim]``): a
-    multiplier on each head's output, or on each of its elements; ``slopes`` (float32 ``[heads]``): ``slopes[h] *
-    (p - j)`` is taken off the scaled score of query ``p`` and key ``j``; ``chunk`` > 0: a query at ``p`` sees keys from ``p //
-    chunk * chunk`` on; ``sigmoid_bias`` (float32 ``[heads]``): a key's weight is ``sigmoid(s + bias_h)``, not normalised, in
-    the place of a softmax.  ``v_pages=None``: the values are the first ``value_dim`` elements of the key rows."""
+def _check_generic_attention(q, k_pages, v_pages, out, heads, kv_heads, head_dim, value_dim, gate, slopes, sink_values, sigmoid_bias):
+    """The checks of the two kernels for any head size; returns the value pages and width, the gate's width and the value stride."""
     value_dim = head_dim if value_dim is None else value_dim
     gate_width = 1
     if gate is not None:
@@ -518,6 +506,26 @@ def paged_attention_generic(
     if k_pages.shape[1:] != (kv_heads, k_pages.shape[2], head_dim):
         raise KernelError(f"key pages {tuple(k_pages.shape)} do not fit the head sizes")
     _need(q, None, "q"), _need(out, q.dtype, "out"), _need(k_pages, q.dtype, "k_pages"), _need(v_pages, q.dtype, "v_pages")
+    return v_pages, value_dim, gate_width, value_stride
+
+
+def paged_attention_generic(
+    q, k_pages, v_pages, block_table, entry_of_token, positions, out, heads, kv_heads, head_dim, scale, window,
+    value_dim: int | None = None, sink: bool = False, gate: torch.Tensor | None = None,
+    slopes: torch.Tensor | None = None, sink_values: torch.Tensor | None = None, softcap: float = 0.0, chunk: int = 0,
+    sigmoid_bias: torch.Tensor | None = None,
+) -> None:
+    """One warp per (token, head), any head size; ``softcap`` > 0: a scaled score ``s`` becomes ``softcap * tanh(s /
+    softcap)``; ``value_dim``: width of a value head when it differs;
+    ``sink``: one more participant of score zero and no value in the softmax, or of the learned score
+    ``sink_values[h]`` (float32 ``[heads]``); ``gate`` (float32 ``[T, heads]`` or ``[T, heads * value_dim]``): a
+    multiplier on each head's output, or on each of its elements; ``slopes`` (float32 ``[heads]``): ``slopes[h] *
+    (p - j)`` is taken off the scaled score of query ``p`` and key ``j``; ``chunk`` > 0: a query at ``p`` sees keys from ``p //
+    chunk * chunk`` on; ``sigmoid_bias`` (float32 ``[heads]``): a key's weight is ``sigmoid(s + bias_h)``, not normalised, in
+    the place of a softmax.  ``v_pages=None``: the values are the first ``value_dim`` elements of the key rows."""
+    v_pages, value_dim, gate_width, value_stride = _check_generic_attention(
+        q, k_pages, v_pages, out, heads, kv_heads, head_dim, value_dim, gate, slopes, sink_values, sigmoid_bias
+    )
     _need(block_table, torch.int32, "block_table"), _need(entry_of_token, torch.int32, "entry_of_token")
     _need(positions, torch.int32, "positions")
     fn = _fn(
@@ -532,6 +540,44 @@ def paged_attention_generic(
         _ptr(slopes), _ptr(sink_values), float(softcap or 0.0), int(chunk), _ptr(sigmoid_bias), _stream(),
     )  # fmt: skip
     _check(code, "paged_attention_generic")
+
+
+def attention_rows_supports(q, k_pages, v_pages, out, head_dim: int, value_dim: int | None) -> bool:
+    """Whether float32 attention of these sizes and buffers takes the kernel whose blocks share every key among many rows."""
+    value_dim = head_dim if value_dim is None else value_dim
+    fn = load_library("attention_generic").me_paged_attention_rows_supports
+    fn.argtypes, fn.restype = [c_int] * 4, c_int
+    values = k_pages if v_pages is None else v_pages
+    return bool(fn(head_dim, value_dim, head_dim if v_pages is None else value_dim, 1 if v_pages is None else 0)) and all(
+        t.data_ptr() % 16 == 0 for t in (q, k_pages, values, out)
+    )
+
+
+def paged_attention_rows(
+    q, k_pages, v_pages, block_table, ctx, out, heads, kv_heads, head_dim, scale, window,
+    value_dim: int | None = None, sink: bool = False, gate: torch.Tensor | None = None,
+    slopes: torch.Tensor | None = None, sink_values: torch.Tensor | None = None, softcap: float = 0.0, chunk: int = 0,
+    sigmoid_bias: torch.Tensor | None = None,
+) -> None:  # fmt: skip
+    """:func:`paged_attention_generic` in float32 with its bits, every key fetched once for 64 or 16 (token, head) rows
+    of an entry.  The context gives ``cu_tokens``, ``num_entries``, ``max_query_len`` and ``positions`` (ascending within an entry)."""
+    v_pages, value_dim, gate_width, value_stride = _check_generic_attention(
+        q, k_pages, v_pages, out, heads, kv_heads, head_dim, value_dim, gate, slopes, sink_values, sigmoid_bias
+    )
+    _need(q, torch.float32, "q"), _need(block_table, torch.int32, "block_table"), _need(ctx.positions, torch.int32, "positions")
+    _need(ctx.cu_tokens, torch.int32, "cu_tokens")
+    fn = _fn(
+        "attention_generic",
+        "me_paged_attention_rows",
+        [c_void_p] * 7 + [c_float] + [c_int] * 9 + [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p],
+    )
+    code = fn(
+        _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), _ptr(ctx.cu_tokens), _ptr(ctx.positions), _ptr(out), scale,
+        ctx.num_entries, ctx.max_query_len, heads, kv_heads, head_dim, k_pages.shape[2], block_table.shape[1], window, value_dim,
+        1 if (sink or sink_values is not None) else 0, _ptr(gate), gate_width, value_stride, _ptr(slopes), _ptr(sink_values),
+        float(softcap or 0.0), int(chunk), _ptr(sigmoid_bias), _stream(),
+    )  # fmt: skip
+    _check(code, "paged_attention_rows")
 
 
 def paged_attention(
@@ -556,6 +602,12 @@ def paged_attention(
                 slopes=slopes, sink_values=sink_values, softcap=softcap, chunk=chunk, sigmoid_bias=sigmoid_bias,
             )  # fmt: skip
             return
+    if q.dtype == torch.float32 and attention_rows_supports(q, k_pages, v_pages, out, head_dim, value_dim):
+        paged_attention_rows(
+            q, k_pages, v_pages, block_table, ctx, out, heads, kv_heads, head_dim, scale, window, value_dim=value_dim, sink=sink,
+            gate=gate, slopes=slopes, sink_values=sink_values, softcap=softcap, chunk=chunk, sigmoid_bias=sigmoid_bias,
+        )  # fmt: skip
+        return
     paged_attention_generic(
         q, k_pages, v_pages, block_table, ctx.entry_of_token, ctx.positions, out, heads, kv_heads, head_dim,
         scale, window, value_dim=value_dim, sink=sink, gate=gate, slopes=slopes, sink_values=sink_values, softcap=softcap,
