@@ -62,6 +62,10 @@ struct SplitParams {
     int tokens, outs, inner;
     int k_blocks, per_segment;
     int clustered;  // the segments of a tile are the CTAs of a cluster along z
+    // Grouped product: the weight holds `group_rows` rows per group, one group after the other, and token tile b belongs to
+    // group group_of_block[b] (negative: it holds no rows and its CTAs return at once).  `outs` counts one group's features.
+    const int* group_of_block;
+    int group_rows;
 };
 
 __device__ __forceinline__ uint32_t upper_pair(float even, float odd) {  // bfloat16 pair, the even k in the low half
@@ -111,9 +115,9 @@ __device__ __noinline__ float plain_sum(const float* x, const float* w, int inne
     }
     return sum;
 }
-__device__ __forceinline__ float finite_or_again(const SplitParams& p, int t, int n, float v) {
+__device__ __forceinline__ float finite_or_again(const SplitParams& p, int t, int w_row, float v) {
     if (fabsf(v) <= 3.402823466e38f) return v;
-    return plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(n) * p.inner, p.inner);
+    return plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(w_row) * p.inner, p.inner);
 }
 
 template <int NT>
@@ -135,6 +139,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int kb_begin = p.clustered ? blockIdx.z * p.per_segment : 0;
     const int kb_end = p.clustered ? min(kb_begin + p.per_segment, p.k_blocks) : p.k_blocks;
     const int blocks = kb_end - kb_begin;
+    int w0 = n0;  // first weight row of the tile
+    if (p.group_of_block != nullptr) {
+        pdl_wait();  // a kernel before this one wrote the groups
+        const int group = p.group_of_block[blockIdx.x];
+        if (group < 0) return;  // every CTA of the tile (and of its cluster): nothing has been set up yet
+        w0 = group * p.group_rows + n0;
+    }
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], CONVERTERS / 32); }
@@ -159,8 +170,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 uint8_t* at = raw + (i % C::STAGES) * C::RAW_BYTES;
                 mbar_expect_tx(&full[i % C::STAGES], C::RAW_BYTES);
                 const int k = (kb_begin + i) * SPLIT_K;
-                tma_load_2d(at, &map_w, k, n0, &full[i % C::STAGES]);
-                tma_load_2d(at + C::W_BYTES / 2, &map_w, k + SPLIT_K / 2, n0, &full[i % C::STAGES]);
+                tma_load_2d(at, &map_w, k, w0, &full[i % C::STAGES]);
+                tma_load_2d(at + C::W_BYTES / 2, &map_w, k + SPLIT_K / 2, w0, &full[i % C::STAGES]);
             };
             auto load_x = [&](int i) {
                 uint8_t* at = raw + (i % C::STAGES) * C::RAW_BYTES + C::W_BYTES;
@@ -329,7 +340,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
             for (int c = 0; c < COLUMNS; ++c) {
                 const int t = t0 + column + c;
-                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, n, total[c]);
+                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, w0 + row, total[c]);
             }
         }
     }
@@ -352,7 +363,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                 for (int s = 1; s < MAX_SEGMENTS; ++s)
                     if (s < segments) part[0] += part[s];
-                p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, n, part[0]);
+                p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, w0 + row, part[0]);
             }
         }
         cluster_sync();  // the others may still read this CTA's part
@@ -425,10 +436,11 @@ static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, cons
 }
 
 // out[t][n] = sum_k x[t][k] * w[n][k]; `segments` ranges of k blocks whose sums are added in ascending order, in one
-// CTA or (`clustered`) in a cluster's CTAs.  `map_x` has boxes of `tile` (16 or 64) rows.
+// CTA or (`clustered`) in a cluster's CTAs.  With `group_of_block` a grouped product: `tile` rows of x to a group.  `map_x` has boxes of `tile` (16 or 64) rows.
 ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x, const float* w, float* out, int tokens, int outs,
-                            int inner, int tile, int segments, int clustered, cudaStream_t stream) {
+                            int inner, int tile, int segments, int clustered, const int* group_of_block, int group_rows, cudaStream_t stream) {
     if (tokens <= 0 || outs <= 0) return 0;
+    if (group_of_block != nullptr && (group_rows < outs || tokens % tile)) return ME_ERR_ARGUMENT;
     if (inner <= 0 || inner % 4 != 0 || segments < 1 || segments > MAX_SEGMENTS) return ME_ERR_ARGUMENT;
     SplitParams p = {};
     p.x = x, p.w = w, p.out = out;
@@ -436,6 +448,7 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     p.k_blocks = (inner + SPLIT_K - 1) / SPLIT_K;
     p.per_segment = (p.k_blocks + segments - 1) / segments;
     p.clustered = clustered && segments > 1;
+    p.group_of_block = group_of_block, p.group_rows = group_rows;
     if ((segments - 1) * p.per_segment >= p.k_blocks) return ME_ERR_ARGUMENT;  // a segment would be empty
     alignas(64) CUtensorMap w_map, x_map;
     memcpy(&w_map, map_w, sizeof(w_map));

@@ -252,7 +252,7 @@ def _split_library():
         lib = load_library("gemm_split")
         lib.me_make_tensor_map_f32.argtypes = [c_void_p, c_void_p, c_ulonglong, c_ulonglong, c_uint]
         lib.me_make_tensor_map_f32.restype = c_int
-        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 6 + [c_void_p]
+        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_int, c_void_p]
         lib.me_gemm_split.restype = c_int
         lib.me_gemm_split_take_error.argtypes = [ctypes.POINTER(c_int)]
         lib.me_gemm_split_take_error.restype = c_int
@@ -278,24 +278,31 @@ def split_segments(outs: int, inner: int) -> int:
     return -(-k_blocks // per_segment)
 
 
-def split_side_by_side(tokens: int, outs: int, segments: int) -> bool:
+def split_tile(tokens: int) -> int:
+    return SPLIT_TILES[0] if tokens <= SPLIT_TILES[0] else SPLIT_TILES[1]
+
+
+def split_side_by_side(tokens: int, outs: int, segments: int, tile: int | None = None) -> bool:
     """Whether a tile's segments run in the CTAs of a cluster (few tiles) or one after the other in a CTA; the bits are the
     same.  Side by side when that takes fewer rounds of resident CTAs, a round being one segment long."""
-    tile = SPLIT_TILES[0] if tokens <= SPLIT_TILES[0] else SPLIT_TILES[1]
+    tile = tile or split_tile(tokens)
     slots = NUM_SMS * (2 if tile == SPLIT_TILES[0] else 1)
     ctas = -(-outs // BLOCK_N) * -(-tokens // tile)
     return -(-ctas * segments // slots) < -(-ctas // slots) * segments
 
 
 class SplitPlan:
-    """A float32 weight for :func:`gemm_split`."""
+    """A float32 weight for :func:`gemm_split`, or, with ``group_rows`` rows for each group, for :func:`gemm_split_grouped`."""
 
-    def __init__(self, weight: torch.Tensor):
+    def __init__(self, weight: torch.Tensor, group_rows: int | None = None):
         if not split_supports(weight):
             raise RuntimeError(f"the float32 tensor-core product takes a contiguous float32 CUDA weight whose width is a multiple of 4 and at least {SPLIT_MIN_INNER}")
         self.weight = weight
         self.rows, self.inner = weight.shape
-        self.segments = split_segments(self.rows, self.inner)
+        if group_rows is not None and (group_rows < 1 or self.rows % group_rows):
+            raise RuntimeError(f"{self.rows} weight rows do not form groups of {group_rows}")
+        self.group_rows = group_rows
+        self.segments = split_segments(group_rows or self.rows, self.inner)
         self.map = _make_map_f32(weight, BLOCK_N)
 
 
@@ -311,6 +318,16 @@ def _make_map_f32(tensor: torch.Tensor, box_rows: int) -> ctypes.Array:
 _split_activation_maps: dict[tuple[int, int, int, int], ctypes.Array] = {}
 
 
+def _split_activation_map(x: torch.Tensor, tile: int) -> ctypes.Array:
+    key = (x.data_ptr(), x.shape[0], x.shape[1], tile)
+    held = _split_activation_maps.get(key)
+    if held is None:
+        if len(_split_activation_maps) > 8192:
+            _split_activation_maps.clear()
+        held = _split_activation_maps[key] = _make_map_f32(x, tile)
+    return held
+
+
 def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side: bool | None = None) -> None:
     """``out[T, rows] = x @ weight^T`` in float32 (three bfloat16 pieces of each operand, see gemm_split.cu).
     ``side_by_side`` pins where a tile's segments run instead of the rule's choice: the kernel tests run both."""
@@ -319,22 +336,43 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side
         raise RuntimeError(f"activation {tuple(x.shape)} {x.dtype} does not fit a float32 weight of width {plan.inner}")
     if out.dtype != torch.float32 or tuple(out.shape) != (tokens, plan.rows) or not out.is_contiguous():
         raise RuntimeError(f"output {tuple(out.shape)} does not fit [{tokens}, {plan.rows}] float32")
-    tile = SPLIT_TILES[0] if tokens <= SPLIT_TILES[0] else SPLIT_TILES[1]
-    key = (x.data_ptr(), tokens, plan.inner, tile)
-    held = _split_activation_maps.get(key)
-    if held is None:
-        if len(_split_activation_maps) > 8192:
-            _split_activation_maps.clear()
-        held = _split_activation_maps[key] = _make_map_f32(x, tile)
+    tile = split_tile(tokens)
     if side_by_side is None:
         side_by_side = split_side_by_side(tokens, plan.rows, plan.segments)
     code = _split_library().me_gemm_split(
-        plan.map, held, x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,
-        plan.segments, 1 if side_by_side else 0, _ops_stream(),
+        plan.map, _split_activation_map(x, tile), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,
+        plan.segments, 1 if side_by_side else 0, None, 0, _ops_stream(),
     )  # fmt: skip
     _count_launch()
     if code != 0:
         raise RuntimeError(f"float32 tensor-core product failed to launch (code {code})")
+
+
+def gemm_split_grouped(
+    plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, group_of_block: torch.Tensor, pad: int, filled: int, side_by_side: bool | None = None
+) -> None:
+    """A float32 product over rows that are sorted by group: the plan's weight holds ``plan.group_rows`` rows per group, run ``b``
+    of ``pad`` rows of ``x`` (one of ``SPLIT_TILES``) belongs to group ``group_of_block[b]`` (int32 on the device; negative: no rows
+    there), ``out[t] = x[t] @ weight_of_group^T``.  A row's bits depend on the row and its group's weight alone.  ``filled``:
+    about how many runs hold rows, for the choice of the form."""
+    rows, outs = x.shape[0], plan.group_rows
+    if outs is None:
+        raise RuntimeError("this plan was not made for a grouped product")
+    if x.dtype != torch.float32 or not x.is_contiguous() or x.dim() != 2 or x.shape[1] != plan.inner or x.data_ptr() % 16:
+        raise RuntimeError(f"activation {tuple(x.shape)} {x.dtype} does not fit a float32 weight of width {plan.inner}")
+    if out.dtype != torch.float32 or tuple(out.shape) != (rows, outs) or not out.is_contiguous():
+        raise RuntimeError(f"output {tuple(out.shape)} does not fit [{rows}, {outs}] float32")
+    if pad not in SPLIT_TILES or rows % pad or group_of_block.dtype != torch.int32 or group_of_block.numel() < rows // pad:
+        raise RuntimeError("the rows of a grouped product come in runs of a token tile with one int32 group each")
+    if side_by_side is None:
+        side_by_side = split_side_by_side(max(1, min(filled, rows // pad)) * pad, outs, plan.segments, pad)
+    code = _split_library().me_gemm_split(
+        plan.map, _split_activation_map(x, pad), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, plan.inner, pad,
+        plan.segments, 1 if side_by_side else 0, group_of_block.data_ptr(), outs, _ops_stream(),
+    )  # fmt: skip
+    _count_launch()
+    if code != 0:
+        raise RuntimeError(f"grouped float32 tensor-core product failed to launch (code {code})")
 
 
 GROUP_PAD = 128  # rows of a run of the sorted rows that belongs to one group: the token tile of the grouped product

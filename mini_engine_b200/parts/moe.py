@@ -20,7 +20,7 @@ multiplied by ``sigmoid(W_sg h)``, one number per token, formed in 32-bit with t
 How it runs, two forms; neither has a shape that depends on the choice, so both can be captured in a graph, and in
 both a token's result does not depend on the rest of the batch.
 
-* *All units, masked* (few tokens, float32, sizes that the tensor-core product does not take): all units' gate and
+* *All units, masked* (few tokens in bfloat16, sizes that the tensor-core products do not take): all units' gate and
   up matrices are one row-concatenated weight and all down matrices one column-concatenated weight.  The routing
   kernel leaves a dense map ``[T, units]`` of weights (zero for units that a token did not choose); the activation
   kernel multiplies every unit's features by its weight for the token; the down product then *is* the weighted sum
@@ -30,7 +30,9 @@ both a token's result does not depend on the rest of the batch.
   in an array sorted by unit, each unit's run padded to whole tiles of 128 rows; the tokens' inputs are gathered
   into it; a grouped tensor-core product whose tiles read the weights of their run's unit forms the gated
   activations (the gate in its epilogue), a second one the down products, and a last kernel adds a token's rows
-  with their weights in the order of its choices.  Only chosen units are computed.
+  with their weights in the order of its choices.  Only chosen units are computed.  In float32 every step takes this
+  form, with runs padded to 16 or 64 rows and the activation as a kernel of its own: a token's bits then do not depend on
+  how many tokens its step holds.
 """
 
 from __future__ import annotations
@@ -47,6 +49,9 @@ from mini_engine_b200.weights.loader import WeightSpec
 # From this many tokens on a bfloat16 step sorts its rows by unit and computes only chosen units.  Below, the
 # masked form's two products over all units cost less than the sorted form's five launches and padded tiles.
 SORTED_MIN_TOKENS = 256
+# Rows of a run in float32: the token tiles of its grouped product, by how many rows a unit has on average.  16-row tiles
+# stream a unit's weights from two CTAs per SM; 64 rows read them once for four times the rows.
+SORTED_PAD_FEW, SORTED_PAD_MANY = 16, 64
 
 
 @register("feed_forward", "routed_experts")
@@ -116,6 +121,7 @@ class RoutedExperts(FeedForward):
         self.shared_gate_up: GatedLinear | ActivatedLinear | None = None
         self.correction_values: torch.Tensor | None = None
         self.shared_down: Linear | None = None
+        self.sorted32 = False  # float32: every step's rows are sorted by unit
         self.sorted_gate_up = self.sorted_down = None  # plans of the grouped products, when the sizes allow them
 
     def _name(self, unit: int, which: str) -> str:
@@ -146,8 +152,10 @@ class RoutedExperts(FeedForward):
         ups = [tensors[self._name(unit, "up")] for unit in range(self.units)]
         downs = [tensors[self._name(unit, "down")] for unit in range(self.units)]
         gates = [tensors[self._name(unit, "gate")] for unit in range(self.units)] if self.gated else []
-        self.gate_up = Linear(torch.cat(gates + ups, dim=0).contiguous())  # [all gates | all ups]
-        self.down = Linear(torch.cat(downs, dim=1).contiguous())
+        self.sorted32 = ops.split_gemm_supports(ups[0]) and ops.split_gemm_supports(downs[0])
+        if not self.sorted32:
+            self.gate_up = Linear(torch.cat(gates + ups, dim=0).contiguous())  # [all gates | all ups]
+            self.down = Linear(torch.cat(downs, dim=1).contiguous())
         self.router = tensors[self.prefix + self.names["router"]]
         if self.has_shared_gate:  # one more row of the router's product
             self.router = torch.cat((self.router, tensors[self.prefix + self.names["shared_gate"]]), dim=0).contiguous()
@@ -165,6 +173,10 @@ class RoutedExperts(FeedForward):
             else:
                 self.shared_gate_up = ActivatedLinear(tensors[shared + self.names["up"]], self.activation)
             self.shared_down = Linear(tensors[shared + self.names["down"]])
+        if self.sorted32:
+            rows = [torch.cat((gate, up), dim=0) for gate, up in zip(gates, ups)] if self.gated else ups
+            self.sorted_gate_up = ops.SplitPlan(torch.cat(rows, dim=0).contiguous(), group_rows=rows[0].shape[0])
+            self.sorted_down = ops.SplitPlan(torch.cat(downs, dim=0).contiguous(), group_rows=self.hidden)
         if ups[0].dtype == torch.bfloat16 and ops.tensor_core_gemm_supports(self.inter, self.hidden) and ops.tensor_core_gemm_supports(self.hidden, self.inter):
             # unit after unit: [gate rows; up rows] of each (or its up rows alone), and the down matrices stacked by rows
             rows = [torch.cat((gate, up), dim=0) for gate, up in zip(gates, ups)] if self.gated else ups
@@ -207,7 +219,7 @@ class RoutedExperts(FeedForward):
     def _sorted(self, tokens: int) -> bool:
         # Many tokens: only chosen units are computed.  Very few: only chosen units' weights are read.  The choice
         # depends on the token count alone, so a captured step always takes the form it was captured with.
-        return self.sorted_gate_up is not None and (tokens >= SORTED_MIN_TOKENS or 2 * tokens * self.top <= self.units)
+        return self.sorted32 or self.sorted_gate_up is not None and (tokens >= SORTED_MIN_TOKENS or 2 * tokens * self.top <= self.units)
 
     def _forward_routed(self, h: torch.Tensor, ctx: StepContext, chosen, chosen_weight, weights) -> torch.Tensor:
         if self._sorted(h.shape[0]):
@@ -226,6 +238,8 @@ class RoutedExperts(FeedForward):
     def _sorted_products(self, h: torch.Tensor, ctx: StepContext, chosen: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
         """The chosen units' outputs, row by row in an order sorted by unit, and the row of every (token, choice)."""
         tokens, pad = h.shape[0], ops.GROUP_PAD
+        if self.sorted32:
+            pad = SORTED_PAD_FEW if tokens * self.top <= SORTED_PAD_FEW * self.units else SORTED_PAD_MANY
         # every unit's run may end in a partly filled tile; the capacity is a function of the step's token count alone
         capacity = -(-(tokens * self.top + self.units * (pad - 1)) // pad) * pad
         grow = ctx.workspace.growing
@@ -236,6 +250,17 @@ class RoutedExperts(FeedForward):
         rows = grow("routed.rows", (capacity, self.hidden), h.dtype)
         ops.gather_rows(h, token_of, rows)
         act = grow("routed.sorted_act", (capacity, self.inter), h.dtype)
+        if self.sorted32:
+            filled = tokens * self.top // pad + min(self.units, tokens * self.top) // 2
+            both = grow("routed.sorted_both", (1, capacity, self.sorted_gate_up.group_rows), torch.float32)
+            ops.gemm_split_grouped(self.sorted_gate_up, rows, both[0], unit_of_block, pad, filled)
+            if self.gated:
+                ops.swiglu(both, act, self.gate_slope, self.limit, self.up_offset)
+            else:
+                ops.activation(both, act, self.activation)
+            down = grow("routed.sorted_down", (capacity, self.hidden), torch.float32)
+            ops.gemm_split_grouped(self.sorted_down, act, down, unit_of_block, pad, filled)
+            return down, row_of
         if self.gated:
             ops.gemm_tensor_core_grouped(
                 self.sorted_gate_up, rows, act, unit_of_block, 2 * self.inter, self.inter, dual_rows=self.inter,

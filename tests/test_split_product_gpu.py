@@ -89,3 +89,40 @@ def test_weights_that_tma_cannot_address_are_refused_by_the_rule():
     assert not tc.split_supports(torch.randn(4, 130, device="cuda"))
     assert not tc.split_supports(torch.randn(4, 60, device="cuda"))
     assert not tc.split_supports(torch.randn(4, 128, device="cuda").to(torch.bfloat16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,units,top,outs,inner", [(1, 4, 1, 64, 64), (9, 8, 2, 130, 260), (70, 5, 3, 384, 1100), (300, 8, 2, 200, 520)])
+def test_grouped_product_gives_the_bits_of_each_groups_own(tokens, units, top, outs, inner):
+    """Rows sorted by unit, one unit without rows, choices outside the units; runs of 16 and of 64 rows, segments side by
+    side and one after the other: every row has the bits of the product of its own unit's weight alone."""
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(tokens)
+    h, w = torch.randn(tokens, inner, device="cuda"), torch.randn(units, outs, inner, device="cuda")
+    scores = torch.rand(tokens, units + 1)
+    scores[:, min(2, units - 1)] = -1.0  # nobody's choice unless all are needed
+    chosen = scores.topk(top, dim=1).indices.to(torch.int32).cuda()  # `units` itself: outside
+    alone = []
+    for u in range(units):
+        out = torch.empty(tokens, outs, device="cuda")
+        tc.gemm_split(tc.SplitPlan(w[u].clone()), h, out)
+        alone.append(out)
+    plan = tc.SplitPlan(w.reshape(units * outs, inner), group_rows=outs)
+    for pad in (16, 64):
+        capacity = -(-(tokens * top + units * (pad - 1)) // pad) * pad
+        ints = lambda *shape: torch.empty(shape, dtype=torch.int32, device="cuda")  # noqa: E731
+        row_of, token_of, unit_of_block = ints(tokens, top), ints(capacity), ints(capacity // pad)
+        ops.sort_by_unit(chosen=chosen, units=units, pad=pad, row_of=row_of, token_of=token_of, unit_of_block=unit_of_block)
+        rows = torch.empty(capacity, inner, device="cuda")
+        ops.gather_rows(h, token_of, rows)
+        for side_by_side in (False, True):
+            out = torch.full((capacity, outs), float("nan"), device="cuda")
+            tc.gemm_split_grouped(plan, rows, out, unit_of_block, pad, units, side_by_side)
+            assert tc.take_error() == 0
+            for t in range(tokens):
+                for u, row in zip(chosen[t].tolist(), row_of[t].tolist()):
+                    assert (row < 0) == (u >= units)
+                    if row >= 0:
+                        assert torch.equal(out[row], alone[u][t])
