@@ -48,7 +48,7 @@ struct PrepArgs {
 constexpr int PREP_TOKENS = 8;
 
 __global__ void __launch_bounds__(256) gla_prepare_kernel(PrepArgs a) {
-    extern __shared__ float low[];  // [PREP_TOKENS][rank]
+    extern __shared__ __align__(16) float low[];  // [PREP_TOKENS][rank]
     const int first = blockIdx.x * PREP_TOKENS;
     const int count = min(PREP_TOKENS, a.tokens - first);
     pdl_trigger();
@@ -66,23 +66,45 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(PrepArgs a) {
         float z[PREP_TOKENS];
 #pragma unroll
         for (int t = 0; t < PREP_TOKENS; ++t) z[t] = 0.0f;
-        for (int r = 0; r < a.rank; ++r) {
+        // 16 rows of A2 are fetched together, ahead of the sums (in ascending r).
+        int r = 0;
+        for (; r + 16 <= a.rank && a.rank % 4 == 0; r += 16) {
+            float w[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) w[j] = a.a2t[static_cast<size_t>(r + j) * items + i];
+#pragma unroll
+            for (int j = 0; j < 16; j += 4)
+#pragma unroll
+                for (int t = 0; t < PREP_TOKENS; ++t) {
+                    const float4 x = *reinterpret_cast<const float4*>(low + t * a.rank + r + j);  // rows behind `count` are not used
+                    z[t] = fmaf(w[j], x.x, z[t]);
+                    z[t] = fmaf(w[j + 1], x.y, z[t]);
+                    z[t] = fmaf(w[j + 2], x.z, z[t]);
+                    z[t] = fmaf(w[j + 3], x.w, z[t]);
+                }
+        }
+        for (; r < a.rank; ++r) {
             const float w = a.a2t[static_cast<size_t>(r) * items + i];
 #pragma unroll
-            for (int t = 0; t < PREP_TOKENS; ++t)
-                if (t < count) z[t] = fmaf(w, low[t * a.rank + r], z[t]);
+            for (int t = 0; t < PREP_TOKENS; ++t) z[t] = fmaf(w, low[t * a.rank + r], z[t]);
         }
         const float bias = a.a2_bias[i];
         const int head = i / a.dim, d = i % a.dim;
+        float q_sum[PREP_TOKENS], k_sum[PREP_TOKENS];
+#pragma unroll
+        for (int t = 0; t < PREP_TOKENS; ++t) q_sum[t] = k_sum[t] = 0.0f;
+        for (int p = 0; p < a.splits; ++p)
+#pragma unroll
+            for (int t = 0; t < PREP_TOKENS; ++t) {
+                if (t >= count) continue;
+                const float* row = a.proj + p * a.split_stride + static_cast<size_t>(first + t) * a.width + i;
+                q_sum[t] += row[a.q_col];
+                k_sum[t] += row[a.k_col];
+            }
 #pragma unroll
         for (int t = 0; t < PREP_TOKENS; ++t) {
             if (t >= count) break;
-            const float* row = a.proj + static_cast<size_t>(first + t) * a.width + i;
-            float q = 0.0f, k = 0.0f;
-            for (int p = 0; p < a.splits; ++p) {
-                q += row[p * a.split_stride + a.q_col];
-                k += row[p * a.split_stride + a.k_col];
-            }
+            const float q = q_sum[t], k = k_sum[t];
             float* dst = a.prepared + (static_cast<size_t>(first + t) * a.heads + head) * (a.row ? a.row : 3 * a.dim) + d;
             dst[0] = q * a.q_scale;
             dst[a.dim] = k;
@@ -92,12 +114,17 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(PrepArgs a) {
     if (!a.row) return;
     const int values = a.heads * a.vdim;
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < values; i += gridDim.y * blockDim.x) {
-        for (int t = 0; t < count; ++t) {
-            const float* src = a.proj + static_cast<size_t>(first + t) * a.width + a.v_col + i;
-            float v = 0.0f;
-            for (int p = 0; p < a.splits; ++p) v += src[p * a.split_stride];
-            a.prepared[(static_cast<size_t>(first + t) * a.heads + i / a.vdim) * a.row + 3 * a.dim + i % a.vdim] = v;
-        }
+        float v[PREP_TOKENS];
+#pragma unroll
+        for (int t = 0; t < PREP_TOKENS; ++t) v[t] = 0.0f;
+        for (int p = 0; p < a.splits; ++p)
+#pragma unroll
+            for (int t = 0; t < PREP_TOKENS; ++t)
+                if (t < count) v[t] += a.proj[p * a.split_stride + static_cast<size_t>(first + t) * a.width + a.v_col + i];
+        const int head = i / a.vdim, e = i % a.vdim;
+#pragma unroll
+        for (int t = 0; t < PREP_TOKENS; ++t)
+            if (t < count) a.prepared[(static_cast<size_t>(first + t) * a.heads + head) * a.row + 3 * a.dim + e] = v[t];
     }
 }
 
@@ -279,7 +306,7 @@ ME_EXPORT int me_gla_scan(const float* proj, int splits, long long split_stride,
     if (chunk_min > 0) p.row = 3 * dim + vdim, p.v_col = v_col, p.vdim = vdim;
     // The channels of a token block are spread over several blocks as well: a thread's chain (its rows of A2, then the
     // decays of eight tokens) is long, and only many warps to an SM hide it.  2,048 tokens of 32 heads of 128: 254 us with
-    // one block per eight tokens, 176 with 16.
+    // one block per eight tokens, 176 with 16, 109 with rows of A2 and sums fetched together.
     const int token_blocks = (tokens + PREP_TOKENS - 1) / PREP_TOKENS;
     const int channel_blocks = std::min((heads * dim + 255) / 256, 16);
     const int code = launch_kernel(gla_prepare_kernel, dim3(token_blocks, channel_blocks), 256,
