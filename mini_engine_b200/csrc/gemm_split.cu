@@ -38,22 +38,26 @@ constexpr int MAX_SEGMENTS = 8;
 
 __device__ int g_split_error = 0;  // 0 ok; else (role << 8) | detail of the first failure seen
 
-// NT: tokens per CTA.
+// NT: tokens per CTA.  The tiles pass through the roles in units, whole k blocks or (128 tokens, for which tensor memory has
+// no room otherwise) halves of 32 k; two buffers of pieces, so that the converters write one while the MMAs read the other.
 template <int NT>
 struct SplitConfig {
-    static constexpr int W_BYTES = SPLIT_ROWS * SPLIT_K * 4;
-    static constexpr int X_BYTES = NT * SPLIT_K * 4;
-    static constexpr int RAW_BYTES = W_BYTES + X_BYTES;
-    static constexpr int PIECES_BYTES = 3 * NT * SPLIT_K * 2;
-    // 16 tokens: 36 KB raw blocks, two CTAs to an SM (one CTA with five blocks in flight was 30 % slower: a block's
-    // way through the roles is what takes the time); 64 tokens: 48 KB, one CTA
-    static constexpr int STAGES = NT > 16 ? 3 : 2;
-    // tensor memory: two buffers of w0 x0, the 2^-8 and the 2^-16 terms, two buffers of the weights' pieces
-    static constexpr int SMALL_COLUMN = 2 * NT, A_COLUMN = 4 * NT, A_COLUMNS = 3 * SPLIT_K / 2;
-    static constexpr int TMEM_COLUMNS = 4 * NT + 2 * A_COLUMNS <= 256 ? 256 : 512;
-    static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + 2 * PIECES_BYTES + 1024 + 128;
+    static constexpr int UNITS = NT >= 128 ? 2 : 1, UNIT_K = SPLIT_K / UNITS;  // units to a block
+    static constexpr int BOXES = UNIT_K / 32;                                  // a TMA box is 32 k wide
+    static constexpr int W_BYTES = SPLIT_ROWS * UNIT_K * 4, X_BYTES = NT * UNIT_K * 4, RAW_BYTES = W_BYTES + X_BYTES;  // raw tiles of a unit
+    static constexpr int PIECES_BYTES = 3 * NT * SPLIT_K * 2;  // of a block: rows of 128 bytes, of which a half takes 64
+    static constexpr int PIECES_BUFFERS = 2 / UNITS;
+    // 16 tokens: 36 KB a unit, two CTAs to an SM (one CTA with five units in flight was 30 % slower: a unit's way through the
+    // roles is what takes the time); 64 tokens: 48 KB; 128: 32 KB
+    static constexpr int STAGES = NT <= 16 ? 2 : NT <= 64 ? 3 : 5;
+    // tensor memory: w0 x0 of one or two blocks, the 2^-8 and the 2^-16 terms, the weights' pieces of two units
+    static constexpr int MAINS = UNITS == 1 ? 2 : 1;
+    static constexpr int SMALL_COLUMN = MAINS * NT, A_COLUMN = SMALL_COLUMN + 2 * NT, A_PIECE = UNIT_K / 2, A_COLUMNS = 3 * A_PIECE;
+    static constexpr int TMEM_COLUMNS = A_COLUMN + 2 * A_COLUMNS <= 256 ? 256 : 512;
+    static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + PIECES_BUFFERS * PIECES_BYTES + 1024 + 256;
+    static_assert(A_COLUMN + 2 * A_COLUMNS <= TMEM_COLUMNS, "tensor memory");
+    static_assert(STAGES * RAW_BYTES >= NT * SPLIT_ROWS * 4, "the cluster's exchange reuses the raw tiles");
 };
-static_assert(SplitConfig<16>::RAW_BYTES * SplitConfig<16>::STAGES >= 16 * SPLIT_ROWS * 4, "the cluster's exchange reuses the raw tiles");
 
 struct SplitParams {
     const float* x;
@@ -61,6 +65,7 @@ struct SplitParams {
     float* out;
     int tokens, outs, inner;
     int k_blocks, per_segment;
+    int vector_out;  // rows of the output start on 16 bytes and hold whole float4
     int clustered;  // the segments of a tile are the CTAs of a cluster along z
     // Grouped product: the weight holds `group_rows` rows per group, one group after the other, and token tile b belongs to
     // group group_of_block[b] (negative: it holds no rows and its CTAs return at once).  `outs` counts one group's features.
@@ -81,11 +86,11 @@ __device__ __forceinline__ float4 lds128(uint32_t address) {
 __device__ __forceinline__ void sts128(uint32_t address, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(address), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ float ld_cluster_f32(uint32_t address, uint32_t rank) {
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t address, uint32_t rank) {
     uint32_t remote;
-    float v;
+    float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(address), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
     return v;
 }
 __device__ __forceinline__ void tcgen05_st8(uint32_t taddr, const uint32_t* r) {
@@ -127,18 +132,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     extern __shared__ uint8_t smem_raw[];
     uint8_t* raw = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* pieces = raw + C::STAGES * C::RAW_BYTES;
-    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + 2 * C::PIECES_BYTES);  // raw tiles arrived
-    uint64_t* empty = full + C::STAGES;                                          // raw tiles read by the workers
-    uint64_t* ready = empty + C::STAGES;                                         // [2] pieces written
-    uint64_t* done = ready + 2;                                                  // [2] MMAs retired
-    uint64_t* taken = done + 2;                                                  // [2] sums out of tensor memory
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + 2);
+    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + C::PIECES_BUFFERS * C::PIECES_BYTES);  // raw tiles arrived
+    uint64_t* empty = full + C::STAGES;                                                         // raw tiles read by the converters
+    uint64_t* ready = empty + C::STAGES;                                                        // [2] a unit's pieces written
+    uint64_t* done = ready + 2;                                                                 // [2] its MMAs retired
+    uint64_t* taken = done + 2;                                                                 // [MAINS] a block's sums out of tensor memory
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + C::MAINS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.x * NT, n0 = blockIdx.y * SPLIT_ROWS;
     const int kb_begin = p.clustered ? blockIdx.z * p.per_segment : 0;
     const int kb_end = p.clustered ? min(kb_begin + p.per_segment, p.k_blocks) : p.k_blocks;
-    const int blocks = kb_end - kb_begin;
+    const int blocks = kb_end - kb_begin, units = C::UNITS * blocks;
     int w0 = n0;  // first weight row of the tile
     if (p.group_of_block != nullptr) {
         pdl_wait();  // a kernel before this one wrote the groups
@@ -149,7 +154,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], CONVERTERS / 32); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&ready[b], CONVERTERS / 32); mbar_init(&done[b], 1); mbar_init(&taken[b], TAKERS / 32); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&ready[b], CONVERTERS / 32); mbar_init(&done[b], 1); }
+        for (int b = 0; b < C::MAINS; ++b) mbar_init(&taken[b], TAKERS / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tcgen05_alloc(tmem_holder, C::TMEM_COLUMNS);
@@ -166,32 +172,30 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // ------------------------------------------------------------- TMA producer
         if (lane == 0) {
             pdl_trigger();
-            auto load_w = [&](int i) {
-                uint8_t* at = raw + (i % C::STAGES) * C::RAW_BYTES;
-                mbar_expect_tx(&full[i % C::STAGES], C::RAW_BYTES);
-                const int k = (kb_begin + i) * SPLIT_K;
-                tma_load_2d(at, &map_w, k, w0, &full[i % C::STAGES]);
-                tma_load_2d(at + C::W_BYTES / 2, &map_w, k + SPLIT_K / 2, w0, &full[i % C::STAGES]);
+            auto load_w = [&](int u) {
+                mbar_expect_tx(&full[u % C::STAGES], C::RAW_BYTES);
+                for (int box = 0; box < C::BOXES; ++box)
+                    tma_load_2d(raw + (u % C::STAGES) * C::RAW_BYTES + box * SPLIT_ROWS * 128, &map_w, kb_begin * SPLIT_K + u * C::UNIT_K + 32 * box, w0,
+                                &full[u % C::STAGES]);
             };
-            auto load_x = [&](int i) {
-                uint8_t* at = raw + (i % C::STAGES) * C::RAW_BYTES + C::W_BYTES;
-                const int k = (kb_begin + i) * SPLIT_K;
-                tma_load_2d(at, &map_x, k, t0, &full[i % C::STAGES]);
-                tma_load_2d(at + C::X_BYTES / 2, &map_x, k + SPLIT_K / 2, t0, &full[i % C::STAGES]);
+            auto load_x = [&](int u) {
+                for (int box = 0; box < C::BOXES; ++box)
+                    tma_load_2d(raw + (u % C::STAGES) * C::RAW_BYTES + C::W_BYTES + box * NT * 128, &map_x, kb_begin * SPLIT_K + u * C::UNIT_K + 32 * box, t0,
+                                &full[u % C::STAGES]);
             };
-            const int early = min(blocks, C::STAGES);  // weights are written by no kernel: ahead of the wait
-            for (int i = 0; i < early; ++i) load_w(i);
+            const int early = min(units, C::STAGES);  // weights are written by no kernel: ahead of the wait
+            for (int u = 0; u < early; ++u) load_w(u);
             pdl_wait();
-            for (int i = 0; i < early; ++i) load_x(i);
+            for (int u = 0; u < early; ++u) load_x(u);
             int issued = early;
-            for (int i = early; i < blocks; ++i, ++issued) {
-                if (!mbar_wait(&empty[i % C::STAGES], ((i / C::STAGES) & 1) ^ 1)) { atomicCAS(&g_split_error, 0, (1 << 8)); break; }
-                load_w(i);
-                load_x(i);
+            for (int u = early; u < units; ++u, ++issued) {
+                if (!mbar_wait(&empty[u % C::STAGES], ((u / C::STAGES) & 1) ^ 1)) { atomicCAS(&g_split_error, 0, (1 << 8)); break; }
+                load_w(u);
+                load_x(u);
             }
             // Copies in flight must land before the shared memory is released; on the normal path the converters saw them.
-            if (issued < blocks || g_split_error != 0) {
-                for (int i = max(issued - C::STAGES, 0); i < issued; ++i) mbar_wait(&full[i % C::STAGES], (i / C::STAGES) & 1);
+            if (issued < units || g_split_error != 0) {
+                for (int u = max(issued - C::STAGES, 0); u < issued; ++u) mbar_wait(&full[u % C::STAGES], (u / C::STAGES) & 1);
             }
         }
     } else if (warp == 1) {
@@ -199,78 +203,90 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (lane == 0) {
             constexpr uint32_t one = make_idesc(NT), two = make_idesc(2 * NT);
             const uint32_t small = tmem_base + C::SMALL_COLUMN;
-            for (int i = 0, at = 0; i < blocks; ++i) {
-                bool go = mbar_wait(&ready[i & 1], (i >> 1) & 1);
-                if (i >= 2) go = go && mbar_wait(&taken[i & 1], ((i >> 1) & 1) ^ 1);
-                if (i > 0 && at == 0) go = go && mbar_wait(&taken[(i - 1) & 1], ((i - 1) >> 1) & 1);  // the small terms too
-                if (!go) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
+            auto wait_taken = [&](int block) { return block < 0 || mbar_wait(&taken[block % C::MAINS], (block / C::MAINS) & 1); };
+            for (int u = 0, at = 0; u < units; ++u) {
+                const int half = u % C::UNITS, block = u / C::UNITS;
+                const bool fresh = half == 0 && at == 0;  // a segment starts its own sums: the last one's must be out
+                if (!mbar_wait(&ready[u & 1], (u >> 1) & 1) || (fresh && !wait_taken(block - 1))) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
                 tcgen05_fence_after();
-                const uint32_t a = tmem_base + C::A_COLUMN + (i & 1) * C::A_COLUMNS, main_sum = tmem_base + (i & 1) * NT;
-                const uint64_t x0 = smem_desc_sw128(smem_u32(pieces + (i & 1) * C::PIECES_BYTES));
-                const uint64_t x1 = x0 + ((NT * 128) >> 4);
-                // one kind of product after the other: MMAs into the same columns follow each other without a gap
-                const uint32_t w1 = a + SPLIT_K / 2, w2 = w1 + SPLIT_K / 2;
-                constexpr int STEPS = SPLIT_K / 16;  // 8 columns of the weights' pieces, 32 bytes of the tokens'
+                const uint32_t a = tmem_base + C::A_COLUMN + (u & 1) * C::A_COLUMNS, main_sum = tmem_base + block % C::MAINS * NT;
+                const uint64_t b = smem_desc_sw128(smem_u32(pieces + (C::UNITS == 1 ? (u & 1) * C::PIECES_BYTES : 0))) + 4 * half;
+                // The small terms of 32 k, then of the next: MMAs into the same columns follow each other without a gap, and the
+                // widest come last, so that the next unit's waits pass while they run.  A step of 16 k is 8 columns of the weights'
+                // pieces and 32 bytes of the tokens'.
+                bool go = true;
 #pragma unroll
-                for (int k = 0; k < STEPS; ++k) tcgen05_mma_bf16_ts(small, a + 8 * k, x1 + 2 * k, two, at > 0 || k > 0);
+                for (int box = 0; box < C::BOXES; ++box) {
+                    const uint32_t w0_piece = a + 16 * box, w1_piece = w0_piece + C::A_PIECE, w2_piece = w1_piece + C::A_PIECE;
+                    const uint64_t x0 = b + 4 * box, x1 = x0 + ((NT * 128) >> 4);
+                    tcgen05_mma_bf16_ts(small, w1_piece, x0, two, !fresh || box > 0);
+                    tcgen05_mma_bf16_ts(small, w1_piece + 8, x0 + 2, two, 1);
+                    tcgen05_mma_bf16_ts(small + NT, w2_piece, x0, one, 1);
+                    tcgen05_mma_bf16_ts(small + NT, w2_piece + 8, x0 + 2, one, 1);
+                    if (box == C::BOXES - 1) {
+                        if (half == 0 && !wait_taken(block - C::MAINS)) { go = false; break; }  // the takers have had their time
+                        tcgen05_fence_after();
 #pragma unroll
-                for (int k = 0; k < STEPS; ++k) tcgen05_mma_bf16_ts(small, w1 + 8 * k, x0 + 2 * k, two, 1);
-#pragma unroll
-                for (int k = 0; k < STEPS; ++k) tcgen05_mma_bf16_ts(small + NT, w2 + 8 * k, x0 + 2 * k, one, 1);
-#pragma unroll
-                for (int k = 0; k < STEPS; ++k) tcgen05_mma_bf16_ts(main_sum, a + 8 * k, x0 + 2 * k, one, k > 0);
-                tcgen05_commit(&done[i & 1]);
-                if (++at == p.per_segment) at = 0;  // a new segment starts its own sums
+                        for (int k = 0; k < C::UNIT_K / 16; ++k) tcgen05_mma_bf16_ts(main_sum, a + 8 * k, b + 2 * k, one, half > 0 || k > 0);
+                    }
+                    tcgen05_mma_bf16_ts(small, w0_piece, x1, two, 1);
+                    tcgen05_mma_bf16_ts(small, w0_piece + 8, x1 + 2, two, 1);
+                }
+                if (!go) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
+                tcgen05_commit(&done[u & 1]);
+                if (half == C::UNITS - 1 && ++at == p.per_segment) at = 0;
             }
         }
     } else if (warp < 2 + CONVERTERS / 32) {
         // ----------------------------------------------------------------- converters
-        const int worker = threadIdx.x - 64, half = worker >> 7;  // which half of a block's k
+        // A thread takes 16 or 32 weights of a row.
+        const int worker = threadIdx.x - 64, run = worker >> 7;
         const int row = quarter * 32 + lane;
-        for (int i = 0; i < blocks; ++i) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&full[i % C::STAGES], (i / C::STAGES) & 1));
+        for (int u = 0; u < units; ++u) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[u % C::STAGES], (u / C::STAGES) & 1));
             if (!ok) break;
-            const uint32_t w_tile = smem_u32(raw + (i % C::STAGES) * C::RAW_BYTES), x_tile = w_tile + C::W_BYTES;
-            const uint32_t x_pieces = smem_u32(pieces + (i & 1) * C::PIECES_BYTES);
-            // 32 of the row's 64 weights, 16 at a time; TMA put 16-byte chunk c of row r at c ^ (r % 8)
-            const uint32_t from = w_tile + half * (C::W_BYTES / 2) + row * 128;
-            const uint32_t to = lanes + C::A_COLUMN + (i & 1) * C::A_COLUMNS + half * 16;
+            const uint32_t w_tile = smem_u32(raw + (u % C::STAGES) * C::RAW_BYTES), x_tile = w_tile + C::W_BYTES;
+            const uint32_t from_row = w_tile + (C::BOXES == 2 ? run * SPLIT_ROWS * 128 : 0) + row * 128;
+            const uint32_t to = lanes + C::A_COLUMN + (u & 1) * C::A_COLUMNS + run * (C::UNIT_K / 4);
 #pragma unroll
-            for (int run = 0; run < 2; ++run) {
-                uint32_t w0[8], w1[8], w2[8];
+            for (int part = 0; part < C::BOXES; ++part) {  // 16 weights; TMA put 16-byte chunk c of row r at c ^ (r % 8)
+                const int first_chunk = 4 * (C::BOXES == 2 ? part : run);
+                uint32_t piece0[8], piece1[8], piece2[8];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const float4 v = lds128(from + (((4 * run + c) ^ (row & 7)) << 4));
+                    const float4 v = lds128(from_row + (((first_chunk + c) ^ (row & 7)) << 4));
                     const float4 r = make_float4(below_upper(v.x), below_upper(v.y), below_upper(v.z), below_upper(v.w));
-                    w0[2 * c] = upper_pair(v.x, v.y), w0[2 * c + 1] = upper_pair(v.z, v.w);
-                    w1[2 * c] = upper_pair(r.x, r.y), w1[2 * c + 1] = upper_pair(r.z, r.w);
-                    w2[2 * c] = upper_pair(below_upper(r.x), below_upper(r.y));
-                    w2[2 * c + 1] = upper_pair(below_upper(r.z), below_upper(r.w));
+                    piece0[2 * c] = upper_pair(v.x, v.y), piece0[2 * c + 1] = upper_pair(v.z, v.w);
+                    piece1[2 * c] = upper_pair(r.x, r.y), piece1[2 * c + 1] = upper_pair(r.z, r.w);
+                    piece2[2 * c] = upper_pair(below_upper(r.x), below_upper(r.y));
+                    piece2[2 * c + 1] = upper_pair(below_upper(r.z), below_upper(r.w));
                 }
-                if (run == 0 && i >= 2) {  // the MMAs of block i - 2 have read these buffers
-                    ok = __all_sync(0xffffffffu, mbar_wait(&done[i & 1], ((i >> 1) & 1) ^ 1));
+                if (part == 0 && u >= 2) {  // the MMAs of two units ago have read these buffers
+                    ok = __all_sync(0xffffffffu, mbar_wait(&done[u & 1], ((u >> 1) & 1) ^ 1));
                     if (!ok) break;
                     tcgen05_fence_after();
                 }
-                tcgen05_st8(to + 8 * run, w0);
-                tcgen05_st8(to + 8 * run + SPLIT_K / 2, w1);
-                tcgen05_st8(to + 8 * run + SPLIT_K, w2);
+                tcgen05_st8(to + 8 * part, piece0);
+                tcgen05_st8(to + 8 * part + C::A_PIECE, piece1);
+                tcgen05_st8(to + 8 * part + 2 * C::A_PIECE, piece2);
             }
             if (!ok) break;
+            const uint32_t x_pieces = smem_u32(pieces + (C::UNITS == 1 ? (u & 1) * C::PIECES_BYTES : 0));
 #pragma unroll
-            for (int unit = worker; unit < NT * 8; unit += CONVERTERS) {
-                // 8 k values of a token: two raw chunks to one 16-byte chunk of each piece
-                const int t = unit >> 3, chunk = unit & 7, side = chunk >> 2;
-                const uint32_t x_from = x_tile + side * (C::X_BYTES / 2) + t * 128;
+            for (int item = worker; item < NT * C::UNIT_K / 8; item += CONVERTERS) {
+                // 8 k values of a token: two raw chunks to one 16-byte chunk of each piece.  Eight lanes are four chunks of tokens t
+                // and t + 4, whose pieces fall into different banks; so do their raw chunks, read in opposite order.
+                const int box = item / (NT * 4), chunk = item & 3, upper = (item >> 2) & 1, t = ((item >> 3) & 3) + 4 * upper + 8 * (item % (NT * 4) >> 5);
+                const uint32_t from = x_tile + box * NT * 128 + t * 128;
+                const float4 one = lds128(from + (((2 * chunk + upper) ^ (t & 7)) << 4));
+                const float4 other = lds128(from + (((2 * chunk + (upper ^ 1)) ^ (t & 7)) << 4));
                 float4 v[2];
-                // the sides take their chunks in opposite order: the eight lanes of a row then meet all banks
-                const float4 first = lds128(x_from + (((2 * (chunk & 3) + side) ^ (t & 7)) << 4));
-                const float4 second = lds128(x_from + (((2 * (chunk & 3) + (side ^ 1)) ^ (t & 7)) << 4));
-                v[0] = side ? second : first;
-                v[1] = side ? first : second;
+                v[0] = upper ? other : one;
+                v[1] = upper ? one : other;
+                const int to_chunk = 4 * (C::UNITS == 1 ? box : u & 1) + chunk;
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
-                    sts128(x_pieces + q * NT * 128 + t * 128 + ((chunk ^ (t & 7)) << 4),
+                    sts128(x_pieces + q * NT * 128 + t * 128 + ((to_chunk ^ (t & 7)) << 4),
                            make_uint4(upper_pair(v[0].x, v[0].y), upper_pair(v[0].z, v[0].w), upper_pair(v[1].x, v[1].y),
                                       upper_pair(v[1].z, v[1].w)));
 #pragma unroll
@@ -283,8 +299,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&ready[i & 1]);
-                mbar_arrive(&empty[i % C::STAGES]);
+                mbar_arrive(&ready[u & 1]);
+                mbar_arrive(&empty[u % C::STAGES]);
             }
         }
         if (!ok && lane == 0) atomicCAS(&g_split_error, 0, (3 << 8));
@@ -293,19 +309,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // The sums of a block out of tensor memory and added up; at the end of a segment the small terms join them.
         constexpr int COLUMNS = NT / 2;
         const int row = quarter * 32 + lane, n = n0 + row, column = (warp - 2 - CONVERTERS / 32) / 4 * COLUMNS;
-        float sum[COLUMNS], total[COLUMNS];  // of the running segment, of the finished ones
+        // With 128 tokens a thread's registers hold one sum per column: its CTA runs one segment (see me_gemm_split).
+        constexpr bool MANY = NT < 128;
+        float sum[COLUMNS], total[MANY ? COLUMNS : 1] = {};  // of the running segment, of the finished ones
         int at = 0;
         bool first = true;
 #pragma unroll
-        for (int c = 0; c < COLUMNS; ++c) sum[c] = total[c] = 0.0f;
+        for (int c = 0; c < COLUMNS; ++c) sum[c] = 0.0f;
         for (int i = 0; i < blocks; ++i) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&done[i & 1], (i >> 1) & 1));
+            const int u = i * C::UNITS + C::UNITS - 1;  // the block's last unit
+            ok = __all_sync(0xffffffffu, mbar_wait(&done[u & 1], (u >> 1) & 1));
             if (!ok) break;
             tcgen05_fence_after();
 #pragma unroll
             for (int c0 = 0; c0 < COLUMNS; c0 += 8) {
                 float got[8];
-                tcgen05_ld8(lanes + (i & 1) * NT + column + c0, got);
+                tcgen05_ld8(lanes + i % C::MAINS * NT + column + c0, got);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) sum[c0 + c] += got[c];
             }
@@ -319,28 +338,33 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const float part = sum[c0 + c] + (low[c] + lower[c]);
-                        total[c0 + c] = first ? part : total[c0 + c] + part;
-                        sum[c0 + c] = 0.0f;
+                        if constexpr (MANY) {
+                            total[c0 + c] = first ? part : total[c0 + c] + part;
+                            sum[c0 + c] = 0.0f;
+                        } else {
+                            sum[c0 + c] = part;
+                        }
                     }
                 }
                 first = false;
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&taken[i & 1]);
+            if (lane == 0) mbar_arrive(&taken[i % C::MAINS]);
         }
+        auto result = [&](int c) { return MANY ? total[MANY ? c : 0] : sum[c]; };
         if (!ok && lane == 0) atomicCAS(&g_split_error, 0, (4 << 8));
         pdl_wait();  // the output may still be read by a kernel before this one
         if (p.clustered && ok) {
             // every MMA and load of this CTA has ended: the raw tiles make room for the exchange
             float* exchange = reinterpret_cast<float*>(raw);
 #pragma unroll
-            for (int c = 0; c < COLUMNS; ++c) exchange[(column + c) * SPLIT_ROWS + row] = total[c];
+            for (int c = 0; c < COLUMNS; ++c) exchange[(column + c) * SPLIT_ROWS + row] = result(c);
         } else if (ok && n < p.outs) {
 #pragma unroll
             for (int c = 0; c < COLUMNS; ++c) {
                 const int t = t0 + column + c;
-                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, w0 + row, total[c]);
+                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, w0 + row, result(c));
             }
         }
     }
@@ -351,19 +375,30 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         cluster_sync();
         if (warp >= 2 && warp < 2 + CONVERTERS / 32 && ok) {
             pdl_wait();
-            const int worker = threadIdx.x - 64, row = worker & 127, segments = gridDim.z;
-            for (int c = 2 * blockIdx.z + (worker >> 7); c < NT; c += 2 * segments) {
-                const int t = t0 + c, n = n0 + row;
+            // Four rows of a column at a time, shared out among the cluster's CTAs.
+            const int segments = gridDim.z;
+            for (int item = threadIdx.x - 64 + CONVERTERS * blockIdx.z; item < NT * (SPLIT_ROWS / 4); item += CONVERTERS * segments) {
+                const int c = item / (SPLIT_ROWS / 4), row = item % (SPLIT_ROWS / 4) * 4, t = t0 + c, n = n0 + row;
                 if (t >= p.tokens || n >= p.outs) continue;
                 const uint32_t from = smem_u32(raw) + (c * SPLIT_ROWS + row) * 4;
-                float part[MAX_SEGMENTS];
+                float4 part[MAX_SEGMENTS];
 #pragma unroll
                 for (int s = 0; s < MAX_SEGMENTS; ++s)
-                    if (s < segments) part[s] = ld_cluster_f32(from, s);
+                    if (s < segments) part[s] = ld_cluster_f32x4(from, s);
+                float4 y = part[0];
 #pragma unroll
                 for (int s = 1; s < MAX_SEGMENTS; ++s)
-                    if (s < segments) part[0] += part[s];
-                p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, w0 + row, part[0]);
+                    if (s < segments) y.x += part[s].x, y.y += part[s].y, y.z += part[s].z, y.w += part[s].w;
+                const float v[4] = {finite_or_again(p, t, w0 + row, y.x), n + 1 < p.outs ? finite_or_again(p, t, w0 + row + 1, y.y) : 0.0f,
+                                    n + 2 < p.outs ? finite_or_again(p, t, w0 + row + 2, y.z) : 0.0f, n + 3 < p.outs ? finite_or_again(p, t, w0 + row + 3, y.w) : 0.0f};
+                float* to = p.out + static_cast<size_t>(t) * p.outs + n;
+                if (p.vector_out) {
+                    *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (n + i < p.outs) to[i] = v[i];
+                }
             }
         }
         cluster_sync();  // the others may still read this CTA's part
@@ -448,6 +483,7 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     p.k_blocks = (inner + SPLIT_K - 1) / SPLIT_K;
     p.per_segment = (p.k_blocks + segments - 1) / segments;
     p.clustered = clustered && segments > 1;
+    p.vector_out = outs % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
     p.group_of_block = group_of_block, p.group_rows = group_rows;
     if ((segments - 1) * p.per_segment >= p.k_blocks) return ME_ERR_ARGUMENT;  // a segment would be empty
     alignas(64) CUtensorMap w_map, x_map;
@@ -455,6 +491,7 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     memcpy(&x_map, map_x, sizeof(x_map));
     if (tile == 16) return launch_split<16>(w_map, x_map, p, segments, stream);
     if (tile == 64) return launch_split<64>(w_map, x_map, p, segments, stream);
+    if (tile == 128 && (p.clustered || segments == 1)) return launch_split<128>(w_map, x_map, p, segments, stream);
     return ME_ERR_ARGUMENT;
 }
 

@@ -238,7 +238,13 @@ def gemm_swiglu(
 
 # ------------------------------------------------------------------------------ float32
 
-SPLIT_TILES = (16, 64)  # tokens per CTA: up to 16 two CTAs share an SM and stream weights, else one
+# Tokens per CTA (up to 16 two CTAs share an SM and stream weights, else one) and the time of a k block, in blocks of 64 tokens
+# (1.13 us).  A round of CTAs costs SPLIT_START blocks beside them, a cluster's exchange SPLIT_EXCHANGE for each segment of 128
+# tokens.  Measured forms, us (64 tokens to a CTA and segments one after the other; 64 side by side; 128): 256 tokens x 6,144 x
+# 4,096 155, 154, 123; x 24,576 x 4,096 459, -, 324; x 4,096 x 4,096 80, 106, 83; 512 x 2,048 x 2,048 45, 100, 68; 512 x 9,216 x
+# 2,048 169, 198, 133; 64 x 6,144 x 4,096 78, 62, 80.
+SPLIT_TILES = {16: 1.0, 64: 1.0, 128: 1.44}
+SPLIT_START, SPLIT_EXCHANGE = 4.0, 0.8
 SPLIT_MIN_K_BLOCKS = 4  # of a segment
 # Shorter reductions stay on CUDA cores: a chain of fmaf over so few terms is as exact as the short chain of the tensor
 # core (relative error at 64: 1.5e-7 against 1.2e-7; at 4: 4e-8 against 7e-8), and nothing is to be gained.
@@ -278,17 +284,25 @@ def split_segments(outs: int, inner: int) -> int:
     return -(-k_blocks // per_segment)
 
 
-def split_tile(tokens: int) -> int:
-    return SPLIT_TILES[0] if tokens <= SPLIT_TILES[0] else SPLIT_TILES[1]
-
-
-def split_side_by_side(tokens: int, outs: int, segments: int, tile: int | None = None) -> bool:
-    """Whether a tile's segments run in the CTAs of a cluster (few tiles) or one after the other in a CTA; the bits are the
-    same.  Side by side when that takes fewer rounds of resident CTAs, a round being one segment long."""
-    tile = tile or split_tile(tokens)
-    slots = NUM_SMS * (2 if tile == SPLIT_TILES[0] else 1)
-    ctas = -(-outs // BLOCK_N) * -(-tokens // tile)
-    return -(-ctas * segments // slots) < -(-ctas // slots) * segments
+def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | None = None) -> tuple[int, bool]:
+    """Tokens per CTA (or the given ``tile``), and whether a tile's segments run in the CTAs of a cluster or one after the other in a
+    CTA; the bits are the same in every form.  The form whose rounds of resident CTAs take least time."""
+    blocks = -(-inner // BLOCK_K)
+    per_segment = -(-blocks // segments)
+    # A cluster lies within a group of 16 to 18 SMs, of which there are eight: some SMs stay out of large clusters.
+    in_clusters = NUM_SMS if segments <= 2 else 8 * (17 // segments) * segments
+    forms = []
+    for rows, cost in SPLIT_TILES.items():
+        if (rows != tile) if tile is not None else (rows == 16) != (tokens <= 16) or (rows == 128 and tokens <= 64):
+            continue
+        per_sm = 2 if rows == 16 else 1
+        ctas = -(-outs // BLOCK_N) * -(-tokens // rows)
+        if rows < 128 or segments == 1:
+            forms.append((-(-ctas // (per_sm * NUM_SMS)) * (blocks * cost + SPLIT_START), rows, False))
+        if segments > 1:
+            rounds = -(-ctas * segments // (per_sm * in_clusters))
+            forms.append((rounds * (per_segment * cost + SPLIT_START + SPLIT_EXCHANGE * segments * rows / 128), rows, True))
+    return min(forms)[1:]
 
 
 class SplitPlan:
@@ -328,17 +342,15 @@ def _split_activation_map(x: torch.Tensor, tile: int) -> ctypes.Array:
     return held
 
 
-def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side: bool | None = None) -> None:
+def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[int, bool] | None = None) -> None:
     """``out[T, rows] = x @ weight^T`` in float32 (three bfloat16 pieces of each operand, see gemm_split.cu).
-    ``side_by_side`` pins where a tile's segments run instead of the rule's choice: the kernel tests run both."""
+    ``form`` pins the tokens per CTA and where a tile's segments run instead of the rule's choice: the kernel tests run all."""
     tokens = x.shape[0]
     if x.dtype != torch.float32 or not x.is_contiguous() or x.dim() != 2 or x.shape[1] != plan.inner or x.data_ptr() % 16:
         raise RuntimeError(f"activation {tuple(x.shape)} {x.dtype} does not fit a float32 weight of width {plan.inner}")
     if out.dtype != torch.float32 or tuple(out.shape) != (tokens, plan.rows) or not out.is_contiguous():
         raise RuntimeError(f"output {tuple(out.shape)} does not fit [{tokens}, {plan.rows}] float32")
-    tile = split_tile(tokens)
-    if side_by_side is None:
-        side_by_side = split_side_by_side(tokens, plan.rows, plan.segments)
+    tile, side_by_side = split_form(tokens, plan.rows, plan.inner, plan.segments) if form is None else form
     code = _split_library().me_gemm_split(
         plan.map, _split_activation_map(x, tile), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,
         plan.segments, 1 if side_by_side else 0, None, 0, _ops_stream(),
@@ -365,7 +377,7 @@ def gemm_split_grouped(
     if pad not in SPLIT_TILES or rows % pad or group_of_block.dtype != torch.int32 or group_of_block.numel() < rows // pad:
         raise RuntimeError("the rows of a grouped product come in runs of a token tile with one int32 group each")
     if side_by_side is None:
-        side_by_side = split_side_by_side(max(1, min(filled, rows // pad)) * pad, outs, plan.segments, pad)
+        side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad)[1]
     code = _split_library().me_gemm_split(
         plan.map, _split_activation_map(x, pad), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, plan.inner, pad,
         plan.segments, 1 if side_by_side else 0, group_of_block.data_ptr(), outs, _ops_stream(),

@@ -47,15 +47,16 @@ def test_split_product(tokens, outs, inner):
         return float(((y.double() - want) / want.norm(dim=1, keepdim=True)).norm())
 
     out = torch.full((tokens, outs), float("nan"), device="cuda")
-    tc.gemm_split(plan, x, out, side_by_side=False)
+    tc.gemm_split(plan, x, out, (64, False))
     assert tc.take_error() == 0
     # no less exact than the fmaf chain; a quarter more for the few outputs of the small shapes
     assert error(out) <= 1.25 * error(simt)
-    # the same bits with the segments in a cluster, and for rows of another batch (another token tile)
-    other = torch.full((tokens, outs), float("nan"), device="cuda")
-    tc.gemm_split(plan, x, other, side_by_side=True)
-    assert tc.take_error() == 0
-    assert torch.equal(out, other)
+    # the same bits with the segments in a cluster, with another token tile, and for rows of another batch
+    for form in [(16, False), (16, True), (64, True), (128, plan.segments > 1)]:
+        other = torch.full((tokens, outs), float("nan"), device="cuda")
+        tc.gemm_split(plan, x, other, form)
+        assert tc.take_error() == 0
+        assert torch.equal(out, other), form
     for rows in (slice(tokens // 2, tokens // 2 + 1), slice(0, min(tokens, 16)), slice(tokens // 3, tokens)):
         part = torch.empty(len(range(*rows.indices(tokens))), outs, device="cuda")
         tc.gemm_split(plan, x[rows].clone(), part)
