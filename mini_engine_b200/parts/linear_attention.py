@@ -123,11 +123,10 @@ class GatedLinearAttention(Mixer):
         # Long entries run in chunks of tokens side by side.  In float32 every entry walks: a token's bits there do not depend on
         # how its request was cut.  A step's longest entry is known on the host.
         chunk_min, records, row = 0, None, 3 * self.dim
-        if (
-            ctx.dtype == torch.bfloat16 and ctx.max_query_len >= CHUNKED_MIN_TOKENS
-            and ops.state_chunks_support(self.dim, self.vdim, self.heads * self.dim * self.vdim)
-        ):  # fmt: skip
-            chunk_min, row = CHUNKED_MIN_TOKENS, 3 * self.dim + self.vdim
+        if ctx.dtype == torch.bfloat16 and ops.state_chunks_support(self.dim, self.vdim, self.heads * self.dim * self.vdim):
+            row += self.vdim  # one size whatever the step, so that the buffer is allocated once
+            chunk_min = CHUNKED_MIN_TOKENS if ctx.max_query_len >= CHUNKED_MIN_TOKENS else 0
+        if chunk_min:
             chunks = tokens // ops.STATE_CHUNK + ctx.num_entries
             records = ctx.workspace.growing("gla.records", (chunks, self.heads * ops.state_record_floats("gated", self.dim)), torch.float32)
         prepared = ctx.buffer("gla.prepared", (tokens, self.heads * row), torch.float32)
