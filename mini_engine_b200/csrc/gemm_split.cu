@@ -22,11 +22,11 @@
 // shared memory, so that one MMA multiplies a piece of the weights by several pieces of the tokens), eight taker warps add
 // the sums of a block up while the MMAs of the next run.
 //
-// What bounds it: a block takes about 1,500 cycles whatever its tokens: the 16 MMAs hold the thread that issues them
-// 58 cycles each, waits for the other roles come on top, and the converters need 1,000 to 1,100.  Beside the CUDA-core
-// kernel: 256 x 24,576 x 4,096 (tokens, outs, inner) 2,378 -> 431 us (120 TFLOP/s), 256 x 4,096 x 12,288 1,714 -> 207,
-// 512 x 2,048 x 5,632 760 -> 102; 8 x 24,576 x 4,096 807 -> 92 (4.4 TB/s of weights), 8 x 4,096 x 4,096 377 -> 24,
-// 1 x 151,936 x 1,024 919 -> 110 (5.7 TB/s).
+// What bounds it: a k block takes about 2,000 cycles with 16 or 64 tokens and 2,500 with 128.  The MMAs take 85 to 90 cycles
+// each beside the converters, 58 alone (both work on tensor memory and shared memory), the converters 1,050 to 1,100 a block,
+// and the waits between the roles come on top.  Beside the CUDA-core kernel (tokens x outs x inner): 256 x 24,576 x 4,096
+// 2,378 -> 324 us (159 TFLOP/s), 256 x 4,096 x 12,288 1,714 -> 202, 512 x 2,048 x 5,632 760 -> 107; 8 x 24,576 x 4,096
+// 807 -> 94 (4.3 TB/s of weights), 8 x 4,096 x 4,096 377 -> 25, 1 x 151,936 x 1,024 919 -> 112 (5.6 TB/s).
 #include "tcgen05.cuh"
 
 constexpr int SPLIT_ROWS = 128;  // output features per CTA
