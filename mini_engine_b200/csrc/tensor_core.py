@@ -350,6 +350,8 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
         raise RuntimeError(f"activation {tuple(x.shape)} {x.dtype} does not fit a float32 weight of width {plan.inner}")
     if out.dtype != torch.float32 or tuple(out.shape) != (tokens, plan.rows) or not out.is_contiguous():
         raise RuntimeError(f"output {tuple(out.shape)} does not fit [{tokens}, {plan.rows}] float32")
+    if tokens == 0:
+        return
     tile, side_by_side = split_form(tokens, plan.rows, plan.inner, plan.segments) if form is None else form
     code = _split_library().me_gemm_split(
         plan.map, _split_activation_map(x, tile), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,

@@ -82,6 +82,23 @@ def test_infinities_and_nan_come_out_as_in_one_chain():
 
 
 @pytest.mark.gpu
+def test_activations_off_16_bytes_and_no_tokens():
+    """A product of the parts takes both: the first on CUDA cores, the second without a launch."""
+    from mini_engine_b200.engine.workspace import Workspace
+    from mini_engine_b200.parts.linear import Linear
+
+    class Context:
+        workspace = Workspace(8, "cuda")
+
+    torch.manual_seed(5)
+    linear = Linear(torch.randn(70, 64, device="cuda"))
+    x = torch.randn(3 * 64 + 1, device="cuda")[1:].view(3, 64)
+    out = linear.forward(x, Context, "out")[0].clone()
+    assert torch.allclose(out.double(), x.double() @ linear.weight.double().T, rtol=1e-5, atol=1e-4)
+    assert linear.forward(x[:0].clone(), Context, "out").shape == (1, 0, 70)
+
+
+@pytest.mark.gpu
 def test_weights_that_tma_cannot_address_are_refused_by_the_rule():
     tc = tensor_core()
     base = torch.randn(4 * 128 + 1, device="cuda")
