@@ -654,16 +654,22 @@ ME_EXPORT int me_mixed_attention(const void* q, const void* k_pages, const void*
 //
 // A block takes eight consecutive tokens of an entry and all heads; a warp one KV head with its GROUP query heads, two heads
 // to the 16 rows of a product, so its keys, values, scores and output stay with it.  The first walk over the key tiles
-// gives every row's maximum and denominator, the second forms the normalised weights, leaves them in shared memory as two
-// bfloat16 terms (their sum is the weight to 17 bits), mixes them there as products [heads x heads] . [heads x
-// (query, key)], each warp its own columns and in place, and applies them to the values.  Nothing but the output is
-// written.  The distance bias is taken per (head, distance), 39 distances a tile of 32 keys, instead of per score.  Products are m16n8k16 with float32 sums.
+// gives every row's maximum and denominator, the second forms the normalised weights, leaves them in shared memory as three
+// bfloat16 terms (their sum is the float32 weight, all 24 bits), mixes them there as products [heads x heads] . [heads x
+// (query, key)], each warp its own columns and in place, and applies the mixed weights, again three terms, to the values.
+// Nothing but the output is written.  The distance bias is taken per (head, distance), 39 distances a tile of 32 keys, instead
+// of per score.  Products are m16n8k16 with float32 sums.
+//
+// The terms are rounded to nearest, so a term is at most 2^-8 of the number before it: of the nine products of the mixing
+// matrix's and the weights' terms the six largest are formed, the others are below 2^-24 of a product.  The tensor core
+// truncates when it adds: the products with 16 keys' values leave it and are added to the output with rounding.
 //
 // Bound by the instructions a warp issues around its products (exponentials, masks, the split of the weights), with
 // one block to an SM; see the figures at launch_mixed_tiles.  A tile of eight tokens, since the output of four heads and
 // 16 tokens would take every register of a warp.
 constexpr int TILE_Q = 8, TILE_K = 32, TILE_DIM = 128;
 constexpr int BIAS_SPAN = TILE_Q + TILE_K;  // distances within a tile, one spare
+constexpr int TERMS = 3;                    // bfloat16 terms of a float32 number
 
 template <int KV, int GROUP>
 struct MixTile {
@@ -671,7 +677,7 @@ struct MixTile {
     static constexpr int PITCH = TILE_Q * TILE_K + 8;  // weights of a head, 16 bytes of padding: rows fall into different banks
     static constexpr int TALK_PITCH = HEADS + 8;
     static constexpr int KV_BYTES = TILE_K * TILE_DIM * 2;
-    static constexpr int SMEM = 2 * KV * KV_BYTES + 2 * HEADS * PITCH * 2 + 2 * HEADS * TALK_PITCH * 2 + HEADS * BIAS_SPAN * 4;
+    static constexpr int SMEM = 2 * KV * KV_BYTES + TERMS * HEADS * PITCH * 2 + TERMS * HEADS * TALK_PITCH * 2 + HEADS * BIAS_SPAN * 4;
 };
 
 struct MixTileArgs {
@@ -680,9 +686,13 @@ struct MixTileArgs {
     const int* cu_tokens;  // [entries + 1]
 };
 
-__device__ __forceinline__ void two_terms(float x, float y, uint32_t& high, uint32_t& low) {
-    high = pack_bf16(x, y);
-    low = pack_bf16(x - __uint_as_float(high << 16), y - __uint_as_float(high & 0xffff0000u));
+// x and y as pairs of bfloat16 terms, the largest first
+__device__ __forceinline__ void terms_of(float x, float y, uint32_t (&term)[TERMS]) {
+#pragma unroll
+    for (int i = 0; i < TERMS; ++i) {
+        term[i] = pack_bf16(x, y);
+        x -= __uint_as_float(term[i] << 16), y -= __uint_as_float(term[i] & 0xffff0000u);
+    }
 }
 
 template <int KV, int GROUP>
@@ -695,9 +705,9 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, q = lane >> 2;
     __nv_bfloat16* keys = reinterpret_cast<__nv_bfloat16*>(mix_tile_shared) + warp * (C::KV_BYTES / 2);
     __nv_bfloat16* values = keys + KV * (C::KV_BYTES / 2);
-    __nv_bfloat16* weights = reinterpret_cast<__nv_bfloat16*>(mix_tile_shared) + 2 * KV * (C::KV_BYTES / 2);  // [2][HEADS][PITCH]
-    __nv_bfloat16* talk = weights + 2 * HEADS * C::PITCH;                                               // [2][HEADS][TALK_PITCH]
-    float* bias = reinterpret_cast<float*>(talk + 2 * HEADS * C::TALK_PITCH) + warp * GROUP * BIAS_SPAN;
+    __nv_bfloat16* weights = reinterpret_cast<__nv_bfloat16*>(mix_tile_shared) + 2 * KV * (C::KV_BYTES / 2);  // [TERMS][HEADS][PITCH]
+    __nv_bfloat16* talk = weights + TERMS * HEADS * C::PITCH;                                           // [TERMS][HEADS][TALK_PITCH]
+    float* bias = reinterpret_cast<float*>(talk + TERMS * HEADS * C::TALK_PITCH) + warp * GROUP * BIAS_SPAN;
     constexpr int PLANE = HEADS * C::PITCH, TALK_PLANE = HEADS * C::TALK_PITCH;
 
     const int entry = blockIdx.y, begin = m.cu_tokens[entry];
@@ -706,11 +716,11 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
     if (count <= 0) return;
     const int head0 = warp * GROUP;
     for (int i = threadIdx.x; i < HEADS * HEADS; i += KV * 32) {
-        const float t = m.talk[i];
-        const __nv_bfloat16 high = __float2bfloat16_rn(t);
-        const int at = i / HEADS * C::TALK_PITCH + i % HEADS;
-        talk[at] = high;
-        talk[TALK_PLANE + at] = __float2bfloat16_rn(t - __bfloat162float(high));
+        uint32_t term[TERMS];
+        terms_of(m.talk[i], 0.0f, term);
+#pragma unroll
+        for (int plane = 0; plane < TERMS; ++plane)
+            talk[plane * TALK_PLANE + i / HEADS * C::TALK_PITCH + i % HEADS] = __ushort_as_bfloat16(static_cast<unsigned short>(term[plane]));
     }
     const int p0 = a.positions[begin + first], p_last = p0 + count - 1;
     const int* table = a.block_table + static_cast<size_t>(entry) * a.table_width;
@@ -868,12 +878,12 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
                             const float v = s[r][n][2 * h + e];
                             w[e] = v == -INFINITY ? 0.0f : expf(v - top[r][h]) * total[r][h];
                         }
-                        uint32_t high, low;
-                        two_terms(w[0], w[1], high, low);
+                        uint32_t term[TERMS];
+                        terms_of(w[0], w[1], term);
                         // columns of a head: (8 keys, query, key), so that a query's eight keys are one 16-byte row
                         __nv_bfloat16* to = weights + (head0 + 2 * r + h) * C::PITCH + ((half * 2 + n) * TILE_Q + q) * 8 + 2 * quad;
-                        *reinterpret_cast<uint32_t*>(to) = high;
-                        *reinterpret_cast<uint32_t*>(to + PLANE) = low;
+#pragma unroll
+                        for (int plane = 0; plane < TERMS; ++plane) *reinterpret_cast<uint32_t*>(to + plane * PLANE) = term[plane];
                     }
         }
         __syncwarp();
@@ -882,42 +892,35 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
         __syncthreads();  // every head's weights
 #pragma unroll
         for (int column = warp; column < TILE_Q * TILE_K / 8; column += KV) {
-            uint32_t high[HEADS / 8], low[HEADS / 8];  // B operands: eight (query, key) columns of all heads
-            {
-                uint32_t b[4];
-                if constexpr (HEADS == 32) {
-                    ldmatrix_x4_trans(b, weights + lane * C::PITCH + column * 8);
+            uint32_t b[TERMS][HEADS / 8];  // B operands: eight (query, key) columns of all heads
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) high[j] = b[j];
-                    ldmatrix_x4_trans(b, weights + PLANE + lane * C::PITCH + column * 8);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) low[j] = b[j];
-                } else {
-                    ldmatrix_x4_trans(b, weights + (lane >> 4) * PLANE + (lane & 15) * C::PITCH + column * 8);
-                    high[0] = b[0], high[1] = b[1], low[0] = b[2], low[1] = b[3];
-                }
+            for (int plane = 0; plane < TERMS; ++plane) {
+                if constexpr (HEADS == 32) ldmatrix_x4_trans(b[plane], weights + plane * PLANE + lane * C::PITCH + column * 8);
+                else ldmatrix_x2_trans(b[plane], weights + plane * PLANE + (lane & 15) * C::PITCH + column * 8);
             }
             __syncwarp();  // the columns are read before their mixed weights take their place
 #pragma unroll
             for (int r = 0; r < HEADS / 16; ++r) {
+                uint32_t t[TERMS][HEADS / 16][4];
+#pragma unroll
+                for (int plane = 0; plane < TERMS; ++plane)
+#pragma unroll
+                    for (int k = 0; k < HEADS / 16; ++k)
+                        ldmatrix_x4(t[plane][k], talk + plane * TALK_PLANE + (r * 16 + (lane & 15)) * C::TALK_PITCH + k * 16 + (lane >> 4) * 8);
                 float mixed[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                for (int k = 0; k < HEADS / 16; ++k) {
-                    uint32_t t[4];
-                    const int at = (r * 16 + (lane & 15)) * C::TALK_PITCH + k * 16 + (lane >> 4) * 8;
-                    ldmatrix_x4(t, talk + TALK_PLANE + at);
-                    mma_bf16(mixed, t, high[2 * k], high[2 * k + 1]);
-                    ldmatrix_x4(t, talk + at);
-                    mma_bf16(mixed, t, low[2 * k], low[2 * k + 1]);
-                    mma_bf16(mixed, t, high[2 * k], high[2 * k + 1]);
-                }
+                for (int level = TERMS - 1; level >= 0; --level)  // the smallest products first
+#pragma unroll
+                    for (int k = 0; k < HEADS / 16; ++k)
+#pragma unroll
+                        for (int plane = 0; plane <= level; ++plane) mma_bf16(mixed, t[plane][k], b[level - plane][2 * k], b[level - plane][2 * k + 1]);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    uint32_t top_term, low_term;
-                    two_terms(mixed[2 * h], mixed[2 * h + 1], top_term, low_term);
+                    uint32_t term[TERMS];
+                    terms_of(mixed[2 * h], mixed[2 * h + 1], term);
                     __nv_bfloat16* to = weights + (r * 16 + q + 8 * h) * C::PITCH + column * 8 + 2 * quad;
-                    *reinterpret_cast<uint32_t*>(to) = top_term;
-                    *reinterpret_cast<uint32_t*>(to + PLANE) = low_term;
+#pragma unroll
+                    for (int plane = 0; plane < TERMS; ++plane) *reinterpret_cast<uint32_t*>(to + plane * PLANE) = term[plane];
                 }
             }
         }
@@ -925,11 +928,11 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
         __syncthreads();  // every column's mixed weights; each warp reads its own heads' and overwrites them alone
 #pragma unroll
         for (int k = 0; k < TILE_K / 16; ++k) {
-            uint32_t w[ROWS][2][4];
+            uint32_t w[ROWS][TERMS][4];
 #pragma unroll
             for (int r = 0; r < ROWS; ++r)
 #pragma unroll
-                for (int plane = 0; plane < 2; ++plane)
+                for (int plane = 0; plane < TERMS; ++plane)
                     ldmatrix_x4(w[r][plane], weights + plane * PLANE + (head0 + 2 * r + ((lane >> 3) & 1)) * C::PITCH +
                                                  ((2 * k + (lane >> 4)) * TILE_Q + (lane & 7)) * 8);
 #pragma unroll
@@ -937,12 +940,16 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
                 uint32_t b[4];
                 ldmatrix_x4_trans(b, values + swizzled<TILE_DIM>(k * 16 + (lane & 15), 2 * n + (lane >> 4)) * 8);
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r)
+                for (int r = 0; r < ROWS; ++r) {
+                    float part[2][4] = {};
 #pragma unroll
-                    for (int plane = 1; plane >= 0; --plane) {
-                        mma_bf16(out[r][2 * n], w[r][plane], b[0], b[1]);
-                        mma_bf16(out[r][2 * n + 1], w[r][plane], b[2], b[3]);
+                    for (int plane = TERMS - 1; plane >= 0; --plane) {
+                        mma_bf16(part[0], w[r][plane], b[0], b[1]);
+                        mma_bf16(part[1], w[r][plane], b[2], b[3]);
                     }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) out[r][2 * n][c] += part[0][c], out[r][2 * n + 1][c] += part[1][c];
+                }
             }
         }
         __syncwarp();
@@ -961,9 +968,10 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
         }
 }
 
-// Against the two kernels above on one prompt of 2,048 tokens (window 1,024, 64 kept): 32 heads of 8 KV heads 7,795 -> 548 us,
-// 16 heads 5,294 -> 308 us; 700 tokens behind 800: 3,448 -> 356 and 2,363 -> 198 us.  Error against float64 the same (1.66e-3,
-// the output's rounding to bfloat16).
+// Against the two kernels above as they were, on one prompt of 2,048 tokens (window 1,024, 64 kept): 32 heads of 8 KV heads
+// 7,795 -> 699 us, 16 heads 5,294 -> 376 us; 700 tokens behind 800: 3,448 -> 455 and 2,363 -> 245 us (with weights and mixing
+// matrix in two terms, 17 bits, 569, 330, 377 and 216 us: the third term's products cost a fifth and are what keeps 32 bits).  Error
+// against float64 the same (1.66e-3, the output's rounding to bfloat16), also where the heads' weights cancel.
 template <int KV, int GROUP>
 static int launch_mixed_tiles(const MixTileArgs& m, int entries, int longest, cudaStream_t stream) {
     static SharedMemoryOptIn opt_in;
