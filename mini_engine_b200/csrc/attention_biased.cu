@@ -19,6 +19,7 @@
 #include "mma_sync.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 struct BiasedArgs {
     const void* q;           // [tokens][heads][dim]
@@ -664,6 +665,10 @@ ME_EXPORT int me_mixed_attention(const void* q, const void* k_pages, const void*
 // matrix's and the weights' terms the six largest are formed, the others are below 2^-24 of a product.  The tensor core
 // truncates when it adds: the products with 16 keys' values leave it and are added to the output with rounding.
 //
+// A key that a query does not see has the weight zero in a product, which an infinity or NaN among its values would carry to
+// that query.  So a block whose output holds one walks again: keys with such values are then taken out of the product and
+// added to the queries that see them alone.
+//
 // Bound by the instructions a warp issues around its products (exponentials, masks, the split of the weights), with
 // one block to an SM; see the figures at launch_mixed_tiles.  A tile of eight tokens, since the output of four heads and
 // 16 tokens would take every register of a warp.
@@ -851,112 +856,153 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
 
     // Second walk.
     float out[ROWS][TILE_DIM / 8][4];
+    // Values that hold an infinity or NaN: out of the product, and to the queries that see their key.
+    auto add_apart = [&](int start) {
+        bool odd_lane = false;
+        for (int chunk = 0; chunk < TILE_DIM / 8; ++chunk) {
+            const uint4 x = *reinterpret_cast<const uint4*>(values + swizzled<TILE_DIM>(lane, chunk) * 8);
+            for (const uint32_t pair : {x.x, x.y, x.z, x.w}) odd_lane = odd_lane || (pair & 0x7f80u) == 0x7f80u || (pair & 0x7f800000u) == 0x7f800000u;
+        }
+        for (uint32_t odd = __ballot_sync(0xffffffffu, odd_lane); odd; odd &= odd - 1) {
+            const int j = __ffs(odd) - 1, distance = p0 + q - start - j;
+            if (q < count && distance >= 0 && (distance < a.window || start + j < a.keep_first)) {
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const __nv_bfloat16* from = weights + (head0 + 2 * r + h) * C::PITCH + ((j >> 3) * TILE_Q + q) * 8 + (j & 7);
+                        const float w = __bfloat162float(from[0]) + (__bfloat162float(from[PLANE]) + __bfloat162float(from[2 * PLANE]));
+#pragma unroll
+                        for (int n = 0; n < TILE_DIM / 8; ++n) {
+                            const uint32_t v = *reinterpret_cast<const uint32_t*>(values + swizzled<TILE_DIM>(j, n) * 8 + 2 * quad);
+                            out[r][n][2 * h] = fmaf(w, __uint_as_float(v << 16), out[r][n][2 * h]);
+                            out[r][n][2 * h + 1] = fmaf(w, __uint_as_float(v & 0xffff0000u), out[r][n][2 * h + 1]);
+                        }
+                    }
+            }
+            __syncwarp();
+            if (lane < TILE_DIM / 8) *reinterpret_cast<uint4*>(values + swizzled<TILE_DIM>(j, lane) * 8) = make_uint4(0u, 0u, 0u, 0u);
+            __syncwarp();
+        }
+    };
+    auto walk = [&](auto apart) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+            for (int n = 0; n < TILE_DIM / 8; ++n)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) out[r][n][c] = 0.0f;
+        there = fetch(k_pages, keys, 0);
+        fetch(v_pages, values, 0);
+        for (int i = 0; i < tiles; ++i) {
+            cp_async_wait<1>();
+            distances(i);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float s[ROWS][2][4];
+                scores(keys, i, half, there, s);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            float w[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const float v = s[r][n][2 * h + e];
+                                w[e] = v == -INFINITY ? 0.0f : expf(v - top[r][h]) * total[r][h];
+                            }
+                            uint32_t term[TERMS];
+                            terms_of(w[0], w[1], term);
+                            // columns of a head: (8 keys, query, key), so that a query's eight keys are one 16-byte row
+                            __nv_bfloat16* to = weights + (head0 + 2 * r + h) * C::PITCH + ((half * 2 + n) * TILE_Q + q) * 8 + 2 * quad;
+#pragma unroll
+                            for (int plane = 0; plane < TERMS; ++plane) *reinterpret_cast<uint32_t*>(to + plane * PLANE) = term[plane];
+                        }
+            }
+            __syncwarp();
+            if (i + 1 < tiles) there = fetch(k_pages, keys, i + 1);
+            else cp_async_commit();
+            __syncthreads();  // every head's weights
+#pragma unroll
+            for (int column = warp; column < TILE_Q * TILE_K / 8; column += KV) {
+                uint32_t b[TERMS][HEADS / 8];  // B operands: eight (query, key) columns of all heads
+#pragma unroll
+                for (int plane = 0; plane < TERMS; ++plane) {
+                    if constexpr (HEADS == 32) ldmatrix_x4_trans(b[plane], weights + plane * PLANE + lane * C::PITCH + column * 8);
+                    else ldmatrix_x2_trans(b[plane], weights + plane * PLANE + (lane & 15) * C::PITCH + column * 8);
+                }
+                __syncwarp();  // the columns are read before their mixed weights take their place
+#pragma unroll
+                for (int r = 0; r < HEADS / 16; ++r) {
+                    uint32_t t[TERMS][HEADS / 16][4];
+#pragma unroll
+                    for (int plane = 0; plane < TERMS; ++plane)
+#pragma unroll
+                        for (int k = 0; k < HEADS / 16; ++k)
+                            ldmatrix_x4(t[plane][k], talk + plane * TALK_PLANE + (r * 16 + (lane & 15)) * C::TALK_PITCH + k * 16 + (lane >> 4) * 8);
+                    float mixed[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int level = TERMS - 1; level >= 0; --level)  // the smallest products first
+#pragma unroll
+                        for (int k = 0; k < HEADS / 16; ++k)
+#pragma unroll
+                            for (int plane = 0; plane <= level; ++plane) mma_bf16(mixed, t[plane][k], b[level - plane][2 * k], b[level - plane][2 * k + 1]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t term[TERMS];
+                        terms_of(mixed[2 * h], mixed[2 * h + 1], term);
+                        __nv_bfloat16* to = weights + (r * 16 + q + 8 * h) * C::PITCH + column * 8 + 2 * quad;
+#pragma unroll
+                        for (int plane = 0; plane < TERMS; ++plane) *reinterpret_cast<uint32_t*>(to + plane * PLANE) = term[plane];
+                    }
+                }
+            }
+            cp_async_wait<1>();
+            __syncthreads();  // every column's mixed weights; each warp reads its own heads' and overwrites them alone
+            if constexpr (decltype(apart)::value) add_apart(tile_start(i));
+#pragma unroll
+            for (int k = 0; k < TILE_K / 16; ++k) {
+                uint32_t w[ROWS][TERMS][4];
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int plane = 0; plane < TERMS; ++plane)
+                        ldmatrix_x4(w[r][plane], weights + plane * PLANE + (head0 + 2 * r + ((lane >> 3) & 1)) * C::PITCH +
+                                                     ((2 * k + (lane >> 4)) * TILE_Q + (lane & 7)) * 8);
+#pragma unroll
+                for (int n = 0; n < TILE_DIM / 16; ++n) {
+                    uint32_t b[4];
+                    ldmatrix_x4_trans(b, values + swizzled<TILE_DIM>(k * 16 + (lane & 15), 2 * n + (lane >> 4)) * 8);
+#pragma unroll
+                    for (int r = 0; r < ROWS; ++r) {
+                        float part[2][4] = {};
+#pragma unroll
+                        for (int plane = TERMS - 1; plane >= 0; --plane) {
+                            mma_bf16(part[0], w[r][plane], b[0], b[1]);
+                            mma_bf16(part[1], w[r][plane], b[2], b[3]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) out[r][2 * n][c] += part[0][c], out[r][2 * n + 1][c] += part[1][c];
+                    }
+                }
+            }
+            __syncwarp();
+            if (i + 1 < tiles) fetch(v_pages, values, i + 1);
+            else cp_async_commit();
+        }
+        cp_async_wait<0>();
+    };
+    walk(std::false_type{});
+    bool finite = true;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
 #pragma unroll
         for (int n = 0; n < TILE_DIM / 8; ++n)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) out[r][n][c] = 0.0f;
-    there = fetch(k_pages, keys, 0);
-    fetch(v_pages, values, 0);
-    for (int i = 0; i < tiles; ++i) {
-        cp_async_wait<1>();
-        distances(i);
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float s[ROWS][2][4];
-            scores(keys, i, half, there, s);
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                for (int n = 0; n < 2; ++n)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        float w[2];
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const float v = s[r][n][2 * h + e];
-                            w[e] = v == -INFINITY ? 0.0f : expf(v - top[r][h]) * total[r][h];
-                        }
-                        uint32_t term[TERMS];
-                        terms_of(w[0], w[1], term);
-                        // columns of a head: (8 keys, query, key), so that a query's eight keys are one 16-byte row
-                        __nv_bfloat16* to = weights + (head0 + 2 * r + h) * C::PITCH + ((half * 2 + n) * TILE_Q + q) * 8 + 2 * quad;
-#pragma unroll
-                        for (int plane = 0; plane < TERMS; ++plane) *reinterpret_cast<uint32_t*>(to + plane * PLANE) = term[plane];
-                    }
-        }
-        __syncwarp();
-        if (i + 1 < tiles) there = fetch(k_pages, keys, i + 1);
-        else cp_async_commit();
-        __syncthreads();  // every head's weights
-#pragma unroll
-        for (int column = warp; column < TILE_Q * TILE_K / 8; column += KV) {
-            uint32_t b[TERMS][HEADS / 8];  // B operands: eight (query, key) columns of all heads
-#pragma unroll
-            for (int plane = 0; plane < TERMS; ++plane) {
-                if constexpr (HEADS == 32) ldmatrix_x4_trans(b[plane], weights + plane * PLANE + lane * C::PITCH + column * 8);
-                else ldmatrix_x2_trans(b[plane], weights + plane * PLANE + (lane & 15) * C::PITCH + column * 8);
-            }
-            __syncwarp();  // the columns are read before their mixed weights take their place
-#pragma unroll
-            for (int r = 0; r < HEADS / 16; ++r) {
-                uint32_t t[TERMS][HEADS / 16][4];
-#pragma unroll
-                for (int plane = 0; plane < TERMS; ++plane)
-#pragma unroll
-                    for (int k = 0; k < HEADS / 16; ++k)
-                        ldmatrix_x4(t[plane][k], talk + plane * TALK_PLANE + (r * 16 + (lane & 15)) * C::TALK_PITCH + k * 16 + (lane >> 4) * 8);
-                float mixed[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int level = TERMS - 1; level >= 0; --level)  // the smallest products first
-#pragma unroll
-                    for (int k = 0; k < HEADS / 16; ++k)
-#pragma unroll
-                        for (int plane = 0; plane <= level; ++plane) mma_bf16(mixed, t[plane][k], b[level - plane][2 * k], b[level - plane][2 * k + 1]);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t term[TERMS];
-                    terms_of(mixed[2 * h], mixed[2 * h + 1], term);
-                    __nv_bfloat16* to = weights + (r * 16 + q + 8 * h) * C::PITCH + column * 8 + 2 * quad;
-#pragma unroll
-                    for (int plane = 0; plane < TERMS; ++plane) *reinterpret_cast<uint32_t*>(to + plane * PLANE) = term[plane];
-                }
-            }
-        }
-        cp_async_wait<1>();
-        __syncthreads();  // every column's mixed weights; each warp reads its own heads' and overwrites them alone
-#pragma unroll
-        for (int k = 0; k < TILE_K / 16; ++k) {
-            uint32_t w[ROWS][TERMS][4];
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                for (int plane = 0; plane < TERMS; ++plane)
-                    ldmatrix_x4(w[r][plane], weights + plane * PLANE + (head0 + 2 * r + ((lane >> 3) & 1)) * C::PITCH +
-                                                 ((2 * k + (lane >> 4)) * TILE_Q + (lane & 7)) * 8);
-#pragma unroll
-            for (int n = 0; n < TILE_DIM / 16; ++n) {
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, values + swizzled<TILE_DIM>(k * 16 + (lane & 15), 2 * n + (lane >> 4)) * 8);
-#pragma unroll
-                for (int r = 0; r < ROWS; ++r) {
-                    float part[2][4] = {};
-#pragma unroll
-                    for (int plane = TERMS - 1; plane >= 0; --plane) {
-                        mma_bf16(part[0], w[r][plane], b[0], b[1]);
-                        mma_bf16(part[1], w[r][plane], b[2], b[3]);
-                    }
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) out[r][2 * n][c] += part[0][c], out[r][2 * n + 1][c] += part[1][c];
-                }
-            }
-        }
-        __syncwarp();
-        if (i + 1 < tiles) fetch(v_pages, values, i + 1);
-        else cp_async_commit();
-    }
-    cp_async_wait<0>();
+            for (int c = 0; c < 4; ++c) finite = finite && fabsf(out[r][n][c]) < INFINITY;
+    if (__syncthreads_or(!finite)) walk(std::true_type{});
     if (q >= count) return;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)

@@ -11,9 +11,9 @@ from test_pimezen_gpu import paged, plain_attention
 pytestmark = pytest.mark.gpu
 
 
-def tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size, alike=False):
+def tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size, alike=False, odd=()):
     """Requests ``(past, new)`` in one step through both forms; returns (tiles, rows, float64) of all new tokens.  ``alike``: the
-    heads' weights differ by about a thousandth and are mixed with signs that cancel, so that only their last bits are left."""
+    heads' weights differ by about a thousandth and are mixed with signs that cancel, so that only their last bits are left.  ``odd``: values ``(request, token, KV head, column, value)``."""
     from mini_engine_b200.csrc import ops
 
     dim, dtype = 128, torch.bfloat16
@@ -30,6 +30,9 @@ def tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size, ali
         if alike:
             k = k[:, :1].expand(-1, kv_heads, -1).clone()
             q = torch.where(torch.rand(q.shape) < 0.05, q[:, :1] * (1 + 2.0**-7), q[:, :1]).to(dtype).float()
+        for request, token, head, column, value in odd:
+            if request == i:
+                v[token, head, column] = value
         count = 2 * (-(-total // page_size)) + 1
         k_pages, table = paged(k, page_size, count, torch.Generator().manual_seed(i))
         v_pages, _ = paged(v, page_size, count, torch.Generator().manual_seed(i))
@@ -90,6 +93,20 @@ def test_mixed_heads_keep_32_bits_of_every_weight(heads, kv_heads):
     scale = want.norm()
     assert float((rows - want).norm() / scale) < 2.5e-3
     assert float((tiles - want).norm()) < 1.02 * float((rows - want).norm())
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(32, 8), (16, 8), (16, 4)])
+def test_values_that_are_not_finite_reach_only_the_queries_that_see_their_key(heads, kv_heads):
+    """A kept key, keys inside windows and the last key of a portion, behind and ahead of queries of the same tile."""
+    inf, nan = float("inf"), float("nan")
+    odd = [(0, 2, 1, 3, inf), (0, 21, 0, 5, nan), (0, 21, 0, 100, -inf), (0, 27, 3, 64, inf), (0, 39, 2, 0, nan), (1, 45, 1, 127, -inf)]
+    torch.manual_seed(heads)
+    tiles, rows, _ = tiles_and_rows([(0, 40), (37, 12)], heads, kv_heads, 12, 6, 16, odd=odd)
+    assert rows.isnan().any() and rows.isinf().any()
+    assert torch.equal(tiles.isnan(), rows.isnan())
+    assert torch.equal(torch.where(tiles.isinf(), tiles, 0.0), torch.where(rows.isinf(), rows, 0.0))
+    finite = rows.isfinite()
+    assert float((tiles - rows)[finite].norm() / rows[finite].norm()) < 2.5e-3  # both rounded to bfloat16
 
 
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 24), (3, 64, 128), (2, 128, 128), (1, 100, 36)])
