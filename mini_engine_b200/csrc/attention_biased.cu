@@ -499,11 +499,16 @@ constexpr int MIX_GROUP = 8;    // query heads per KV head, at most
 constexpr int MIX_COLUMNS = 8;  // value elements per lane, at most: vdim <= 256
 
 // GROUP and COLUMNS: MIX_GROUP and MIX_COLUMNS, or as many as the sizes need, so that nothing is shuffled and added for heads
-// and columns that are not there.  What the warps of a block wait for is memory: eight heads' scores and four keys' values are
-// fetched at a time, ahead of the arithmetic, whose order is that of one at a time.  Eight decoded tokens behind 16 to 2,048, 16 heads
-// in 8 KV heads: 90 -> 60 us.
+// and columns that are not there.  What the warps of a block wait for is memory: AT_ONCE heads' scores and KEYS keys' values are
+// fetched ahead of the arithmetic, whose order is that of one at a time.  Four keys pay while their values and the sums leave
+// registers for many warps: with 4 x 4 or more sums a lane, one key at a time is faster but for sixteen warps of 8 x 4.  Both
+// kernels, us, every head and key at full width and one by one | this form (decoded tokens of 1,088 visible keys, bfloat16 unless
+// said): 16 heads in 8 KV heads of 128, 32 tokens: 243 | 127; 32 heads in 8: 298 | 179; 16 in 4: 124 | 99; 16 in 2: 118 | 101; 16 in
+// 8 with values of 256: 290 | 169 (four keys at a time: 570), float32 429 | 400; 8 in 1 with values of 192: 93 | 93 (151).
 template <typename T, int WARPS, int GROUP, int COLUMNS>
 __global__ void __launch_bounds__(WARPS * 32) attention_mix_values_kernel(ScoreArgs s, const float* __restrict__ talk) {
+    constexpr int KEYS = COLUMNS == 4 && (GROUP == 2 || (GROUP == 8 && WARPS == 16)) ? 4 : 1;
+    constexpr int AT_ONCE = GROUP == 8 && COLUMNS == 8 ? 4 : 8;
     const BiasedArgs& a = s.a;
     extern __shared__ __align__(16) float mix_shared[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -548,7 +553,6 @@ __global__ void __launch_bounds__(WARPS * 32) attention_mix_values_kernel(ScoreA
                 if (page >= 0) {
                     value_row = ((static_cast<long long>(page) * a.kv_heads + kv) * a.page_size + key % a.page_size) * vd;
                     const float* column = rows + (run == 0 ? key : kept_end + (key - lowest));
-                    constexpr int AT_ONCE = 8;
                     for (int g0 = 0; g0 < heads; g0 += AT_ONCE) {  // ascending g: the order of the mixed sum
                         float score[AT_ONCE];
 #pragma unroll
@@ -565,7 +569,6 @@ __global__ void __launch_bounds__(WARPS * 32) attention_mix_values_kernel(ScoreA
                     }
                 }
             }
-            constexpr int KEYS = 4;
             for (int j0 = 0; j0 < 32; j0 += KEYS) {
                 long long rj[KEYS];
                 float v[KEYS][COLUMNS];
@@ -624,7 +627,11 @@ static int launch_two_kernels(const ScoreArgs& s, const float* talk, cudaStream_
     if (smem1 > 48 * 1024 || smem2 > 200 * 1024) return ME_ERR_UNSUPPORTED;
     int code = launch_kernel_in_order(attention_scores_kernel<T, WARPS>, a.tokens * a.heads, WARPS * 32, smem1, stream, s);
     if (code) return code;
-    if (a.vdim > 128) return launch_mix_values<T, WARPS, MIX_GROUP, MIX_COLUMNS>(s, talk, smem2, stream);
+    if (a.vdim > 128) {
+        if (group <= 2) return launch_mix_values<T, WARPS, 2, MIX_COLUMNS>(s, talk, smem2, stream);
+        if (group <= 4) return launch_mix_values<T, WARPS, 4, MIX_COLUMNS>(s, talk, smem2, stream);
+        return launch_mix_values<T, WARPS, MIX_GROUP, MIX_COLUMNS>(s, talk, smem2, stream);
+    }
     if (group <= 2) return launch_mix_values<T, WARPS, 2, 4>(s, talk, smem2, stream);
     if (group <= 4) return launch_mix_values<T, WARPS, 4, 4>(s, talk, smem2, stream);
     return launch_mix_values<T, WARPS, MIX_GROUP, 4>(s, talk, smem2, stream);

@@ -6,7 +6,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from test_pimezen_gpu import paged, plain_attention
+from test_pimezen_gpu import paged, plain_attention, run_attention
 
 pytestmark = pytest.mark.gpu
 
@@ -107,6 +107,22 @@ def test_values_that_are_not_finite_reach_only_the_queries_that_see_their_key(he
     assert torch.equal(torch.where(tiles.isinf(), tiles, 0.0), torch.where(rows.isinf(), rows, 0.0))
     finite = rows.isfinite()
     assert float((tiles - rows)[finite].norm() / rows[finite].norm()) < 2.5e-3  # both rounded to bfloat16
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,vdim", [(3, 3, 129), (4, 2, 256), (8, 2, 200), (3, 1, 64), (7, 1, 96), (8, 1, 192), (16, 2, 128)])
+def test_every_form_of_the_two_kernels(heads, kv_heads, vdim, dtype):
+    """Groups and value widths on both sides of the forms' bounds (2, 4 and 8 heads; 128 and 256 columns), heads that are no
+    multiple of the scores fetched at a time; a long step (two warps in bfloat16) and a short one (sixteen)."""
+    torch.manual_seed(heads + vdim)
+    count, dim = 600, 24
+    q, k, v = (torch.randn(count, h, d).to(dtype).float() for h, d in ((heads, dim), (kv_heads, dim), (kv_heads, vdim)))
+    r1, r2, talk = torch.rand(heads), torch.rand(heads) + 0.1, torch.randn(heads, heads)
+    want = plain_attention(q, k, v, r1, r2, talk, dim**-0.5, 50, 7)
+    for positions in (list(range(count)), [0, 31, 64, 599]):
+        got = run_attention(q, k, v, r1, r2, talk, dim**-0.5, 50, 7, positions, dtype)  # the one-pass form beside the two kernels
+        error = float((got - want[positions]).norm() / want[positions].norm())
+        assert error < (2e-6 if dtype == torch.float32 else 2.5e-3)  # sums of 57 weighted values; the output's rounding
 
 
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 24), (3, 64, 128), (2, 128, 128), (1, 100, 36)])
