@@ -413,11 +413,29 @@ ME_EXPORT int me_biased_attention(const void* q, const void* k_pages, const void
 // scores, heads x group for the mixing, group x vdim for the values, each once.  Tiles go to warps by tile
 // number and partial results are added in ascending order, as above.
 
+// Which entries of a step the tile kernel below takes, for a step that runs both forms: those that bring at least `eighths` / 8 of
+// the keys that their last token sees, or `most` tokens.  An entry's few tokens behind many keys fill few blocks of tiles, each of
+// which walks all of the keys; see me_mixed_attention_tiles.
+struct TileRule {
+    const int* cu_tokens;  // [entries + 1]; null: the kernel takes every entry
+    int eighths, most;
+};
+
+constexpr int TILE_Q = 8, TILE_K = 32, TILE_DIM = 128;  // of the tile kernel
+
+__device__ __forceinline__ bool takes_tiles(const TileRule& rule, const BiasedArgs& a, int entry) {
+    const int begin = rule.cu_tokens[entry], count = rule.cu_tokens[entry + 1] - begin;
+    if (count < TILE_Q) return false;
+    const long long keys = min(static_cast<long long>(a.positions[begin + count - 1]) + 1, static_cast<long long>(a.window) + a.keep_first);
+    return count >= rule.most || 8ll * count >= keys * rule.eighths;
+}
+
 struct ScoreArgs {
     BiasedArgs a;
     float* scores;  // [tokens][heads][stride]
     float* stats;   // [tokens][heads][2] maximum, denominator
     int stride;     // most keys a query can see
+    TileRule tiles;  // entries that are left to the tile kernel
 };
 
 template <typename T, int WARPS>
@@ -433,6 +451,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_scores_kernel(ScoreArgs 
     pdl_trigger();
     const float r1 = a.r1 ? a.r1[head] : 0.0f, r2 = a.r1 ? a.r2[head] : 0.0f;
     pdl_wait();
+    if (s.tiles.cu_tokens && takes_tiles(s.tiles, a, a.entry_of_token[token])) return;
     const int own_kv = head / (a.heads / a.kv_heads);
     const int position = a.positions[token];
     const int* table = a.block_table + static_cast<size_t>(a.entry_of_token[token]) * a.table_width;
@@ -521,6 +540,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_mix_values_kernel(ScoreA
     pdl_trigger();
     for (int i = threadIdx.x; i < group * heads; i += WARPS * 32) mixing[i] = talk[(kv * group + i / heads) * heads + i % heads];
     pdl_wait();
+    if (s.tiles.cu_tokens && takes_tiles(s.tiles, a, a.entry_of_token[token])) return;
     for (int g = threadIdx.x; g < heads; g += WARPS * 32) {
         const float* st = s.stats + (static_cast<size_t>(token) * heads + g) * 2;
         top[g] = st[0];
@@ -638,23 +658,25 @@ static int launch_two_kernels(const ScoreArgs& s, const float* talk, cudaStream_
 }
 
 // Mixed attention in two kernels.  `scores` holds tokens * heads * stride floats, `stats` tokens * heads * 2;
-// `stride` is the most keys a query of this step can see.  out: [tokens][heads][vdim] of the pages' type.
+// `stride` is the most keys a query of this step can see.  out: [tokens][heads][vdim] of the pages' type.  With `cu_tokens` the
+// entries that TileRule gives to the tile kernel are left alone; `expected`: about how many tokens then remain, else all.
 ME_EXPORT int me_mixed_attention(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                  const int* entry_of_token, const int* positions, const float* r1, const float* r2,
                                  const float* talk, float* scores, float* stats, int stride, void* out, int type,
                                  float scale, int tokens, int heads, int kv_heads, int dim, int vdim, int page_size,
-                                 int table_width, int window, int keep_first, cudaStream_t stream) {
+                                 int table_width, int window, int keep_first, const int* cu_tokens, int eighths, int most,
+                                 int expected, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (heads % kv_heads || heads / kv_heads > MIX_GROUP || vdim > 32 * MIX_COLUMNS || dim < 1 || vdim < 1) return ME_ERR_UNSUPPORTED;
     if ((r1 == nullptr) != (r2 == nullptr) || window < 0 || keep_first < 0 || talk == nullptr || stride < 1) return ME_ERR_ARGUMENT;
     if (static_cast<long long>(tokens) * heads > 0x7fffffffll) return ME_ERR_UNSUPPORTED;
     ScoreArgs s{{q, k_pages, v_pages, block_table, entry_of_token, positions, r1, r2, out, scale, tokens, heads,
                  kv_heads, dim, vdim, page_size, table_width, window, keep_first, 0},
-                scores, stats, stride};
+                scores, stats, stride, {cu_tokens, eighths, most}};
     // float32: four warps always (the same bits for a token in a prompt and decoded alone); bfloat16: two
     // warps when the step has blocks enough to fill the GPU, sixteen when it has few.
     if (type != ME_BF16) return launch_two_kernels<float, 4>(s, talk, stream);
-    if (static_cast<long long>(tokens) * kv_heads >= 1024) return launch_two_kernels<__nv_bfloat16, 2>(s, talk, stream);
+    if (static_cast<long long>(expected) * kv_heads >= 1024) return launch_two_kernels<__nv_bfloat16, 2>(s, talk, stream);
     return launch_two_kernels<__nv_bfloat16, 16>(s, talk, stream);
 }
 
@@ -679,7 +701,6 @@ ME_EXPORT int me_mixed_attention(const void* q, const void* k_pages, const void*
 // Bound by the instructions a warp issues around its products (exponentials, masks, the split of the weights), with
 // one block to an SM; see the figures at launch_mixed_tiles.  A tile of eight tokens, since the output of four heads and
 // 16 tokens would take every register of a warp.
-constexpr int TILE_Q = 8, TILE_K = 32, TILE_DIM = 128;
 constexpr int BIAS_SPAN = TILE_Q + TILE_K;  // distances within a tile, one spare
 constexpr int TERMS = 3;                    // bfloat16 terms of a float32 number
 
@@ -696,6 +717,7 @@ struct MixTileArgs {
     BiasedArgs a;
     const float* talk;
     const int* cu_tokens;  // [entries + 1]
+    TileRule rule;         // which entries, all without its own cu_tokens
 };
 
 // x and y as pairs of bfloat16 terms, the largest first
@@ -725,7 +747,7 @@ __global__ void __launch_bounds__(KV * 32, 1) mixed_attention_tiles_kernel(MixTi
     const int entry = blockIdx.y, begin = m.cu_tokens[entry];
     const int first = static_cast<int>(gridDim.x - 1 - blockIdx.x) * TILE_Q;  // the last tokens see the most keys: they go first
     const int count = min(m.cu_tokens[entry + 1] - begin - first, TILE_Q);
-    if (count <= 0) return;
+    if (count <= 0 || (m.rule.cu_tokens && !takes_tiles(m.rule, a, entry))) return;
     const int head0 = warp * GROUP;
     for (int i = threadIdx.x; i < HEADS * HEADS; i += KV * 32) {
         uint32_t term[TERMS];
@@ -1034,11 +1056,13 @@ static int launch_mixed_tiles(const MixTileArgs& m, int entries, int longest, cu
 }
 
 // The same result from tiles of tokens; bfloat16, 128-wide heads, the (kv_heads, group) pairs below.  The tokens of entry e are
-// cu_tokens[e] .. cu_tokens[e + 1], at consecutive positions; none has more than `longest`.
+// cu_tokens[e] .. cu_tokens[e + 1], at consecutive positions; none has more than `longest`.  `most` > 0: only the entries that
+// TileRule gives to this kernel, which the two kernels above then leave alone.
 ME_EXPORT int me_mixed_attention_tiles(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                        const int* cu_tokens, const int* positions, const float* r1, const float* r2,
                                        const float* talk, void* out, float scale, int entries, int longest, int heads, int kv_heads,
-                                       int dim, int vdim, int page_size, int table_width, int window, int keep_first, cudaStream_t stream) {
+                                       int dim, int vdim, int page_size, int table_width, int window, int keep_first, int eighths,
+                                       int most, cudaStream_t stream) {
     if (entries <= 0 || longest <= 0) return 0;
     if (dim != TILE_DIM || vdim != TILE_DIM || kv_heads < 1 || heads % kv_heads || entries > 65535) return ME_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(k_pages) % 16 || reinterpret_cast<uintptr_t>(v_pages) % 16 || reinterpret_cast<uintptr_t>(q) % 4 || reinterpret_cast<uintptr_t>(out) % 4)
@@ -1046,7 +1070,7 @@ ME_EXPORT int me_mixed_attention_tiles(const void* q, const void* k_pages, const
     if ((r1 == nullptr) != (r2 == nullptr) || window < 1 || keep_first < 0 || talk == nullptr) return ME_ERR_ARGUMENT;
     MixTileArgs m{{q, k_pages, v_pages, block_table, nullptr, positions, r1, r2, out, scale, 0, heads, kv_heads, dim, vdim,
                    page_size, table_width, window, keep_first, 0},
-                  talk, cu_tokens};
+                  talk, cu_tokens, {most > 0 ? cu_tokens : nullptr, eighths, most}};
     const int group = heads / kv_heads;
     if (kv_heads == 8 && group == 4) return launch_mixed_tiles<8, 4>(m, entries, longest, stream);
     if (kv_heads == 8 && group == 2) return launch_mixed_tiles<8, 2>(m, entries, longest, stream);

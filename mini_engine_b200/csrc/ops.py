@@ -844,12 +844,14 @@ MIXED_ATTENTION_MAX_GROUP, MIXED_ATTENTION_MAX_VALUE_DIM = 8, 256
 def mixed_attention(
     *, q, k_pages, v_pages, block_table, entry_of_token, positions, out, heads: int, kv_heads: int, head_dim: int,
     value_dim: int, scale: float, window: int, keep_first: int, r1: torch.Tensor | None, r2: torch.Tensor | None,
-    talk: torch.Tensor, scores: torch.Tensor, stats: torch.Tensor, stride: int,
+    talk: torch.Tensor, scores: torch.Tensor, stats: torch.Tensor, stride: int, besides_tiles: torch.Tensor | None = None,
+    expected: int | None = None,
 ) -> None:  # fmt: skip
     """The attention of :func:`biased_attention` with mixed heads, in two kernels that keep the scores
     (``scores``: float32 scratch of ``T * heads * stride`` values, ``stride`` the most keys a query can see;
     ``stats``: ``T * heads * 2``) and apply every value once.  Groups of up to 8 query heads per KV head,
-    value heads up to 256 wide."""
+    value heads up to 256 wide.  ``besides_tiles``: the step's ``cu_tokens``; entries that :func:`mixed_attention_tiles` takes
+    with ``by_entry`` are left to it, and about ``expected`` tokens remain (what the kernels' width goes by)."""
     _need(q, None, "q"), _need(out, q.dtype, "out"), _need(k_pages, q.dtype, "k_pages"), _need(v_pages, q.dtype, "v_pages")
     _need(block_table, torch.int32, "block_table"), _need(entry_of_token, torch.int32, "entry_of_token")
     _need(positions, torch.int32, "positions"), _need(talk, torch.float32, "talk")
@@ -864,33 +866,67 @@ def mixed_attention(
         raise KernelError(f"pages {tuple(k_pages.shape)}, {tuple(v_pages.shape)} do not fit the head sizes")
     if talk.shape != (heads, heads) or scores.numel() < tokens * heads * stride or stats.numel() < tokens * heads * 2:
         raise KernelError("talk must be [heads, heads]; scores and stats must hold the step's (token, head) pairs")
+    eighths, most = (0, 0) if besides_tiles is None else MIXED_TILES[kv_heads, heads // kv_heads]
+    if besides_tiles is not None:
+        _need(besides_tiles, torch.int32, "besides_tiles")
     fn = _fn(
         "attention_biased",
         "me_mixed_attention",
-        [c_void_p] * 11 + [c_int, c_void_p, c_int, c_float] + [c_int] * 9 + [c_void_p],
+        [c_void_p] * 11 + [c_int, c_void_p, c_int, c_float] + [c_int] * 9 + [c_void_p, c_int, c_int, c_int, c_void_p],
     )
     code = fn(
         _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), _ptr(entry_of_token), _ptr(positions), _ptr(r1), _ptr(r2),
         _ptr(talk), _ptr(scores), _ptr(stats), int(stride), _ptr(out), _type_code(q.dtype), float(scale), tokens, heads,
-        kv_heads, head_dim, value_dim, k_pages.shape[2], block_table.shape[1], int(window), int(keep_first), _stream(),
+        kv_heads, head_dim, value_dim, k_pages.shape[2], block_table.shape[1], int(window), int(keep_first), _ptr(besides_tiles),
+        eighths, most, tokens if expected is None else expected, _stream(),
     )  # fmt: skip
     _check(code, "mixed_attention")
 
 
-MIXED_TILES = {(8, 4), (8, 2), (4, 4)}  # (KV heads, query heads of each) that the tile kernel is built for
+# (KV heads, query heads of each) that the tile kernel is built for, and which entries take it where both forms run: those that
+# bring so many eighths of the keys that they see, or so many tokens.  A tile walks all of its keys, twice, on one SM, however few
+# its tokens are; the two kernels take a time per token.  Measured, us, tiles | two kernels, one entry behind 2,048 (a window of
+# 1,024 and 64 kept keys): 32 heads in 8: 64 tokens 424 | 300, 96 424 | 429, 127 436 | 527; 16 in 8: 64 224 | 194, 96 224 | 270;
+# 16 in 4: 96 313 | 228, 192 313 | 394; behind 512: 32 in 8 64 223 | 167, 96 236 | 246; 16 in 8 64 120 | 110, 96 126 | 153; 16 in 4
+# 127 189 | 160, 192 201 | 241; whole prompts of 16 and 64 tokens: 24 | 26 and 36 | 62, 14 | 20 and 21 | 46, 18 | 20 and 27 | 36.
+MIXED_TILES = {(8, 4): (3, 96), (8, 2): (2, 80), (4, 4): (6, 144)}
+MIXED_TILES_START = 24  # tokens that take the two kernels as long as their two launches
+MIXED_TILES_MIN_TOKENS = 8  # of an entry: a tile takes as long with one token in it as with eight
 
 
 def mixed_attention_tiles_supports(dtype: torch.dtype, heads: int, kv_heads: int, head_dim: int, value_dim: int) -> bool:
     return dtype == torch.bfloat16 and head_dim == value_dim == 128 and heads % kv_heads == 0 and (kv_heads, heads // kv_heads) in MIXED_TILES
 
 
+def mixed_attention_forms(
+    kv_heads: int, heads: int, *, tokens: int, entries: int, decoded: int, least: int, longest: int, portion_keys: int, keys: int
+) -> tuple[bool, bool]:
+    """Whether a step takes the tiles, and whether it takes the two kernels; with both each entry runs in its own form, one after the
+    other.  ``decoded`` of its ``entries`` bring one token, the others ``least`` to ``longest``; a token sees at most ``keys`` keys, a
+    portion's ``portion_keys``.  A form that no entry can take is not launched (an eager launch is 15 us of the host).  More
+    tokens than any entry needs for tiles run in tiles all together where that is faster: the tiles' time, which goes with
+    the keys, grows from ``portion_keys`` to ``keys``, and the two kernels' time for the decoded tokens is spared.  32 heads in 8,
+    us, all in tiles | each its own: 32 decoded behind 2,048 beside a portion of 512 behind 512 442 | 592; eight beside a
+    prompt of 192 422 | 161."""
+    eighths, most = MIXED_TILES[kv_heads, heads // kv_heads]
+    takes = lambda count: count >= MIXED_TILES_MIN_TOKENS and (count >= most or 8 * count >= eighths * portion_keys)  # noqa: E731
+    if longest < MIXED_TILES_MIN_TOKENS:
+        return False, True
+    together = tokens > most and (MIXED_TILES_START + decoded) * keys >= (MIXED_TILES_START + most) * (keys - portion_keys)
+    if together or (not decoded and takes(least)):
+        return True, False
+    return entries - decoded > 1 or takes(longest), True
+
+
 def mixed_attention_tiles(
     *, q, k_pages, v_pages, block_table, cu_tokens, longest: int, positions, out, heads: int, kv_heads: int, head_dim: int,
     value_dim: int, scale: float, window: int, keep_first: int, r1: torch.Tensor | None, r2: torch.Tensor | None, talk: torch.Tensor,
+    by_entry: bool = False,
 ) -> None:  # fmt: skip
     """The attention of :func:`mixed_attention` from tiles of eight tokens on tensor cores, for the sizes of
     :func:`mixed_attention_tiles_supports`.  An entry's tokens (``cu_tokens``: int32, one more than entries) lie at consecutive
-    positions and are at most ``longest``; ``window`` is positive."""
+    positions and are at most ``longest``; ``window`` is positive.  ``by_entry``: only entries of at least eight tokens that bring
+    the numbers of ``MIXED_TILES``; the others' rows are left as they are."""
     for name, tensor in (("q", q), ("out", out), ("k_pages", k_pages), ("v_pages", v_pages)):
         _need(tensor, torch.bfloat16, name)
     for name, tensor in (("block_table", block_table), ("cu_tokens", cu_tokens), ("positions", positions)):
@@ -906,11 +942,11 @@ def mixed_attention_tiles(
     entries = cu_tokens.shape[0] - 1
     if talk.shape != (heads, heads) or block_table.shape[0] < entries or out.numel() < q.shape[0] * heads * value_dim:
         raise KernelError("talk must be [heads, heads], the block table must have a row per entry, out a value row per token and head")
-    fn = _fn("attention_biased", "me_mixed_attention_tiles", [c_void_p] * 10 + [c_float] + [c_int] * 10 + [c_void_p])
+    fn = _fn("attention_biased", "me_mixed_attention_tiles", [c_void_p] * 10 + [c_float] + [c_int] * 12 + [c_void_p])
     code = fn(
         _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), _ptr(cu_tokens), _ptr(positions), _ptr(r1), _ptr(r2), _ptr(talk),
         _ptr(out), float(scale), entries, int(longest), heads, kv_heads, head_dim, value_dim, k_pages.shape[2],
-        block_table.shape[1], int(window), int(keep_first), _stream(),
+        block_table.shape[1], int(window), int(keep_first), *(MIXED_TILES[kv_heads, heads // kv_heads] if by_entry else (0, 0)), _stream(),
     )  # fmt: skip
     _check(code, "mixed_attention_tiles")
 

@@ -221,11 +221,12 @@ class ModelRunner:
             ctx_len[:real] = start_arr + 1
             fresh[:real] = start_arr == 0
             cursor = real
-            max_q, max_ctx = 1, int(start_arr.max()) + 1
+            max_q, max_ctx, max_portion_ctx = 1, int(start_arr.max()) + 1, 0
         else:
             cursor = 0
             cu[0] = 0
             max_q = max_ctx = 1
+            max_portion_ctx = 0
             for b, entry in enumerate(entries):
                 n = counts[b]
                 end = entry.start + n
@@ -253,6 +254,8 @@ class ModelRunner:
                         raise ValueError(f"entry {b}: wanted place {place} is outside its {n} tokens")
                     wanted_rows.append(cursor + place)
                 max_q, max_ctx = max(max_q, n), max(max_ctx, end)
+                if n > 1:
+                    max_portion_ctx = max(max_portion_ctx, end)
                 cursor += n
         if ids[:real_tokens].min() < 0 or ids[:real_tokens].max() >= self.vocab_size:
             raise ValueError(f"token ids must lie in [0, {self.vocab_size})")
@@ -312,6 +315,8 @@ class ModelRunner:
             num_decode_entries=len(decode_list),
             decode_entries=at(o_kinds, len(decode_list)),
             portion_entries=at(o_kinds + len(decode_list), len(portion_list)),
+            min_portion_len=min((all_counts[b] for b in portion_list), default=2),
+            max_portion_context=max_portion_ctx,
             host={
                 "counts": all_counts,
                 "starts": starts + [0] * (total_entries - real),

@@ -73,10 +73,6 @@ from mini_engine_b200.parts.base import (
 from mini_engine_b200.parts.linear import Linear
 from mini_engine_b200.weights.loader import WeightSpec
 
-# Mixed heads run from tiles of eight tokens on tensor cores when some entry of the step brings this many tokens.  A tile
-# takes as long with one token in it as with eight: below, one block per (token, head) of the two-kernel form is faster.
-MIXING_TILES_MIN_TOKENS = 8
-
 
 @register("mixer", "gqa_attention")
 class GroupedQueryAttention(Mixer):
@@ -333,18 +329,29 @@ class GroupedQueryAttention(Mixer):
         if self.extended:
             out = ctx.buffer("attn.out", (tokens, self.heads * self.value_dim), ctx.dtype)
             # Scores of every visible key are kept between two kernels; a window bounds them whatever the context.
-            # The scratch is sized for the engine's token capacity, so the choice never depends on the batch.
+            # The scratch is sized for the engine's token capacity: whether it fits does not depend on the step.
             stride = (self.window or 0) + self.keep_first
             capacity = max(tokens, ctx.workspace.max_tokens)
-            if self.two_kernel_mixing and self.mixing_tiles and ctx.max_query_len >= MIXING_TILES_MIN_TOKENS:
+            two_kernels = self.two_kernel_mixing and capacity * self.heads * stride * 4 <= 2 << 30
+            tiles, by_entry = self.two_kernel_mixing and self.mixing_tiles and ctx.max_query_len >= ops.MIXED_TILES_MIN_TOKENS, False
+            if tiles and two_kernels:
+                # Which forms run follows from the step's sizes on the host, which entries take which from their own sizes on
+                # the device (a captured step stands for others).
+                tiles, by_entry = ops.mixed_attention_forms(
+                    self.kv_heads, self.heads, tokens=tokens, entries=ctx.num_entries, decoded=ctx.num_decode_entries,
+                    least=ctx.min_portion_len, longest=ctx.max_query_len, portion_keys=min(ctx.max_portion_context, stride),
+                    keys=min(ctx.max_context_len, stride),
+                )  # fmt: skip
+            if tiles:
                 ops.mixed_attention_tiles(
                     q=q, k_pages=cache.k, v_pages=cache.v, block_table=ctx.block_tables[cache.group], cu_tokens=ctx.cu_tokens,
                     longest=ctx.max_query_len, positions=ctx.positions, out=out, heads=self.heads, kv_heads=self.kv_heads, head_dim=d,
                     value_dim=self.value_dim, scale=self.scale, window=self.window, keep_first=self.keep_first, r1=self.r1,
-                    r2=self.r2, talk=self.talk,
+                    r2=self.r2, talk=self.talk, by_entry=by_entry,
                 )  # fmt: skip
-                return self.out.forward(out, ctx, "attn.o")
-            if self.two_kernel_mixing and capacity * self.heads * stride * 4 <= 2 << 30:
+                if not by_entry:
+                    return self.out.forward(out, ctx, "attn.o")
+            if two_kernels:
                 scores = ctx.buffer("attn.scores", (tokens, self.heads * stride), torch.float32)
                 stats = ctx.buffer("attn.stats", (tokens, self.heads * 2), torch.float32)
                 ops.mixed_attention(
@@ -352,7 +359,7 @@ class GroupedQueryAttention(Mixer):
                     entry_of_token=ctx.entry_of_token, positions=ctx.positions, out=out, heads=self.heads,
                     kv_heads=self.kv_heads, head_dim=d, value_dim=self.value_dim, scale=self.scale, window=self.window,
                     keep_first=self.keep_first, r1=self.r1, r2=self.r2, talk=self.talk, scores=scores, stats=stats,
-                    stride=stride,
+                    stride=stride, besides_tiles=ctx.cu_tokens if tiles else None, expected=ctx.num_decode_entries if tiles else None,
                 )  # fmt: skip
                 return self.out.forward(out, ctx, "attn.o")
             spread = None

@@ -191,6 +191,8 @@ class StepContext:
     num_decode_entries: int = 0  # entries that bring exactly one token ...
     decode_entries: torch.Tensor | None = None  # ... their numbers, ascending (int32)
     portion_entries: torch.Tensor | None = None  # the numbers of the entries that bring more
+    min_portion_len: int = 2  # the fewest tokens of an entry that brings more, and ...
+    max_portion_context: int = 0  # ... the longest context of one
     host: Mapping[str, Any] = field(default_factory=dict)  # host copies for parts written in Python
     embedding_state: torch.Tensor | None = None  # [slots + 1, *shape]: per-request state of the embedding part
     memo: dict = field(default_factory=dict)  # what parts compute once per step and share between layers

@@ -164,3 +164,30 @@ def test_prefix_hits_need_the_kept_pages_too():
     manager.free(req)
     hit = manager.match_prefix(tokens)[0]
     assert len(hit) == 5 and hit[0] != NULL_PAGE and hit[1:4] == [NULL_PAGE] * 3 and hit[4] != NULL_PAGE
+
+
+@pytest.mark.parametrize("kv_heads,heads", [(8, 32), (8, 16), (4, 16)])
+def test_which_forms_of_the_mixed_heads_a_step_takes(kv_heads, heads):
+    """Few tokens: each entry its own form, and none that no entry can take.  Many: portions that see as many keys as the decoded
+    entries beside them take tiles together; decoded entries far behind a fresh prompt only when there are many of them."""
+    from mini_engine_b200.csrc import ops
+
+    eighths, most = ops.MIXED_TILES[kv_heads, heads // kv_heads]
+    least_behind = -(-eighths * 64 // 8)  # tokens of an entry that sees 64 keys
+
+    def forms(portions, portion_keys, decoded=0, keys=0):
+        return ops.mixed_attention_forms(
+            kv_heads, heads, tokens=sum(portions) + decoded, entries=len(portions) + decoded, decoded=decoded, least=min(portions, default=2),
+            longest=max(portions, default=1), portion_keys=portion_keys, keys=max(keys, portion_keys),
+        )  # fmt: skip
+
+    tiles, rows, both = (True, False), (False, True), (True, True)
+    assert forms([], 0, 8, 500) == rows and forms([7, 5], 7, 3, 500) == rows
+    assert forms([8], 8) == tiles and forms([8], 1088) == rows  # a whole prompt, a portion far behind
+    assert forms([least_behind], 64) == tiles and forms([least_behind - 1], 64) == rows
+    assert forms([least_behind] * 2, 64) == tiles and forms([least_behind, least_behind - 1], 64) == both
+    assert forms([20], 20, 1, 900) == both and forms([20], 900, 1, 900) == rows and forms([20], 900, most, 900) == tiles
+    assert forms([most // 2] * 2, 1088) == both and forms([most // 2] * 3, 1088) == tiles
+    assert forms([2016], 1088, 32, 1088) == tiles and forms([292], 200, 8, 1088) == both
+    fewest = [min(d for d in range(1, 1000) if forms([2000], keys, d, 1088) == tiles) for keys in (8, 200, 600, 1000, 1088)]
+    assert fewest == sorted(fewest, reverse=True) and most - 3 <= fewest[0] <= most and fewest[-1] == 1

@@ -6,16 +6,18 @@ from __future__ import annotations
 import pytest
 import torch
 
-from test_pimezen_gpu import paged, plain_attention, run_attention
+import plain_pimezen as plain
+import schedules
+from test_pimezen_gpu import (
+    TOLERANCE, branch, compare, expected_logits, layer, load_plain, paged, plain_attention, random_ids, replay, run_attention,
+)  # fmt: skip
 
 pytestmark = pytest.mark.gpu
 
 
-def tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size, alike=False, odd=()):
-    """Requests ``(past, new)`` in one step through both forms; returns (tiles, rows, float64) of all new tokens.  ``alike``: the
+def inputs_of(requests, heads, kv_heads, window, keep_first, page_size, alike=False, odd=()):
+    """Requests ``(past, new)`` in one step: arguments of both forms, of each alone, and float64 of all new tokens.  ``alike``: the
     heads' weights differ by about a thousandth and are mixed with signs that cancel, so that only their last bits are left.  ``odd``: values ``(request, token, KV head, column, value)``."""
-    from mini_engine_b200.csrc import ops
-
     dim, dtype = 128, torch.bfloat16
     r1, r2, talk = torch.rand(heads) * 2, torch.rand(heads) + 0.1, torch.randn(heads, heads)
     if alike:
@@ -51,17 +53,26 @@ def tiles_and_rows(requests, heads, kv_heads, window, keep_first, page_size, ali
         positions=torch.tensor(positions, dtype=torch.int32, device="cuda"), heads=heads, kv_heads=kv_heads, head_dim=dim,
         value_dim=dim, scale=dim**-0.5, window=window, keep_first=keep_first, r1=cuda(r1), r2=cuda(r2), talk=cuda(talk),
     )  # fmt: skip
-    tiles, rows = (torch.full((n, heads * dim), float("nan"), dtype=dtype, device="cuda") for _ in range(2))
-    ops.mixed_attention_tiles(
-        **shared, out=tiles, cu_tokens=torch.tensor(cu, dtype=torch.int32, device="cuda"), longest=max(new for _, new in requests)
-    )
     entry = torch.cat([torch.full((new,), i, dtype=torch.int32) for i, (_, new) in enumerate(requests)])
-    ops.mixed_attention(
-        **shared, out=rows, entry_of_token=cuda(entry), scores=torch.full((n * heads * stride,), float("nan"), device="cuda"),
+    cu_tokens = torch.tensor(cu, dtype=torch.int32, device="cuda")
+    for_tiles = dict(cu_tokens=cu_tokens, longest=max(new for _, new in requests))
+    for_rows = dict(
+        entry_of_token=cuda(entry), scores=torch.full((n * heads * stride,), float("nan"), device="cuda"),
         stats=torch.empty(n * heads * 2, device="cuda"), stride=stride,
     )  # fmt: skip
+    return shared, for_tiles, for_rows, torch.cat(wants).reshape(n, -1).double()
+
+
+def tiles_and_rows(*args, **options):
+    """The step of :func:`inputs_of` through each form; (tiles, two kernels, float64)."""
+    from mini_engine_b200.csrc import ops
+
+    shared, for_tiles, for_rows, want = inputs_of(*args, **options)
+    tiles, rows = (torch.full(want.shape, float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ops.mixed_attention_tiles(**shared, **for_tiles, out=tiles)
+    ops.mixed_attention(**shared, **for_rows, out=rows)
     torch.cuda.synchronize()
-    return tiles.double().cpu(), rows.double().cpu(), torch.cat(wants).reshape(n, -1).double()
+    return tiles.double().cpu(), rows.double().cpu(), want
 
 
 @pytest.mark.parametrize("heads,kv_heads", [(32, 8), (16, 8), (16, 4)])
@@ -123,6 +134,100 @@ def test_every_form_of_the_two_kernels(heads, kv_heads, vdim, dtype):
         got = run_attention(q, k, v, r1, r2, talk, dim**-0.5, 50, 7, positions, dtype)  # the one-pass form beside the two kernels
         error = float((got - want[positions]).norm() / want[positions].norm())
         assert error < (2e-6 if dtype == torch.float32 else 2.5e-3)  # sums of 57 weighted values; the output's rounding
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(32, 8), (16, 8), (16, 4)])
+def test_each_entry_takes_one_form(heads, kv_heads):
+    """With both forms in a step an entry comes from the form that its tokens and keys choose, none from both, none from neither."""
+    from mini_engine_b200.csrc import ops
+
+    window, keep_first = 500, 20
+    eighths, most = ops.MIXED_TILES[kv_heads, heads // kv_heads]
+    edge = -(-520 * eighths // 8)  # tokens behind a full window from which on tiles are taken
+    edge = min(edge, most)
+    requests = [(0, 7), (0, 8), (600, 1), (700, edge - 1), (700, edge), (3, 1), (64, 24), (30, 40)]
+    shared, for_tiles, for_rows, _ = inputs_of(requests, heads, kv_heads, window, keep_first, 16)
+    tokens = for_rows["entry_of_token"].shape[0]
+    tiles, rows, both, fewer = (torch.full((tokens, heads * 128), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(4))
+    ops.mixed_attention_tiles(**shared, **for_tiles, out=tiles)
+    ops.mixed_attention(**shared, **for_rows, out=rows)
+    ops.mixed_attention_tiles(**shared, **for_tiles, out=both, by_entry=True)
+    ops.mixed_attention(**shared, **for_rows, out=both, besides_tiles=for_tiles["cu_tokens"])
+    ops.mixed_attention(**shared, **for_rows, out=fewer, besides_tiles=for_tiles["cu_tokens"])
+    begin = 0
+    for past, new in requests:
+        span = slice(begin, begin + new)
+        in_tiles = new >= 8 and (new >= most or 8 * new >= eighths * min(past + new, window + keep_first))
+        assert torch.equal(both[span], (tiles if in_tiles else rows)[span]), (past, new)
+        assert torch.equal(fewer[span], torch.full_like(fewer[span], 7.0) if in_tiles else rows[span]), (past, new)
+        begin += new
+
+
+# Three layers of the sizes that the tile kernel is built for, with kept keys and windows shorter than the prompts.
+CONFIG_TILES = {
+    "architecture": "Pimezen", "vocab": 96, "width": 64, "norm": {"eps": 1e-5},
+    "layers": [
+        layer(branch(16, 8, 128, 128, 0.08, 40, 6), {"heads": 2, "dim": 16, "vdim": 32, "tau": 8.0, "decay_rank": 4}, 1.0, 0.7,
+              {"kind": "dense", "ff": 96, "limit": 2.0}),
+        layer(branch(16, 4, 128, 128, 0.08, 33, 17), {"heads": 1, "dim": 32, "vdim": 64, "tau": 4.0, "decay_rank": 2}, 0.8, 1.0, None),
+        layer(branch(32, 8, 128, 128, 0.08, 70, 0), {"heads": 2, "dim": 16, "vdim": 16, "tau": 12.0, "decay_rank": 8}, 1.2, 0.5,
+              {"kind": "dense", "ff": 64, "limit": 1.0}),
+    ],
+}  # fmt: skip
+
+
+@pytest.fixture(scope="module")
+def tiles_folder(tmp_path_factory):
+    from mini_engine_b200.config import PimezenConfig
+    from mini_engine_b200.weights import write_random_model
+
+    folder = tmp_path_factory.mktemp("pimezen_tiles")
+    write_random_model(folder, PimezenConfig.from_dict(CONFIG_TILES), seed=23, dtype=torch.bfloat16, scale=12.0)
+    return folder
+
+
+@pytest.fixture
+def tile_calls(monkeypatch):
+    """Which steps take tiles, and whether by entry."""
+    from mini_engine_b200.csrc import ops
+
+    calls, run = [], ops.mixed_attention_tiles
+    monkeypatch.setattr(ops, "mixed_attention_tiles", lambda **args: (calls.append(args.get("by_entry", False)), run(**args)))
+    return calls
+
+
+@pytest.mark.parametrize("schedule", ["whole", "tail_one_by_one", "changing_portions", "mixed"])
+def test_a_model_whose_sizes_reach_the_tiles(schedule, tiles_folder, tile_calls):
+    requests = {f"r{i}": random_ids(700 + i, n, 96) for i, n in enumerate([150, 64, 17, 230, 5, 9, 90])}
+    steps = getattr(schedules, schedule)(requests)
+    got = replay(tiles_folder, "bfloat16", steps)
+    compare(got, expected_logits(tiles_folder, requests), requests, "bfloat16")
+    assert True in tile_calls if schedule == "mixed" else set(tile_calls) == {False}  # by entry beside other entries only
+
+
+def test_the_tiles_through_the_engine_with_and_without_graphs(tiles_folder, tile_calls):
+    """Lone prompts and second portions from captured steps (a dummy entry beside them), decoded entries beside a portion, slots
+    and pages used again: every token within the tolerance of the plain logits' largest."""
+    from mini_engine_b200 import EngineConfig, LLMEngine, SamplingParams
+
+    weights, config = load_plain(tiles_folder)
+    prompts = [random_ids(60 + i, n, 96) for i, n in enumerate((5, 9, 70, 130, 33, 100))]
+    for graphs in (True, False):
+        engine = LLMEngine.from_pretrained(
+            tiles_folder, EngineConfig(block_size=16, num_blocks=96, max_model_len=256, max_num_seqs=3, max_num_batched_tokens=112,
+                                       dtype=torch.bfloat16, cuda_graphs=graphs)  # fmt: skip
+        )
+        tile_calls.clear()
+        alone = [engine.generate([prompt], SamplingParams(max_tokens=6, ignore_eos=True))[0] for prompt in prompts]
+        assert (engine.stats.prompt_graph_steps > 0) == graphs
+        together = engine.generate(prompts, SamplingParams(max_tokens=12, ignore_eos=True))
+        assert True in tile_calls
+        for prompt, tokens in [*zip(prompts, alone), *zip(prompts, together)]:
+            logits = plain.forward_logits(weights, config, (prompt + tokens)[:-1])
+            slack = 2 * TOLERANCE["bfloat16"] * float(logits.abs().max())
+            for i, token in enumerate(tokens):
+                row = logits[len(prompt) - 1 + i]
+                assert float(row.max() - row[token]) <= slack, f"graphs {graphs}: token {i} of a {len(prompt)}-token prompt"
 
 
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 24), (3, 64, 128), (2, 128, 128), (1, 100, 36)])
