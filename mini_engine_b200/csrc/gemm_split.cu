@@ -1,20 +1,31 @@
 // y[t][n] = sum_k x[t][k] * w[n][k] in float32 on the 5th-generation tensor cores, for the float32 path.
 //
-// Arithmetic.  Every float32 operand is the exact sum of three bfloat16 values: its upper 16 bits, the upper 16 bits
-// of what is left, and what is left then (8 + 8 + 8 bits of the 24; truncation, so nothing overflows).  Of the nine
-// products of the pieces the six largest are formed (tcgen05.mma multiplies bfloat16 exactly and adds in float32):
+// Arithmetic.  A float32 operand of 2^-110 and more (or zero) is the exact sum of three bfloat16 values: the operand rounded to
+// nearest, what is left rounded to nearest, and what is left then (8 + 8 + 8 bits and two signs).  A piece is at most 2^-8,
+// the third 2^-17 of the operand.  Of the nine products of the pieces the six largest are formed (tcgen05.mma multiplies
+// bfloat16 exactly and adds in float32):
 //   w0 x0  |  w0 x1 + w1 x0  |  w0 x2 + w1 x1 + w2 x0
-// The three dropped ones are below 2^-24 of a product.  Weights, activations and sums are 32-bit in memory: the pieces
-// exist in shared and tensor memory only.  The tensor core truncates when it adds, so its chain is kept short: the
-// sum of w0 x0 over 64 k is taken out of tensor memory and added with rounding in registers; the small terms (2^-8 and
-// 2^-16 of the products) run over a whole segment of the reduction.  Error against float64 (norm of the difference
-// over norm of the result, normal operands) beside that of one fmaf chain per output (gemm_simt.cu):
-//   inner 64: 1.2e-7, 1.5e-7;  2,048: 1.4e-7, 8.0e-7;  4,096 in one segment: 2.2e-7, 1.2e-6;  12,288: 1.9e-7, 2.0e-6.
+// The three dropped ones are together at most 2^-24 of a product, of either sign (0.09 x 2^-24 in the mean square over all
+// mantissas; pieces that are cut instead of rounded have the operand's sign and drop up to 2^-21).  Weights, activations and
+// sums are 32-bit in memory: the pieces exist in shared and tensor memory only.  The tensor core truncates when it adds, so its
+// chain is kept short: the sum of w0 x0 over 64 k is taken out of tensor memory and added with rounding in registers; the
+// small terms (2^-8 and 2^-16 of the products) run over a whole segment of the reduction.  Error against float64 (norm of the
+// difference over norm of the result, 64 x 512 outputs) | that of one fmaf chain per output (gemm_simt.cu), by inner size:
+//                        64                  2,048               12,288
+//   normal operands      6.9e-8 | 1.5e-7     9.9e-8 | 8.1e-7     1.3e-7 | 2.0e-6
+//   one sign             9.0e-8 | 1.2e-7     9.3e-8 | 7.0e-7     9.1e-8 | 1.5e-6
+//   sums that cancel     4.6e-4 | 1.4e-3     7.3e-4 | 8.2e-3     1.1e-3 | 2.0e-2
+//   one operand in ten   3.8e-8 | 4.4e-8     7.3e-8 | 1.8e-7     9.8e-8 | 4.4e-7
+//   one operand 1e4 of the others
+//                        1.1e-7 | 1.3e-7     1.4e-7 | 8.0e-7     1.6e-7 | 2.0e-6
+//   one operand alone    2.6e-8 | 2.6e-8     2.6e-8 | 2.5e-8     2.6e-8 | 2.5e-8 (at most 8.6e-8 | 6.0e-8 of an output)
+// Smaller operands lose what falls under 2^-134, so an output below 2^-90 is formed again as below.
 //
 // An output's sum is formed in an order that depends on (outs, inner) alone: 64-wide k blocks in ascending order
 // within a segment, segments in ascending order, whether the segments of a tile run one after the other in a CTA or
 // side by side in the CTAs of a cluster.  A row's bits therefore do not depend on what else is in the batch.
-// A sum that comes out infinite or NaN (a piece of an infinity is NaN) is formed again with fmaf in ascending k.
+// A sum that comes out infinite or NaN (a piece of an infinity is NaN, and that of a value that rounds to one) is formed again
+// with fmaf in ascending k.
 //
 // Orientation and roles follow the bfloat16 product (gemm_tcgen05.cu): 128 weight rows are the A operand, the tokens
 // the narrow B operand.  Warp 0 loads raw float32 tiles with TMA, warp 1 issues the MMAs, eight converter warps make the
@@ -26,7 +37,8 @@
 // each beside the converters, 58 alone (both work on tensor memory and shared memory), the converters 1,050 to 1,100 a block,
 // and the waits between the roles come on top.  Beside the CUDA-core kernel (tokens x outs x inner): 256 x 24,576 x 4,096
 // 2,378 -> 324 us (159 TFLOP/s), 256 x 4,096 x 12,288 1,714 -> 202, 512 x 2,048 x 5,632 760 -> 107; 8 x 24,576 x 4,096
-// 807 -> 94 (4.3 TB/s of weights), 8 x 4,096 x 4,096 377 -> 25, 1 x 151,936 x 1,024 919 -> 112 (5.6 TB/s).
+// 807 -> 94 (4.3 TB/s of weights), 8 x 4,096 x 4,096 377 -> 25, 1 x 151,936 x 1,024 919 -> 112 (5.6 TB/s); these with pieces that were cut.  Rounded ones against cut ones, in turn and
+// behind a flushed L2: 256 x 24,576 x 4,096 338 -> 325, 256 x 4,096 x 12,288 215 -> 205, 8 x 24,576 x 4,096 106 -> 102, others the same.
 #include "tcgen05.cuh"
 
 constexpr int SPLIT_ROWS = 128;  // output features per CTA
@@ -76,7 +88,15 @@ struct SplitParams {
 __device__ __forceinline__ uint32_t upper_pair(float even, float odd) {  // bfloat16 pair, the even k in the low half
     return __byte_perm(__float_as_uint(even), __float_as_uint(odd), 0x7632);
 }
-__device__ __forceinline__ float below_upper(float v) { return v - __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t rounded_pair(float even, float odd) {
+    const __nv_bfloat162 pair = __floats2bfloat162_rn(even, odd);
+    return *reinterpret_cast<const uint32_t*>(&pair);
+}
+// What a pair of pieces leaves of four values.
+__device__ __forceinline__ float4 without(float4 v, uint32_t xy, uint32_t zw) {
+    return make_float4(v.x - __uint_as_float(xy << 16), v.y - __uint_as_float(xy & 0xffff0000u), v.z - __uint_as_float(zw << 16),
+                       v.w - __uint_as_float(zw & 0xffff0000u));
+}
 
 __device__ __forceinline__ float4 lds128(uint32_t address) {
     float4 v;
@@ -108,7 +128,7 @@ __device__ __forceinline__ void tcgen05_ld8(uint32_t taddr, float* v) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// The sum of one output again, for one that came out infinite or NaN.
+// The sum of one output again, for one that came out infinite, NaN or so small that pieces may have fallen under the range.
 __device__ __noinline__ float plain_sum(const float* x, const float* w, int inner) {
     float sum = 0.0f;
     for (int k = 0; k < inner; k += 4) {
@@ -120,8 +140,8 @@ __device__ __noinline__ float plain_sum(const float* x, const float* w, int inne
     }
     return sum;
 }
-__device__ __forceinline__ float finite_or_again(const SplitParams& p, int t, int w_row, float v) {
-    if (fabsf(v) <= 3.402823466e38f) return v;
+__device__ __forceinline__ float sound_or_again(const SplitParams& p, int t, int w_row, float v) {
+    if (fabsf(v) <= 3.402823466e38f && (fabsf(v) >= 0x1p-90f || v == 0.0f)) return v;
     return plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(w_row) * p.inner, p.inner);
 }
 
@@ -255,11 +275,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float4 v = lds128(from_row + (((first_chunk + c) ^ (row & 7)) << 4));
-                    const float4 r = make_float4(below_upper(v.x), below_upper(v.y), below_upper(v.z), below_upper(v.w));
-                    piece0[2 * c] = upper_pair(v.x, v.y), piece0[2 * c + 1] = upper_pair(v.z, v.w);
-                    piece1[2 * c] = upper_pair(r.x, r.y), piece1[2 * c + 1] = upper_pair(r.z, r.w);
-                    piece2[2 * c] = upper_pair(below_upper(r.x), below_upper(r.y));
-                    piece2[2 * c + 1] = upper_pair(below_upper(r.z), below_upper(r.w));
+                    piece0[2 * c] = rounded_pair(v.x, v.y), piece0[2 * c + 1] = rounded_pair(v.z, v.w);
+                    const float4 r = without(v, piece0[2 * c], piece0[2 * c + 1]);
+                    piece1[2 * c] = rounded_pair(r.x, r.y), piece1[2 * c + 1] = rounded_pair(r.z, r.w);
+                    const float4 rest = without(r, piece1[2 * c], piece1[2 * c + 1]);
+                    piece2[2 * c] = upper_pair(rest.x, rest.y), piece2[2 * c + 1] = upper_pair(rest.z, rest.w);
                 }
                 if (part == 0 && u >= 2) {  // the MMAs of two units ago have read these buffers
                     ok = __all_sync(0xffffffffu, mbar_wait(&done[u & 1], ((u >> 1) & 1) ^ 1));
@@ -286,12 +306,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 const int to_chunk = 4 * (C::UNITS == 1 ? box : u & 1) + chunk;
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
-                    sts128(x_pieces + q * NT * 128 + t * 128 + ((to_chunk ^ (t & 7)) << 4),
-                           make_uint4(upper_pair(v[0].x, v[0].y), upper_pair(v[0].z, v[0].w), upper_pair(v[1].x, v[1].y),
-                                      upper_pair(v[1].z, v[1].w)));
+                    uint32_t pair[4];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        v[h] = make_float4(below_upper(v[h].x), below_upper(v[h].y), below_upper(v[h].z), below_upper(v[h].w));
+                    for (int h = 0; h < 2; ++h) {
+                        pair[2 * h] = q < 2 ? rounded_pair(v[h].x, v[h].y) : upper_pair(v[h].x, v[h].y);
+                        pair[2 * h + 1] = q < 2 ? rounded_pair(v[h].z, v[h].w) : upper_pair(v[h].z, v[h].w);
+                        v[h] = without(v[h], pair[2 * h], pair[2 * h + 1]);
+                    }
+                    sts128(x_pieces + q * NT * 128 + t * 128 + ((to_chunk ^ (t & 7)) << 4), make_uint4(pair[0], pair[1], pair[2], pair[3]));
                 }
             }
             tcgen05_wait_st();
@@ -364,7 +386,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
             for (int c = 0; c < COLUMNS; ++c) {
                 const int t = t0 + column + c;
-                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = finite_or_again(p, t, w0 + row, result(c));
+                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = sound_or_again(p, t, w0 + row, result(c));
             }
         }
     }
@@ -389,8 +411,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                 for (int s = 1; s < MAX_SEGMENTS; ++s)
                     if (s < segments) y.x += part[s].x, y.y += part[s].y, y.z += part[s].z, y.w += part[s].w;
-                const float v[4] = {finite_or_again(p, t, w0 + row, y.x), n + 1 < p.outs ? finite_or_again(p, t, w0 + row + 1, y.y) : 0.0f,
-                                    n + 2 < p.outs ? finite_or_again(p, t, w0 + row + 2, y.z) : 0.0f, n + 3 < p.outs ? finite_or_again(p, t, w0 + row + 3, y.w) : 0.0f};
+                const float v[4] = {sound_or_again(p, t, w0 + row, y.x), n + 1 < p.outs ? sound_or_again(p, t, w0 + row + 1, y.y) : 0.0f,
+                                    n + 2 < p.outs ? sound_or_again(p, t, w0 + row + 2, y.z) : 0.0f, n + 3 < p.outs ? sound_or_again(p, t, w0 + row + 3, y.w) : 0.0f};
                 float* to = p.out + static_cast<size_t>(t) * p.outs + n;
                 if (p.vector_out) {
                     *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);

@@ -79,6 +79,63 @@ def test_infinities_and_nan_come_out_as_in_one_chain():
     assert torch.equal(torch.isnan(out), torch.isnan(want))
     odd = torch.isinf(want)
     assert odd.any() and torch.equal(out[odd], want[odd]) and not torch.isinf(out[~odd]).any()
+    small = torch.isfinite(want) & ((torch.arange(40, device="cuda")[:, None] == 8) | (torch.arange(130, device="cuda") == 11))
+    small &= want.abs() < 2.0**-90  # row 8 and column 11 hold nothing else but the rows of huge and odd values
+    assert small.sum() > 150 and torch.equal(out[small], want[small])  # their pieces fall under bfloat16's range: one chain
+
+
+def operands(kind, tokens, outs, inner):
+    normal = lambda *shape: torch.randn(*shape, device="cuda")  # noqa: E731
+    x, w = normal(tokens, inner), normal(outs, inner)
+    if kind == "one sign":
+        return x.abs(), w.abs()
+    if kind == "between 1 and 2":
+        return torch.rand_like(x) + 1, torch.rand_like(w) + 1
+    if kind == "largest dropped when cut":  # 1 + 2^-7 - 2^-23: all lower bits set
+        return torch.full_like(x, 1 + 2.0**-7 - 2.0**-23), torch.full_like(w, 1 + 2.0**-7 - 2.0**-23)
+    at = torch.randint(0, inner, (tokens,), device="cuda")
+    rows = torch.arange(tokens, device="cuda")
+    if kind == "one alone":
+        alone = torch.zeros_like(x)
+        alone[rows, at] = x[rows, at]
+        return alone, w
+    if kind == "one dominates":
+        x[rows, at] *= 1e4
+        return x, w
+    if kind == "one in ten":
+        x = torch.relu(x).square()
+        x[:, torch.rand(inner, device="cuda") < 0.9] = 0
+        return x, w
+    half = inner // 2
+    x[:, half : 2 * half] = x[:, :half]
+    w[:, half : 2 * half] = -w[:, :half] * (1 + 1e-4 * normal(outs, half))
+    return x, w  # "cancels"
+
+
+KINDS = ["one sign", "between 1 and 2", "largest dropped when cut", "one alone", "one dominates", "one in ten", "cancels"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("inner", [64, 260, 2048, 12288])
+def test_operands_that_do_not_average_out(kind, inner):
+    """No less exact than one fmaf chain whatever the operands; a tenth more for a product that stands alone, whose dropped part
+    (0.09 x 2^-24 in the mean square, 2^-24 at most) joins one rounding (2^-24 / sqrt(12) of the mean operand), and for draws."""
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(inner)
+    x, w = operands(kind, 70, 300, inner)
+    out, simt = torch.empty(70, 300, device="cuda"), torch.empty(70, 300, device="cuda")
+    tc.gemm_split(tc.SplitPlan(w), x, out)
+    ops.gemm_simt(x, w, simt)
+    assert tc.take_error() == 0
+    want = x.double() @ w.double().T
+    error = lambda y: float((y.double() - want).norm() / want.norm())  # noqa: E731
+    assert error(out) <= 1.1 * error(simt)
+    # of the products' absolute sum: what is dropped, a rounding per block of 64 and at the end, truncation within a block
+    size = x.double().abs() @ w.double().abs().T
+    assert float(((out.double() - want).abs() / size)[size > 0].max()) <= (inner / 64 + 16) * 2.0**-24
 
 
 @pytest.mark.gpu
