@@ -145,7 +145,8 @@ __device__ __forceinline__ float sound_or_again(const SplitParams& p, int t, int
     return plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(w_row) * p.inner, p.inner);
 }
 
-template <int NT>
+// WITHHELD: no tile is ever loaded and waits end after a few polls, so that a test can take the way of a kernel that gives up.
+template <int NT, bool WITHHELD = false>
 __global__ void __launch_bounds__(SPLIT_THREADS, NT <= 16 ? 2 : 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SplitParams p) {
     using C = SplitConfig<NT>;
@@ -187,18 +188,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
 
     bool ok = true;
+    auto wait = [](uint64_t* bar, uint32_t parity) { return WITHHELD ? mbar_wait(bar, parity, 512) : mbar_wait(bar, parity); };
 
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer
         if (lane == 0) {
             pdl_trigger();
             auto load_w = [&](int u) {
+                if (WITHHELD) return;
                 mbar_expect_tx(&full[u % C::STAGES], C::RAW_BYTES);
                 for (int box = 0; box < C::BOXES; ++box)
                     tma_load_2d(raw + (u % C::STAGES) * C::RAW_BYTES + box * SPLIT_ROWS * 128, &map_w, kb_begin * SPLIT_K + u * C::UNIT_K + 32 * box, w0,
                                 &full[u % C::STAGES]);
             };
             auto load_x = [&](int u) {
+                if (WITHHELD) return;
                 for (int box = 0; box < C::BOXES; ++box)
                     tma_load_2d(raw + (u % C::STAGES) * C::RAW_BYTES + C::W_BYTES + box * NT * 128, &map_x, kb_begin * SPLIT_K + u * C::UNIT_K + 32 * box, t0,
                                 &full[u % C::STAGES]);
@@ -209,25 +213,24 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             for (int u = 0; u < early; ++u) load_x(u);
             int issued = early;
             for (int u = early; u < units; ++u, ++issued) {
-                if (!mbar_wait(&empty[u % C::STAGES], ((u / C::STAGES) & 1) ^ 1)) { atomicCAS(&g_split_error, 0, (1 << 8)); break; }
+                if (!wait(&empty[u % C::STAGES], ((u / C::STAGES) & 1) ^ 1)) { atomicCAS(&g_split_error, 0, (1 << 8)); break; }
                 load_w(u);
                 load_x(u);
             }
-            // Copies in flight must land before the shared memory is released; on the normal path the converters saw them.
-            if (issued < units || g_split_error != 0) {
-                for (int u = max(issued - C::STAGES, 0); u < issued; ++u) mbar_wait(&full[u % C::STAGES], (u / C::STAGES) & 1);
-            }
+            // Copies in flight must land before the shared memory is released, also when another role has given up.
+            for (int u = max(issued - C::STAGES, 0); u < issued; ++u) wait(&full[u % C::STAGES], (u / C::STAGES) & 1);
         }
     } else if (warp == 1) {
         // --------------------------------------------------------------- MMA issuer
         if (lane == 0) {
             constexpr uint32_t one = make_idesc(NT), two = make_idesc(2 * NT);
             const uint32_t small = tmem_base + C::SMALL_COLUMN;
-            auto wait_taken = [&](int block) { return block < 0 || mbar_wait(&taken[block % C::MAINS], (block / C::MAINS) & 1); };
+            int sent = 0;  // units whose MMAs were issued
+            auto wait_taken = [&](int block) { return block < 0 || wait(&taken[block % C::MAINS], (block / C::MAINS) & 1); };
             for (int u = 0, at = 0; u < units; ++u) {
                 const int half = u % C::UNITS, block = u / C::UNITS;
                 const bool fresh = half == 0 && at == 0;  // a segment starts its own sums: the last one's must be out
-                if (!mbar_wait(&ready[u & 1], (u >> 1) & 1) || (fresh && !wait_taken(block - 1))) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
+                if (!wait(&ready[u & 1], (u >> 1) & 1) || (fresh && !wait_taken(block - 1))) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
                 tcgen05_fence_after();
                 const uint32_t a = tmem_base + C::A_COLUMN + (u & 1) * C::A_COLUMNS, main_sum = tmem_base + block % C::MAINS * NT;
                 const uint64_t b = smem_desc_sw128(smem_u32(pieces + (C::UNITS == 1 ? (u & 1) * C::PIECES_BYTES : 0))) + 4 * half;
@@ -252,10 +255,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     tcgen05_mma_bf16_ts(small, w0_piece, x1, two, 1);
                     tcgen05_mma_bf16_ts(small, w0_piece + 8, x1 + 2, two, 1);
                 }
-                if (!go) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
                 tcgen05_commit(&done[u & 1]);
+                ++sent;
+                if (!go) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
                 if (half == C::UNITS - 1 && ++at == p.per_segment) at = 0;
             }
+            // MMAs in flight read shared memory and write tensor memory: they end before either is given back.
+            for (int u = max(sent - 2, 0); u < sent; ++u) wait(&done[u & 1], (u >> 1) & 1);
         }
     } else if (warp < 2 + CONVERTERS / 32) {
         // ----------------------------------------------------------------- converters
@@ -263,7 +269,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int worker = threadIdx.x - 64, run = worker >> 7;
         const int row = quarter * 32 + lane;
         for (int u = 0; u < units; ++u) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&full[u % C::STAGES], (u / C::STAGES) & 1));
+            ok = __all_sync(0xffffffffu, wait(&full[u % C::STAGES], (u / C::STAGES) & 1));
             if (!ok) break;
             const uint32_t w_tile = smem_u32(raw + (u % C::STAGES) * C::RAW_BYTES), x_tile = w_tile + C::W_BYTES;
             const uint32_t from_row = w_tile + (C::BOXES == 2 ? run * SPLIT_ROWS * 128 : 0) + row * 128;
@@ -282,7 +288,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     piece2[2 * c] = upper_pair(rest.x, rest.y), piece2[2 * c + 1] = upper_pair(rest.z, rest.w);
                 }
                 if (part == 0 && u >= 2) {  // the MMAs of two units ago have read these buffers
-                    ok = __all_sync(0xffffffffu, mbar_wait(&done[u & 1], ((u >> 1) & 1) ^ 1));
+                    ok = __all_sync(0xffffffffu, wait(&done[u & 1], ((u >> 1) & 1) ^ 1));
                     if (!ok) break;
                     tcgen05_fence_after();
                 }
@@ -340,7 +346,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         for (int c = 0; c < COLUMNS; ++c) sum[c] = 0.0f;
         for (int i = 0; i < blocks; ++i) {
             const int u = i * C::UNITS + C::UNITS - 1;  // the block's last unit
-            ok = __all_sync(0xffffffffu, mbar_wait(&done[u & 1], (u >> 1) & 1));
+            ok = __all_sync(0xffffffffu, wait(&done[u & 1], (u >> 1) & 1));
             if (!ok) break;
             tcgen05_fence_after();
 #pragma unroll
@@ -463,10 +469,10 @@ ME_EXPORT int me_make_tensor_map_f32(void* out, const void* base, unsigned long 
     return 0;
 }
 
-template <int NT>
+template <int NT, bool WITHHELD = false>
 static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, const SplitParams& p, int segments, cudaStream_t stream) {
     using C = SplitConfig<NT>;
-    auto kernel = gemm_split_kernel<NT>;
+    auto kernel = gemm_split_kernel<NT, WITHHELD>;
     static SharedMemoryOptIn opt_in;
     if (const int e = opt_in(kernel, C::SMEM_BYTES)) return e;
     const dim3 grid((p.tokens + NT - 1) / NT, (p.outs + SPLIT_ROWS - 1) / SPLIT_ROWS, p.clustered ? segments : 1);
@@ -493,9 +499,11 @@ static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, cons
 }
 
 // out[t][n] = sum_k x[t][k] * w[n][k]; `segments` ranges of k blocks whose sums are added in ascending order, in one
-// CTA or (`clustered`) in a cluster's CTAs.  With `group_of_block` a grouped product: `tile` rows of x to a group.  `map_x` has boxes of `tile` (16 or 64) rows.
+// CTA or (`clustered`) in a cluster's CTAs.  With `group_of_block` a grouped product: `tile` rows of x to a group.  `map_x` has boxes
+// of `tile` rows: 16, 64, or 128 where a CTA runs one segment (one in all, or `clustered`).  `withheld`: every wait runs out (for tests).
 ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x, const float* w, float* out, int tokens, int outs,
-                            int inner, int tile, int segments, int clustered, const int* group_of_block, int group_rows, cudaStream_t stream) {
+                            int inner, int tile, int segments, int clustered, const int* group_of_block, int group_rows, int withheld,
+                            cudaStream_t stream) {
     if (tokens <= 0 || outs <= 0) return 0;
     if (group_of_block != nullptr && (group_rows < outs || tokens % tile)) return ME_ERR_ARGUMENT;
     if (inner <= 0 || inner % 4 != 0 || segments < 1 || segments > MAX_SEGMENTS) return ME_ERR_ARGUMENT;
@@ -511,6 +519,7 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     alignas(64) CUtensorMap w_map, x_map;
     memcpy(&w_map, map_w, sizeof(w_map));
     memcpy(&x_map, map_x, sizeof(x_map));
+    if (withheld) return tile == 16 ? launch_split<16, true>(w_map, x_map, p, segments, stream) : ME_ERR_ARGUMENT;
     if (tile == 16) return launch_split<16>(w_map, x_map, p, segments, stream);
     if (tile == 64) return launch_split<64>(w_map, x_map, p, segments, stream);
     if (tile == 128 && (p.clustered || segments == 1)) return launch_split<128>(w_map, x_map, p, segments, stream);

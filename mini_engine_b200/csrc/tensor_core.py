@@ -258,7 +258,7 @@ def _split_library():
         lib = load_library("gemm_split")
         lib.me_make_tensor_map_f32.argtypes = [c_void_p, c_void_p, c_ulonglong, c_ulonglong, c_uint]
         lib.me_make_tensor_map_f32.restype = c_int
-        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_int, c_void_p]
+        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_int, c_int, c_void_p]
         lib.me_gemm_split.restype = c_int
         lib.me_gemm_split_take_error.argtypes = [ctypes.POINTER(c_int)]
         lib.me_gemm_split_take_error.restype = c_int
@@ -355,7 +355,7 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
     tile, side_by_side = split_form(tokens, plan.rows, plan.inner, plan.segments) if form is None else form
     code = _split_library().me_gemm_split(
         plan.map, _split_activation_map(x, tile), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,
-        plan.segments, 1 if side_by_side else 0, None, 0, _ops_stream(),
+        plan.segments, 1 if side_by_side else 0, None, 0, 0, _ops_stream(),
     )  # fmt: skip
     _count_launch()
     if code != 0:
@@ -382,7 +382,7 @@ def gemm_split_grouped(
         side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad)[1]
     code = _split_library().me_gemm_split(
         plan.map, _split_activation_map(x, pad), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, plan.inner, pad,
-        plan.segments, 1 if side_by_side else 0, group_of_block.data_ptr(), outs, _ops_stream(),
+        plan.segments, 1 if side_by_side else 0, group_of_block.data_ptr(), outs, 0, _ops_stream(),
     )  # fmt: skip
     _count_launch()
     if code != 0:
@@ -435,6 +435,20 @@ def wait_probe(polls: int = 4096) -> bool:
     if code != 0:
         raise RuntimeError(f"the wait probe failed to launch (code {code})")
     return bool(returned.item())
+
+
+def split_wait_probe(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side: bool) -> None:
+    """The float32 product with every tile withheld: all waits of its roles run out after a few polls, the kernel records that,
+    gives its tensor memory back and returns without a result.  Exists so that the give-up path can be tested."""
+    if x.shape[1] != plan.inner or tuple(out.shape) != (x.shape[0], plan.rows) or not (x.is_contiguous() and out.is_contiguous()):
+        raise RuntimeError("the probe takes the arguments of a product")
+    code = _split_library().me_gemm_split(
+        plan.map, _split_activation_map(x, 16), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), x.shape[0], plan.rows, plan.inner, 16,
+        plan.segments, 1 if side_by_side else 0, None, 0, 1, _ops_stream(),
+    )  # fmt: skip
+    _count_launch()
+    if code != 0:
+        raise RuntimeError(f"the wait probe failed to launch (code {code})")
 
 
 def take_error() -> int:

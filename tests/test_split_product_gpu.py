@@ -201,3 +201,29 @@ def test_grouped_product_gives_the_bits_of_each_groups_own(tokens, units, top, o
                     assert (row < 0) == (u >= units)
                     if row >= 0:
                         assert torch.equal(out[row], alone[u][t])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("side_by_side", [False, True])
+def test_a_wait_that_runs_out_is_reported_and_leaves_the_device_usable(side_by_side):
+    """The product with its tiles withheld: every role gives up, the CTAs of a cluster meet all the same, the error reaches the host
+    once, and tensor memory is free for the next product (512 columns an SM would be gone after two leaks)."""
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(6)
+    x, w = torch.randn(20, 1100, device="cuda"), torch.randn(300, 1100, device="cuda")
+    plan = tc.SplitPlan(w)
+    assert plan.segments > 1 and tc.take_error() == 0
+    out = torch.full((20, 300), 7.0, device="cuda")
+    for _ in range(8):
+        tc.split_wait_probe(plan, x, out, side_by_side)
+    torch.cuda.synchronize()
+    assert bool((out == 7.0).all())  # nothing is written
+    with pytest.raises(ops.KernelError, match="limit of a wait"):
+        ops.raise_on_device_error()
+    assert tc.take_error() == 0
+    for form in [(16, side_by_side), (128, True)]:
+        tc.gemm_split(plan, x, out, form)
+        assert float((out.double() - x.double() @ w.double().T).abs().max()) < 1e-3
+    assert tc.take_error() == 0
