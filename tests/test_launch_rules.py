@@ -116,3 +116,23 @@ def test_graph_buckets_cover_every_batch_up_to_the_cap(max_batch):
     for batch in range(1, max_batch + 1):
         bucket = next(b for b in buckets if b >= batch)
         assert bucket - batch < max(16, bucket // 2 + 1)
+
+
+@pytest.mark.parametrize("enabled", [True, False])
+def test_collection_stays_off_until_the_last_capture_ends(enabled):
+    """Two engines capture at once: the first to end must not start the collector under the other."""
+    import gc
+
+    from mini_engine_b200.engine.graphs import _NoCollection
+
+    was = gc.isenabled()
+    try:
+        gc.enable() if enabled else gc.disable()
+        first, second = _NoCollection(), _NoCollection()
+        first.__enter__(), second.__enter__()
+        first.__exit__(None, None, None)
+        assert not gc.isenabled()
+        second.__exit__(None, None, None)
+        assert gc.isenabled() == enabled
+    finally:
+        gc.enable() if was else gc.disable()
