@@ -898,6 +898,12 @@ def mixed_attention_tiles_supports(dtype: torch.dtype, heads: int, kv_heads: int
     return dtype == torch.bfloat16 and head_dim == value_dim == 128 and heads % kv_heads == 0 and (kv_heads, heads // kv_heads) in MIXED_TILES
 
 
+def mixed_attention_tiles_take(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether the tile kernel takes these buffers: it copies rows in pieces of 16 bytes and reads and writes in pairs.  The other
+    forms take any."""
+    return all(t.data_ptr() % 16 == 0 for t in (k_pages, v_pages)) and all(t.data_ptr() % 4 == 0 for t in (q, out))
+
+
 def mixed_attention_forms(
     kv_heads: int, heads: int, *, tokens: int, entries: int, decoded: int, least: int, longest: int, portion_keys: int, keys: int
 ) -> tuple[bool, bool]:
@@ -983,7 +989,8 @@ def gla_scan(
     scratch of ``T * heads * 3 * dim`` values (q, k and decay of every token, made by a first kernel).  ``chunk_min`` > 0:
     entries of at least that many tokens run in chunks of ``STATE_CHUNK`` tokens (:func:`state_chunks_support` says for
     which sizes), with ``records [chunks, heads * state_record_floats("gated", dim)]`` as scratch for all of their chunks and
-    ``prepared`` of ``T * heads * (3 * dim + vdim)`` values; the other entries walk token by token."""
+    ``prepared`` of ``T * heads * (3 * dim + vdim)`` values; the other entries walk token by token, and all do when a buffer that
+    the chunks read and write in pieces of 16 bytes starts off them."""
     _need(proj, torch.float32, "proj"), _need(a2t, torch.float32, "a2t"), _need(a2_bias, torch.float32, "a2_bias")
     _need(state, torch.float32, "state"), _need(out, torch.float32, "out"), _need(prepared, torch.float32, "prepared")
     rank, tokens = a2t.shape[0], proj.shape[1]
@@ -996,6 +1003,8 @@ def gla_scan(
         _need(records, torch.float32, "records")
         if not state_chunks_support(dim, vdim, slot_floats) or records.dim() != 2 or records.shape[1] != heads * state_record_floats("gated", dim):
             raise KernelError("gla_scan: the chunks' records or the head sizes do not fit")
+        if any(t.data_ptr() % 16 for t in (state, out, prepared, records)):
+            chunk_min = 0
     fn = _fn(
         "linear_attention",
         "me_gla_scan",

@@ -334,6 +334,7 @@ class GroupedQueryAttention(Mixer):
             capacity = max(tokens, ctx.workspace.max_tokens)
             two_kernels = self.two_kernel_mixing and capacity * self.heads * stride * 4 <= 2 << 30
             tiles, by_entry = self.two_kernel_mixing and self.mixing_tiles and ctx.max_query_len >= ops.MIXED_TILES_MIN_TOKENS, False
+            tiles = tiles and ops.mixed_attention_tiles_take(q, cache.k, cache.v, out)
             if tiles and two_kernels:
                 # Which forms run follows from the step's sizes on the host, which entries take which from their own sizes on
                 # the device (a captured step stands for others).

@@ -191,3 +191,17 @@ def test_which_forms_of_the_mixed_heads_a_step_takes(kv_heads, heads):
     assert forms([2016], 1088, 32, 1088) == tiles and forms([292], 200, 8, 1088) == both
     fewest = [min(d for d in range(1, 1000) if forms([2000], keys, d, 1088) == tiles) for keys in (8, 200, 600, 1000, 1088)]
     assert fewest == sorted(fewest, reverse=True) and most - 3 <= fewest[0] <= most and fewest[-1] == 1
+
+
+@pytest.mark.parametrize("off", [(0, 0, 0, 0), (2, 0, 0, 6), (1, 0, 0, 0), (0, 4, 0, 0), (0, 0, 1, 0), (0, 0, 0, 3), (8, 8, 16, 8)])
+def test_buffers_that_the_tiles_take(off):
+    """Pages on 16 bytes, queries and outputs on 4; everything else goes to the forms that take any start."""
+    import torch
+
+    from mini_engine_b200.csrc import ops
+
+    base = torch.empty(64, dtype=torch.bfloat16)
+    assert base.data_ptr() % 16 == 0
+    q, k, v, out = (base[n:] for n in off)
+    taken = off[0] % 2 == 0 and off[1] % 8 == 0 and off[2] % 8 == 0 and off[3] % 2 == 0
+    assert ops.mixed_attention_tiles_take(q, k, v, out) == taken

@@ -250,8 +250,9 @@ def test_gated_recurrence_in_chunks(heads, dim, vdim, counts, starts):
     slots, fresh = list(range(len(counts))), [1 if start == 0 else 0 for start in starts]
     first = torch.randn(len(counts) + 1, heads, dim, vdim)
     results = []
-    for chunk_min in (0, 33):
-        state, out = first.clone().cuda(), torch.full((tokens, heads * vdim), float("nan"), device="cuda")
+    for chunk_min, off in ((0, 0), (33, 0), (33, 1)):  # `off` floats: states that do not start on 16 bytes walk
+        state, out = torch.empty(first.numel() + off, device="cuda")[off:].view(first.shape), torch.full((tokens, heads * vdim), float("nan"), device="cuda")
+        state.copy_(first)
         prepared = torch.full((tokens * heads * (3 * dim + vdim),), float("nan"), device="cuda")
         chunks = tokens // ops.STATE_CHUNK + len(counts)
         records = torch.full((chunks, heads * ops.state_record_floats("gated", dim)), float("nan"), device="cuda")
@@ -275,7 +276,8 @@ def test_gated_recurrence_in_chunks(heads, dim, vdim, counts, starts):
             t += 1
         states[slot] = s
     want = torch.stack(want)
-    (walk, walk_state), (chunked, chunk_state) = results
+    (walk, walk_state), (chunked, chunk_state), (walked, walked_state) = results
+    assert torch.equal(walked, walk) and torch.equal(walked_state, walk_state)
     for got, exact in ((walk, want), (chunked, want), (walk_state, states), (chunk_state, states)):
         assert float((got - exact).norm() / exact.norm()) < 2e-6  # sums of float32, up to 200 terms a state element
     # entries below the minimum walk in both
