@@ -168,9 +168,12 @@ __device__ __forceinline__ void column_product(const float* in, int in_head, con
 }
 
 // A thread has one output column of the block's eight tokens and the block all columns of a head; NARROW (few tokens): a block
-// has 32 columns (blockIdx.z), a warp two of the tokens, so that a step of a few tokens runs on many SMs.  The bits are the same.
-template <typename InT, typename T, bool NARROW>
-__global__ void __launch_bounds__(128) head_product_kernel(HeadProductArgs a) {
+// has 32 columns (blockIdx.z), a warp two of the tokens, so that a step of a few tokens runs on many SMs.  MANY: registers are
+// cut so that ten blocks fit an SM instead of seven.  The bits are the same.
+constexpr int HP_RESIDENT = 7, HP_MANY_RESIDENT = 10;
+
+template <typename InT, typename T, bool NARROW, bool MANY>
+__global__ void __launch_bounds__(128, MANY ? HP_MANY_RESIDENT : 0) head_product_kernel(HeadProductArgs a) {
     extern __shared__ __align__(16) float staged[];  // [HP_TOKENS][inner + tail]
     const int head = blockIdx.y, first = blockIdx.x * HP_TOKENS;
     const int count = min(HP_TOKENS, a.tokens - first);
@@ -232,11 +235,20 @@ ME_EXPORT int me_head_product(const void* in, int in_type, int splits, long long
     dim3 grid((tokens + HP_TOKENS - 1) / HP_TOKENS, heads);
     // Blocks of a whole head fill the GPU from about two to an SM on.  Eight tokens, 16 heads of 512 x 128 and 128 x 512:
     // 135 us for either with whole heads, 43 us in blocks of 32 columns.
-    const bool narrow = static_cast<long long>(grid.x) * heads < 2 * 148 && outs > 32;
+    const long long blocks = static_cast<long long>(grid.x) * heads;
+    const bool narrow = blocks < 2 * 148 && outs > 32;
     if (narrow) grid.z = (outs + 31) / 32;
+    // Seven blocks to an SM keep the weights that are fetched together in registers, ten do not but may take fewer rounds.  32 heads
+    // of 64 x 64 beside 64, 300 tokens (1,216 blocks): 22.5 us with seven, 18.4 with ten; 2,048 tokens: 82.7, 72.6; 16 heads of 512
+    // x 128, 300 tokens (608 blocks): 61, 68.
+    const int fit = static_cast<int>(227 * 1024 / (smem + 1024));
+    auto rounds = [&](int resident) { return (blocks + 148 * std::min(resident, fit) - 1) / (148 * std::min(resident, fit)); };
+    const bool many = !narrow && rounds(HP_MANY_RESIDENT) < rounds(HP_RESIDENT);
 #define ME_LAUNCH_HEAD_PRODUCT(IN, T)                                                                              \
     {                                                                                                              \
-        auto kernel = narrow ? head_product_kernel<IN, T, true> : head_product_kernel<IN, T, false>;               \
+        auto kernel = narrow ? head_product_kernel<IN, T, true, false>                                             \
+                      : many ? head_product_kernel<IN, T, false, true>                                             \
+                             : head_product_kernel<IN, T, false, false>;                                           \
         if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         return launch_kernel(kernel, grid, 128, smem, stream, a);                                                  \
     }
