@@ -193,18 +193,20 @@ __global__ void __launch_bounds__(32) gla_scan_kernel(ScanArgs a) {
     auto stage_tile = [&](int chunk, int buffer) {  // q, k, decay of tokens chunk .. chunk + count
         const int count = min(SCAN_CHUNK, end - chunk);
         float* tile = tiles + buffer * TILE;
+        const float* from = a.prepared + (static_cast<size_t>(chunk) * a.heads + head) * row;
+        const int step = a.heads * row;  // floats between two tokens; a tile's offsets fit 32 bits
         if (vector) {
             const int quads = 3 * dim / 4;
             for (int i = lane; i < count * quads; i += 32) {
                 const int t = i / quads, j = (i % quads) * 4;
                 const int which = j / dim, d = j % dim;
-                copy_async_16(tile + (t * 3 + which) * DIMP + d,
-                              a.prepared + (static_cast<size_t>(chunk + t) * a.heads + head) * row + j);
+                copy_async_16(tile + (t * 3 + which) * DIMP + d, from + t * step + j);
             }
         } else {
+#pragma unroll 4
             for (int i = lane; i < count * 3 * dim; i += 32) {
                 const int t = i / (3 * dim), j = i % (3 * dim);
-                tile[(t * 3 + j / dim) * DIMP + j % dim] = a.prepared[(static_cast<size_t>(chunk + t) * a.heads + head) * row + j];
+                tile[(t * 3 + j / dim) * DIMP + j % dim] = from[t * step + j];
             }
         }
         copy_async_commit();
