@@ -234,6 +234,25 @@ __device__ __forceinline__ void copy_async_16(float* shared_dst, const float* gl
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory"); }
 
+// Four columns of a row of the reading product again, for a row that came out infinite or NaN: a later token's value has the
+// coefficient zero, which an infinity or NaN among the values carries to every row, so those terms are left out.  The order of
+// the sums is the walk's.
+template <int DIM, int ROWS>
+__device__ __noinline__ float4 sums_without_later_values(const float* stage, const float* held, const float* v, int row, int t, int column) {
+    constexpr int TERMS = (DIM + CHUNK) / WALK_WARPS;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int part = 0; part < WALK_WARPS; ++part) {
+        float4 share = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int term = part * TERMS; term < (part + 1) * TERMS && term <= DIM + t; ++term) {
+            const float w = stage[term * ROWS + row];
+            const float4 x = *reinterpret_cast<const float4*>((term < DIM ? held + term * COLUMNS : v + (term - DIM) * COLUMNS) + column);
+            share = make_float4(fmaf(w, x.x, share.x), fmaf(w, x.y, share.y), fmaf(w, x.z, share.z), fmaf(w, x.w, share.w));
+        }
+        sum = part == 0 ? share : make_float4(sum.x + share.x, sum.y + share.y, sum.z + share.z, sum.w + share.w);
+    }
+    return sum;
+}
+
 // One block of eight warps per (entry, head, 32 value columns).  A thread of the first four warps owns a tile of 4 channels x 4
 // columns of the state (two of them at 128 channels) in registers, and shares it with the block through shared memory.  What
 // the two products of a chunk read from shared memory is what they cost, so that a thread takes tiles as large as its registers
@@ -351,6 +370,10 @@ __global__ void __launch_bounds__(WALK_THREADS) chunk_walk_kernel(ChunkArgs a) {
             for (int part = 1; part < WALK_WARPS; ++part) {
                 const float4 x = *reinterpret_cast<const float4*>(partial + (part * ROWS + row) * COLUMNS + 4 * strip);
                 z.x += x.x, z.y += x.y, z.z += x.z, z.w += x.w;
+            }
+            if constexpr (RULE == RULE_GATED) {
+                if (!(fabsf(z.x) < INFINITY && fabsf(z.y) < INFINITY && fabsf(z.z) < INFINITY && fabsf(z.w) < INFINITY))
+                    z = sums_without_later_values<DIM, ROWS>(stage, held, v, row, t, 4 * strip);
             }
             if (REMOVES && row < CHUNK) {
                 *reinterpret_cast<float4*>(minus_y + row * COLUMNS + 4 * strip) = make_float4(-z.x, -z.y, -z.z, -z.w);

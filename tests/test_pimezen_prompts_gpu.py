@@ -230,6 +230,36 @@ def test_the_tiles_through_the_engine_with_and_without_graphs(tiles_folder, tile
                 assert float(row.max() - row[token]) <= slack, f"graphs {graphs}: token {i} of a {len(prompt)}-token prompt"
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("token", [32, 40, 63])
+def test_a_value_that_is_not_finite_leaves_earlier_tokens_of_its_chunk_alone(token, value):
+    """Its own column from that token on is spoilt, as token by token, and nothing else."""
+    from test_pimezen_gpu import FakeContext
+
+    from mini_engine_b200.csrc import ops
+
+    torch.manual_seed(token)
+    heads, dim, vdim, tokens, rank = 2, 64, 40, 70, 4
+    columns = {"q": 0, "k": heads * dim, "v": 2 * heads * dim, "g": 2 * heads * dim + heads * vdim, "a": 2 * heads * (dim + vdim)}
+    proj = torch.randn(1, tokens, columns["a"] + rank, device="cuda")
+    proj[0, token, columns["v"] + vdim + 7] = value  # head 1, column 7
+    a2t, bias = torch.randn(rank, heads * dim, device="cuda"), torch.randn(heads * dim, device="cuda")
+    outs = []
+    for chunk_min in (0, 33):
+        state, out = torch.zeros(2, heads, dim, vdim, device="cuda"), torch.full((tokens, heads * vdim), 7.0, device="cuda")
+        ops.gla_scan(
+            proj=proj, columns=columns, a2t=a2t, a2_bias=bias, ctx=FakeContext([tokens], [0], [1]), state=state, out=out,
+            prepared=torch.empty(tokens * heads * (3 * dim + vdim), device="cuda"), q_scale=1.0, tau=6.0, heads=heads, dim=dim, vdim=vdim,
+            chunk_min=chunk_min, records=torch.empty(6, heads * ops.state_record_floats("gated", dim), device="cuda") if chunk_min else None,
+        )  # fmt: skip
+        outs.append((out.cpu().double(), state[0].cpu().double()))
+    (walk, walk_state), (chunks, chunk_state) = outs
+    assert not walk[token:, vdim + 7].isfinite().any()
+    assert torch.equal(chunks.isfinite(), walk.isfinite()) and torch.equal(chunk_state.isfinite(), walk_state.isfinite())
+    there = walk.isfinite()
+    assert float((chunks - walk)[there].norm() / walk[there].norm()) < 2e-6
+
+
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 8, 24), (3, 64, 128), (2, 128, 128), (1, 100, 36)])
 @pytest.mark.parametrize("counts,starts", [([33], [0]), ([48, 5], [7, 0]), ([1, 200, 34], [3, 0, 50])])
 def test_gated_recurrence_in_chunks(heads, dim, vdim, counts, starts):
