@@ -698,9 +698,10 @@ ME_EXPORT int me_mixed_attention(const void* q, const void* k_pages, const void*
 // that query.  So a block whose output holds one walks again: keys with such values are then taken out of the product and
 // added to the queries that see them alone.
 //
-// Bound by the instructions a warp issues around its products (exponentials, masks, the split of the weights), with
-// one block to an SM; see the figures at launch_mixed_tiles.  A tile of eight tokens, since the output of four heads and
-// 16 tokens would take every register of a warp.
+// Bound by the latency of a warp's own chains: registers and shared memory leave one block and two warps a scheduler, of which
+// one issues every 4.6 cycles (1.9 of them the fixed latency of the instruction before); the tensor pipe is active 30 % of the
+// time (profiles/mixed_attention_tiles_kernel_prefill_2048.md); figures at launch_mixed_tiles.  A tile of eight tokens, since the
+// output of four heads and 16 tokens would take every register of a warp.
 constexpr int BIAS_SPAN = TILE_Q + TILE_K;  // distances within a tile, one spare
 constexpr int TERMS = 3;                    // bfloat16 terms of a float32 number
 

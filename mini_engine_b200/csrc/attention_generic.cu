@@ -146,8 +146,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) paged_attention_generic_kerne
 // R x 32 scores (a thread 2 rows x 4 keys, or 1 x 2), a warp takes whole rows for the softmax, and a thread keeps one quad
 // of value elements of R * QP / 256 rows.  A tile that some row sees in part marks the weights of unseen keys, and
 // their values are left out (they may be anything); a tile that all rows see whole is not looked at twice.
-// Bound by the multiply-adds at R = 64 (256 FMA of a tile's 32 keys and a head of 128 per row and lane), by the latency of
-// a tile's chains at R = 16; see the figures at launch_rows.
+// Bound by latency: eight warps to an SM for steps of this size (512 tokens are 128 blocks), each of which issues every 4.8 cycles
+// at R = 64 and every 6 at R = 16 and waits for shared memory most (1.5 and 2.2 cycles; profiles/paged_attention_rows_kernel.md);
+// figures at launch_rows.
 constexpr int ROW_THREADS = 256;
 constexpr uint32_t UNSEEN = 0x80000000u;  // the weight -0: a key that the row does not see
 

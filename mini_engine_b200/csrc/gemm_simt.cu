@@ -1,10 +1,11 @@
 // y[t][n] = sum_k x[t][k] * w[n][k] on CUDA cores, for any sizes.
 //
-// This is the true 32-bit matrix product of the float32 path (no tensor cores, no TF32) and
-// the fallback of the bfloat16 path for shapes that TMA cannot address.  Every output element
-// is one accumulator updated with fmaf for k = 0, 1, 2, ... in ascending order, so a row's
-// result is bit-identical whatever other rows share the launch: splitting a prompt into
-// portions or batching it with other requests cannot change a single bit.
+// The product of the shapes that the tensor-core kernels do not take: bfloat16 widths that TMA
+// cannot address, and in float32 (whose other products are gemm_split.cu's) inner sizes under 64
+// or no multiple of 4, and weights or activations that do not start on 16 bytes.  Every output
+// element is one accumulator updated with fmaf for k = 0, 1, 2, ... in ascending order, so a row's
+// result is bit-identical whatever other rows share the launch: splitting a prompt into portions
+// or batching it with other requests cannot change a single bit.
 //
 // The weight keeps the checkpoint's [out, in] layout (torch Linear,
 // src/mini_engine/model.py:97-100 of YuvGev00/mini-engine).

@@ -39,7 +39,7 @@ struct PrepArgs {
     int q_col, k_col, a_col;  // first column of q [heads*dim], k [heads*dim], low-rank sums [rank]
     const float* a2t;         // [rank][heads*dim]
     const float* a2_bias;     // [heads*dim]
-    float* prepared;          // [tokens][heads][3][dim]
+    float* prepared;          // [tokens][heads][3][dim], or rows of `row` floats (below)
     float q_scale, inv_tau;
     int tokens, heads, dim, rank;
     int row = 0, v_col = 0, vdim = 0;  // row > 0: prepared[token][head] is `row` floats, q, k, decay and the vdim value sums

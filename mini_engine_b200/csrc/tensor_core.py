@@ -246,8 +246,8 @@ def gemm_swiglu(
 SPLIT_TILES = {16: 1.0, 64: 1.0, 128: 1.44}
 SPLIT_START, SPLIT_EXCHANGE = 4.0, 0.8
 SPLIT_MIN_K_BLOCKS = 4  # of a segment
-# Shorter reductions stay on CUDA cores: a chain of fmaf over so few terms is as exact as the short chain of the tensor
-# core (relative error at 64: 1.5e-7 against 1.2e-7; at 4: 4e-8 against 7e-8), and nothing is to be gained.
+# Shorter reductions stay on CUDA cores: a chain of fmaf over so few terms is about as exact as the short chain of the tensor
+# core (relative error of normal operands at 64: 1.5e-7 against 0.7e-7), and nothing is to be gained.
 SPLIT_MIN_INNER = 64
 _split_lib = None
 
@@ -268,7 +268,8 @@ def _split_library():
 
 def split_supports(weight: torch.Tensor) -> bool:
     """TMA wants a 16-byte aligned start and row pitch: ``inner`` a multiple of 4 float32 values.  A property of the weight
-    alone: every step of a model takes the same kernel."""
+    alone: every step of a model takes the same kernel (but for activations that do not start on 16 bytes, which
+    :class:`parts.linear.Linear` sends to the CUDA cores; the workspace's always do)."""
     return (
         weight.dtype == torch.float32 and weight.is_cuda and weight.is_contiguous()
         and weight.shape[1] % 4 == 0 and weight.shape[1] >= SPLIT_MIN_INNER and weight.data_ptr() % 16 == 0

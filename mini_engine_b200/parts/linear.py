@@ -9,11 +9,11 @@ YuvGev00/mini-engine) and pick the kernel:
   2,048-token prompt and a single decoded token; for few tokens the reduction axis is
   split over several CTAs and the result comes back as ``S`` partial sums that the consumer
   adds in a fixed order.
-* float32 with ``in`` a multiple of 4: the tensor-core kernel on three bfloat16 pieces of each
-  operand (their exact sum), with the sums in an order that depends on the weight's shape alone,
-  so a row's result never depends on which other rows are in the batch.
-* shapes that TMA cannot address: a CUDA-core kernel that adds the products of one output
-  element in ascending ``k`` with one accumulator.
+* float32 with ``in`` a multiple of 4 and at least 64: the tensor-core kernel on three bfloat16
+  pieces of each operand (their sum down to 2^-134), with the sums in an order that depends on
+  the weight's shape alone, so a row's result never depends on which other rows are in the batch.
+* other shapes, and tensors that do not start on 16 bytes: a CUDA-core kernel that adds the
+  products of one output element in ascending ``k`` with one accumulator.
 """
 
 from __future__ import annotations
