@@ -54,9 +54,14 @@ class Workspace:
 
     def growing(self, name: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """A buffer of exactly ``shape`` that grows on demand instead of being sized for the
-        token capacity (logits: ``[rows, vocab]`` is large and ``rows`` is usually small)."""
-        flat = self._flat(name, math.prod(shape), dtype)
-        return flat[: math.prod(shape)].view(shape)
+        token capacity (logits: ``[rows, vocab]`` is large and ``rows`` is usually small).  It grows
+        by half at least, so that steps of ever longer prompts do not leave one buffer behind for
+        every length: all that it has ever replaced is less than twice what it holds."""
+        elements = math.prod(shape)
+        held = self._buffers.get((name, dtype))
+        if held is not None and held.numel() < elements:
+            self._flat(name, max(elements, held.numel() + held.numel() // 2), dtype)
+        return self._flat(name, elements, dtype)[:elements].view(shape)
 
     def zeroed(self, name: str, count: int) -> torch.Tensor:
         """``count`` int32 values that are zero when first handed out.  Kernels that use them

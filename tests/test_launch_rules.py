@@ -136,3 +136,24 @@ def test_collection_stays_off_until_the_last_capture_ends(enabled):
         assert gc.isenabled() == enabled
     finally:
         gc.enable() if was else gc.disable()
+
+
+def test_a_growing_buffer_does_not_leave_one_behind_for_every_size():
+    """Ever longer prompts: what was replaced stays allocated (a captured graph may use it), so it must not add up."""
+    import torch
+
+    from mini_engine_b200.engine.workspace import Workspace
+
+    workspace = Workspace(64, "cpu")
+    for rows in range(1, 400):
+        view = workspace.growing("records", (rows, 50), torch.float32)
+        assert view.shape == (rows, 50)
+    assert workspace.bytes_held() < 4.5 * 400 * 50 * 4  # half more than asked for, and twice that replaced
+    first = workspace.growing("once", (1000, 3), torch.int32)
+    assert workspace.growing("once", (1000, 3), torch.int32).data_ptr() == first.data_ptr()
+    workspace.frozen = True
+    try:
+        workspace.growing("once", (1001, 3), torch.int32)
+        raise AssertionError("a frozen workspace grew")
+    except RuntimeError:
+        pass
