@@ -263,7 +263,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && has_work) {
+        if (has_work && elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(TC_KEYS);        // S[128 x 128] = Q K^T, K-major operands
             constexpr uint32_t idesc_o = make_idesc(TC_DIM, true);   // O[128 x 128] += P V, V is MN-major
             bool ok = mbar_wait(q_full, 0);
@@ -671,7 +671,7 @@ attention_tcgen05_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && has_work) {
+        if (has_work && elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(TC_KEYS);       // S[128 x 128] = Q K^T, K-major operands
             constexpr uint32_t idesc_o = make_idesc(TC_DIM, true);  // O[128 x 128] += P V, V is MN-major
             // An MMA instruction holds the thread that issues it for 54 cycles whatever its size, and

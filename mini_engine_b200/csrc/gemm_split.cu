@@ -192,7 +192,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_trigger();
             auto load_w = [&](int u) {
                 if (WITHHELD) return;
@@ -222,7 +222,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
     } else if (warp == 1) {
         // --------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t one = make_idesc(NT), two = make_idesc(2 * NT);
             const uint32_t small = tmem_base + C::SMALL_COLUMN;
             int sent = 0;  // units whose MMAs were issued

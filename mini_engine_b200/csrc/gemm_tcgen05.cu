@@ -144,7 +144,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_trigger();
             // Weights are written by no kernel, so the first stages' weight tiles are requested
             // before the preceding kernel has finished; the activations wait for it.
@@ -181,7 +181,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
     } else if (warp == 1) {
         // --------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(BLOCK_T);
             bool ok = true;
             for (int i = 0; i < iterations && ok; ++i) {
@@ -339,7 +339,7 @@ gemm_tcgen05_stacked_swiglu_kernel(const __grid_constant__ CUtensorMap map_w, co
     bool ok = true;  // of the epilogue warps: the sums are there
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_trigger();
             const int early = min(iterations, C::STAGES);
             for (int i = 0; i < early; ++i) {
@@ -367,7 +367,7 @@ gemm_tcgen05_stacked_swiglu_kernel(const __grid_constant__ CUtensorMap map_w, co
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(BLOCK_T);
             for (int i = 0; i < iterations; ++i) {
                 const int stage = i % C::STAGES;
@@ -531,7 +531,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     const uint32_t tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_trigger();
             const int early = min(iterations, C::STAGES);
             for (int i = 0; i < early; ++i) {
@@ -554,7 +554,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = make_idesc_pair(width);
             bool ok = true;
             for (int i = 0; i < iterations && ok; ++i) {
@@ -708,7 +708,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
     const uint32_t tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_trigger();
             int it = 0;  // k blocks loaded so far, over all items: stage = it % STAGES
             bool waited = false, ok = true;
@@ -747,7 +747,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
             if (!waited) pdl_wait();
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             int it = 0, j = 0;
             bool ok = true;
             for (int item = pair; item < p.items && ok; item += pairs, ++j) {

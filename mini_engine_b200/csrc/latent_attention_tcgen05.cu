@@ -156,7 +156,7 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && has_work) {
+        if (has_work && elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(LT_KEYS);  // S[128 x 64] = Q K^T, K-major operands
             const uint32_t idesc_o = make_idesc(half_columns, true);  // O[128 x R/2] += P C, C is MN-major
             const uint32_t c_tile = smem_u32(k_tile) + c_first * LT_K_BLOCK;  // this CTA's columns

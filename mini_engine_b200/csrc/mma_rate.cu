@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(128) mma_rate_kernel(long long* out, int iters
     if (PAIR) cluster_sync();
     tcgen05_fence_after();
     const uint32_t tmem = *holder;
-    if (threadIdx.x == 0 && rank == 0) {
+    if (threadIdx.x < 32 && rank == 0 && elect_one()) {
         const uint32_t idesc = PAIR ? (make_idesc_pair(N) | (MN ? (1u << 16) : 0u)) : make_idesc(N, MN != 0);
         const uint64_t a_desc = smem_desc_sw128(smem_u32(a_tile));
         const uint64_t b_desc = MN ? smem_desc_sw128_mn(smem_u32(b_tile), 16384) : smem_desc_sw128(smem_u32(b_tile));

@@ -44,6 +44,16 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(inner), "r"(row), "r"(smem_u32(bar))
         : "memory");
 }
+// One thread of a converged warp, the same one every time.  The warp that issues MMAs, commits or tile loads branches on this and
+// not on a lane number: behind elect.sync the compiler knows that a single thread runs and keeps the operands of these
+// instructions in uniform registers; behind a comparison it does not.  Cycles that an MMA of K = 16 holds its thread, by N, lane 0 |
+// elected (csrc/mma_rate.cu): 16 48.6 | 9.0, 32 48.6 | 16.0, 64 48.6 | 32.0 (both operands in shared memory 53.6 | 48.0), from 128 on
+// what the pipe takes, N / 2, either way.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t chosen;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+    return chosen != 0;
+}
 __device__ __forceinline__ void tcgen05_alloc(uint32_t* holder, uint32_t columns) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(columns) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
