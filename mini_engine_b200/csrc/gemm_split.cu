@@ -7,7 +7,8 @@
 //   w0 x0  |  w0 x1 + w1 x0  |  w0 x2 + w1 x1 + w2 x0
 // The three dropped ones are together at most 2^-24 of a product, of either sign (0.09 x 2^-24 in the mean square over all
 // mantissas; pieces that are cut instead of rounded have the operand's sign and drop up to 2^-21).  Weights, activations and
-// sums are 32-bit in memory: the pieces exist in shared and tensor memory only.  The tensor core truncates when it adds, so its
+// sums are 32-bit in memory; the weights' pieces exist in tensor memory only, the tokens' ones (all three, so every bit of a token) in
+// shared memory or a scratch buffer.  The tensor core truncates when it adds, so its
 // chain is kept short: the sum of w0 x0 over 64 k is taken out of tensor memory and added with rounding in registers; the
 // small terms (2^-8 and 2^-16 of the products) run over a whole segment of the reduction.  Error against float64 (norm of the
 // difference over norm of the result, 64 x 512 outputs) | that of one fmaf chain per output (gemm_simt.cu), by inner size:
@@ -28,45 +29,55 @@
 // with fmaf in ascending k.
 //
 // Orientation and roles follow the bfloat16 product (gemm_tcgen05.cu): 128 weight rows are the A operand, the tokens
-// the narrow B operand.  Warp 0 loads raw float32 tiles with TMA, warp 1 issues the MMAs, eight converter warps make the
-// pieces (weights: a thread's row goes to tensor memory, where A is read from; tokens: three stacked bfloat16 tiles in
-// shared memory, so that one MMA multiplies a piece of the weights by several pieces of the tokens), eight taker warps add
-// the sums of a block up while the MMAs of the next run.
+// the narrow B operand.  Warp 0 loads raw float32 tiles with TMA, warp 1 issues the MMAs, converter warps make the pieces of the
+// weights (a thread's row goes to tensor memory, where A is read from), taker warps add the sums of a block up while the MMAs of the
+// next run.  The tokens' pieces are three stacked bfloat16 tiles in shared memory, so that one MMA multiplies a piece of the weights
+// by several pieces of the tokens.  Up to 16 tokens the converters make them too; for more, a kernel before this one makes them once
+// for all feature tiles (split_rows_kernel) and they arrive by TMA.
 //
-// What bounds it: a k block takes about 2,000 cycles with 16 or 64 tokens and 2,500 with 128.  The MMAs take 85 to 90 cycles
-// each beside the converters, 58 alone (both work on tensor memory and shared memory), the converters 1,050 to 1,100 a block,
-// and the waits between the roles come on top.  Beside the CUDA-core kernel (tokens x outs x inner): 256 x 24,576 x 4,096
-// 2,378 -> 324 us (159 TFLOP/s), 256 x 4,096 x 12,288 1,714 -> 202, 512 x 2,048 x 5,632 760 -> 107; 8 x 24,576 x 4,096
-// 807 -> 94 (4.3 TB/s of weights), 8 x 4,096 x 4,096 377 -> 25, 1 x 151,936 x 1,024 919 -> 112 (5.6 TB/s); these with pieces that were cut.  Rounded ones against cut ones, in turn and
-// behind a flushed L2: 256 x 24,576 x 4,096 338 -> 325, 256 x 4,096 x 12,288 215 -> 205, 8 x 24,576 x 4,096 106 -> 102, others the same.
+// What bounds it: the issuing thread.  Alone, the MMAs of a k block take 768 cycles with 64 tokens and 1,536 with 128; the thread's one
+// look at a barrier per unit takes 190 cycles on an idle SM and about 400 beside the converters, since it queues behind the MMAs
+// (csrc/mma_rate.cu measures the MMAs alone), and the last MMAs before it cover half of that.  A block takes 1,300 cycles with 64 tokens,
+// 2,300 with 128.  So the thread looks once a unit, at one barrier that takes the arrivals of converters, takers and TMA together, and the
+// widest MMAs come last.  Two groups of eight converter warps work on alternate units: one group (with the tokens to convert as well)
+// took 2,000 to 2,700 cycles a block from the arrival of a tile to its last piece.  us of a product (plain stream order, behind a flushed L2; one group of
+// converters and waits of their own | this form; of the 64-token and wider ones 5 are split_rows_kernel and its launch): 256 x 24,576 x 4,096 320 | 260
+// (198 TFLOP/s), 256 x 4,096 x 12,288 199 | 149, 512 x 2,048 x 6,144 115 | 78, 512 x 2,048 x 2,048 46 | 33, 1,024 sorted rows in 8 groups x 6,144 x 2,048
+// 259 | 185, 64 x 2,048 x 9,216 55 | 41, 8 x 24,576 x 4,096 92 | 81 (5.0 TB/s of weights), 8 x 2,048 x 2,048 13.7 | 11.2.
 #include "tcgen05.cuh"
 
 constexpr int SPLIT_ROWS = 128;  // output features per CTA
 constexpr int SPLIT_K = 64;      // k per block: two 128-byte rows of float32, one of bfloat16
-constexpr int CONVERTERS = 256;  // threads: two warps per quarter of tensor memory's lanes
-constexpr int TAKERS = 256;      // threads: two warps per quarter
-constexpr int SPLIT_THREADS = 64 + CONVERTERS + TAKERS;
+constexpr int CONVERTERS = 256;  // threads of a group of converters: two warps per quarter of tensor memory's lanes
 constexpr int MAX_SEGMENTS = 8;
+constexpr int RING = 4;          // barriers of units in flight
 
 __device__ int g_split_error = 0;  // 0 ok; else (role << 8) | detail of the first failure seen
 
 // NT: tokens per CTA.  The tiles pass through the roles in units, whole k blocks or (128 tokens, for which tensor memory has
-// no room otherwise) halves of 32 k; two buffers of pieces, so that the converters write one while the MMAs read the other.
-template <int NT>
+// no room otherwise) halves of 32 k; the weights' pieces have two buffers, so that the converters write one while the MMAs read the other.
+// PRE: the tokens' pieces were made by split_rows_kernel and arrive by TMA, a block at a time; else the raw tokens arrive with
+// the raw weights and the converters make their pieces too.
+template <int NT, bool PRE>
 struct SplitConfig {
+    static constexpr int GROUPS = NT <= 16 ? 1 : 2;  // of converters: unit u is group u % GROUPS's
+    static constexpr int TAKERS = NT <= 16 ? 128 : 256, COLUMNS = NT * 128 / TAKERS;  // threads; columns of one
+    static constexpr int FIRST_CONVERTER = GROUPS == 2 ? 4 : 2, FIRST_TAKER = FIRST_CONVERTER + GROUPS * CONVERTERS / 32;  // warps
+    static constexpr int THREADS = FIRST_TAKER * 32 + TAKERS, CTAS = NT <= 16 ? 2 : 1;
     static constexpr int UNITS = NT >= 128 ? 2 : 1, UNIT_K = SPLIT_K / UNITS;  // units to a block
-    static constexpr int BOXES = UNIT_K / 32;                                  // a TMA box is 32 k wide
-    static constexpr int W_BYTES = SPLIT_ROWS * UNIT_K * 4, X_BYTES = NT * UNIT_K * 4, RAW_BYTES = W_BYTES + X_BYTES;  // raw tiles of a unit
-    static constexpr int PIECES_BYTES = 3 * NT * SPLIT_K * 2;  // of a block: rows of 128 bytes, of which a half takes 64
-    static constexpr int PIECES_BUFFERS = 2 / UNITS;
-    // 16 tokens: 36 KB a unit, two CTAs to an SM (one CTA with five units in flight was 30 % slower: a unit's way through the
-    // roles is what takes the time); 64 tokens: 48 KB; 128: 32 KB
-    static constexpr int STAGES = NT <= 16 ? 2 : NT <= 64 ? 3 : 5;
+    static constexpr int BOXES = UNIT_K / 32;                                  // a TMA box of float32 is 32 k wide
+    static constexpr int W_BYTES = SPLIT_ROWS * UNIT_K * 4, X_BYTES = PRE ? 0 : NT * UNIT_K * 4, RAW_BYTES = W_BYTES + X_BYTES;  // of a unit
+    static constexpr int PIECES_BYTES = 3 * NT * SPLIT_K * 2;  // of a block's tokens
+    static constexpr int X_BUFFERS = PRE && NT <= 64 ? 3 : 2;  // blocks of them
+    static constexpr int STAGES = NT <= 16 ? 2 : NT <= 64 ? (PRE ? 4 : 3) : 8;
     // tensor memory: w0 x0 of one or two blocks, the 2^-8 and the 2^-16 terms, the weights' pieces of two units
     static constexpr int MAINS = UNITS == 1 ? 2 : 1;
     static constexpr int SMALL_COLUMN = MAINS * NT, A_COLUMN = SMALL_COLUMN + 2 * NT, A_PIECE = UNIT_K / 2, A_COLUMNS = 3 * A_PIECE;
     static constexpr int TMEM_COLUMNS = A_COLUMN + 2 * A_COLUMNS <= 256 ? 256 : 512;
-    static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + PIECES_BUFFERS * PIECES_BYTES + 1024 + 256;
+    static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + X_BUFFERS * PIECES_BYTES + 1024 + 256;
+    static constexpr int READY_ARRIVALS = CONVERTERS / 32 + (PRE ? 1 : 0);  // of a unit; more where a block begins, see the takers
+    static_assert((2 * STAGES + 2 * RING + 2 * MAINS + 1) * 8 + 4 <= 256, "barriers");
+    static_assert(PRE == (NT > 16), "more tokens than 16 come as pieces");
     static_assert(A_COLUMN + 2 * A_COLUMNS <= TMEM_COLUMNS, "tensor memory");
     static_assert(STAGES * RAW_BYTES >= NT * SPLIT_ROWS * 4, "the cluster's exchange reuses the raw tiles");
 };
@@ -93,9 +104,18 @@ __device__ __forceinline__ uint32_t rounded_pair(float even, float odd) {
     return *reinterpret_cast<const uint32_t*>(&pair);
 }
 // What a pair of pieces leaves of four values.
+__device__ __forceinline__ float2 without(float2 v, uint32_t pair) {  // both at once; exact, as a piece is a part of its value
+    const float2 piece = make_float2(__uint_as_float(pair << 16), __uint_as_float(pair & 0xffff0000u)), minus = make_float2(-1.0f, -1.0f);
+    float2 rest;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(rest))
+        : "l"(reinterpret_cast<const unsigned long long&>(piece)), "l"(reinterpret_cast<const unsigned long long&>(minus)),
+          "l"(reinterpret_cast<const unsigned long long&>(v)));
+    return rest;
+}
 __device__ __forceinline__ float4 without(float4 v, uint32_t xy, uint32_t zw) {
-    return make_float4(v.x - __uint_as_float(xy << 16), v.y - __uint_as_float(xy & 0xffff0000u), v.z - __uint_as_float(zw << 16),
-                       v.w - __uint_as_float(zw & 0xffff0000u));
+    const float2 a = without(make_float2(v.x, v.y), xy), b = without(make_float2(v.z, v.w), zw);
+    return make_float4(a.x, a.y, b.x, b.y);
 }
 
 __device__ __forceinline__ float4 lds128(uint32_t address) {
@@ -129,8 +149,9 @@ __device__ __forceinline__ void tcgen05_ld8(uint32_t taddr, float* v) {
 }
 
 // The sum of one output again, for one that came out infinite, NaN or so small that pieces may have fallen under the range.
-__device__ __noinline__ float plain_sum(const float* x, const float* w, int inner) {
+__device__ __forceinline__ float plain_sum(const float* x, const float* w, int inner) {
     float sum = 0.0f;
+#pragma unroll 1
     for (int k = 0; k < inner; k += 4) {
         const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
         sum = fmaf(a.x, b.x, sum);
@@ -140,25 +161,40 @@ __device__ __noinline__ float plain_sum(const float* x, const float* w, int inne
     }
     return sum;
 }
-__device__ __forceinline__ float sound_or_again(const SplitParams& p, int t, int w_row, float v) {
-    if (fabsf(v) <= 3.402823466e38f && (fabsf(v) >= 0x1p-90f || v == 0.0f)) return v;
-    return plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(w_row) * p.inner, p.inner);
+__device__ __forceinline__ bool sound(float v) { return fabsf(v) <= 3.402823466e38f && (fabsf(v) >= 0x1p-90f || v == 0.0f); }
+__device__ __forceinline__ void form_again(const SplitParams& p, int t, int w_row, int n) {
+    p.out[static_cast<size_t>(t) * p.outs + n] = plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(w_row) * p.inner, p.inner);
+}
+// What the threads of four warps hold at most from now on; the roles' shares stand where the roles part.
+template <int REGISTERS>
+__device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGISTERS)); }
+template <int REGISTERS>
+__device__ __forceinline__ void registers_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGISTERS)); }
+
+// The three pieces of four values, each as two pairs.
+__device__ __forceinline__ void pieces_of(float4 v, uint32_t* p0, uint32_t* p1, uint32_t* p2) {
+    p0[0] = rounded_pair(v.x, v.y), p0[1] = rounded_pair(v.z, v.w);
+    const float4 r = without(v, p0[0], p0[1]);
+    p1[0] = rounded_pair(r.x, r.y), p1[1] = rounded_pair(r.z, r.w);
+    const float4 rest = without(r, p1[0], p1[1]);
+    p2[0] = upper_pair(rest.x, rest.y), p2[1] = upper_pair(rest.z, rest.w);
 }
 
 // WITHHELD: no tile is ever loaded and waits end after a few polls, so that a test can take the way of a kernel that gives up.
-template <int NT, bool WITHHELD = false>
-__global__ void __launch_bounds__(SPLIT_THREADS, NT <= 16 ? 2 : 1)
+template <int NT, bool PRE, bool WITHHELD = false>
+__global__ void __launch_bounds__(SplitConfig<NT, PRE>::THREADS, SplitConfig<NT, PRE>::CTAS)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SplitParams p) {
-    using C = SplitConfig<NT>;
+    using C = SplitConfig<NT, PRE>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* raw = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* pieces = raw + C::STAGES * C::RAW_BYTES;
-    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + C::PIECES_BUFFERS * C::PIECES_BYTES);  // raw tiles arrived
-    uint64_t* empty = full + C::STAGES;                                                         // raw tiles read by the converters
-    uint64_t* ready = empty + C::STAGES;                                                        // [2] a unit's pieces written
-    uint64_t* done = ready + 2;                                                                 // [2] its MMAs retired
-    uint64_t* taken = done + 2;                                                                 // [MAINS] a block's sums out of tensor memory
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + C::MAINS);
+    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + C::X_BUFFERS * C::PIECES_BYTES);  // raw tiles arrived
+    uint64_t* empty = full + C::STAGES;   // raw tiles read by the converters
+    uint64_t* ready = empty + C::STAGES;  // [RING] all that a unit's MMAs need is there
+    uint64_t* done = ready + RING;        // [RING] its MMAs retired
+    uint64_t* mains = done + RING;        // [MAINS] a block's w0 x0 complete
+    uint64_t* taken = mains + C::MAINS;   // a segment's small terms out of tensor memory
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.x * NT, n0 = blockIdx.y * SPLIT_ROWS;
@@ -175,8 +211,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], CONVERTERS / 32); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&ready[b], CONVERTERS / 32); mbar_init(&done[b], 1); }
-        for (int b = 0; b < C::MAINS; ++b) mbar_init(&taken[b], TAKERS / 32);
+        // The issuer waits once a unit: a wait holds it for 190 cycles and more, which only the last MMAs before it cover.  So a unit's
+        // barrier also takes the arrivals of the tokens' pieces and of the takers who have emptied the sums that it overwrites:
+        // in the first unit of a block if that is a unit of its own (barriers 0 and 2 of four if a block has two units).
+        for (int b = 0; b < RING; ++b) {
+            const bool opens = b % C::UNITS == 0;
+            mbar_init(&ready[b], CONVERTERS / 32 + (opens ? C::TAKERS / 32 + (PRE ? 1 : 0) : 0));
+            mbar_init(&done[b], 1);
+        }
+        for (int b = 0; b < C::MAINS; ++b) mbar_init(&mains[b], 1);
+        mbar_init(taken, C::TAKERS / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tcgen05_alloc(tmem_holder, C::TMEM_COLUMNS);
@@ -190,6 +234,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     bool ok = true;
     auto wait = [](uint64_t* bar, uint32_t parity) { return WITHHELD ? mbar_wait(bar, parity, 512) : mbar_wait(bar, parity); };
 
+    // Two groups of converters: 128 x 56 + 512 x 56 + 256 x 112 registers, which is what 896 threads of 72 start with.
+    if (C::GROUPS == 2 && warp < C::FIRST_CONVERTER) registers_down<56>();
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer
         if (elect_one()) {
@@ -201,74 +247,116 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     tma_load_2d(raw + (u % C::STAGES) * C::RAW_BYTES + box * SPLIT_ROWS * 128, &map_w, kb_begin * SPLIT_K + u * C::UNIT_K + 32 * box, w0,
                                 &full[u % C::STAGES]);
             };
-            auto load_x = [&](int u) {
+            auto load_x = [&](int u) {  // raw tokens
                 if (WITHHELD) return;
                 for (int box = 0; box < C::BOXES; ++box)
                     tma_load_2d(raw + (u % C::STAGES) * C::RAW_BYTES + C::W_BYTES + box * NT * 128, &map_x, kb_begin * SPLIT_K + u * C::UNIT_K + 32 * box, t0,
                                 &full[u % C::STAGES]);
             };
+            auto load_pieces = [&](int b) {
+                uint64_t* bar = &ready[b * C::UNITS % RING];
+                mbar_expect_tx(bar, C::PIECES_BYTES);
+                for (int q = 0; q < 3; ++q)
+                    tma_load_2d(pieces + b % C::X_BUFFERS * C::PIECES_BYTES + q * NT * 128, &map_x, (kb_begin + b) * SPLIT_K, q * p.tokens + t0, bar);
+            };
             const int early = min(units, C::STAGES);  // weights are written by no kernel: ahead of the wait
             for (int u = 0; u < early; ++u) load_w(u);
             pdl_wait();
-            for (int u = 0; u < early; ++u) load_x(u);
-            int issued = early;
-            for (int u = early; u < units; ++u, ++issued) {
-                if (!wait(&empty[u % C::STAGES], ((u / C::STAGES) & 1) ^ 1)) { atomicCAS(&g_split_error, 0, (1 << 8)); break; }
-                load_w(u);
-                load_x(u);
+            int issued = early, x_issued = 0;
+            bool go = true;
+            if constexpr (PRE) {
+                for (; x_issued < min(blocks, C::X_BUFFERS); ++x_issued) load_pieces(x_issued);
+                // A block's pieces take the place of the block X_BUFFERS before, whose last unit must be done.  Weights go first: their
+                // room comes free with a unit's conversion, ahead of its MMAs.  A unit is converted at most two units ahead of
+                // them, so whenever this thread waits for room for weights, all pieces that the MMAs need until then are on their way.
+                auto room_for_pieces = [&]() { return (x_issued - C::X_BUFFERS + 1) * C::UNITS - 1; };  // the unit that gives it
+                for (int u = early; u < units || x_issued < blocks;) {
+                    if (u < units) {
+                        if (!wait(&empty[u % C::STAGES], ((u / C::STAGES) & 1) ^ 1)) { go = false; break; }
+                        load_w(u);
+                        issued = ++u;
+                    } else {
+                        const int last = room_for_pieces();
+                        if (!wait(&done[last % RING], (last / RING) & 1)) { go = false; break; }
+                    }
+                    while (x_issued < blocks) {
+                        const int last = room_for_pieces();
+                        if (!mbar_try_wait(&done[last % RING], (last / RING) & 1)) break;
+                        load_pieces(x_issued);
+                        ++x_issued;
+                    }
+                }
+            } else {
+                for (int u = 0; u < early; ++u) load_x(u);
+                for (int u = early; u < units; ++u, ++issued) {
+                    if (!wait(&empty[u % C::STAGES], ((u / C::STAGES) & 1) ^ 1)) { go = false; break; }
+                    load_w(u);
+                    load_x(u);
+                }
             }
+            if (!go) atomicCAS(&g_split_error, 0, (1 << 8));
             // Copies in flight must land before the shared memory is released, also when another role has given up.
             for (int u = max(issued - C::STAGES, 0); u < issued; ++u) wait(&full[u % C::STAGES], (u / C::STAGES) & 1);
+            if (PRE && (!go || g_split_error != 0)) {  // on the normal path the MMAs have waited for the pieces
+                const long long until = clock64() + 100000;  // their barriers may miss other arrivals for good: 50 us, no copy takes that long
+                while (clock64() < until) __nanosleep(1000);
+            }
         }
     } else if (warp == 1) {
         // --------------------------------------------------------------- MMA issuer
         if (elect_one()) {
             constexpr uint32_t one = make_idesc(NT), two = make_idesc(2 * NT);
+            constexpr uint64_t PIECE = (NT * 128) >> 4;  // from a piece of the tokens to the next, in descriptor units
             const uint32_t small = tmem_base + C::SMALL_COLUMN;
+            const uint64_t x_pieces = smem_desc_sw128(smem_u32(pieces));
             int sent = 0;  // units whose MMAs were issued
-            auto wait_taken = [&](int block) { return block < 0 || wait(&taken[block % C::MAINS], (block / C::MAINS) & 1); };
-            for (int u = 0, at = 0; u < units; ++u) {
+            for (int u = 0, at = 0, segment = 0; u < units; ++u) {
                 const int half = u % C::UNITS, block = u / C::UNITS;
-                const bool fresh = half == 0 && at == 0;  // a segment starts its own sums: the last one's must be out
-                if (!wait(&ready[u & 1], (u >> 1) & 1) || (fresh && !wait_taken(block - 1))) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
+                const bool fresh = half == 0 && at == 0;  // a segment starts its own small terms
+                if (!wait(&ready[u % RING], (u / RING) & 1)) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
                 tcgen05_fence_after();
                 const uint32_t a = tmem_base + C::A_COLUMN + (u & 1) * C::A_COLUMNS, main_sum = tmem_base + block % C::MAINS * NT;
-                const uint64_t b = smem_desc_sw128(smem_u32(pieces + (C::UNITS == 1 ? (u & 1) * C::PIECES_BYTES : 0))) + 4 * half;
-                // The small terms of 32 k, then of the next: MMAs into the same columns follow each other without a gap, and the
-                // widest come last, so that the next unit's waits pass while they run.  A step of 16 k is 8 columns of the weights'
-                // pieces and 32 bytes of the tokens'.
+                const uint64_t b = x_pieces + block % C::X_BUFFERS * (C::PIECES_BYTES >> 4) + 4 * half;
+                // A step of 16 k is 8 columns of the weights' pieces and 32 bytes of the tokens'.  The block's own sums come first, so
+                // that the takers have them while the small terms run; MMAs of both small sums come last: while the last of them run
+                // the wait for the next unit passes.  MMAs into the same columns follow each other without a gap.
+#pragma unroll
+                for (int k = 0; k < C::UNIT_K / 16; ++k) tcgen05_mma_bf16_ts(main_sum, a + 8 * k, b + 2 * k, one, half > 0 || k > 0);
+                if (half == C::UNITS - 1) tcgen05_commit(&mains[block % C::MAINS]);
                 bool go = true;
-#pragma unroll
-                for (int box = 0; box < C::BOXES; ++box) {
-                    const uint32_t w0_piece = a + 16 * box, w1_piece = w0_piece + C::A_PIECE, w2_piece = w1_piece + C::A_PIECE;
-                    const uint64_t x0 = b + 4 * box, x1 = x0 + ((NT * 128) >> 4);
-                    tcgen05_mma_bf16_ts(small, w1_piece, x0, two, !fresh || box > 0);
-                    tcgen05_mma_bf16_ts(small, w1_piece + 8, x0 + 2, two, 1);
-                    tcgen05_mma_bf16_ts(small + NT, w2_piece, x0, one, 1);
-                    tcgen05_mma_bf16_ts(small + NT, w2_piece + 8, x0 + 2, one, 1);
-                    if (box == C::BOXES - 1) {
-                        if (half == 0 && !wait_taken(block - C::MAINS)) { go = false; break; }  // the takers have had their time
-                        tcgen05_fence_after();
-#pragma unroll
-                        for (int k = 0; k < C::UNIT_K / 16; ++k) tcgen05_mma_bf16_ts(main_sum, a + 8 * k, b + 2 * k, one, half > 0 || k > 0);
-                    }
-                    tcgen05_mma_bf16_ts(small, w0_piece, x1, two, 1);
-                    tcgen05_mma_bf16_ts(small, w0_piece + 8, x1 + 2, two, 1);
+                if (fresh && segment > 0) {
+                    go = wait(taken, (segment & 1) ^ 1);
+                    tcgen05_fence_after();
                 }
-                tcgen05_commit(&done[u & 1]);
+                if (go) {
+#pragma unroll
+                    for (int k = 0; k < C::UNIT_K / 16; k += 2) {  // 32 k after 32 k: the order is the same in every form
+                        tcgen05_mma_bf16_ts(small, a + C::A_PIECE + 8 * k, b + 2 * k, two, !fresh || k > 0);
+                        tcgen05_mma_bf16_ts(small, a + C::A_PIECE + 8 * k + 8, b + 2 * k + 2, two, 1);
+                        tcgen05_mma_bf16_ts(small + NT, a + 2 * C::A_PIECE + 8 * k, b + 2 * k, one, 1);
+                        tcgen05_mma_bf16_ts(small + NT, a + 2 * C::A_PIECE + 8 * k + 8, b + 2 * k + 2, one, 1);
+                        tcgen05_mma_bf16_ts(small, a + 8 * k, b + PIECE + 2 * k, two, 1);
+                        tcgen05_mma_bf16_ts(small, a + 8 * k + 8, b + PIECE + 2 * k + 2, two, 1);
+                    }
+                }
+                tcgen05_commit(&done[u % RING]);
                 ++sent;
                 if (!go) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
-                if (half == C::UNITS - 1 && ++at == p.per_segment) at = 0;
+                if (half == C::UNITS - 1 && ++at == p.per_segment) at = 0, ++segment;
             }
             // MMAs in flight read shared memory and write tensor memory: they end before either is given back.
-            for (int u = max(sent - 2, 0); u < sent; ++u) wait(&done[u & 1], (u >> 1) & 1);
+            for (int u = max(sent - RING, 0); u < sent; ++u) wait(&done[u % RING], (u / RING) & 1);
         }
-    } else if (warp < 2 + CONVERTERS / 32) {
+    } else if (warp < C::FIRST_CONVERTER) {
+        // warps that fill the first group of four up
+    } else if (warp < C::FIRST_TAKER) {
         // ----------------------------------------------------------------- converters
         // A thread takes 16 or 32 weights of a row.
-        const int worker = threadIdx.x - 64, run = worker >> 7;
+        if constexpr (C::GROUPS == 2) registers_down<56>();
+        const int group = (warp - C::FIRST_CONVERTER) / (CONVERTERS / 32);
+        const int worker = threadIdx.x - C::FIRST_CONVERTER * 32 - group * CONVERTERS, run = worker >> 7;
         const int row = quarter * 32 + lane;
-        for (int u = 0; u < units; ++u) {
+        for (int u = group; u < units; u += C::GROUPS) {
             ok = __all_sync(0xffffffffu, wait(&full[u % C::STAGES], (u / C::STAGES) & 1));
             if (!ok) break;
             const uint32_t w_tile = smem_u32(raw + (u % C::STAGES) * C::RAW_BYTES), x_tile = w_tile + C::W_BYTES;
@@ -279,16 +367,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 const int first_chunk = 4 * (C::BOXES == 2 ? part : run);
                 uint32_t piece0[8], piece1[8], piece2[8];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float4 v = lds128(from_row + (((first_chunk + c) ^ (row & 7)) << 4));
-                    piece0[2 * c] = rounded_pair(v.x, v.y), piece0[2 * c + 1] = rounded_pair(v.z, v.w);
-                    const float4 r = without(v, piece0[2 * c], piece0[2 * c + 1]);
-                    piece1[2 * c] = rounded_pair(r.x, r.y), piece1[2 * c + 1] = rounded_pair(r.z, r.w);
-                    const float4 rest = without(r, piece1[2 * c], piece1[2 * c + 1]);
-                    piece2[2 * c] = upper_pair(rest.x, rest.y), piece2[2 * c + 1] = upper_pair(rest.z, rest.w);
-                }
+                for (int c = 0; c < 4; ++c)
+                    pieces_of(lds128(from_row + (((first_chunk + c) ^ (row & 7)) << 4)), piece0 + 2 * c, piece1 + 2 * c, piece2 + 2 * c);
                 if (part == 0 && u >= 2) {  // the MMAs of two units ago have read these buffers
-                    ok = __all_sync(0xffffffffu, wait(&done[u & 1], ((u >> 1) & 1) ^ 1));
+                    ok = __all_sync(0xffffffffu, wait(&done[(u - 2) % RING], ((u - 2) / RING) & 1));
                     if (!ok) break;
                     tcgen05_fence_after();
                 }
@@ -297,37 +379,30 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 tcgen05_st8(to + 8 * part + 2 * C::A_PIECE, piece2);
             }
             if (!ok) break;
-            const uint32_t x_pieces = smem_u32(pieces + (C::UNITS == 1 ? (u & 1) * C::PIECES_BYTES : 0));
+            if constexpr (!PRE) {
+                const uint32_t x_pieces = smem_u32(pieces + u % C::X_BUFFERS * C::PIECES_BYTES);
 #pragma unroll
-            for (int item = worker; item < NT * C::UNIT_K / 8; item += CONVERTERS) {
-                // 8 k values of a token: two raw chunks to one 16-byte chunk of each piece.  Eight lanes are four chunks of tokens t
-                // and t + 4, whose pieces fall into different banks; so do their raw chunks, read in opposite order.
-                const int box = item / (NT * 4), chunk = item & 3, upper = (item >> 2) & 1, t = ((item >> 3) & 3) + 4 * upper + 8 * (item % (NT * 4) >> 5);
-                const uint32_t from = x_tile + box * NT * 128 + t * 128;
-                const float4 one = lds128(from + (((2 * chunk + upper) ^ (t & 7)) << 4));
-                const float4 other = lds128(from + (((2 * chunk + (upper ^ 1)) ^ (t & 7)) << 4));
-                float4 v[2];
-                v[0] = upper ? other : one;
-                v[1] = upper ? one : other;
-                const int to_chunk = 4 * (C::UNITS == 1 ? box : u & 1) + chunk;
+                for (int item = worker; item < NT * C::UNIT_K / 8; item += CONVERTERS) {
+                    // 8 k values of a token: two raw chunks to one 16-byte chunk of each piece.  Eight lanes are four chunks of tokens t
+                    // and t + 4, whose pieces fall into different banks; so do their raw chunks, read in opposite order.
+                    const int box = item / (NT * 4), chunk = item & 3, upper = (item >> 2) & 1, t = ((item >> 3) & 3) + 4 * upper + 8 * (item % (NT * 4) >> 5);
+                    const uint32_t from = x_tile + box * NT * 128 + t * 128;
+                    const float4 one = lds128(from + (((2 * chunk + upper) ^ (t & 7)) << 4));
+                    const float4 other = lds128(from + (((2 * chunk + (upper ^ 1)) ^ (t & 7)) << 4));
+                    uint32_t out[3][4];
+                    pieces_of(upper ? other : one, out[0], out[1], out[2]);
+                    pieces_of(upper ? one : other, out[0] + 2, out[1] + 2, out[2] + 2);
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    uint32_t pair[4];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        pair[2 * h] = q < 2 ? rounded_pair(v[h].x, v[h].y) : upper_pair(v[h].x, v[h].y);
-                        pair[2 * h + 1] = q < 2 ? rounded_pair(v[h].z, v[h].w) : upper_pair(v[h].z, v[h].w);
-                        v[h] = without(v[h], pair[2 * h], pair[2 * h + 1]);
-                    }
-                    sts128(x_pieces + q * NT * 128 + t * 128 + ((to_chunk ^ (t & 7)) << 4), make_uint4(pair[0], pair[1], pair[2], pair[3]));
+                    for (int q = 0; q < 3; ++q)
+                        sts128(x_pieces + q * NT * 128 + t * 128 + (((4 * box + chunk) ^ (t & 7)) << 4), make_uint4(out[q][0], out[q][1], out[q][2], out[q][3]));
                 }
             }
             tcgen05_wait_st();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read shared memory as the async proxy
+            if (!PRE) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read shared memory as the async proxy
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&ready[u & 1]);
+                mbar_arrive(&ready[u % RING]);
                 mbar_arrive(&empty[u % C::STAGES]);
             }
         }
@@ -335,29 +410,37 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     } else {
         // ------------------------------------------------------------------- takers
         // The sums of a block out of tensor memory and added up; at the end of a segment the small terms join them.
-        constexpr int COLUMNS = NT / 2;
-        const int row = quarter * 32 + lane, n = n0 + row, column = (warp - 2 - CONVERTERS / 32) / 4 * COLUMNS;
+        if constexpr (C::GROUPS == 2) registers_up<112>();
+        constexpr int COLUMNS = C::COLUMNS;
+        const int row = quarter * 32 + lane, n = n0 + row, column = (warp - C::FIRST_TAKER) / 4 * COLUMNS;
         // With 128 tokens a thread's registers hold one sum per column: its CTA runs one segment (see me_gemm_split).
         constexpr bool MANY = NT < 128;
         float sum[COLUMNS], total[MANY ? COLUMNS : 1] = {};  // of the running segment, of the finished ones
-        int at = 0;
-        bool first = true;
+        int at = 0, segment = 0;
 #pragma unroll
         for (int c = 0; c < COLUMNS; ++c) sum[c] = 0.0f;
+        if (lane == 0)
+            for (int b = 0; b < C::MAINS; ++b) mbar_arrive(&ready[b * C::UNITS]);  // nothing lies in tensor memory yet
         for (int i = 0; i < blocks; ++i) {
-            const int u = i * C::UNITS + C::UNITS - 1;  // the block's last unit
-            ok = __all_sync(0xffffffffu, wait(&done[u & 1], (u >> 1) & 1));
+            ok = __all_sync(0xffffffffu, wait(&mains[i % C::MAINS], (i / C::MAINS) & 1));
             if (!ok) break;
             tcgen05_fence_after();
 #pragma unroll
-            for (int c0 = 0; c0 < COLUMNS; c0 += 8) {
-                float got[8];
-                tcgen05_ld8(lanes + i % C::MAINS * NT + column + c0, got);
+            for (int c0 = 0; c0 < COLUMNS; c0 += 16) {
+                float got[16];
+                tcgen05_ld16(lanes + i % C::MAINS * NT + column + c0, got);
 #pragma unroll
-                for (int c = 0; c < 8; ++c) sum[c0 + c] += got[c];
+                for (int c = 0; c < 16; ++c) sum[c0 + c] += got[c];
             }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[(i + C::MAINS) * C::UNITS % RING]);  // for the block that takes this one's columns
             if (++at == p.per_segment || i + 1 == blocks) {
                 at = 0;
+                const int u = i * C::UNITS + C::UNITS - 1;  // the block's last unit
+                ok = __all_sync(0xffffffffu, wait(&done[u % RING], (u / RING) & 1));
+                if (!ok) break;
+                tcgen05_fence_after();
 #pragma unroll
                 for (int c0 = 0; c0 < COLUMNS; c0 += 8) {
                     float low[8], lower[8];
@@ -367,18 +450,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     for (int c = 0; c < 8; ++c) {
                         const float part = sum[c0 + c] + (low[c] + lower[c]);
                         if constexpr (MANY) {
-                            total[c0 + c] = first ? part : total[c0 + c] + part;
+                            total[c0 + c] = segment == 0 ? part : total[c0 + c] + part;
                             sum[c0 + c] = 0.0f;
                         } else {
                             sum[c0 + c] = part;
                         }
                     }
                 }
-                first = false;
+                ++segment;
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(taken);
             }
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&taken[i % C::MAINS]);
         }
         auto result = [&](int c) { return MANY ? total[MANY ? c : 0] : sum[c]; };
         if (!ok && lane == 0) atomicCAS(&g_split_error, 0, (4 << 8));
@@ -389,11 +472,17 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
             for (int c = 0; c < COLUMNS; ++c) exchange[(column + c) * SPLIT_ROWS + row] = result(c);
         } else if (ok && n < p.outs) {
+            unsigned long long odd = 0;  // columns to be formed again
 #pragma unroll
             for (int c = 0; c < COLUMNS; ++c) {
                 const int t = t0 + column + c;
-                if (t < p.tokens) p.out[static_cast<size_t>(t) * p.outs + n] = sound_or_again(p, t, w0 + row, result(c));
+                if (t < p.tokens) {
+                    p.out[static_cast<size_t>(t) * p.outs + n] = result(c);
+                    if (!sound(result(c))) odd |= 1ull << c;
+                }
             }
+#pragma unroll 1
+            for (; odd != 0; odd &= odd - 1) form_again(p, t0 + column + __ffsll(odd) - 1, w0 + row, n);
         }
     }
     tcgen05_fence_before();
@@ -401,11 +490,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (warp == 1) tcgen05_dealloc(tmem_base, C::TMEM_COLUMNS);
     if (p.clustered) {
         cluster_sync();
-        if (warp >= 2 && warp < 2 + CONVERTERS / 32 && ok) {
+        if (warp >= C::FIRST_CONVERTER && warp < C::FIRST_CONVERTER + CONVERTERS / 32 && ok) {
             pdl_wait();
             // Four rows of a column at a time, shared out among the cluster's CTAs.
             const int segments = gridDim.z;
-            for (int item = threadIdx.x - 64 + CONVERTERS * blockIdx.z; item < NT * (SPLIT_ROWS / 4); item += CONVERTERS * segments) {
+            for (int item = threadIdx.x - C::FIRST_CONVERTER * 32 + CONVERTERS * blockIdx.z; item < NT * (SPLIT_ROWS / 4); item += CONVERTERS * segments) {
                 const int c = item / (SPLIT_ROWS / 4), row = item % (SPLIT_ROWS / 4) * 4, t = t0 + c, n = n0 + row;
                 if (t >= p.tokens || n >= p.outs) continue;
                 const uint32_t from = smem_u32(raw) + (c * SPLIT_ROWS + row) * 4;
@@ -417,8 +506,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                 for (int s = 1; s < MAX_SEGMENTS; ++s)
                     if (s < segments) y.x += part[s].x, y.y += part[s].y, y.z += part[s].z, y.w += part[s].w;
-                const float v[4] = {sound_or_again(p, t, w0 + row, y.x), n + 1 < p.outs ? sound_or_again(p, t, w0 + row + 1, y.y) : 0.0f,
-                                    n + 2 < p.outs ? sound_or_again(p, t, w0 + row + 2, y.z) : 0.0f, n + 3 < p.outs ? sound_or_again(p, t, w0 + row + 3, y.w) : 0.0f};
+                const float v[4] = {y.x, y.y, y.z, y.w};
                 float* to = p.out + static_cast<size_t>(t) * p.outs + n;
                 if (p.vector_out) {
                     *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
@@ -427,6 +515,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     for (int i = 0; i < 4; ++i)
                         if (n + i < p.outs) to[i] = v[i];
                 }
+                unsigned odd = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) odd |= sound(v[i]) ? 0u : 1u << i;
+#pragma unroll 1
+                for (int i = 0; i < 4 && n + i < p.outs; ++i)
+                    if (odd >> i & 1) form_again(p, t, w0 + row + i, n + i);
             }
         }
         cluster_sync();  // the others may still read this CTA's part
@@ -451,35 +545,75 @@ static EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// A [rows][inner] float32 matrix, tiles of box_rows x 32 in the 128-byte swizzle; elements outside read as zero.
-ME_EXPORT int me_make_tensor_map_f32(void* out, const void* base, unsigned long long rows, unsigned long long inner, unsigned int box_rows) {
+static int make_map(void* out, const void* base, CUtensorMapDataType type, int element, unsigned long long rows, unsigned long long inner,
+                    unsigned long long pitch, unsigned int box_rows) {
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return ME_ERR_UNSUPPORTED;
-    if (inner % 4 != 0 || reinterpret_cast<uintptr_t>(base) % 16 != 0 || box_rows > 256) return ME_ERR_ARGUMENT;
+    if (pitch % 16 != 0 || reinterpret_cast<uintptr_t>(base) % 16 != 0 || box_rows > 256) return ME_ERR_ARGUMENT;
     alignas(64) CUtensorMap map;
     const cuuint64_t dims[2] = {inner, rows};
-    const cuuint64_t strides[1] = {inner * 4};
-    const cuuint32_t box[2] = {SPLIT_K / 2, box_rows};
+    const cuuint64_t strides[1] = {pitch};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / element), box_rows};
     const cuuint32_t element_strides[2] = {1, 1};
-    const CUresult result = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
-                                   element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult result = encode(&map, type, 2, const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (result != CUDA_SUCCESS) return ME_ERR_ARGUMENT;
     memcpy(out, &map, sizeof(map));
     return 0;
 }
 
-template <int NT, bool WITHHELD = false>
+// A [rows][inner] float32 matrix, tiles of box_rows x 32 in the 128-byte swizzle; elements outside read as zero.
+ME_EXPORT int me_make_tensor_map_f32(void* out, const void* base, unsigned long long rows, unsigned long long inner, unsigned int box_rows) {
+    return make_map(out, base, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, rows, inner, inner * 4, box_rows);
+}
+
+// The pieces that split_rows_kernel wrote of `rows` tokens, tiles of box_rows x 64.
+ME_EXPORT int me_make_tensor_map_pieces(void* out, const void* base, unsigned long long rows, unsigned long long inner, unsigned int box_rows) {
+    return make_map(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3 * rows, inner, (inner + 7) / 8 * 16, box_rows);
+}
+
+// pieces[q][t][k] of x[t][k], rows of the pieces padded to whole 16 bytes.  A thread makes 8 values' pieces; bound by the
+// latency of one load and of the launch.
+constexpr int ROWS_THREADS = 256;
+__global__ void __launch_bounds__(ROWS_THREADS)
+split_rows_kernel(const float* __restrict__ x, uint4* __restrict__ pieces, int tokens, int inner) {
+    pdl_trigger();
+    pdl_wait();
+    const int chunks = (inner + 7) / 8;
+    const long long total = static_cast<long long>(tokens) * chunks;
+    for (long long i = static_cast<long long>(blockIdx.x) * ROWS_THREADS + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * ROWS_THREADS) {
+        const long long t = i / chunks;
+        const int k = static_cast<int>(i - t * chunks) * 8;
+        const float* from = x + t * inner + k;  // inner is a multiple of 4
+        const float4 a = *reinterpret_cast<const float4*>(from);
+        const float4 b = k + 4 < inner ? *reinterpret_cast<const float4*>(from + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint32_t out[3][4];
+        pieces_of(a, out[0], out[1], out[2]);
+        pieces_of(b, out[0] + 2, out[1] + 2, out[2] + 2);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) pieces[q * total + i] = make_uint4(out[q][0], out[q][1], out[q][2], out[q][3]);
+    }
+}
+
+static int split_rows(const float* x, void* pieces, int tokens, int inner, cudaStream_t stream) {
+    if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(pieces) % 16 != 0) return ME_ERR_ARGUMENT;
+    const long long total = static_cast<long long>(tokens) * ((inner + 7) / 8);
+    const long long wanted = (total + ROWS_THREADS - 1) / ROWS_THREADS;
+    const int blocks = static_cast<int>(wanted < 148 * 8 ? wanted : 148 * 8);
+    return launch_kernel(split_rows_kernel, dim3(blocks), dim3(ROWS_THREADS), 0, stream, x, static_cast<uint4*>(pieces), tokens, inner);
+}
+
+template <int NT, bool PRE, bool WITHHELD = false>
 static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, const SplitParams& p, int segments, cudaStream_t stream) {
-    using C = SplitConfig<NT>;
-    auto kernel = gemm_split_kernel<NT, WITHHELD>;
+    using C = SplitConfig<NT, PRE>;
+    auto kernel = gemm_split_kernel<NT, PRE, WITHHELD>;
     static SharedMemoryOptIn opt_in;
     if (const int e = opt_in(kernel, C::SMEM_BYTES)) return e;
     const dim3 grid((p.tokens + NT - 1) / NT, (p.outs + SPLIT_ROWS - 1) / SPLIT_ROWS, p.clustered ? segments : 1);
     if (grid.y > 65535) return ME_ERR_UNSUPPORTED;
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
-    config.blockDim = dim3(SPLIT_THREADS);
+    config.blockDim = dim3(C::THREADS);
     config.dynamicSmemBytes = C::SMEM_BYTES;
     config.stream = stream;
     cudaLaunchAttribute attributes[2];
@@ -499,10 +633,12 @@ static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, cons
 }
 
 // out[t][n] = sum_k x[t][k] * w[n][k]; `segments` ranges of k blocks whose sums are added in ascending order, in one
-// CTA or (`clustered`) in a cluster's CTAs.  With `group_of_block` a grouped product: `tile` rows of x to a group.  `map_x` has boxes
-// of `tile` rows: 16, 64, or 128 where a CTA runs one segment (one in all, or `clustered`).  `withheld`: every wait runs out (for tests).
+// CTA or (`clustered`) in a cluster's CTAs.  With `group_of_block` a grouped product: `tile` rows of x to a group.  `tile` tokens to a CTA: 16
+// (`map_x` has boxes of as many rows of x), or 64, or 128 where a CTA runs one segment (one in all, or `clustered`): these come with room for the
+// tokens' `pieces` (3 x tokens x inner bfloat16, rows padded to 16 bytes), which are made first, and `map_x` is that of the pieces.
+// `withheld`: every wait runs out (for tests).
 ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x, const float* w, float* out, int tokens, int outs,
-                            int inner, int tile, int segments, int clustered, const int* group_of_block, int group_rows, int withheld,
+                            int inner, int tile, void* pieces, int segments, int clustered, const int* group_of_block, int group_rows, int withheld,
                             cudaStream_t stream) {
     if (tokens <= 0 || outs <= 0) return 0;
     if (group_of_block != nullptr && (group_rows < outs || tokens % tile)) return ME_ERR_ARGUMENT;
@@ -519,10 +655,12 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     alignas(64) CUtensorMap w_map, x_map;
     memcpy(&w_map, map_w, sizeof(w_map));
     memcpy(&x_map, map_x, sizeof(x_map));
-    if (withheld) return tile == 16 ? launch_split<16, true>(w_map, x_map, p, segments, stream) : ME_ERR_ARGUMENT;
-    if (tile == 16) return launch_split<16>(w_map, x_map, p, segments, stream);
-    if (tile == 64) return launch_split<64>(w_map, x_map, p, segments, stream);
-    if (tile == 128 && (p.clustered || segments == 1)) return launch_split<128>(w_map, x_map, p, segments, stream);
+    if (pieces != nullptr)
+        if (const int e = split_rows(x, pieces, tokens, inner, stream)) return e;
+    if (withheld) return tile == 16 && !pieces ? launch_split<16, false, true>(w_map, x_map, p, segments, stream) : ME_ERR_ARGUMENT;
+    if (tile == 16 && !pieces) return launch_split<16, false>(w_map, x_map, p, segments, stream);
+    if (tile == 64 && pieces) return launch_split<64, true>(w_map, x_map, p, segments, stream);
+    if (tile == 128 && pieces && (p.clustered || segments == 1)) return launch_split<128, true>(w_map, x_map, p, segments, stream);
     return ME_ERR_ARGUMENT;
 }
 

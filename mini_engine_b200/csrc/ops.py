@@ -447,14 +447,14 @@ def SplitPlan(weight: torch.Tensor, group_rows: int | None = None):
     return tensor_core.SplitPlan(weight, group_rows)
 
 
-def gemm_split(plan, x: torch.Tensor, out: torch.Tensor) -> None:
+def gemm_split(plan, x: torch.Tensor, out: torch.Tensor, workspace=None) -> None:
     """``out[T, N] = x[T, K] @ weight[N, K]^T`` in float32 on the tensor cores."""
-    tensor_core.gemm_split(plan, x, out)
+    tensor_core.gemm_split(plan, x, out, workspace=workspace)
 
 
-def gemm_split_grouped(plan, x: torch.Tensor, out: torch.Tensor, group_of_block: torch.Tensor, pad: int, filled: int) -> None:
+def gemm_split_grouped(plan, x: torch.Tensor, out: torch.Tensor, group_of_block: torch.Tensor, pad: int, filled: int, workspace=None) -> None:
     """A float32 product over rows sorted by group (see :func:`tensor_core.gemm_split_grouped`)."""
-    tensor_core.gemm_split_grouped(plan, x, out, group_of_block, pad, filled)
+    tensor_core.gemm_split_grouped(plan, x, out, group_of_block, pad, filled, workspace=workspace)
 
 
 def tensor_core_gemm_supports(outs: int, inner: int) -> bool:

@@ -238,13 +238,16 @@ def gemm_swiglu(
 
 # ------------------------------------------------------------------------------ float32
 
-# Tokens per CTA (up to 16 two CTAs share an SM and stream weights, else one) and the time of a k block, in blocks of 64 tokens
-# (1.13 us).  A round of CTAs costs SPLIT_START blocks beside them, a cluster's exchange SPLIT_EXCHANGE for each segment of 128
-# tokens.  Measured forms, us (64 tokens to a CTA and segments one after the other; 64 side by side; 128): 256 tokens x 6,144 x
-# 4,096 155, 154, 123; x 24,576 x 4,096 459, -, 324; x 4,096 x 4,096 80, 106, 83; 512 x 2,048 x 2,048 45, 100, 68; 512 x 9,216 x
-# 2,048 169, 198, 133; 64 x 6,144 x 4,096 78, 62, 80.
-SPLIT_TILES = {16: 1.0, 64: 1.0, 128: 1.44}
-SPLIT_START, SPLIT_EXCHANGE = 4.0, 0.8
+# Tokens per CTA (up to 16 two CTAs share an SM, else one) and the us of a k block.  A round of CTAs costs SPLIT_START beside them, a
+# cluster's exchange SPLIT_EXCHANGE for each segment of 128 tokens.  Clusters of 1 to 8 CTAs that are resident at a time with one CTA
+# to an SM (cudaOccupancyMaxActiveClusters on a B200; with two to an SM twice as many and a few more).  Measured forms, us (64 tokens to a
+# CTA and segments one after the other; 64 side by side; 128): 256 tokens x 6,144 x 4,096 98, 107, 99; x 24,576 x 4,096 306, -, 260; x
+# 4,096 x 4,096 54, 81, 71; 512 x 2,048 x 2,048 33, 84, 64; 512 x 9,216 x 2,048 115, 145, 114; 512 x 2,048 x 9,216 115, 170, 142;
+# 128 x 2,048 x 2,048 32, 30, 27; 64 x 2,048 x 9,216 101, 41, 55; 40 x 6,144 x 2,048 30, 30, 40.
+SPLIT_TILES = {16: 1.0, 64: 0.70, 128: 1.25}
+SPLIT_START, SPLIT_EXCHANGE = 5.0, 0.25
+SPLIT_CLUSTERS = (NUM_SMS, 74, 45, 33, 26, 22, 15, 15)
+SPLIT_PIECES_MIN_TILE = 64  # tokens per CTA from which on their pieces are made ahead, by a kernel of their own
 SPLIT_MIN_K_BLOCKS = 4  # of a segment
 # Shorter reductions stay on CUDA cores: a chain of fmaf over so few terms is about as exact as the short chain of the tensor
 # core (relative error of normal operands at 64: 1.5e-7 against 0.7e-7), and nothing is to be gained.
@@ -258,7 +261,9 @@ def _split_library():
         lib = load_library("gemm_split")
         lib.me_make_tensor_map_f32.argtypes = [c_void_p, c_void_p, c_ulonglong, c_ulonglong, c_uint]
         lib.me_make_tensor_map_f32.restype = c_int
-        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_int, c_int, c_void_p]
+        lib.me_make_tensor_map_pieces.argtypes = [c_void_p, c_void_p, c_ulonglong, c_ulonglong, c_uint]
+        lib.me_make_tensor_map_pieces.restype = c_int
+        lib.me_gemm_split.argtypes = [c_void_p] * 5 + [c_int] * 4 + [c_void_p] + [c_int] * 2 + [c_void_p, c_int, c_int, c_void_p]
         lib.me_gemm_split.restype = c_int
         lib.me_gemm_split_take_error.argtypes = [ctypes.POINTER(c_int)]
         lib.me_gemm_split_take_error.restype = c_int
@@ -290,8 +295,6 @@ def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | No
     CTA; the bits are the same in every form.  The form whose rounds of resident CTAs take least time."""
     blocks = -(-inner // BLOCK_K)
     per_segment = -(-blocks // segments)
-    # A cluster lies within a group of 16 to 18 SMs, of which there are eight: some SMs stay out of large clusters.
-    in_clusters = NUM_SMS if segments <= 2 else 8 * (17 // segments) * segments
     forms = []
     for rows, cost in SPLIT_TILES.items():
         if (rows != tile) if tile is not None else (rows == 16) != (tokens <= 16) or (rows == 128 and tokens <= 64):
@@ -301,7 +304,7 @@ def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | No
         if rows < 128 or segments == 1:
             forms.append((-(-ctas // (per_sm * NUM_SMS)) * (blocks * cost + SPLIT_START), rows, False))
         if segments > 1:
-            rounds = -(-ctas * segments // (per_sm * in_clusters))
+            rounds = -(-ctas // (per_sm * SPLIT_CLUSTERS[segments - 1]))
             forms.append((rounds * (per_segment * cost + SPLIT_START + SPLIT_EXCHANGE * segments * rows / 128), rows, True))
     return min(forms)[1:]
 
@@ -318,34 +321,36 @@ class SplitPlan:
             raise RuntimeError(f"{self.rows} weight rows do not form groups of {group_rows}")
         self.group_rows = group_rows
         self.segments = split_segments(group_rows or self.rows, self.inner)
-        self.map = _make_map_f32(weight, BLOCK_N)
+        self.map = _make_split_map(_split_library().me_make_tensor_map_f32, weight, self.rows, self.inner, BLOCK_N)
 
 
-def _make_map_f32(tensor: torch.Tensor, box_rows: int) -> ctypes.Array:
+def _make_split_map(make, tensor: torch.Tensor, rows: int, inner: int, box_rows: int) -> ctypes.Array:
     holder = (ctypes.c_ubyte * 128)()
-    rows, inner = tensor.shape
-    code = _split_library().me_make_tensor_map_f32(holder, tensor.data_ptr(), rows, inner, box_rows)
+    code = make(holder, tensor.data_ptr(), rows, inner, box_rows)
     if code != 0:
         raise RuntimeError(f"could not make a TMA descriptor for a {rows} x {inner} float32 matrix (code {code})")
     return holder
 
 
-_split_activation_maps: dict[tuple[int, int, int, int], ctypes.Array] = {}
+_split_activation_maps: dict[tuple[int, int, int, int, bool], ctypes.Array] = {}
 
 
-def _split_activation_map(x: torch.Tensor, tile: int) -> ctypes.Array:
-    key = (x.data_ptr(), x.shape[0], x.shape[1], tile)
+def _split_activation_map(x: torch.Tensor, tile: int, rows: int = 0, inner: int = 0) -> ctypes.Array:
+    """Of a float32 matrix, or (``rows`` given) of the pieces of one of ``rows`` x ``inner`` values."""
+    key = (x.data_ptr(), rows or x.shape[0], inner or x.shape[1], tile, rows > 0)
     held = _split_activation_maps.get(key)
     if held is None:
         if len(_split_activation_maps) > 8192:
             _split_activation_maps.clear()
-        held = _split_activation_maps[key] = _make_map_f32(x, tile)
+        make = _split_library().me_make_tensor_map_pieces if rows else _split_library().me_make_tensor_map_f32
+        held = _split_activation_maps[key] = _make_split_map(make, x, key[1], key[2], tile)
     return held
 
 
-def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[int, bool] | None = None) -> None:
+def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[int, bool] | None = None, workspace=None) -> None:
     """``out[T, rows] = x @ weight^T`` in float32 (three bfloat16 pieces of each operand, see gemm_split.cu).
-    ``form`` pins the tokens per CTA and where a tile's segments run instead of the rule's choice: the kernel tests run all."""
+    ``form`` pins the tokens per CTA and where a tile's segments run instead of the rule's choice: the kernel tests run all.
+    The tokens' pieces, where they are made ahead, lie in a buffer of the ``workspace``."""
     tokens = x.shape[0]
     if x.dtype != torch.float32 or not x.is_contiguous() or x.dim() != 2 or x.shape[1] != plan.inner or x.data_ptr() % 16:
         raise RuntimeError(f"activation {tuple(x.shape)} {x.dtype} does not fit a float32 weight of width {plan.inner}")
@@ -354,9 +359,25 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
     if tokens == 0:
         return
     tile, side_by_side = split_form(tokens, plan.rows, plan.inner, plan.segments) if form is None else form
+    _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, 0, workspace)
+
+
+def _launch_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, outs: int, tile: int, side_by_side: bool, group_of_block, group_rows: int, workspace) -> None:
+    rows, inner = x.shape
+    pieces = None
+    if tile >= SPLIT_PIECES_MIN_TILE:
+        count = 3 * rows * (-(-inner // 8) * 8)
+        if workspace is None:
+            held = torch.empty(count, dtype=torch.bfloat16, device=x.device)
+        else:
+            held = workspace.growing("split.pieces", (count,), torch.bfloat16)
+        pieces, x_map = held.data_ptr(), _split_activation_map(held, tile, rows, inner)
+        _count_launch()
+    else:
+        x_map = _split_activation_map(x, tile)
     code = _split_library().me_gemm_split(
-        plan.map, _split_activation_map(x, tile), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), tokens, plan.rows, plan.inner, tile,
-        plan.segments, 1 if side_by_side else 0, None, 0, 0, _ops_stream(),
+        plan.map, x_map, x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, inner, tile, pieces,
+        plan.segments, 1 if side_by_side else 0, group_of_block, group_rows, 0, _ops_stream(),
     )  # fmt: skip
     _count_launch()
     if code != 0:
@@ -364,8 +385,9 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
 
 
 def gemm_split_grouped(
-    plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, group_of_block: torch.Tensor, pad: int, filled: int, side_by_side: bool | None = None
-) -> None:
+    plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, group_of_block: torch.Tensor, pad: int, filled: int, side_by_side: bool | None = None,
+    workspace=None,
+) -> None:  # fmt: skip
     """A float32 product over rows that are sorted by group: the plan's weight holds ``plan.group_rows`` rows per group, run ``b``
     of ``pad`` rows of ``x`` (one of ``SPLIT_TILES``) belongs to group ``group_of_block[b]`` (int32 on the device; negative: no rows
     there), ``out[t] = x[t] @ weight_of_group^T``.  A row's bits depend on the row and its group's weight alone.  ``filled``:
@@ -381,13 +403,7 @@ def gemm_split_grouped(
         raise RuntimeError("the rows of a grouped product come in runs of a token tile with one int32 group each")
     if side_by_side is None:
         side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad)[1]
-    code = _split_library().me_gemm_split(
-        plan.map, _split_activation_map(x, pad), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, plan.inner, pad,
-        plan.segments, 1 if side_by_side else 0, group_of_block.data_ptr(), outs, 0, _ops_stream(),
-    )  # fmt: skip
-    _count_launch()
-    if code != 0:
-        raise RuntimeError(f"grouped float32 tensor-core product failed to launch (code {code})")
+    _launch_split(plan, x, out, outs, pad, side_by_side, group_of_block.data_ptr(), outs, workspace)
 
 
 GROUP_PAD = 128  # rows of a run of the sorted rows that belongs to one group: the token tile of the grouped product
@@ -444,7 +460,7 @@ def split_wait_probe(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_b
     if x.shape[1] != plan.inner or tuple(out.shape) != (x.shape[0], plan.rows) or not (x.is_contiguous() and out.is_contiguous()):
         raise RuntimeError("the probe takes the arguments of a product")
     code = _split_library().me_gemm_split(
-        plan.map, _split_activation_map(x, 16), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), x.shape[0], plan.rows, plan.inner, 16,
+        plan.map, _split_activation_map(x, 16), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), x.shape[0], plan.rows, plan.inner, 16, None,
         plan.segments, 1 if side_by_side else 0, None, 0, 1, _ops_stream(),
     )  # fmt: skip
     _count_launch()

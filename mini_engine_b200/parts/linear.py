@@ -75,7 +75,7 @@ class Linear:
         if self.tensor_core:
             ops.gemm_tensor_core(self.plan, x, out, splits)
         elif self.split_plan is not None and x.data_ptr() % 16 == 0:
-            ops.gemm_split(self.split_plan, x, out[0])
+            ops.gemm_split(self.split_plan, x, out[0], ctx.workspace)
         else:
             ops.gemm_simt(x, self.weight, out[0])
         return out

@@ -253,13 +253,13 @@ class RoutedExperts(FeedForward):
         if self.sorted32:
             filled = tokens * self.top // pad + min(self.units, tokens * self.top) // 2
             both = grow("routed.sorted_both", (1, capacity, self.sorted_gate_up.group_rows), torch.float32)
-            ops.gemm_split_grouped(self.sorted_gate_up, rows, both[0], unit_of_block, pad, filled)
+            ops.gemm_split_grouped(self.sorted_gate_up, rows, both[0], unit_of_block, pad, filled, ctx.workspace)
             if self.gated:
                 ops.swiglu(both, act, self.gate_slope, self.limit, self.up_offset)
             else:
                 ops.activation(both, act, self.activation)
             down = grow("routed.sorted_down", (capacity, self.hidden), torch.float32)
-            ops.gemm_split_grouped(self.sorted_down, act, down, unit_of_block, pad, filled)
+            ops.gemm_split_grouped(self.sorted_down, act, down, unit_of_block, pad, filled, ctx.workspace)
             return down, row_of
         if self.gated:
             ops.gemm_tensor_core_grouped(
