@@ -346,6 +346,195 @@ __global__ void __launch_bounds__(ROW_THREADS) paged_attention_rows_kernel(RowAr
     }
 }
 
+// ------------------------------------------------------------------ float32, few rows an entry (decoded tokens)
+//
+// The same bits for entries of at most 16 (token, head) rows per KV head, in two kernels.  In the kernel above such an entry is one block, whose tiles
+// follow each other: a tile of 32 keys takes the latency of a chain over the head, of a softmax and of a chain over its keys, 4 us
+// at heads of 128 and 11 over latent rows of 576, while most SMs are idle.  Only what a row's order of operations demands is serial here:
+// the scores of all tiles are independent (first kernel, a block to a tile), a tile's maximum needs its own scores, its weights the
+// running maximum, and the chains over the keys are separate for every value element (second kernel, a block to 64 value columns).
+// Eight decoded tokens behind 17 to 512, 16 heads in 8 KV heads of 128: 68 -> FIGA us; over latent rows of 576 with 512 values 179 -> FIGB.
+constexpr int FEW_ROWS = 16, FEW_TILES = 4, FEW_KEYS = 32 * FEW_TILES, FEW_COLUMNS = 64;  // rows of a block; tiles and keys of a step of the second kernel
+
+struct FewRows {
+    const AttnArgs& a;
+    int begin, rows, group, kv, lowest, last, tile0;  // of the block's entry and KV head
+    __device__ FewRows(const RowArgs& m, int entry, int kv_head) : a(m.a), group(m.a.heads / m.a.kv_heads), kv(kv_head) {
+        begin = m.cu_tokens[entry];
+        rows = (m.cu_tokens[entry + 1] - begin) * group;
+        if (rows <= 0) return;
+        lowest = lowest_of(position_of(0)), last = position_of(rows - 1);
+        tile0 = lowest / 32 * 32;
+    }
+    __device__ int position_of(int r) const { return a.positions[begin + r / group]; }
+    __device__ int head_of(int r) const { return kv * group + r % group; }
+    __device__ size_t item_of(int r) const { return static_cast<size_t>(begin + r / group) * a.heads + head_of(r); }
+    __device__ int lowest_of(int position) const {
+        const int low = a.window > 0 ? max(position - a.window + 1, 0) : 0;
+        return a.chunk > 0 ? max(low, position / a.chunk * a.chunk) : low;
+    }
+    __device__ int page_of(const int* table, int key) const { return key >= lowest && key <= last ? table[key / a.page_size] : -1; }
+    __device__ size_t cached_row(int page, int key) const { return (static_cast<size_t>(page) * a.kv_heads + kv) * a.page_size + key % a.page_size; }
+};
+
+// scores[token][head][key - tile0] = q . k, for the tiles blockIdx.x, + gridDim.x, ... of the entry.
+__global__ void __launch_bounds__(ROW_THREADS) few_rows_scores_kernel(RowArgs m, float* scores, int capacity) {
+    extern __shared__ __align__(16) float few_shared[];
+    const AttnArgs& a = m.a;
+    const int d = a.head_dim, kp = d + 4;
+    float *q = few_shared, *keys = q + FEW_ROWS * kp;  // [FEW_ROWS][kp], [32][kp]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_trigger();
+    pdl_wait();
+    const FewRows e(m, blockIdx.z, blockIdx.y);
+    if (e.rows <= 0 || e.tile0 + 32 * static_cast<int>(blockIdx.x) > e.last) return;
+    const int* table = a.block_table + static_cast<size_t>(blockIdx.z) * a.table_width;
+    for (int i = tid; i < e.rows * (d / 4); i += ROW_THREADS) {
+        const int r = i / (d / 4), x = i % (d / 4) * 4;
+        *reinterpret_cast<float4*>(q + r * kp + x) = *reinterpret_cast<const float4*>(static_cast<const float*>(a.q) + e.item_of(r) * d + x);
+    }
+    for (int tile = e.tile0 + 32 * blockIdx.x; tile <= e.last; tile += 32 * gridDim.x) {
+        __syncthreads();  // the keys of the tile before are read
+        const int key = tile + (tid >> 3), page = e.page_of(table, key);
+        const float* from = static_cast<const float*>(a.k_pages) + (page >= 0 ? e.cached_row(page, key) * d : 0);
+        for (int x = (tid & 7) * 4; x < d; x += 32) cp_async_16(keys + (tid >> 3) * kp + x, from + x, page >= 0);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        for (int r = warp; r < e.rows; r += 2 * (ROW_THREADS / 32)) {  // a key to a lane, two rows at a time
+            const int other = r + ROW_THREADS / 32 < e.rows ? r + ROW_THREADS / 32 : r;
+            const float *k = keys + lane * kp, *q0 = q + r * kp, *q1 = q + other * kp;
+            float dot0 = 0.0f, dot1 = 0.0f;
+#pragma unroll 8
+            for (int x = 0; x < d; x += 4) {
+                const float4 kk = *reinterpret_cast<const float4*>(k + x), u = *reinterpret_cast<const float4*>(q0 + x), v = *reinterpret_cast<const float4*>(q1 + x);
+                dot0 = fmaf(u.x, kk.x, dot0), dot1 = fmaf(v.x, kk.x, dot1);
+                dot0 = fmaf(u.y, kk.y, dot0), dot1 = fmaf(v.y, kk.y, dot1);
+                dot0 = fmaf(u.z, kk.z, dot0), dot1 = fmaf(v.z, kk.z, dot1);
+                dot0 = fmaf(u.w, kk.w, dot0), dot1 = fmaf(v.w, kk.w, dot1);
+            }
+            scores[e.item_of(r) * capacity + (tile - e.tile0) + lane] = dot0;
+            scores[e.item_of(other) * capacity + (tile - e.tile0) + lane] = dot1;
+        }
+    }
+}
+
+// Softmax and values of 64 value columns.  A step is four tiles: every (row, tile) gets a warp of its own for the scores' maximum and, with the
+// running maximum known, for the weights; then a thread adds a quad of columns of one row up over the step's keys.
+__global__ void __launch_bounds__(ROW_THREADS) few_rows_values_kernel(RowArgs m, const float* scores, int capacity) {
+    extern __shared__ __align__(16) float few_values[];
+    float(*values)[FEW_KEYS][FEW_COLUMNS] = reinterpret_cast<float(*)[FEW_KEYS][FEW_COLUMNS]>(few_values);  // [2]
+    __shared__ __align__(16) float weights[FEW_ROWS][FEW_KEYS];
+    __shared__ float tile_max[FEW_ROWS][FEW_TILES], tile_sum[FEW_ROWS][FEW_TILES], tile_scale[FEW_ROWS][FEW_TILES], row_max[FEW_ROWS], row_sum[FEW_ROWS];
+    __shared__ int key_there[2][FEW_KEYS];
+    const AttnArgs& a = m.a;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, column0 = blockIdx.x * FEW_COLUMNS, columns = min(FEW_COLUMNS, a.value_dim - column0);
+    pdl_trigger();
+    pdl_wait();
+    const FewRows e(m, blockIdx.z, blockIdx.y);
+    if (e.rows <= 0) return;
+    const int* table = a.block_table + static_cast<size_t>(blockIdx.z) * a.table_width;
+    const bool sigmoid = a.sigmoid_bias != nullptr;
+    if (tid < FEW_ROWS) row_max[tid] = -INFINITY, row_sum[tid] = 0.0f;
+    auto fetch = [&](int first, int buffer) {  // two threads to a key
+        const int j = tid >> 1, key = first + j, page = e.page_of(table, key);
+        const float* from = static_cast<const float*>(a.v_pages) + (page >= 0 ? e.cached_row(page, key) * a.value_stride + column0 : 0);
+        for (int x = (tid & 1) * 4; x < columns; x += 8) cp_async_16(&values[buffer][j][x], from + x, page >= 0);
+        if ((tid & 1) == 0) key_there[buffer][j] = page >= 0;
+        cp_async_commit();
+    };
+    const int my_row = tid / (FEW_COLUMNS / 4), quad = tid % (FEW_COLUMNS / 4) * 4;
+    const bool adds = my_row < e.rows && quad < columns;
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int buffer = 0;
+    fetch(e.tile0, 0);
+    for (int first = e.tile0; first <= e.last; first += FEW_KEYS, buffer ^= 1) {
+        if (first + FEW_KEYS <= e.last) fetch(first + FEW_KEYS, buffer ^ 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        for (int i = warp; i < e.rows * FEW_TILES; i += ROW_THREADS / 32) {
+            const int r = i / FEW_TILES, t = i % FEW_TILES, key = first + 32 * t + lane, position = e.position_of(r), head = e.head_of(r);
+            const bool seen = key_there[buffer][32 * t + lane] != 0 && key >= e.lowest_of(position) && key <= position;
+            float score = -INFINITY;
+            if (seen) {
+                score = scores[e.item_of(r) * capacity + (key - e.tile0)] * a.scale;
+                if (a.softcap > 0.0f) score = a.softcap * tanhf(score / a.softcap);
+                if (a.slopes) score -= a.slopes[head] * static_cast<float>(position - key);
+            }
+            if (sigmoid) {
+                weights[r][32 * t + lane] = seen ? 1.0f / (1.0f + expf(-(score + a.sigmoid_bias[head]))) : __uint_as_float(UNSEEN);
+            } else {
+                weights[r][32 * t + lane] = seen ? score : __uint_as_float(UNSEEN);
+                const float best = warp_max(score);
+                if (lane == 0) tile_max[r][t] = best;
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, seen);
+            if (lane == 0) tile_sum[r][t] = __uint_as_float(mask);  // which keys the row sees, until the sums take its place
+        }
+        __syncthreads();
+        if (!sigmoid) {
+            for (int i = warp; i < e.rows * FEW_TILES; i += ROW_THREADS / 32) {
+                const int r = i / FEW_TILES, t = i % FEW_TILES;
+                float old_max = row_max[r];
+                for (int before = 0; before < t; ++before) old_max = fmaxf(old_max, tile_max[r][before]);
+                const float new_max = fmaxf(old_max, tile_max[r][t]);
+                float rescale = 1.0f, sum = 0.0f;
+                if (new_max != -INFINITY) {  // uniform across the warp
+                    const bool seen = __float_as_uint(tile_sum[r][t]) >> lane & 1;
+                    rescale = expf(old_max - new_max);
+                    const float weight = seen ? expf(weights[r][32 * t + lane] - new_max) : 0.0f;
+                    sum = warp_sum(weight);
+                    if (seen) weights[r][32 * t + lane] = weight;
+                } else {
+                    weights[r][32 * t + lane] = __uint_as_float(UNSEEN);
+                }
+                __syncwarp();
+                if (lane == 0) tile_scale[r][t] = rescale, tile_sum[r][t] = sum;
+            }
+            __syncthreads();
+            if (tid < e.rows) {
+                float best = row_max[tid], sum = row_sum[tid];
+                for (int t = 0; t < FEW_TILES; ++t) {
+                    best = fmaxf(best, tile_max[tid][t]);
+                    if (best != -INFINITY) sum = sum * tile_scale[tid][t] + tile_sum[tid][t];
+                }
+                row_max[tid] = best, row_sum[tid] = sum;
+            }
+        }
+        if (adds) {
+            for (int t = 0; t < FEW_TILES; ++t) {
+                if (!sigmoid) {
+                    const float f = tile_scale[my_row][t];
+                    acc.x *= f, acc.y *= f, acc.z *= f, acc.w *= f;
+                }
+#pragma unroll 8
+                for (int j = 32 * t; j < 32 * t + 32; ++j) {
+                    const float w = weights[my_row][j];
+                    const float4 v = *reinterpret_cast<const float4*>(&values[buffer][j][quad]);
+                    if (__float_as_uint(w) == UNSEEN) continue;
+                    acc.x = fmaf(w, v.x, acc.x), acc.y = fmaf(w, v.y, acc.y), acc.z = fmaf(w, v.z, acc.z), acc.w = fmaf(w, v.w, acc.w);
+                }
+            }
+        }
+        __syncthreads();  // the next copies overwrite this buffer, the next step the weights
+    }
+    cp_async_wait<0>();
+    if (!adds) return;
+    const int head = e.head_of(my_row);
+    float denom = row_sum[my_row];
+    if (a.sink) denom += expf((a.sink_values ? a.sink_values[head] : 0.0f) - row_max[my_row]);  // the silent participant
+    float inv = sigmoid ? 1.0f : 1.0f / denom;
+    const size_t at = e.item_of(my_row);
+    if (a.gate && a.gate_width == 1) inv *= a.gate[at];
+    float4 y = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+    if (a.gate && a.gate_width > 1) {
+        const float* g = a.gate + at * a.gate_width + column0 + quad;
+        y.x *= g[0], y.y *= g[1], y.z *= g[2], y.w *= g[3];
+    }
+    *reinterpret_cast<float4*>(static_cast<float*>(a.out) + at * a.value_dim + column0 + quad) = y;
+}
+
 static size_t rows_shared_bytes(const AttnArgs& a, int rows) {
     const size_t kp = a.head_dim + 4, vp = a.k_pages == a.v_pages ? 0 : a.value_dim + 4;
     return (rows * kp + 64 * (kp + vp) + static_cast<size_t>(rows) * 36) * sizeof(float);
@@ -383,13 +572,14 @@ ME_EXPORT int me_paged_attention_rows_supports(int head_dim, int value_dim, int 
 }
 
 // The attention of me_paged_attention_generic in float32, with its bits.  The tokens of entry e are cu_tokens[e] ..
-// cu_tokens[e + 1], in ascending position; no entry has more than `longest`.
+// cu_tokens[e + 1], in ascending position; no entry has more than `longest`.  With `scores` (room for tokens x heads x `capacity`
+// floats, a multiple of 32 that no entry's visible keys, from their tile's start on, pass) entries of at most 16 rows take the two kernels for few rows.
 ME_EXPORT int me_paged_attention_rows(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                       const int* cu_tokens, const int* positions, void* out, float scale, int entries, int longest,
                                       int heads, int kv_heads, int head_dim, int page_size, int table_width, int window,
                                       int value_dim, int sink, const float* gate, int gate_width, int value_stride,
                                       const float* slopes, const float* sink_values, float softcap, int chunk,
-                                      const float* sigmoid_bias, cudaStream_t stream) {
+                                      const float* sigmoid_bias, float* scores, int capacity, cudaStream_t stream) {
     if (entries <= 0 || longest <= 0) return 0;
     if (gate && gate_width != 1 && gate_width != value_dim) return ME_ERR_ARGUMENT;
     if (value_stride < value_dim || chunk < 0 || (sigmoid_bias && sink)) return ME_ERR_ARGUMENT;
@@ -402,6 +592,17 @@ ME_EXPORT int me_paged_attention_rows(const void* q, const void* k_pages, const 
     // 64 rows share a key where an entry brings that many; else 16, whose tiles take a third of the time.  Two blocks of
     // 64 rows fit an SM up to heads of 128.
     const long long rows = static_cast<long long>(longest) * (heads / kv_heads);
+    if (scores != nullptr) {
+        const size_t bytes = (FEW_ROWS + 32) * static_cast<size_t>(head_dim + 4) * sizeof(float);
+        if (rows > FEW_ROWS || capacity < 32 || capacity % 32 || kv_heads > 65535 || entries > 65535 || bytes > 200 * 1024) return ME_ERR_ARGUMENT;
+        static SharedMemoryOptIn opt_in, values_opt_in;
+        if (const int e = opt_in(few_rows_scores_kernel, 200 * 1024)) return e;
+        if (const int e = values_opt_in(few_rows_values_kernel, 2 * FEW_KEYS * FEW_COLUMNS * sizeof(float))) return e;
+        const int tiles = capacity / 32 < 64 ? capacity / 32 : 64;
+        if (const int e = launch_kernel(few_rows_scores_kernel, dim3(tiles, kv_heads, entries), ROW_THREADS, bytes, stream, m, scores, capacity)) return e;
+        return launch_kernel(few_rows_values_kernel, dim3((value_dim + FEW_COLUMNS - 1) / FEW_COLUMNS, kv_heads, entries), ROW_THREADS,
+                             2 * FEW_KEYS * FEW_COLUMNS * sizeof(float), stream, m, scores, capacity);
+    }
     if (rows > 32 && rows_shared_bytes(m.a, 64) <= 113 * 1024) return launch_rows_of<64>(m, entries, longest, stream);
     return launch_rows_of<16>(m, entries, longest, stream);
 }

@@ -562,27 +562,50 @@ def paged_attention_rows(
     q, k_pages, v_pages, block_table, ctx, out, heads, kv_heads, head_dim, scale, window,
     value_dim: int | None = None, sink: bool = False, gate: torch.Tensor | None = None,
     slopes: torch.Tensor | None = None, sink_values: torch.Tensor | None = None, softcap: float = 0.0, chunk: int = 0,
-    sigmoid_bias: torch.Tensor | None = None,
+    sigmoid_bias: torch.Tensor | None = None, scores: torch.Tensor | None = None,
 ) -> None:  # fmt: skip
     """:func:`paged_attention_generic` in float32 with its bits, every key fetched once for 64 or 16 (token, head) rows
-    of an entry.  The context gives ``cu_tokens``, ``num_entries``, ``max_query_len`` and ``positions`` (ascending within an entry)."""
+    of an entry.  The context gives ``cu_tokens``, ``num_entries``, ``max_query_len`` and ``positions`` (ascending within an entry).  With
+    ``scores`` (float32 ``[T, heads, capacity]``, see :func:`few_rows_capacity`) entries of few rows take two kernels whose blocks share their keys out."""
     v_pages, value_dim, gate_width, value_stride = _check_generic_attention(
         q, k_pages, v_pages, out, heads, kv_heads, head_dim, value_dim, gate, slopes, sink_values, sigmoid_bias
     )
     _need(q, torch.float32, "q"), _need(block_table, torch.int32, "block_table"), _need(ctx.positions, torch.int32, "positions")
     _need(ctx.cu_tokens, torch.int32, "cu_tokens")
+    if scores is not None:
+        _need(scores, torch.float32, "scores")
+        if scores.dim() != 3 or scores.shape[0] != q.shape[0] or scores.shape[1] != heads:
+            raise KernelError(f"scores {tuple(scores.shape)} are not [{q.shape[0]}, {heads}, capacity]")
+        _Counter.launches += 1  # one kernel more
     fn = _fn(
         "attention_generic",
         "me_paged_attention_rows",
-        [c_void_p] * 7 + [c_float] + [c_int] * 9 + [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p],
+        [c_void_p] * 7 + [c_float] + [c_int] * 9
+        + [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p, c_int, c_void_p],
     )
     code = fn(
         _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), _ptr(ctx.cu_tokens), _ptr(ctx.positions), _ptr(out), scale,
         ctx.num_entries, ctx.max_query_len, heads, kv_heads, head_dim, k_pages.shape[2], block_table.shape[1], window, value_dim,
         1 if (sink or sink_values is not None) else 0, _ptr(gate), gate_width, value_stride, _ptr(slopes), _ptr(sink_values),
-        float(softcap or 0.0), int(chunk), _ptr(sigmoid_bias), _stream(),
+        float(softcap or 0.0), int(chunk), _ptr(sigmoid_bias), _ptr(scores), 0 if scores is None else scores.shape[2], _stream(),
     )  # fmt: skip
     _check(code, "paged_attention_rows")
+
+
+FEW_ROWS = 16  # (token, head) rows per KV head up to which an entry takes the two kernels for few rows ...
+FEW_ROWS_MIN_CONTEXT = 64  # ... from more keys than this on: two tiles in one block take as long as the second launch
+FEW_ROWS_MAX_SCRATCH = 256 << 20  # bytes of scores; larger steps take the one kernel
+
+
+def few_rows_capacity(tokens: int, longest: int, heads: int, kv_heads: int, context: int, window: int) -> int:
+    """Scores per (token, head) that a step's scratch must hold when its entries, of at most ``longest`` tokens and ``context`` keys,
+    take the two kernels for few rows; 0 when they do not.  Of the sizes alone, so that a captured step takes the form it was captured with."""
+    if window > 0:
+        context = min(context, window + longest + 31)  # from the start of the first visible key's tile on
+    if longest * (heads // kv_heads) > FEW_ROWS or context <= FEW_ROWS_MIN_CONTEXT:
+        return 0
+    capacity = -(-context // 32) * 32
+    return capacity if 4 * tokens * heads * capacity <= FEW_ROWS_MAX_SCRATCH else 0
 
 
 def paged_attention(
@@ -608,9 +631,13 @@ def paged_attention(
             )  # fmt: skip
             return
     if q.dtype == torch.float32 and attention_rows_supports(q, k_pages, v_pages, out, head_dim, value_dim):
+        scores, workspace = None, getattr(ctx, "workspace", None)
+        capacity = 0 if workspace is None else few_rows_capacity(q.shape[0], ctx.max_query_len, heads, kv_heads, ctx.max_context_len, window)
+        if capacity:
+            scores = workspace.growing("attn.row_scores", (q.shape[0], heads, capacity), torch.float32)
         paged_attention_rows(
             q, k_pages, v_pages, block_table, ctx, out, heads, kv_heads, head_dim, scale, window, value_dim=value_dim, sink=sink,
-            gate=gate, slopes=slopes, sink_values=sink_values, softcap=softcap, chunk=chunk, sigmoid_bias=sigmoid_bias,
+            gate=gate, slopes=slopes, sink_values=sink_values, softcap=softcap, chunk=chunk, sigmoid_bias=sigmoid_bias, scores=scores,
         )  # fmt: skip
         return
     paged_attention_generic(
