@@ -166,6 +166,8 @@ def set_programmatic_launch(enabled: bool) -> bool:
     global _programmatic_launch
     with _lock:
         previous, _programmatic_launch = _programmatic_launch, bool(enabled)
+        if previous == _programmatic_launch:  # a library is told when it is loaded and at every change
+            return previous
         for library in _loaded.values():
             if hasattr(library, "me_set_programmatic_launch"):
                 library.me_set_programmatic_launch(ctypes.c_int(1 if enabled else 0))

@@ -33,8 +33,8 @@ def _type_code(dtype: torch.dtype) -> int:
     raise KernelError(f"kernels take float32 or bfloat16, got {dtype}")
 
 
-def _ptr(tensor: torch.Tensor | None) -> c_void_p:
-    return c_void_p(0 if tensor is None else tensor.data_ptr())
+def _ptr(tensor: torch.Tensor | None) -> int:
+    return 0 if tensor is None else tensor.data_ptr()
 
 
 _scoped_stream: c_void_p | None = None
@@ -145,16 +145,16 @@ def _need(tensor: torch.Tensor, dtype: torch.dtype | None, name: str) -> None:
         raise KernelError(f"{name} must be {dtype}, got {tensor.dtype}")
 
 
-_signatures_done: set[str] = set()
+_functions: dict[tuple[str, str], Any] = {}  # with their signatures set; a library stays loaded
 
 
 def _fn(library: str, name: str, argtypes: list[Any]):
-    lib = load_library(library)
-    fn = getattr(lib, name)
-    if name not in _signatures_done:
+    fn = _functions.get((library, name))
+    if fn is None:
+        fn = getattr(load_library(library), name)
         fn.argtypes = argtypes
         fn.restype = c_int
-        _signatures_done.add(name)
+        _functions[(library, name)] = fn
     return fn
 
 
@@ -550,8 +550,7 @@ def paged_attention_generic(
 def attention_rows_supports(q, k_pages, v_pages, out, head_dim: int, value_dim: int | None) -> bool:
     """Whether float32 attention of these sizes and buffers takes the kernel whose blocks share every key among many rows."""
     value_dim = head_dim if value_dim is None else value_dim
-    fn = load_library("attention_generic").me_paged_attention_rows_supports
-    fn.argtypes, fn.restype = [c_int] * 4, c_int
+    fn = _fn("attention_generic", "me_paged_attention_rows_supports", [c_int] * 4)
     values = k_pages if v_pages is None else v_pages
     return bool(fn(head_dim, value_dim, head_dim if v_pages is None else value_dim, 1 if v_pages is None else 0)) and all(
         t.data_ptr() % 16 == 0 for t in (q, k_pages, values, out)

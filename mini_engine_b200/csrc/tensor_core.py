@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 from ctypes import c_int, c_uint, c_ulonglong, c_void_p
+from functools import lru_cache
 
 import torch
 
@@ -91,6 +92,7 @@ def token_tile(tokens: int) -> int:
     return TOKEN_TILES[-1]
 
 
+@lru_cache(maxsize=4096)
 def choose_splits(tokens: int, outs: int, inner: int, max_splits: int = 8) -> int:
     """How many ranges the reduction axis is cut into.  It depends on the sizes only (for a
     given number of tokens the same split is always chosen), and no split is empty."""
@@ -290,6 +292,7 @@ def split_segments(outs: int, inner: int) -> int:
     return -(-k_blocks // per_segment)
 
 
+@lru_cache(maxsize=4096)
 def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | None = None) -> tuple[int, bool]:
     """Tokens per CTA (or the given ``tile``), and whether a tile's segments run in the CTAs of a cluster or one after the other in a
     CTA; the bits are the same in every form.  The form whose rounds of resident CTAs take least time."""

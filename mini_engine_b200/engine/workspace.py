@@ -25,6 +25,22 @@ class Workspace:
         # buffer it was captured with and goes on writing and reading there, so the memory must
         # neither be freed nor given to anyone else.
         self._retired: list[torch.Tensor] = []
+        # The views handed out of each buffer, by how they were asked for: a step asks for some hundred, and making one
+        # (two calls into torch) takes 3 us, a fifth of what the host spends on a launch.
+        self._views: dict[tuple[str, torch.dtype], dict[tuple, torch.Tensor]] = {}
+
+    def _view(self, name: str, dtype: torch.dtype, shape: tuple[int, ...], elements: int) -> torch.Tensor:
+        """``shape`` at the start of the named buffer, which holds at least ``elements``."""
+        flat = self._flat(name, elements, dtype)
+        views = self._views.setdefault((name, dtype), {})
+        if len(views) >= 64:  # steps of many token counts
+            views.clear()
+        view = views[shape] = flat[: math.prod(shape)].view(shape)
+        return view
+
+    def _held_view(self, name: str, dtype: torch.dtype, shape: tuple[int, ...]) -> torch.Tensor | None:
+        views = self._views.get((name, dtype))
+        return None if views is None else views.get(shape)
 
     def _flat(self, name: str, elements: int, dtype: torch.dtype) -> torch.Tensor:
         key = (name, dtype)
@@ -34,6 +50,7 @@ class Workspace:
                 raise RuntimeError(f"workspace buffer {name!r} would have to grow during graph capture")
             if held is not None:
                 self._retired.append(held)
+                self._views.pop(key, None)
             held = torch.empty(elements, dtype=dtype, device=self.device)
             self._buffers[key] = held
         return held
@@ -41,27 +58,32 @@ class Workspace:
     def get(self, name: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """A contiguous view ``shape`` of the named buffer.  The first axis is a token count;
         the buffer is sized for ``max_tokens`` of them."""
-        per_row = math.prod(shape[1:])
-        rows = max(shape[0], self.max_tokens)
-        flat = self._flat(name, rows * per_row, dtype)
-        return flat[: shape[0] * per_row].view(shape)
+        held = self._held_view(name, dtype, shape)
+        if held is not None:
+            return held
+        return self._view(name, dtype, shape, max(shape[0], self.max_tokens) * math.prod(shape[1:]))
 
     def partials(self, name: str, splits: int, tokens: int, width: int) -> torch.Tensor:
         """``[splits, tokens, width]`` float32 for the partial sums of a split product."""
-        rows = max(partial_rows(self.max_tokens), splits * tokens)
-        flat = self._flat(name, rows * width, torch.float32)
-        return flat[: splits * tokens * width].view(splits, tokens, width)
+        shape = (splits, tokens, width)
+        held = self._held_view(name, torch.float32, shape)
+        if held is not None:
+            return held
+        return self._view(name, torch.float32, shape, max(partial_rows(self.max_tokens), splits * tokens) * width)
 
     def growing(self, name: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """A buffer of exactly ``shape`` that grows on demand instead of being sized for the
         token capacity (logits: ``[rows, vocab]`` is large and ``rows`` is usually small).  It grows
         by half at least, so that steps of ever longer prompts do not leave one buffer behind for
         every length: all that it has ever replaced is less than twice what it holds."""
+        view = self._held_view(name, dtype, shape)
+        if view is not None:
+            return view
         elements = math.prod(shape)
         held = self._buffers.get((name, dtype))
         if held is not None and held.numel() < elements:
             self._flat(name, max(elements, held.numel() + held.numel() // 2), dtype)
-        return self._flat(name, elements, dtype)[:elements].view(shape)
+        return self._view(name, dtype, shape, elements)
 
     def zeroed(self, name: str, count: int) -> torch.Tensor:
         """``count`` int32 values that are zero when first handed out.  Kernels that use them
@@ -73,6 +95,7 @@ class Workspace:
                 raise RuntimeError(f"workspace buffer {name!r} would have to grow during graph capture")
             if held is not None:
                 self._retired.append(held)
+                self._views.pop(key, None)
             held = torch.zeros(max(count, 1024), dtype=torch.int32, device=self.device)
             self._buffers[key] = held
         return held[:count]
