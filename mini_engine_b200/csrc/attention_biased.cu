@@ -628,6 +628,134 @@ __global__ void __launch_bounds__(WARPS * 32) attention_mix_values_kernel(ScoreA
     }
 }
 
+// The same for bfloat16 values in rows of whole 16-byte pieces, up to 128 wide, when few blocks of sixteen warps run (decoded tokens): a tile's values
+// are on their way into shared memory, all 32 keys at once, while its weights are formed, and a lane adds four neighbouring
+// columns up, so that a key costs a warp one load of values and one of weights instead of four loads and a shuffle per head.  The kernel above fetches four keys at a
+// time, eight trips to memory a tile, behind the scores.  The order of every sum is the same, so are the bits.  16 heads in 8 KV heads of 128, eight tokens behind 16 to
+// 2,048 keys (window 1,024, 64 kept): 61 -> 27 us.
+constexpr int STAGED_WARPS = 16;
+
+template <int GROUP>
+__global__ void __launch_bounds__(STAGED_WARPS * 32) mix_values_staged_kernel(ScoreArgs s, const float* __restrict__ talk) {
+    constexpr int AT_ONCE = 8;
+    const BiasedArgs& a = s.a;
+    extern __shared__ __align__(16) float mix_shared[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int token = blockIdx.x / a.kv_heads, kv = blockIdx.x % a.kv_heads;
+    const int heads = a.heads, group = heads / a.kv_heads, vd = a.vdim, pieces = vd / 8;
+    float* weights = mix_shared + warp * 32 * GROUP;                                                               // [32][GROUP] of this warp
+    __nv_bfloat16* values = reinterpret_cast<__nv_bfloat16*>(mix_shared + STAGED_WARPS * 32 * GROUP) + warp * 32 * vd;  // [32][vd] of this warp
+    float* partial = mix_shared + STAGED_WARPS * 32 * GROUP;                                                       // [WARPS][group][vd], when all is added
+    float* top = partial + STAGED_WARPS * 16 * vd;                                                                 // [heads]
+    float* inverse = top + heads;                                                                                  // [heads] 1 / denominator
+    float* mixing = inverse + heads;                                                                               // [heads][GROUP] columns of the mixing matrix for this group's heads
+    pdl_trigger();
+    for (int i = threadIdx.x; i < GROUP * heads; i += STAGED_WARPS * 32) mixing[i] = i % GROUP < group ? talk[(kv * group + i % GROUP) * heads + i / GROUP] : 0.0f;
+    pdl_wait();
+    if (s.tiles.cu_tokens && takes_tiles(s.tiles, a, a.entry_of_token[token])) return;
+    for (int g = threadIdx.x; g < heads; g += STAGED_WARPS * 32) {
+        const float* st = s.stats + (static_cast<size_t>(token) * heads + g) * 2;
+        top[g] = st[0];
+        inverse[g] = 1.0f / st[1];
+    }
+    __syncthreads();
+    const int position = a.positions[token];
+    const int* table = a.block_table + static_cast<size_t>(a.entry_of_token[token]) * a.table_width;
+    const __nv_bfloat16* v_pages = static_cast<const __nv_bfloat16*>(a.v_pages);
+    const int lowest = a.window > 0 ? max(position - a.window + 1, 0) : 0;
+    const int kept_end = a.window > 0 ? min(a.keep_first, lowest) : 0;
+    const float* rows = s.scores + static_cast<size_t>(token) * heads * s.stride;
+    float acc[GROUP][4];
+#pragma unroll
+    for (int h = 0; h < GROUP; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[h][i] = 0.0f;
+    for (int run = 0; run < 2; ++run) {
+        const int from = run == 0 ? 0 : lowest, to = run == 0 ? kept_end - 1 : position;  // inclusive
+        for (int tile = (from / 32) * 32; tile <= to; tile += 32) {
+            if ((tile >> 5) % STAGED_WARPS != warp) continue;
+            const int key = tile + lane;
+            long long value_row = -1;  // element offset of this key's values in this KV head
+            if (key >= from && key <= to) {
+                const int page = table[key / a.page_size];
+                if (page >= 0) value_row = ((static_cast<long long>(page) * a.kv_heads + kv) * a.page_size + key % a.page_size) * vd;
+            }
+            const unsigned there = __ballot_sync(0xffffffffu, value_row >= 0);
+            __syncwarp();  // the values of the tile before are read
+            for (int c = lane; c < 32 * pieces; c += 32) {  // all lanes in every turn
+                const int j = c / pieces, piece = c % pieces;
+                const long long row = __shfl_sync(0xffffffffu, value_row, j);
+                cp_async_16(values + j * vd + piece * 8, v_pages + max(row, 0ll) + piece * 8, row >= 0);
+            }
+            cp_async_commit();
+            float mixed[GROUP];
+#pragma unroll
+            for (int h = 0; h < GROUP; ++h) mixed[h] = 0.0f;
+            if (value_row >= 0) {
+                const float* column = rows + (run == 0 ? key : kept_end + (key - lowest));
+                for (int g0 = 0; g0 < heads; g0 += AT_ONCE) {  // ascending g: the order of the mixed sum
+                    float score[AT_ONCE];
+#pragma unroll
+                    for (int i = 0; i < AT_ONCE; ++i) score[i] = g0 + i < heads ? column[static_cast<size_t>(g0 + i) * s.stride] : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < AT_ONCE; ++i) {
+                        const int g = g0 + i;
+                        if (g >= heads) break;
+                        const float w = expf(score[i] - top[g]) * inverse[g];
+#pragma unroll
+                        for (int h = 0; h < GROUP; ++h) mixed[h] = fmaf(mixing[g * GROUP + h], w, mixed[h]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < GROUP; ++h) weights[lane * GROUP + h] = mixed[h];
+            cp_async_wait<0>();
+            __syncwarp();
+            if (lane * 4 < vd) {
+#pragma unroll 8
+                for (int j = 0; j < 32; ++j) {
+                    float w[GROUP];
+#pragma unroll
+                    for (int h = 0; h < GROUP; ++h) w[h] = weights[j * GROUP + h];
+                    const uint2 pair = *reinterpret_cast<const uint2*>(values + j * vd + lane * 4);
+                    if (!(there >> j & 1)) continue;  // uniform across the warp
+                    const float v[4] = {__uint_as_float(pair.x << 16), __uint_as_float(pair.x & 0xffff0000u), __uint_as_float(pair.y << 16), __uint_as_float(pair.y & 0xffff0000u)};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int h = 0; h < GROUP; ++h) acc[h][i] = fmaf(w[h], v[i], acc[h][i]);
+                }
+            }
+        }
+    }
+    __syncthreads();  // the partial sums take the values' place
+    if (lane * 4 < vd)
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h)
+            if (h < group) *reinterpret_cast<float4*>(partial + (warp * group + h) * vd + lane * 4) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+    __syncthreads();
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + (static_cast<size_t>(token) * heads + kv * group) * vd;
+    for (int i = threadIdx.x; i < group * vd; i += STAGED_WARPS * 32) {
+        float sum = 0.0f;
+        for (int w = 0; w < STAGED_WARPS; ++w) sum += partial[w * group * vd + i];
+        out[i] = __float2bfloat16_rn(sum);
+    }
+}
+
+// Whether the staged kernel takes these sizes; its partial sums lie where the values were.
+static bool staged_takes(const ScoreArgs& s) {
+    const BiasedArgs& a = s.a;
+    return a.vdim % 8 == 0 && a.vdim <= 128 && reinterpret_cast<uintptr_t>(a.v_pages) % 16 == 0 && a.heads <= 128;
+}
+
+template <int GROUP>
+static int launch_staged(const ScoreArgs& s, const float* talk, cudaStream_t stream) {
+    const size_t smem = (static_cast<size_t>(STAGED_WARPS) * 32 * GROUP + static_cast<size_t>(STAGED_WARPS) * 16 * s.a.vdim + (2 + GROUP) * s.a.heads) * sizeof(float);
+    static SharedMemoryOptIn opt_in;
+    if (const int code = opt_in(mix_values_staged_kernel<GROUP>, 200 * 1024)) return code;
+    return launch_kernel_in_order(mix_values_staged_kernel<GROUP>, s.a.tokens * s.a.kv_heads, STAGED_WARPS * 32, smem, stream, s, talk);
+}
+
 template <typename T, int WARPS, int GROUP, int COLUMNS>
 static int launch_mix_values(const ScoreArgs& s, const float* talk, size_t smem, cudaStream_t stream) {
     static SharedMemoryOptIn opt_in;
@@ -647,6 +775,13 @@ static int launch_two_kernels(const ScoreArgs& s, const float* talk, cudaStream_
     if (smem1 > 48 * 1024 || smem2 > 200 * 1024) return ME_ERR_UNSUPPORTED;
     int code = launch_kernel_in_order(attention_scores_kernel<T, WARPS>, a.tokens * a.heads, WARPS * 32, smem1, stream, s);
     if (code) return code;
+    if constexpr (std::is_same<T, __nv_bfloat16>::value && WARPS == STAGED_WARPS) {
+        if (staged_takes(s)) {
+            if (group <= 2) return launch_staged<2>(s, talk, stream);
+            if (group <= 4) return launch_staged<4>(s, talk, stream);
+            return launch_staged<MIX_GROUP>(s, talk, stream);
+        }
+    }
     if (a.vdim > 128) {
         if (group <= 2) return launch_mix_values<T, WARPS, 2, MIX_COLUMNS>(s, talk, smem2, stream);
         if (group <= 4) return launch_mix_values<T, WARPS, 4, MIX_COLUMNS>(s, talk, smem2, stream);

@@ -674,11 +674,10 @@ attention_tcgen05_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __
         if (has_work && elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(TC_KEYS);       // S[128 x 128] = Q K^T, K-major operands
             constexpr uint32_t idesc_o = make_idesc(TC_DIM, true);  // O[128 x 128] += P V, V is MN-major
-            // An MMA instruction holds the thread that issues it for 54 cycles whatever its size, and
-            // the pipe needs 64 for 128 x 128 x 16: what the thread does besides must stay under ten
-            // cycles an MMA or the pipe waits for it.  So the operands' descriptors are made once (their
-            // address field is additive: a k step further is a constant more) and the first MMA of a
-            // product, which overwrites, is its own instruction instead of a predicate computed each time.
+            // The pipe needs 64 cycles for 128 x 128 x 16, the thread that issues it less, but looks at barriers cost it 190 cycles
+            // each: what it does besides must stay little or the pipe waits for it.  So the operands' descriptors are made once (their
+            // address field is additive: a k step further is a constant more) and the first MMA of a product, which overwrites, is
+            // its own instruction instead of a predicate computed each time.
             constexpr uint64_t NEXT_TILE = DUO_TILE_BYTES >> 4;  // the second head's queries, the second stage
             const uint64_t q_desc = smem_desc_sw128(smem_u32(q_tiles)), k_desc = smem_desc_sw128(smem_u32(k_tiles));
             const uint64_t v_desc = smem_desc_sw128_mn(smem_u32(v_tiles), TC_HALF_BYTES);
