@@ -64,6 +64,10 @@ struct SplitConfig {
     static constexpr int TAKERS = NT <= 16 ? 128 : 256, COLUMNS = NT * 128 / TAKERS;  // threads; columns of one
     static constexpr int FIRST_CONVERTER = GROUPS == 2 ? 4 : 2, FIRST_TAKER = FIRST_CONVERTER + GROUPS * CONVERTERS / 32;  // warps
     static constexpr int THREADS = FIRST_TAKER * 32 + TAKERS, CTAS = NT <= 16 ? 2 : 1;
+    // Registers of a thread at launch (the most that so many threads leave, what launch_split checks) and in the roles of two groups: the
+    // shares are what the launch has, since more than that would be waited for in vain.
+    static constexpr int LAUNCH_REGISTERS = 65536 / (THREADS * CTAS) / 8 * 8, HELPER_REGISTERS = 56, TAKER_REGISTERS = 112;
+    static_assert(GROUPS == 1 || (THREADS - TAKERS) * HELPER_REGISTERS + TAKERS * TAKER_REGISTERS <= THREADS * LAUNCH_REGISTERS, "register shares");
     static constexpr int UNITS = NT >= 128 ? 2 : 1, UNIT_K = SPLIT_K / UNITS;  // units to a block
     static constexpr int BOXES = UNIT_K / 32;                                  // a TMA box of float32 is 32 k wide
     static constexpr int W_BYTES = SPLIT_ROWS * UNIT_K * 4, X_BYTES = PRE ? 0 : NT * UNIT_K * 4, RAW_BYTES = W_BYTES + X_BYTES;  // of a unit
@@ -165,7 +169,7 @@ __device__ __forceinline__ bool sound(float v) { return fabsf(v) <= 3.402823466e
 __device__ __forceinline__ void form_again(const SplitParams& p, int t, int w_row, int n) {
     p.out[static_cast<size_t>(t) * p.outs + n] = plain_sum(p.x + static_cast<size_t>(t) * p.inner, p.w + static_cast<size_t>(w_row) * p.inner, p.inner);
 }
-// What the threads of four warps hold at most from now on; the roles' shares stand where the roles part.
+// What the threads of four warps hold at most from now on; the roles' shares stand in SplitConfig.
 template <int REGISTERS>
 __device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGISTERS)); }
 template <int REGISTERS>
@@ -234,8 +238,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     bool ok = true;
     auto wait = [](uint64_t* bar, uint32_t parity) { return WITHHELD ? mbar_wait(bar, parity, 512) : mbar_wait(bar, parity); };
 
-    // Two groups of converters: 128 x 56 + 512 x 56 + 256 x 112 registers, which is what 896 threads of 72 start with.
-    if (C::GROUPS == 2 && warp < C::FIRST_CONVERTER) registers_down<56>();
+    if (C::GROUPS == 2 && warp < C::FIRST_CONVERTER) registers_down<C::HELPER_REGISTERS>();
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer
         if (elect_one()) {
@@ -352,7 +355,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     } else if (warp < C::FIRST_TAKER) {
         // ----------------------------------------------------------------- converters
         // A thread takes 16 or 32 weights of a row.
-        if constexpr (C::GROUPS == 2) registers_down<56>();
+        if constexpr (C::GROUPS == 2) registers_down<C::HELPER_REGISTERS>();
         const int group = (warp - C::FIRST_CONVERTER) / (CONVERTERS / 32);
         const int worker = threadIdx.x - C::FIRST_CONVERTER * 32 - group * CONVERTERS, run = worker >> 7;
         const int row = quarter * 32 + lane;
@@ -410,7 +413,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     } else {
         // ------------------------------------------------------------------- takers
         // The sums of a block out of tensor memory and added up; at the end of a segment the small terms join them.
-        if constexpr (C::GROUPS == 2) registers_up<112>();
+        if constexpr (C::GROUPS == 2) registers_up<C::TAKER_REGISTERS>();
         constexpr int COLUMNS = C::COLUMNS;
         const int row = quarter * 32 + lane, n = n0 + row, column = (warp - C::FIRST_TAKER) / 4 * COLUMNS;
         // With 128 tokens a thread's registers hold one sum per column: its CTA runs one segment (see me_gemm_split).
@@ -487,6 +490,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
     tcgen05_fence_before();
     __syncthreads();
+    // What follows is every warp's code, so it must not name a register that the smallest share lacks.  All come back to what they were
+    // launched with: the takers give first, behind the barrier above, so nobody waits for registers that do not come.
+    if constexpr (C::GROUPS == 2) {
+        if (warp >= C::FIRST_TAKER) registers_down<C::LAUNCH_REGISTERS>();
+        else registers_up<C::LAUNCH_REGISTERS>();
+    }
     if (warp == 1) tcgen05_dealloc(tmem_base, C::TMEM_COLUMNS);
     if (p.clustered) {
         cluster_sync();
@@ -609,6 +618,13 @@ static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, cons
     auto kernel = gemm_split_kernel<NT, PRE, WITHHELD>;
     static SharedMemoryOptIn opt_in;
     if (const int e = opt_in(kernel, C::SMEM_BYTES)) return e;
+    if (C::GROUPS == 2) {  // launched with fewer registers, the takers would wait for a share that does not exist
+        static const int registers = [kernel] {
+            cudaFuncAttributes of = {};
+            return cudaFuncGetAttributes(&of, kernel) == cudaSuccess ? of.numRegs : 0;
+        }();
+        if (registers != C::LAUNCH_REGISTERS) return ME_ERR_UNSUPPORTED;
+    }
     const dim3 grid((p.tokens + NT - 1) / NT, (p.outs + SPLIT_ROWS - 1) / SPLIT_ROWS, p.clustered ? segments : 1);
     if (grid.y > 65535) return ME_ERR_UNSUPPORTED;
     cudaLaunchConfig_t config = {};

@@ -227,3 +227,76 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_device_usable(side_by_s
         tc.gemm_split(plan, x, out, form)
         assert float((out.double() - x.double() @ w.double().T).abs().max()) < 1e-3
     assert tc.take_error() == 0
+
+
+# 128 tokens to a CTA, one segment of 65 blocks (its rings go round 32 times, the last block is partial) and eight of 24 in a cluster; 64 to a CTA with
+# segments one after the other, which the rule takes for the first, and of 192 blocks in all
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,outs,inner,form", [(130, 20500, 4100, (128, False)), (200, 520, 12288, (128, True)), (70, 520, 12288, (64, True))])
+def test_long_reductions_give_the_same_bits_in_every_form(tokens, outs, inner, form):
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(7)
+    x, w = torch.randn(tokens, inner, device="cuda"), torch.randn(outs, inner, device="cuda")
+    plan = tc.SplitPlan(w)
+    assert (plan.segments == 1) == (form == (128, False))
+    got = []
+    for chosen in (form, (64, False), form):
+        got.append(torch.full((tokens, outs), float("nan"), device="cuda"))
+        tc.gemm_split(plan, x, got[-1], chosen)
+    assert tc.take_error() == 0
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    simt, want = torch.empty(tokens, outs, device="cuda"), x.double() @ w.double().T
+    ops.gemm_simt(x, w, simt)
+    error = lambda y: float((y.double() - want).norm() / want.norm())  # noqa: E731
+    assert error(got[0]) <= error(simt)  # of one fmaf chain, which is twice as far off at 1,024 already
+
+
+@pytest.mark.gpu
+def test_products_of_many_sizes_share_the_pieces_buffer():
+    """Back to back through one workspace, smaller and larger than the one before; the last two read the same rows."""
+    from mini_engine_b200.engine.workspace import Workspace
+
+    tc = tensor_core()
+    torch.manual_seed(8)
+    workspace = Workspace(16, "cuda")
+    runs = []
+    for tokens, outs, inner in [(300, 520, 1100), (17, 130, 68), (64, 2048, 2048), (130, 520, 4100), (20, 200, 12288), (300, 640, 1100)]:
+        x, w = torch.randn(tokens, inner, device="cuda"), torch.randn(outs, inner, device="cuda")
+        runs.append((tc.SplitPlan(w), x, torch.full((tokens, outs), float("nan"), device="cuda"), torch.empty(tokens, outs, device="cuda")))
+    runs.append((runs[0][0], runs[-1][1], torch.empty(300, 520, device="cuda"), torch.empty(300, 520, device="cuda")))
+    for plan, x, out, _ in runs:
+        tc.gemm_split(plan, x, out, workspace=workspace)
+    for plan, x, _, alone in runs:
+        tc.gemm_split(plan, x, alone)
+    assert tc.take_error() == 0
+    for _, _, out, alone in runs:
+        assert torch.equal(out, alone)
+
+
+@pytest.mark.gpu
+def test_grouped_product_in_runs_of_128_gives_the_bits_of_each_groups_own():
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(9)
+    tokens, units, top, outs, inner, pad = 300, 5, 2, 384, 1100, 128
+    h, w = torch.randn(tokens, inner, device="cuda"), torch.randn(units, outs, inner, device="cuda")
+    chosen = torch.rand(tokens, units).topk(top, dim=1).indices.to(torch.int32).cuda()
+    capacity = -(-(tokens * top + units * (pad - 1)) // pad) * pad
+    ints = lambda *shape: torch.empty(shape, dtype=torch.int32, device="cuda")  # noqa: E731
+    row_of, token_of, unit_of_block = ints(tokens, top), ints(capacity), ints(capacity // pad)
+    ops.sort_by_unit(chosen=chosen, units=units, pad=pad, row_of=row_of, token_of=token_of, unit_of_block=unit_of_block)
+    rows = torch.empty(capacity, inner, device="cuda")
+    ops.gather_rows(h, token_of, rows)
+    plan = tc.SplitPlan(w.reshape(units * outs, inner), group_rows=outs)
+    assert plan.segments > 1
+    out = torch.full((capacity, outs), float("nan"), device="cuda")
+    tc.gemm_split_grouped(plan, rows, out, unit_of_block, pad, units, True)
+    assert tc.take_error() == 0
+    for u in range(units):
+        alone = torch.empty(tokens, outs, device="cuda")
+        tc.gemm_split(tc.SplitPlan(w[u].clone()), h, alone)
+        at, place = (chosen == u).nonzero(as_tuple=True)
+        assert torch.equal(out[row_of[at, place].long()], alone[at])
