@@ -78,9 +78,9 @@ struct SplitConfig {
     static constexpr int MAINS = UNITS == 1 ? 2 : 1;
     static constexpr int SMALL_COLUMN = MAINS * NT, A_COLUMN = SMALL_COLUMN + 2 * NT, A_PIECE = UNIT_K / 2, A_COLUMNS = 3 * A_PIECE;
     static constexpr int TMEM_COLUMNS = A_COLUMN + 2 * A_COLUMNS <= 256 ? 256 : 512;
-    static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + X_BUFFERS * PIECES_BYTES + 1024 + 256;
+    static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + X_BUFFERS * PIECES_BYTES + 1024 + 384;
     static constexpr int READY_ARRIVALS = CONVERTERS / 32 + (PRE ? 1 : 0);  // of a unit; more where a block begins, see the takers
-    static_assert((2 * STAGES + 2 * RING + 2 * MAINS + 1) * 8 + 4 <= 256, "barriers");
+    static_assert((2 * STAGES + 2 * RING + MAINS + 1) * 8 + (2 + THREADS / 32) * 4 <= 384, "barriers, what the roles leave behind");
     static_assert(PRE == (NT > 16), "more tokens than 16 come as pieces");
     static_assert(A_COLUMN + 2 * A_COLUMNS <= TMEM_COLUMNS, "tensor memory");
     static_assert(STAGES * RAW_BYTES >= NT * SPLIT_ROWS * 4, "the cluster's exchange reuses the raw tiles");
@@ -184,7 +184,8 @@ __device__ __forceinline__ void pieces_of(float4 v, uint32_t* p0, uint32_t* p1, 
     p2[0] = upper_pair(rest.x, rest.y), p2[1] = upper_pair(rest.z, rest.w);
 }
 
-// WITHHELD: no tile is ever loaded and waits end after a few polls, so that a test can take the way of a kernel that gives up.
+// WITHHELD: no weights are ever loaded (the tokens' pieces are) and waits end after a few polls, so that a test can take the way of a kernel
+// that gives up, with copies in flight where pieces are made ahead.
 template <int NT, bool PRE, bool WITHHELD = false>
 __global__ void __launch_bounds__(SplitConfig<NT, PRE>::THREADS, SplitConfig<NT, PRE>::CTAS)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SplitParams p) {
@@ -199,6 +200,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     uint64_t* mains = done + RING;        // [MAINS] a block's w0 x0 complete
     uint64_t* taken = mains + C::MAINS;   // a segment's small terms out of tensor memory
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(taken + 1);
+    int* gave_up = reinterpret_cast<int*>(tmem_holder + 1);  // whether some role did
+    int* reached = gave_up + 1;                              // [warps] PRE: the unit or block at which a converter or taker ended
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.x * NT, n0 = blockIdx.y * SPLIT_ROWS;
@@ -214,6 +217,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
 
     if (threadIdx.x == 0) {
+        *gave_up = 0;
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], CONVERTERS / 32); }
         // The issuer waits once a unit: a wait holds it for 190 cycles and more, which only the last MMAs before it cover.  So a unit's
         // barrier also takes the arrivals of the tokens' pieces and of the takers who have emptied the sums that it overwrites:
@@ -236,6 +240,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
 
     bool ok = true;
+    int x_issued = 0;  // of the producer: blocks whose pieces it has asked for
+    auto give_up = [&](int role) {
+        atomicCAS(&g_split_error, 0, role << 8);
+        *gave_up = 1;
+    };
     auto wait = [](uint64_t* bar, uint32_t parity) { return WITHHELD ? mbar_wait(bar, parity, 512) : mbar_wait(bar, parity); };
 
     if (C::GROUPS == 2 && warp < C::FIRST_CONVERTER) registers_down<C::HELPER_REGISTERS>();
@@ -265,7 +274,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const int early = min(units, C::STAGES);  // weights are written by no kernel: ahead of the wait
             for (int u = 0; u < early; ++u) load_w(u);
             pdl_wait();
-            int issued = early, x_issued = 0;
+            int issued = early;
             bool go = true;
             if constexpr (PRE) {
                 for (; x_issued < min(blocks, C::X_BUFFERS); ++x_issued) load_pieces(x_issued);
@@ -297,13 +306,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     load_x(u);
                 }
             }
-            if (!go) atomicCAS(&g_split_error, 0, (1 << 8));
-            // Copies in flight must land before the shared memory is released, also when another role has given up.
+            if (!go) give_up(1);
+            // Copies in flight must land before the shared memory is released, also when another role has given up (pieces: behind the join).
             for (int u = max(issued - C::STAGES, 0); u < issued; ++u) wait(&full[u % C::STAGES], (u / C::STAGES) & 1);
-            if (PRE && (!go || g_split_error != 0)) {  // on the normal path the MMAs have waited for the pieces
-                const long long until = clock64() + 100000;  // their barriers may miss other arrivals for good: 50 us, no copy takes that long
-                while (clock64() < until) __nanosleep(1000);
-            }
         }
     } else if (warp == 1) {
         // --------------------------------------------------------------- MMA issuer
@@ -316,7 +321,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             for (int u = 0, at = 0, segment = 0; u < units; ++u) {
                 const int half = u % C::UNITS, block = u / C::UNITS;
                 const bool fresh = half == 0 && at == 0;  // a segment starts its own small terms
-                if (!wait(&ready[u % RING], (u / RING) & 1)) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
+                if (!wait(&ready[u % RING], (u / RING) & 1)) { give_up(2); break; }
                 tcgen05_fence_after();
                 const uint32_t a = tmem_base + C::A_COLUMN + (u & 1) * C::A_COLUMNS, main_sum = tmem_base + block % C::MAINS * NT;
                 const uint64_t b = x_pieces + block % C::X_BUFFERS * (C::PIECES_BYTES >> 4) + 4 * half;
@@ -344,7 +349,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 }
                 tcgen05_commit(&done[u % RING]);
                 ++sent;
-                if (!go) { atomicCAS(&g_split_error, 0, (2 << 8)); break; }
+                if (!go) { give_up(2); break; }
                 if (half == C::UNITS - 1 && ++at == p.per_segment) at = 0, ++segment;
             }
             // MMAs in flight read shared memory and write tensor memory: they end before either is given back.
@@ -359,7 +364,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int group = (warp - C::FIRST_CONVERTER) / (CONVERTERS / 32);
         const int worker = threadIdx.x - C::FIRST_CONVERTER * 32 - group * CONVERTERS, run = worker >> 7;
         const int row = quarter * 32 + lane;
-        for (int u = group; u < units; u += C::GROUPS) {
+        int u = group;
+        for (; u < units; u += C::GROUPS) {
             ok = __all_sync(0xffffffffu, wait(&full[u % C::STAGES], (u / C::STAGES) & 1));
             if (!ok) break;
             const uint32_t w_tile = smem_u32(raw + (u % C::STAGES) * C::RAW_BYTES), x_tile = w_tile + C::W_BYTES;
@@ -409,7 +415,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 mbar_arrive(&empty[u % C::STAGES]);
             }
         }
-        if (!ok && lane == 0) atomicCAS(&g_split_error, 0, (3 << 8));
+        if (!ok && lane == 0) give_up(3);
+        if (PRE && lane == 0) reached[warp] = u;
     } else {
         // ------------------------------------------------------------------- takers
         // The sums of a block out of tensor memory and added up; at the end of a segment the small terms join them.
@@ -424,6 +431,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         for (int c = 0; c < COLUMNS; ++c) sum[c] = 0.0f;
         if (lane == 0)
             for (int b = 0; b < C::MAINS; ++b) mbar_arrive(&ready[b * C::UNITS]);  // nothing lies in tensor memory yet
+        int taken_blocks = 0;
         for (int i = 0; i < blocks; ++i) {
             ok = __all_sync(0xffffffffu, wait(&mains[i % C::MAINS], (i / C::MAINS) & 1));
             if (!ok) break;
@@ -438,6 +446,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ready[(i + C::MAINS) * C::UNITS % RING]);  // for the block that takes this one's columns
+            ++taken_blocks;
             if (++at == p.per_segment || i + 1 == blocks) {
                 at = 0;
                 const int u = i * C::UNITS + C::UNITS - 1;  // the block's last unit
@@ -467,7 +476,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
         auto result = [&](int c) { return MANY ? total[MANY ? c : 0] : sum[c]; };
-        if (!ok && lane == 0) atomicCAS(&g_split_error, 0, (4 << 8));
+        if (!ok && lane == 0) give_up(4);
+        if (PRE && lane == 0) reached[warp] = taken_blocks;
         pdl_wait();  // the output may still be read by a kernel before this one
         if (p.clustered && ok) {
             // every MMA and load of this CTA has ended: the raw tiles make room for the exchange
@@ -496,6 +506,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (warp >= C::FIRST_TAKER) registers_down<C::LAUNCH_REGISTERS>();
         else registers_up<C::LAUNCH_REGISTERS>();
     }
+    if (PRE && warp == 0 && *gave_up && x_issued > 0) {
+        // Some role gave up, so pieces may still be on their way behind barriers that also wait for arrivals which never come.  Behind the
+        // join nobody else arrives any more: this thread (the producer; the others have asked for none) makes up what is missing, after which a barrier
+        // completes when its bytes have landed.
+        for (int b = max(x_issued - C::X_BUFFERS, 0); b < x_issued; ++b) {
+            const int u = b * C::UNITS;
+            uint64_t* bar = &ready[u % RING];
+            if (mbar_try_wait(bar, (u / RING) & 1)) continue;
+            for (int w = 0; w < CONVERTERS / 32; ++w)
+                if (reached[C::FIRST_CONVERTER + u % C::GROUPS * (CONVERTERS / 32) + w] <= u) mbar_arrive(bar);
+            for (int w = 0; w < C::TAKERS / 32; ++w)
+                if (reached[C::FIRST_TAKER + w] <= b - C::MAINS) mbar_arrive(bar);
+            if (!mbar_wait(bar, (u / RING) & 1)) atomicExch(&g_split_error, 5 << 8);
+        }
+    }
+    __syncwarp();
     if (warp == 1) tcgen05_dealloc(tmem_base, C::TMEM_COLUMNS);
     if (p.clustered) {
         cluster_sync();
@@ -673,10 +699,10 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     memcpy(&x_map, map_x, sizeof(x_map));
     if (pieces != nullptr)
         if (const int e = split_rows(x, pieces, tokens, inner, stream)) return e;
-    if (withheld) return tile == 16 && !pieces ? launch_split<16, false, true>(w_map, x_map, p, segments, stream) : ME_ERR_ARGUMENT;
-    if (tile == 16 && !pieces) return launch_split<16, false>(w_map, x_map, p, segments, stream);
-    if (tile == 64 && pieces) return launch_split<64, true>(w_map, x_map, p, segments, stream);
-    if (tile == 128 && pieces && (p.clustered || segments == 1)) return launch_split<128, true>(w_map, x_map, p, segments, stream);
+    if (tile == 16 && !pieces) return withheld ? launch_split<16, false, true>(w_map, x_map, p, segments, stream) : launch_split<16, false>(w_map, x_map, p, segments, stream);
+    if (tile == 64 && pieces) return withheld ? launch_split<64, true, true>(w_map, x_map, p, segments, stream) : launch_split<64, true>(w_map, x_map, p, segments, stream);
+    if (tile == 128 && pieces && (p.clustered || segments == 1))
+        return withheld ? launch_split<128, true, true>(w_map, x_map, p, segments, stream) : launch_split<128, true>(w_map, x_map, p, segments, stream);
     return ME_ERR_ARGUMENT;
 }
 

@@ -365,7 +365,7 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
     _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, 0, workspace)
 
 
-def _launch_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, outs: int, tile: int, side_by_side: bool, group_of_block, group_rows: int, workspace) -> None:
+def _launch_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, outs: int, tile: int, side_by_side: bool, group_of_block, group_rows: int, workspace, withheld: bool = False) -> None:
     rows, inner = x.shape
     pieces = None
     if tile >= SPLIT_PIECES_MIN_TILE:
@@ -380,7 +380,7 @@ def _launch_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, outs: int
         x_map = _split_activation_map(x, tile)
     code = _split_library().me_gemm_split(
         plan.map, x_map, x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, inner, tile, pieces,
-        plan.segments, 1 if side_by_side else 0, group_of_block, group_rows, 0, _ops_stream(),
+        plan.segments, 1 if side_by_side else 0, group_of_block, group_rows, 1 if withheld else 0, _ops_stream(),
     )  # fmt: skip
     _count_launch()
     if code != 0:
@@ -457,18 +457,12 @@ def wait_probe(polls: int = 4096) -> bool:
     return bool(returned.item())
 
 
-def split_wait_probe(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side: bool) -> None:
-    """The float32 product with every tile withheld: all waits of its roles run out after a few polls, the kernel records that,
-    gives its tensor memory back and returns without a result.  Exists so that the give-up path can be tested."""
+def split_wait_probe(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_by_side: bool, tile: int = 16) -> None:
+    """The float32 product in the form of ``tile`` tokens to a CTA with every weight tile withheld: all waits of its roles run out after a few
+    polls, the kernel records that, gives its tensor memory back and returns without a result.  Exists so that the give-up path can be tested."""
     if x.shape[1] != plan.inner or tuple(out.shape) != (x.shape[0], plan.rows) or not (x.is_contiguous() and out.is_contiguous()):
         raise RuntimeError("the probe takes the arguments of a product")
-    code = _split_library().me_gemm_split(
-        plan.map, _split_activation_map(x, 16), x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), x.shape[0], plan.rows, plan.inner, 16, None,
-        plan.segments, 1 if side_by_side else 0, None, 0, 1, _ops_stream(),
-    )  # fmt: skip
-    _count_launch()
-    if code != 0:
-        raise RuntimeError(f"the wait probe failed to launch (code {code})")
+    _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, 0, None, withheld=True)
 
 
 def take_error() -> int:

@@ -300,3 +300,30 @@ def test_grouped_product_in_runs_of_128_gives_the_bits_of_each_groups_own():
         tc.gemm_split(tc.SplitPlan(w[u].clone()), h, alone)
         at, place = (chosen == u).nonzero(as_tuple=True)
         assert torch.equal(out[row_of[at, place].long()], alone[at])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile,side_by_side", [(64, False), (64, True), (128, True)])
+def test_giving_up_with_pieces_in_flight(tile, side_by_side):
+    """The forms whose tokens arrive as pieces: these are on their way when every role gives up, and have landed before shared memory is
+    given back.  Registers, barriers and tensor memory serve the next products."""
+    from mini_engine_b200.csrc import ops
+
+    tc = tensor_core()
+    torch.manual_seed(10)
+    x, w = torch.randn(150, 1100, device="cuda"), torch.randn(300, 1100, device="cuda")
+    plan = tc.SplitPlan(w)
+    assert plan.segments > 1 and tc.take_error() == 0
+    out, want = torch.full((150, 300), 7.0, device="cuda"), torch.empty(150, 300, device="cuda")
+    tc.gemm_split(plan, x, want, (16, False))
+    for _ in range(8):
+        tc.split_wait_probe(plan, x, out, side_by_side, tile)
+    torch.cuda.synchronize()
+    assert bool((out == 7.0).all())  # nothing is written
+    with pytest.raises(ops.KernelError, match="limit of a wait") as raised:
+        ops.raise_on_device_error()
+    assert f"code {5 << 8}" not in str(raised.value)  # the producer saw its copies land
+    for form in [(tile, side_by_side), (16, True), (128, True)]:
+        tc.gemm_split(plan, x, out, form)
+        assert torch.equal(out, want)
+    assert tc.take_error() == 0
