@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from functools import lru_cache
 from typing import Any
 
 import torch
@@ -596,12 +597,41 @@ FEW_ROWS_MIN_CONTEXT = 64  # ... from more keys than this on: two tiles in one b
 FEW_ROWS_MAX_SCRATCH = 256 << 20  # bytes of scores; larger steps take the one kernel
 
 
-def few_rows_capacity(tokens: int, longest: int, heads: int, kv_heads: int, context: int, window: int) -> int:
+@lru_cache(maxsize=4096)
+def few_rows_pay(entries: int, rows: int, kv_heads: int, head_dim: int, value_dim: int, values_in_keys: bool, context: int) -> bool:
+    """Whether the two kernels are expected to be faster than the one for ``entries`` of ``rows`` rows per KV head behind ``context`` keys.  The one
+    kernel is a block to an entry and KV head, whose time goes with the width of a key and its value; each block beside it on an SM adds
+    0.37 of that.  Of the two kernels the second is a block to 64 value columns, each of which forms the softmax of all rows again; three fit an
+    SM, and the second launch costs 5.5 us.  The constants are fitted to 384 measured shapes (1 to 128 entries, 1 to 16 rows, widths
+    64 to 576, 65 to 2,048 keys): of these 7 take a form that is more than 5 % behind the other, at most 16 %.  us behind 2,048 keys, one kernel |
+    two: 16 heads in 8 KV heads of 128, 8 entries 250 | 114, 128 entries 1,266 | 867; 32 in 8, 32 entries 356 | 333; 16 in 2, 8 252 |
+    136, 96 361 | 298, 128 361 | 456; 24 in 4, 48 358 | 253, 64 358 | 388; 16 over latent rows of 576 with 512 values, 8 666 | 220, 48 670 |
+    425, 64 670 | 663, 128 672 | 1,099; 16 in 2 of 64, 48 186 | 179; behind 128 keys 32 entries of that 18.4 | 23.5."""
+    sms = tensor_core.NUM_SMS
+    shared = 4 * (80 * (head_dim + 4) + (0 if values_in_keys else 64 * (value_dim + 4)) + 576)  # bytes of a block of the one kernel
+    at_a_time = sms * max(1, min(8, (227 << 10) // (shared + 2048)))
+    waves, rest = divmod(entries * kv_heads, at_a_time)
+    wave = lambda blocks: 1.0 + 0.37 * (-(-blocks // sms) - 1) if blocks else 0.0  # noqa: E731
+    one = (100 + 0.55 * (head_dim + value_dim)) * (waves * wave(at_a_time) + wave(rest))
+    value_blocks = entries * kv_heads * -(-value_dim // 64)
+    rounds = -(-value_blocks // (3 * sms))
+    two = (53 + 6.7 * rows) * (1.07 * rounds - 0.07) + (0.22 + 0.025 * rows) * value_blocks
+    return two * context / 2048 + 5.5 < 1.05 * one * context / 2048
+
+
+def few_rows_capacity(
+    tokens: int, longest: int, heads: int, kv_heads: int, context: int, window: int, entries: int = 0, head_dim: int = 0, value_dim: int = 0,
+    values_in_keys: bool = False,
+) -> int:  # fmt: skip
     """Scores per (token, head) that a step's scratch must hold when its entries, of at most ``longest`` tokens and ``context`` keys,
-    take the two kernels for few rows; 0 when they do not.  Of the sizes alone, so that a captured step takes the form it was captured with."""
+    take the two kernels for few rows; 0 when they do not (with ``entries`` and the heads' widths given, also where the one kernel is
+    faster).  Of the sizes alone, so that a captured step takes the form it was captured with."""
     if window > 0:
         context = min(context, window + longest + 31)  # from the start of the first visible key's tile on
-    if longest * (heads // kv_heads) > FEW_ROWS or context <= FEW_ROWS_MIN_CONTEXT:
+    rows = longest * (heads // kv_heads)
+    if rows > FEW_ROWS or context <= FEW_ROWS_MIN_CONTEXT:
+        return 0
+    if entries and not few_rows_pay(entries, rows, kv_heads, head_dim, value_dim, values_in_keys, context):
         return 0
     capacity = -(-context // 32) * 32
     return capacity if 4 * tokens * heads * capacity <= FEW_ROWS_MAX_SCRATCH else 0
@@ -631,7 +661,12 @@ def paged_attention(
             return
     if q.dtype == torch.float32 and attention_rows_supports(q, k_pages, v_pages, out, head_dim, value_dim):
         scores, workspace = None, getattr(ctx, "workspace", None)
-        capacity = 0 if workspace is None else few_rows_capacity(q.shape[0], ctx.max_query_len, heads, kv_heads, ctx.max_context_len, window)
+        capacity = 0
+        if workspace is not None:
+            capacity = few_rows_capacity(
+                q.shape[0], ctx.max_query_len, heads, kv_heads, ctx.max_context_len, window, ctx.num_entries, head_dim, value_dim or head_dim,
+                v_pages is None,
+            )  # fmt: skip
         if capacity:
             scores = workspace.growing("attn.row_scores", (q.shape[0], heads, capacity), torch.float32)
         paged_attention_rows(

@@ -53,3 +53,19 @@ def test_which_steps_take_the_two_kernels():
     assert take(8, 1, 16, 8, 64, 0) == 0 and take(8, 1, 16, 8, 65, 0) == 96
     assert take(8, 1, 16, 8, 4096, 1024) == 1056  # keys behind the window need no room
     assert take(64, 1, 64, 8, 1 << 20, 0) == 0  # more scratch than is kept
+
+
+# entries, heads, KV heads, widths, values in the keys, context, whether the two kernels were measured faster: many entries, whose blocks of value
+# columns each form the softmax again; as many just under three blocks to an SM; short contexts, where the second launch decides
+@pytest.mark.parametrize(
+    "entries,heads,kv_heads,dim,value_dim,in_keys,context,two",
+    [(8, 16, 8, 128, 128, False, 2048, True), (128, 32, 8, 128, 128, False, 2048, True), (96, 16, 2, 128, 128, False, 2048, True),
+     (128, 16, 2, 128, 128, False, 2048, False), (48, 24, 4, 128, 128, False, 512, True), (64, 24, 4, 128, 128, False, 512, False),
+     (8, 16, 1, 576, 512, True, 128, True), (48, 16, 1, 576, 512, True, 2048, True), (128, 16, 1, 576, 512, True, 2048, False),
+     (32, 16, 2, 64, 64, False, 128, False), (32, 16, 2, 64, 64, False, 2048, True)],
+)  # fmt: skip
+def test_the_faster_form_is_taken(entries, heads, kv_heads, dim, value_dim, in_keys, context, two):
+    from mini_engine_b200.csrc import ops
+
+    got = ops.few_rows_capacity(entries, 1, heads, kv_heads, context, 0, entries, dim, value_dim, in_keys)
+    assert got == (context if two else 0)
