@@ -58,6 +58,7 @@ class Workspace:
     def get(self, name: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """A contiguous view ``shape`` of the named buffer.  The first axis is a token count;
         the buffer is sized for ``max_tokens`` of them."""
+        shape = tuple(shape)
         held = self._held_view(name, dtype, shape)
         if held is not None:
             return held
@@ -76,6 +77,7 @@ class Workspace:
         token capacity (logits: ``[rows, vocab]`` is large and ``rows`` is usually small).  It grows
         by half at least, so that steps of ever longer prompts do not leave one buffer behind for
         every length: all that it has ever replaced is less than twice what it holds."""
+        shape = tuple(shape)
         view = self._held_view(name, dtype, shape)
         if view is not None:
             return view

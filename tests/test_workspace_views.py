@@ -25,3 +25,12 @@ def test_views_are_kept_until_their_buffer_is_replaced():
     assert workspace.growing("g", (3, 5), torch.float32).shape == (3, 5)
     for tokens in range(1, 200):  # steps of many token counts
         assert workspace.partials("p", 1, tokens % 16 + 1, 5).shape == (1, tokens % 16 + 1, 5)
+
+
+def test_shapes_may_be_lists():
+    from mini_engine_b200.engine.workspace import Workspace
+
+    workspace = Workspace(8, device="cpu")
+    assert workspace.get("a", [3, 4], torch.float32) is workspace.get("a", (3, 4), torch.float32)
+    assert workspace.growing("g", [2, 5], torch.float32).shape == (2, 5)
+    assert workspace.growing("g", torch.Size([2, 5]), torch.float32) is workspace.growing("g", (2, 5), torch.float32)
