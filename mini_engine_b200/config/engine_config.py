@@ -24,7 +24,9 @@ class EngineConfig:
     seed: int = 0  # seed of temperature sampling
     cuda_graphs: bool = True  # replay captured graphs for decode-only steps
     # When set (0 < f <= 1), num_blocks is ignored and the pool takes this fraction of the device
-    # memory that is free after the weights are loaded.  The reference sizes by num_blocks only.
+    # memory that is free after the weights are loaded.  The reference sizes by num_blocks only.  The steps' activations and scratch
+    # come out of what it leaves; in float32 that includes pieces of the tokens (6 bytes a value of the widest product's input, 512 MB at
+    # most) and scores of decoded tokens (256 MB at most); a buffer that grew on the way keeps less than twice that besides.
     kv_memory_fraction: float | None = None
     # Launch the decode step after the current one before the current one's token ids are read
     # (needs cuda_graphs).  The tokens are the same either way; off is for comparing.  Not in the

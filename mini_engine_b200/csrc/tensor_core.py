@@ -250,6 +250,9 @@ SPLIT_TILES = {16: 1.0, 64: 0.70, 128: 1.25}
 SPLIT_START, SPLIT_EXCHANGE = 5.0, 0.25
 SPLIT_CLUSTERS = (NUM_SMS, 74, 45, 33, 26, 22, 15, 15)
 SPLIT_PIECES_MIN_TILE = 64  # tokens per CTA from which on their pieces are made ahead, by a kernel of their own
+# Bytes of pieces at a time: they come out of what the page pool leaves, so larger steps (from 7,281 tokens of 12,288 on) run in parts.  8,192 x 1,024 x
+# 12,288 in one part and in two 1,390 to 1,480 | 1,530 to 1,640 us, 8,192 x 6,144 x 12,288 8.9 to 9.3 | 8.4 to 8.8 ms.
+SPLIT_PIECES_BYTES = 512 << 20
 SPLIT_MIN_K_BLOCKS = 4  # of a segment
 # Shorter reductions stay on CUDA cores: a chain of fmaf over so few terms is about as exact as the short chain of the tensor
 # core (relative error of normal operands at 64: 1.5e-7 against 0.7e-7), and nothing is to be gained.
@@ -362,29 +365,40 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
     if tokens == 0:
         return
     tile, side_by_side = split_form(tokens, plan.rows, plan.inner, plan.segments) if form is None else form
-    _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, 0, workspace)
+    _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, workspace)
 
 
-def _launch_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, outs: int, tile: int, side_by_side: bool, group_of_block, group_rows: int, workspace, withheld: bool = False) -> None:
+def _launch_split(
+    plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, outs: int, tile: int, side_by_side: bool, groups: torch.Tensor | None, workspace,
+    withheld: bool = False,
+) -> None:  # fmt: skip
     rows, inner = x.shape
-    pieces = None
+    at_once, held = rows, None
     if tile >= SPLIT_PIECES_MIN_TILE:
-        count = 3 * rows * (-(-inner // 8) * 8)
+        # as many rows at a time as their pieces have room, in parts of about the same size
+        width = 3 * (-(-inner // 8) * 8)
+        parts = -(-rows // max(tile, SPLIT_PIECES_BYTES // (2 * width) // tile * tile))
+        at_once = -(-rows // (parts * tile)) * tile
+        count = width * min(at_once, rows)
         if workspace is None:
             held = torch.empty(count, dtype=torch.bfloat16, device=x.device)
         else:
             held = workspace.growing("split.pieces", (count,), torch.bfloat16)
-        pieces, x_map = held.data_ptr(), _split_activation_map(held, tile, rows, inner)
+    for first in range(0, rows, at_once):
+        some = min(at_once, rows - first)
+        if held is None:
+            pieces, x_map = None, _split_activation_map(x, tile)
+        else:
+            pieces, x_map = held.data_ptr(), _split_activation_map(held, tile, some, inner)
+            _count_launch()
+        code = _split_library().me_gemm_split(
+            plan.map, x_map, x.data_ptr() + 4 * first * inner, plan.weight.data_ptr(), out.data_ptr() + 4 * first * outs, some, outs, inner, tile,
+            pieces, plan.segments, 1 if side_by_side else 0, None if groups is None else groups.data_ptr() + 4 * (first // tile),
+            0 if groups is None else outs, 1 if withheld else 0, _ops_stream(),
+        )  # fmt: skip
         _count_launch()
-    else:
-        x_map = _split_activation_map(x, tile)
-    code = _split_library().me_gemm_split(
-        plan.map, x_map, x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, inner, tile, pieces,
-        plan.segments, 1 if side_by_side else 0, group_of_block, group_rows, 1 if withheld else 0, _ops_stream(),
-    )  # fmt: skip
-    _count_launch()
-    if code != 0:
-        raise RuntimeError(f"float32 tensor-core product failed to launch (code {code})")
+        if code != 0:
+            raise RuntimeError(f"float32 tensor-core product failed to launch (code {code})")
 
 
 def gemm_split_grouped(
@@ -406,7 +420,7 @@ def gemm_split_grouped(
         raise RuntimeError("the rows of a grouped product come in runs of a token tile with one int32 group each")
     if side_by_side is None:
         side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad)[1]
-    _launch_split(plan, x, out, outs, pad, side_by_side, group_of_block.data_ptr(), outs, workspace)
+    _launch_split(plan, x, out, outs, pad, side_by_side, group_of_block, workspace)
 
 
 GROUP_PAD = 128  # rows of a run of the sorted rows that belongs to one group: the token tile of the grouped product
@@ -462,7 +476,7 @@ def split_wait_probe(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, side_b
     polls, the kernel records that, gives its tensor memory back and returns without a result.  Exists so that the give-up path can be tested."""
     if x.shape[1] != plan.inner or tuple(out.shape) != (x.shape[0], plan.rows) or not (x.is_contiguous() and out.is_contiguous()):
         raise RuntimeError("the probe takes the arguments of a product")
-    _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, 0, None, withheld=True)
+    _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, None, withheld=True)
 
 
 def take_error() -> int:

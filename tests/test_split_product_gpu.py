@@ -327,3 +327,40 @@ def test_giving_up_with_pieces_in_flight(tile, side_by_side):
         tc.gemm_split(plan, x, out, form)
         assert torch.equal(out, want)
     assert tc.take_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile,side_by_side", [(64, False), (64, True), (128, True)])
+def test_rows_beyond_the_room_for_pieces_run_in_parts(monkeypatch, tile, side_by_side):
+    """The same bits, and no more room however many rows there are; a last part of few rows, room for less than a tile, and groups."""
+    from mini_engine_b200.csrc import ops
+    from mini_engine_b200.engine.workspace import Workspace
+
+    tc = tensor_core()
+    torch.manual_seed(11)
+    x, w = torch.randn(1000, 1100, device="cuda"), torch.randn(300, 1100, device="cuda")
+    plan, want = tc.SplitPlan(w), torch.empty(1000, 300, device="cuda")
+    tc.gemm_split(plan, x, want, (tile, side_by_side))
+    row = 3 * 2 * 1104
+    for room in (row, 200 * row, 331 * row, 999 * row):
+        monkeypatch.setattr(tc, "SPLIT_PIECES_BYTES", room)
+        workspace, out = Workspace(16, "cuda"), torch.full((1000, 300), float("nan"), device="cuda")
+        launches = ops.launch_count()
+        tc.gemm_split(plan, x, out, (tile, side_by_side), workspace)
+        assert ops.launch_count() - launches >= 4
+        assert workspace.bytes_held() <= max(room, tile * row)
+        assert torch.equal(out, want)
+    monkeypatch.setattr(tc, "SPLIT_PIECES_BYTES", 2 * tile * row)
+    groups = torch.tensor([1, -1, 0, 2, 2, 1, 0], dtype=torch.int32, device="cuda")
+    grouped = tc.SplitPlan(w.clone(), group_rows=100)
+    out = torch.full((7 * tile, 100), float("nan"), device="cuda")
+    tc.gemm_split_grouped(grouped, x[: 7 * tile].contiguous(), out, groups, tile, 6, side_by_side)
+    assert tc.take_error() == 0
+    for b, group in enumerate(groups.tolist()):
+        got = out[b * tile : (b + 1) * tile]
+        if group < 0:
+            assert bool(got.isnan().all())
+            continue
+        alone = torch.empty(tile, 100, device="cuda")
+        tc.gemm_split(tc.SplitPlan(w[100 * group : 100 * group + 100].clone()), x[b * tile : (b + 1) * tile].clone(), alone)
+        assert torch.equal(got, alone)
