@@ -542,7 +542,8 @@ static size_t rows_shared_bytes(const AttnArgs& a, int rows) {
 }
 
 // Against one warp per (token, head), a prompt of 512 tokens, 16 heads of 128 in 8 KV heads: 1,361 -> 165 us; 256 tokens, 32
-// heads: 826 -> 143; eight decoded tokens behind 17 to 512: 768 -> 68, over latent rows of 576 with 512 values 768 -> 179 us.
+// heads: 826 -> 143; eight decoded tokens behind 17 to 512 (which now take the two kernels above): 768 -> 68, over latent rows of 576 with 512
+// values 768 -> 179 us.
 template <int R, int QP>
 static int launch_rows(const RowArgs& m, int entries, int longest, cudaStream_t stream) {
     static SharedMemoryOptIn opt_in;

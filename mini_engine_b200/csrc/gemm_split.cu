@@ -56,10 +56,11 @@ __device__ int g_split_error = 0;  // 0 ok; else (role << 8) | detail of the fir
 
 // NT: tokens per CTA.  The tiles pass through the roles in units, whole k blocks or (128 tokens, for which tensor memory has
 // no room otherwise) halves of 32 k; the weights' pieces have two buffers, so that the converters write one while the MMAs read the other.
-// PRE: the tokens' pieces were made by split_rows_kernel and arrive by TMA, a block at a time; else the raw tokens arrive with
+// PRE: the tokens' pieces were made by split_rows_kernel and arrive by TMA, a block at a time; up to 16 tokens the raw tokens arrive with
 // the raw weights and the converters make their pieces too.
-template <int NT, bool PRE>
+template <int NT>
 struct SplitConfig {
+    static constexpr bool PRE = NT > 16;
     static constexpr int GROUPS = NT <= 16 ? 1 : 2;  // of converters: unit u is group u % GROUPS's
     static constexpr int TAKERS = NT <= 16 ? 128 : 256, COLUMNS = NT * 128 / TAKERS;  // threads; columns of one
     static constexpr int FIRST_CONVERTER = GROUPS == 2 ? 4 : 2, FIRST_TAKER = FIRST_CONVERTER + GROUPS * CONVERTERS / 32;  // warps
@@ -72,16 +73,14 @@ struct SplitConfig {
     static constexpr int BOXES = UNIT_K / 32;                                  // a TMA box of float32 is 32 k wide
     static constexpr int W_BYTES = SPLIT_ROWS * UNIT_K * 4, X_BYTES = PRE ? 0 : NT * UNIT_K * 4, RAW_BYTES = W_BYTES + X_BYTES;  // of a unit
     static constexpr int PIECES_BYTES = 3 * NT * SPLIT_K * 2;  // of a block's tokens
-    static constexpr int X_BUFFERS = PRE && NT <= 64 ? 3 : 2;  // blocks of them
-    static constexpr int STAGES = NT <= 16 ? 2 : NT <= 64 ? (PRE ? 4 : 3) : 8;
+    static constexpr int X_BUFFERS = NT == 64 ? 3 : 2;  // blocks of them
+    static constexpr int STAGES = NT <= 16 ? 2 : NT <= 64 ? 4 : 8;
     // tensor memory: w0 x0 of one or two blocks, the 2^-8 and the 2^-16 terms, the weights' pieces of two units
     static constexpr int MAINS = UNITS == 1 ? 2 : 1;
     static constexpr int SMALL_COLUMN = MAINS * NT, A_COLUMN = SMALL_COLUMN + 2 * NT, A_PIECE = UNIT_K / 2, A_COLUMNS = 3 * A_PIECE;
     static constexpr int TMEM_COLUMNS = A_COLUMN + 2 * A_COLUMNS <= 256 ? 256 : 512;
     static constexpr int SMEM_BYTES = STAGES * RAW_BYTES + X_BUFFERS * PIECES_BYTES + 1024 + 384;
-    static constexpr int READY_ARRIVALS = CONVERTERS / 32 + (PRE ? 1 : 0);  // of a unit; more where a block begins, see the takers
     static_assert((2 * STAGES + 2 * RING + MAINS + 1) * 8 + (2 + THREADS / 32) * 4 <= 384, "barriers, what the roles leave behind");
-    static_assert(PRE == (NT > 16), "more tokens than 16 come as pieces");
     static_assert(A_COLUMN + 2 * A_COLUMNS <= TMEM_COLUMNS, "tensor memory");
     static_assert(STAGES * RAW_BYTES >= NT * SPLIT_ROWS * 4, "the cluster's exchange reuses the raw tiles");
 };
@@ -186,10 +185,11 @@ __device__ __forceinline__ void pieces_of(float4 v, uint32_t* p0, uint32_t* p1, 
 
 // WITHHELD: no weights are ever loaded (the tokens' pieces are) and waits end after a few polls, so that a test can take the way of a kernel
 // that gives up, with copies in flight where pieces are made ahead.
-template <int NT, bool PRE, bool WITHHELD = false>
-__global__ void __launch_bounds__(SplitConfig<NT, PRE>::THREADS, SplitConfig<NT, PRE>::CTAS)
+template <int NT, bool WITHHELD = false>
+__global__ void __launch_bounds__(SplitConfig<NT>::THREADS, SplitConfig<NT>::CTAS)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SplitParams p) {
-    using C = SplitConfig<NT, PRE>;
+    using C = SplitConfig<NT>;
+    constexpr bool PRE = C::PRE;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* raw = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* pieces = raw + C::STAGES * C::RAW_BYTES;
@@ -638,10 +638,10 @@ static int split_rows(const float* x, void* pieces, int tokens, int inner, cudaS
     return launch_kernel(split_rows_kernel, dim3(blocks), dim3(ROWS_THREADS), 0, stream, x, static_cast<uint4*>(pieces), tokens, inner);
 }
 
-template <int NT, bool PRE, bool WITHHELD = false>
+template <int NT, bool WITHHELD = false>
 static int launch_split(const CUtensorMap& map_w, const CUtensorMap& map_x, const SplitParams& p, int segments, cudaStream_t stream) {
-    using C = SplitConfig<NT, PRE>;
-    auto kernel = gemm_split_kernel<NT, PRE, WITHHELD>;
+    using C = SplitConfig<NT>;
+    auto kernel = gemm_split_kernel<NT, WITHHELD>;
     static SharedMemoryOptIn opt_in;
     if (const int e = opt_in(kernel, C::SMEM_BYTES)) return e;
     if (C::GROUPS == 2) {  // launched with fewer registers, the takers would wait for a share that does not exist
@@ -699,10 +699,10 @@ ME_EXPORT int me_gemm_split(const void* map_w, const void* map_x, const float* x
     memcpy(&x_map, map_x, sizeof(x_map));
     if (pieces != nullptr)
         if (const int e = split_rows(x, pieces, tokens, inner, stream)) return e;
-    if (tile == 16 && !pieces) return withheld ? launch_split<16, false, true>(w_map, x_map, p, segments, stream) : launch_split<16, false>(w_map, x_map, p, segments, stream);
-    if (tile == 64 && pieces) return withheld ? launch_split<64, true, true>(w_map, x_map, p, segments, stream) : launch_split<64, true>(w_map, x_map, p, segments, stream);
+    if (tile == 16 && !pieces) return withheld ? launch_split<16, true>(w_map, x_map, p, segments, stream) : launch_split<16>(w_map, x_map, p, segments, stream);
+    if (tile == 64 && pieces) return withheld ? launch_split<64, true>(w_map, x_map, p, segments, stream) : launch_split<64>(w_map, x_map, p, segments, stream);
     if (tile == 128 && pieces && (p.clustered || segments == 1))
-        return withheld ? launch_split<128, true, true>(w_map, x_map, p, segments, stream) : launch_split<128, true>(w_map, x_map, p, segments, stream);
+        return withheld ? launch_split<128, true>(w_map, x_map, p, segments, stream) : launch_split<128>(w_map, x_map, p, segments, stream);
     return ME_ERR_ARGUMENT;
 }
 
