@@ -183,6 +183,16 @@ __device__ __forceinline__ void pieces_of(float4 v, uint32_t* p0, uint32_t* p1, 
     p2[0] = upper_pair(rest.x, rest.y), p2[1] = upper_pair(rest.z, rest.w);
 }
 
+// Where a warp meets ahead of each instruction that is warp-wide (.aligned), since lanes go apart at every wait and every arrival of lane 0:
+//   tcgen05.alloc           the branch before it is another warp's (thread 0 is in warp 0)
+//   setmaxnreg, at roles    __syncthreads behind alloc, then branches on the warp's number alone; at the end __syncthreads again
+//   tcgen05.st              __all_sync of the wait for the raw tile, and of the wait for the unit that read these columns before
+//   tcgen05.wait::st        nothing divides lanes between the stores and it: the loop over tokens has as many turns in every lane of a warp
+//   tcgen05.ld, wait::ld    __all_sync of the wait for the block, and at the end of a segment of the wait for its last unit
+//   tcgen05.dealloc         __syncthreads and the __syncwarp behind the producer's last waits
+//   barrier.cluster         __syncwarp in cluster_sync
+// An elected thread's role ends in the branch of its own warp; arrivals on barriers, loads, MMAs and commits are single threads' instructions.
+//
 // WITHHELD: no weights are ever loaded (the tokens' pieces are) and waits end after a few polls, so that a test can take the way of a kernel
 // that gives up, with copies in flight where pieces are made ahead.
 template <int NT, bool WITHHELD = false>

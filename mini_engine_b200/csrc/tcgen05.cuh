@@ -233,7 +233,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     return rank;
 }
+// The instructions are warp-wide: lanes that ran alone (an elected thread's role, an output loop) meet the others first.
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
