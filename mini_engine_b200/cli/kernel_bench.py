@@ -107,18 +107,21 @@ MMA_RATE_CASES = [
 ]
 
 
-def mma_rate(pair: int, a_in_tensor_memory: int, b_mn_major: int, n: int, ctas: int = 148, iters: int = 2000) -> float:
-    """Cycles per MMA of K = 16 when nothing but MMAs runs (csrc/mma_rate.cu)."""
+def mma_rate(
+    pair: int, a_in_tensor_memory: int, b_mn_major: int, n: int, ctas: int = 148, iters: int = 2000, look: int = 0, lane: int = 0
+) -> float:
+    """Cycles per MMA of K = 16 when nothing but MMAs runs (csrc/mma_rate.cu); with ``look`` a wait for a completed barrier behind every
+    four of them, with ``lane`` issued by lane 0 instead of an elected thread."""
     import ctypes
 
     from mini_engine_b200.csrc.build import load_library
 
     lib = load_library("mma_rate")
-    lib.me_mma_rate.argtypes = [ctypes.c_void_p] + [ctypes.c_int] * 6 + [ctypes.c_void_p]
+    lib.me_mma_rate.argtypes = [ctypes.c_void_p] + [ctypes.c_int] * 8 + [ctypes.c_void_p]
     lib.me_mma_rate.restype = ctypes.c_int
     cycles = torch.zeros(1, dtype=torch.int64, device="cuda")
     for _ in range(2):
-        code = lib.me_mma_rate(cycles.data_ptr(), pair, a_in_tensor_memory, b_mn_major, n, ctas, iters, None)
+        code = lib.me_mma_rate(cycles.data_ptr(), pair, a_in_tensor_memory, b_mn_major, n, look, lane, ctas, iters, None)
         if code != 0:
             raise RuntimeError(f"me_mma_rate failed to launch (code {code})")
         torch.cuda.synchronize()
@@ -133,6 +136,13 @@ def bench_mma_rate(args) -> None:
         cycles = mma_rate(pair, in_tmem, mn_major, n)
         m = 256 if pair else 128
         print(f"{label}: {cycles:.1f} cycles per MMA of {m} x {n} x 16, {2 * 128 * n * 16 / cycles:.0f} flop per cycle and SM")
+    for in_tmem, n in ((1, 16), (1, 32), (1, 64), (0, 64)):
+        where = "tensor" if in_tmem else "shared"
+        elected, by_lane = mma_rate(0, in_tmem, 0, n), mma_rate(0, in_tmem, 0, n, lane=1)
+        print(f"one CTA, A in {where} memory, N = {n}: {elected:.1f} cycles per MMA by an elected thread, {by_lane:.1f} by lane 0")
+    for n in (16, 64, 128):
+        alone, looking = mma_rate(0, 1, 0, n), mma_rate(0, 1, 0, n, look=1)
+        print(f"one CTA, A in tensor memory, N = {n}: four MMAs {4 * alone:.0f} cycles, with a look at a completed barrier behind them {4 * looking:.0f}")
 
 
 def attention_context(entries: int, new_tokens: int, context: int):

@@ -674,7 +674,7 @@ attention_tcgen05_duo_kernel(const __grid_constant__ CUtensorMap map_q, const __
         if (has_work && elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(TC_KEYS);       // S[128 x 128] = Q K^T, K-major operands
             constexpr uint32_t idesc_o = make_idesc(TC_DIM, true);  // O[128 x 128] += P V, V is MN-major
-            // The pipe needs 64 cycles for 128 x 128 x 16, the thread that issues it less, but looks at barriers cost it 190 cycles
+            // The pipe needs 64 cycles for 128 x 128 x 16, the thread that issues it less, but looks at barriers cost it 198 cycles
             // each: what it does besides must stay little or the pipe waits for it.  So the operands' descriptors are made once (their
             // address field is additive: a k step further is a constant more) and the first MMA of a product, which overwrites, is
             // its own instruction instead of a predicate computed each time.

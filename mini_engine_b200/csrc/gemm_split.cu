@@ -35,12 +35,13 @@
 // by several pieces of the tokens.  Up to 16 tokens the converters make them too; for more, a kernel before this one makes them once
 // for all feature tiles (split_rows_kernel) and they arrive by TMA.
 //
-// What bounds it: the issuing thread.  Alone, the MMAs of a k block take 768 cycles with 64 tokens and 1,536 with 128; the thread's one
-// look at a barrier per unit takes 190 cycles on an idle SM and about 400 beside the converters, since it queues behind the MMAs
-// (csrc/mma_rate.cu measures the MMAs alone), and the last MMAs before it cover half of that.  A block takes 1,300 cycles with 64 tokens,
-// 2,300 with 128.  So the thread looks once a unit, at one barrier that takes the arrivals of converters, takers and TMA together, and the
-// widest MMAs come last.  Two groups of eight converter warps work on alternate units: one group (with the tokens to convert as well)
-// took 2,000 to 2,700 cycles a block from the arrival of a tile to its last piece.  us of a product (plain stream order, behind a flushed L2; one group of
+// What bounds it: the issuing thread.  Alone, the MMAs of a k block take 768 cycles with 64 tokens and 1,536 with 128.  A look at a barrier takes
+// the thread 198 cycles, also when the barrier has long completed, and only the MMAs issued before run meanwhile (`kernel_bench mma-rate`, an
+// idle SM: four MMAs of 16 or 64 columns 36 and 128 cycles, with a look behind them 198 either way, of 128 columns 256 with and without).
+// A block takes 1,380 cycles with 64 tokens, 2,390 with 128, and 2,830 in both CTAs of an SM with 16 (what each of 64 blocks more takes, with a
+// CTA or two on every SM, at 1,965 MHz).  So the thread looks once a unit, at one barrier that takes the arrivals of converters, takers and TMA
+// together, and the widest MMAs come last.  Two groups of eight converter warps work on alternate units: one group (with the tokens to convert as
+// well) took 2,000 to 2,700 cycles a block from the arrival of a tile to its last piece (clock stamps in a copy).  us of a product (plain stream order, behind a flushed L2; one group of
 // converters and waits of their own | this form; of the 64-token and wider ones 5 are split_rows_kernel and its launch): 256 x 24,576 x 4,096 320 | 260
 // (198 TFLOP/s), 256 x 4,096 x 12,288 199 | 149, 512 x 2,048 x 6,144 115 | 78, 512 x 2,048 x 2,048 46 | 33, 1,024 sorted rows in 8 groups x 6,144 x 2,048
 // 259 | 185, 64 x 2,048 x 9,216 55 | 41, 8 x 24,576 x 4,096 92 | 81 (5.0 TB/s of weights), 8 x 2,048 x 2,048 13.7 | 11.2.
@@ -229,7 +230,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (threadIdx.x == 0) {
         *gave_up = 0;
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], CONVERTERS / 32); }
-        // The issuer waits once a unit: a wait holds it for 190 cycles and more, which only the last MMAs before it cover.  So a unit's
+        // The issuer waits once a unit: a look holds it for 198 cycles, which only the last MMAs before it cover.  So a unit's
         // barrier also takes the arrivals of the tokens' pieces and of the takers who have emptied the sums that it overwrites:
         // in the first unit of a block if that is a unit of its own (barriers 0 and 2 of four if a block has two units).
         for (int b = 0; b < RING; ++b) {

@@ -15,8 +15,9 @@ __device__ __forceinline__ void tcgen05_mma_bf16_ts_pair(uint32_t d_tmem, uint32
         : "memory");
 }
 
-// mode: 0 SS one CTA, 1 TS one CTA, 2 SS pair, 3 TS pair.  B K-major unless mn != 0.
-template <int MODE, int N, int MN>
+// mode: 0 SS one CTA, 1 TS one CTA, 2 SS pair, 3 TS pair.  B K-major unless mn != 0.  look: a wait for a barrier that has long
+// completed behind every four MMAs.  lane: the issuing thread is chosen by its lane number instead of being elected.
+template <int MODE, int N, int MN, bool LOOK, bool LANE>
 __global__ void __launch_bounds__(128) mma_rate_kernel(long long* out, int iters) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -27,7 +28,7 @@ __global__ void __launch_bounds__(128) mma_rate_kernel(long long* out, int iters
     constexpr bool PAIR = MODE >= 2, TS = (MODE & 1) != 0;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0;
     for (int i = threadIdx.x; i < (16384 + 32768) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(tiles)[i] = 0;
-    if (threadIdx.x == 0) { mbar_init(bar, 1); asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+    if (threadIdx.x == 0) { mbar_init(bar, 1); mbar_init(bar + 1, 1); mbar_arrive(bar + 1); asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (threadIdx.x < 32) { if (PAIR) tcgen05_alloc_pair(holder, 512); else tcgen05_alloc(holder, 512); }
     tcgen05_fence_before();
@@ -35,7 +36,7 @@ __global__ void __launch_bounds__(128) mma_rate_kernel(long long* out, int iters
     if (PAIR) cluster_sync();
     tcgen05_fence_after();
     const uint32_t tmem = *holder;
-    if (threadIdx.x < 32 && rank == 0 && elect_one()) {
+    if (threadIdx.x < 32 && rank == 0 && (LANE ? threadIdx.x == 0 : elect_one())) {
         const uint32_t idesc = PAIR ? (make_idesc_pair(N) | (MN ? (1u << 16) : 0u)) : make_idesc(N, MN != 0);
         const uint64_t a_desc = smem_desc_sw128(smem_u32(a_tile));
         const uint64_t b_desc = MN ? smem_desc_sw128_mn(smem_u32(b_tile), 16384) : smem_desc_sw128(smem_u32(b_tile));
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(128) mma_rate_kernel(long long* out, int iters
                     else tcgen05_mma_bf16(tmem, a_desc + (k * 32 >> 4), b_desc + step, idesc, 1u);
                 }
             }
+            if (LOOK) mbar_wait(bar + 1, 0);
         }
         if (PAIR) tcgen05_commit_pair(bar); else tcgen05_commit(bar);
         const bool ok = mbar_wait(bar, 0);
@@ -67,10 +69,10 @@ __global__ void __launch_bounds__(128) mma_rate_kernel(long long* out, int iters
 }
 
 
-template <int MODE, int N, int MN>
+template <int MODE, int N, int MN, bool LOOK, bool LANE>
 static int launch_rate(long long* cycles, int ctas, int iters, cudaStream_t stream) {
     constexpr int SMEM = 16384 + 32768 + 1024 + 256;
-    auto kernel = mma_rate_kernel<MODE, N, MN>;
+    auto kernel = mma_rate_kernel<MODE, N, MN, LOOK, LANE>;
     static SharedMemoryOptIn opt_in;
     if (const int e = opt_in(kernel, SMEM)) return e;
     cudaLaunchConfig_t config = {};
@@ -91,15 +93,21 @@ static int launch_rate(long long* cycles, int ctas, int iters, cudaStream_t stre
 // `cycles` (device, one int64) receives the cycles that CTA 0 needed for 4 * iters MMAs of
 // M = 128 (256 for a pair), N = n, K = 16, or -1 when its bounded wait ran out.
 // pair: 0 one CTA, 1 a CTA pair (cta_group::2; ctas must be even); a_in_tensor_memory: 0 / 1;
-// b_mn_major: the second operand's rows run along the reduction (as values do in attention).
-ME_EXPORT int me_mma_rate(long long* cycles, int pair, int a_in_tensor_memory, int b_mn_major, int n, int ctas, int iters,
+// b_mn_major: the second operand's rows run along the reduction (as values do in attention).  look, lane: see the kernel.
+ME_EXPORT int me_mma_rate(long long* cycles, int pair, int a_in_tensor_memory, int b_mn_major, int n, int look, int lane, int ctas, int iters,
                           cudaStream_t stream) {
     if (ctas < 1 || iters < 1 || (pair && ctas % 2)) return ME_ERR_ARGUMENT;
     const int mode = (pair ? 2 : 0) + (a_in_tensor_memory ? 1 : 0);
-#define ME_RATE_CASE(MODE, N, MN) \
-    if (mode == MODE && n == N && (b_mn_major != 0) == (MN != 0)) return launch_rate<MODE, N, MN>(cycles, ctas, iters, stream);
-    ME_RATE_CASE(0, 64, 0) ME_RATE_CASE(0, 128, 0) ME_RATE_CASE(0, 256, 0) ME_RATE_CASE(1, 128, 1) ME_RATE_CASE(1, 128, 0)
-    ME_RATE_CASE(2, 64, 0) ME_RATE_CASE(2, 128, 0) ME_RATE_CASE(2, 256, 0) ME_RATE_CASE(3, 128, 1) ME_RATE_CASE(3, 128, 0)
+#define ME_RATE_CASE(MODE, N, MN, LOOK, LANE)                                                              \
+    if (mode == MODE && n == N && (b_mn_major != 0) == (MN != 0) && (look != 0) == LOOK && (lane != 0) == LANE) \
+        return launch_rate<MODE, N, MN, LOOK, LANE>(cycles, ctas, iters, stream);
+#define ME_RATE_PLAIN(MODE, N, MN) ME_RATE_CASE(MODE, N, MN, false, false)
+    ME_RATE_PLAIN(0, 64, 0) ME_RATE_PLAIN(0, 128, 0) ME_RATE_PLAIN(0, 256, 0) ME_RATE_PLAIN(1, 128, 1) ME_RATE_PLAIN(1, 128, 0)
+    ME_RATE_PLAIN(2, 64, 0) ME_RATE_PLAIN(2, 128, 0) ME_RATE_PLAIN(2, 256, 0) ME_RATE_PLAIN(3, 128, 1) ME_RATE_PLAIN(3, 128, 0)
+    ME_RATE_PLAIN(1, 16, 0) ME_RATE_PLAIN(1, 32, 0) ME_RATE_PLAIN(1, 64, 0)
+    ME_RATE_CASE(1, 16, 0, false, true) ME_RATE_CASE(1, 32, 0, false, true) ME_RATE_CASE(1, 64, 0, false, true) ME_RATE_CASE(0, 64, 0, false, true)
+    ME_RATE_CASE(1, 16, 0, true, false) ME_RATE_CASE(1, 64, 0, true, false) ME_RATE_CASE(1, 128, 0, true, false)
+#undef ME_RATE_PLAIN
 #undef ME_RATE_CASE
     return ME_ERR_UNSUPPORTED;
 }
