@@ -353,8 +353,10 @@ __global__ void __launch_bounds__(ROW_THREADS) paged_attention_rows_kernel(RowAr
 // at heads of 128 and 11 over latent rows of 576, while most SMs are idle.  Only what a row's order of operations demands is serial here:
 // the scores of all tiles are independent (first kernel, a block to a tile), a tile's maximum needs its own scores, its weights the
 // running maximum, and the chains over the keys are separate for every value element (second kernel, a block to 64 value columns).
-// Eight decoded tokens behind 17 to 512, once with 16 heads in 8 KV heads of 128 and once over latent rows of 576 with 512 values: 68 and 180 us ->
-// 2 x 10 us of scores and 2 x 40 us of values (a step of four tiles takes the latencies of its softmax and of 128 keys' chain, 9 us).
+// Eight decoded tokens, us, the kernel above | these two: 16 heads in 8 KV heads of 128 behind 512 68 | 38, behind 2,048 250 | 114; 16 heads over
+// latent rows of 576 with 512 values 176 | 69 and 666 | 220.  Of the 114 the second kernel takes 76: a step of four tiles takes the
+// latencies of its softmax and of 128 keys' chain, 5 us, in blocks of eight warps of which few are resident.  More entries, and where the one kernel
+// is faster: ops.few_rows_pay.
 constexpr int FEW_ROWS = 16, FEW_TILES = 4, FEW_KEYS = 32 * FEW_TILES, FEW_COLUMNS = 64;  // rows of a block; tiles and keys of a step of the second kernel
 
 struct FewRows {

@@ -947,9 +947,9 @@ def mixed_attention(
 # (KV heads, query heads of each) that the tile kernel is built for, and which entries take it where both forms run: those that
 # bring so many eighths of the keys that they see, or so many tokens.  A tile walks all of its keys, twice, on one SM, however few
 # its tokens are; the two kernels take a time per token.  Measured, us, tiles | two kernels, one entry behind 2,048 (a window of
-# 1,024 and 64 kept keys): 32 heads in 8: 64 tokens 424 | 300, 96 424 | 429, 127 436 | 527; 16 in 8: 64 224 | 194, 96 224 | 270;
-# 16 in 4: 96 313 | 228, 192 313 | 394; behind 512: 32 in 8 64 223 | 167, 96 236 | 246; 16 in 8 64 120 | 110, 96 126 | 153; 16 in 4
-# 127 189 | 160, 192 201 | 241; whole prompts of 16 and 64 tokens: 24 | 26 and 36 | 62, 14 | 20 and 21 | 46, 18 | 20 and 27 | 36.
+# 1,024 and 64 kept keys), L2 flushed: 32 heads in 8: 64 tokens 424 | 321, 80 424 | 390, 96 424 | 462; 16 in 8: 64 225 | 216, 80 225 | 257;
+# 16 in 4: 96 320 | 230, 144 320 | 304, 192 319 | 413; behind 512: 32 in 8 80 236 | 226, 96 236 | 269; 16 in 8 64 121 | 124, 80 127 | 153;
+# 16 in 4 127 188 | 171, 192 205 | 257; whole prompts of 16 and 64 tokens: 27 | 28 and 37 | 75, 16 | 22 and 23 | 54, 21 | 21 and 30 | 40.
 MIXED_TILES = {(8, 4): (3, 96), (8, 2): (2, 80), (4, 4): (6, 144)}
 MIXED_TILES_START = 24  # tokens that take the two kernels as long as their two launches
 MIXED_TILES_MIN_TOKENS = 8  # of an entry: a tile takes as long with one token in it as with eight
@@ -973,8 +973,8 @@ def mixed_attention_forms(
     portion's ``portion_keys``.  A form that no entry can take is not launched (an eager launch is 15 us of the host).  More
     tokens than any entry needs for tiles run in tiles all together where that is faster: the tiles' time, which goes with
     the keys, grows from ``portion_keys`` to ``keys``, and the two kernels' time for the decoded tokens is spared.  32 heads in 8,
-    us, all in tiles | each its own: 32 decoded behind 2,048 beside a portion of 512 behind 512 442 | 592; eight beside a
-    prompt of 192 422 | 161."""
+    us, all in tiles | each its own: 32 decoded behind 2,048 beside a portion of 512 behind 512 432 | 612; eight beside a
+    prompt of 192 424 | 166."""
     eighths, most = MIXED_TILES[kv_heads, heads // kv_heads]
     takes = lambda count: count >= MIXED_TILES_MIN_TOKENS and (count >= most or 8 * count >= eighths * portion_keys)  # noqa: E731
     if longest < MIXED_TILES_MIN_TOKENS:
