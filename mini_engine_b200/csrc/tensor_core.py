@@ -240,14 +240,17 @@ def gemm_swiglu(
 
 # ------------------------------------------------------------------------------ float32
 
-# Tokens per CTA (up to 16 two CTAs share an SM, else one) and the us of a k block.  A round of CTAs costs SPLIT_START beside them, a
-# cluster's exchange SPLIT_EXCHANGE for each segment of 128 tokens.  Clusters of 1 to 8 CTAs that are resident at a time with one CTA
-# to an SM (cudaOccupancyMaxActiveClusters on a B200; with two to an SM twice as many and a few more).  Measured forms, us (64 tokens to a
-# CTA and segments one after the other; 64 side by side; 128): 256 tokens x 6,144 x 4,096 98, 107, 99; x 24,576 x 4,096 306, -, 260; x
-# 4,096 x 4,096 54, 81, 71; 512 x 2,048 x 2,048 33, 84, 64; 512 x 9,216 x 2,048 115, 145, 114; 512 x 2,048 x 9,216 115, 170, 142;
-# 128 x 2,048 x 2,048 32, 30, 27; 64 x 2,048 x 9,216 101, 41, 55; 40 x 6,144 x 2,048 30, 30, 40.
-SPLIT_TILES = {16: 1.0, 64: 0.70, 128: 1.25}
-SPLIT_START, SPLIT_EXCHANGE = 5.0, 0.25
+# Tokens per CTA (with 16 two CTAs share an SM, else one), the us of a k block and of a round of CTAs beside its blocks.  Two CTAs on an SM have
+# SPLIT_SHARED for a block; 64 and 128 tokens have their pieces made by a launch more, SPLIT_PIECES; a cluster's exchange costs SPLIT_EXCHANGE
+# for each segment of 128 tokens.  Clusters of 1 to 8 CTAs that are resident at a time with one CTA to an SM (cudaOccupancyMaxActiveClusters
+# on a B200; with two to an SM twice as many and a few more).  Fitted to 478 shapes (1 to 2,048 tokens, 64 to 32,768 outputs of 64 to
+# 12,288 inputs) in all their forms: for 11 of them another form is more than 5 % faster (27 % at most).  us of 16, 16 side by side | 64, 64 side by side, 128: 17 tokens x
+# 2,048 x 2,048 34, 16 | 38, 30, 32; x 64 x 64 9 | 14, 15; 64 x 1,024 x 1,024 21, 13 | 28, 20, 22; x 2,048 x 512 14, 13 | 22, 20, 22; x 6,144 x
+# 2,048 47, 50 | 38, 40, 50; 128 x 160 x 2,048 34, 15 | 38, 20, 22; 256 x 12,288 x 1,024 116 | 62, 58; 512 x 2,048 x 512 31, 38 | 22, 32, 26 (all with the
+# 7 us of two events and a launch).  Without the 16-token form beyond 16 tokens, small products were up to 29 % behind what they took
+# before pieces were made ahead.
+SPLIT_TILES = {16: (0.80, 3.6), 64: (0.70, 5.8), 128: (1.15, 6.4)}
+SPLIT_SHARED, SPLIT_PIECES, SPLIT_EXCHANGE = 1.06, 3.4, 0.30
 SPLIT_CLUSTERS = (NUM_SMS, 74, 45, 33, 26, 22, 15, 15)
 SPLIT_PIECES_MIN_TILE = 64  # tokens per CTA from which on their pieces are made ahead, by a kernel of their own
 # Bytes of pieces at a time: they come out of what the page pool leaves, so larger steps (from 7,281 tokens of 12,288 on) run in parts.  8,192 x 1,024 x
@@ -302,16 +305,18 @@ def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | No
     blocks = -(-inner // BLOCK_K)
     per_segment = -(-blocks // segments)
     forms = []
-    for rows, cost in SPLIT_TILES.items():
-        if (rows != tile) if tile is not None else (rows == 16) != (tokens <= 16) or (rows == 128 and tokens <= 64):
+    for rows, (block, start) in SPLIT_TILES.items():
+        if (rows != tile) if tile is not None else (rows > 16 and tokens <= 16):
             continue
         per_sm = 2 if rows == 16 else 1
+        pieces = SPLIT_PIECES if rows >= SPLIT_PIECES_MIN_TILE else 0.0
         ctas = -(-outs // BLOCK_N) * -(-tokens // rows)
+        cost = lambda resident: SPLIT_SHARED if rows == 16 and resident > NUM_SMS else block  # noqa: B023, E731
         if rows < 128 or segments == 1:
-            forms.append((-(-ctas // (per_sm * NUM_SMS)) * (blocks * cost + SPLIT_START), rows, False))
+            forms.append((-(-ctas // (per_sm * NUM_SMS)) * (blocks * cost(ctas) + start) + pieces, rows, False))
         if segments > 1:
             rounds = -(-ctas // (per_sm * SPLIT_CLUSTERS[segments - 1]))
-            forms.append((rounds * (per_segment * cost + SPLIT_START + SPLIT_EXCHANGE * segments * rows / 128), rows, True))
+            forms.append((rounds * (per_segment * cost(ctas * segments) + start + SPLIT_EXCHANGE * segments * rows / 128) + pieces, rows, True))
     return min(forms)[1:]
 
 

@@ -63,6 +63,18 @@ def test_split_product(tokens, outs, inner):
         assert torch.equal(part, out[rows])
 
 
+# small products of more than 16 tokens, where the launch that makes pieces counts; larger ones, where weights converted once for many tokens do
+@pytest.mark.parametrize(
+    "tokens,outs,inner,form",
+    [(17, 64, 64, (16, False)), (256, 64, 64, (16, False)), (64, 1024, 1024, (16, True)), (17, 2048, 2048, (16, True)), (128, 160, 2048, (16, True)),
+     (17, 2048, 6144, (16, True)), (512, 2048, 2048, (64, False)), (512, 2048, 512, (64, False)),
+     (64, 2048, 9216, (64, True)), (256, 24576, 4096, (128, False)), (8, 24576, 4096, (16, False))],
+)  # fmt: skip
+def test_the_form_that_was_measured_fastest_is_taken(tokens, outs, inner, form):
+    tc = tensor_core()
+    assert tc.split_form(tokens, outs, inner, tc.split_segments(outs, inner)) == form
+
+
 @pytest.mark.gpu
 def test_infinities_and_nan_come_out_as_in_one_chain():
     from mini_engine_b200.csrc import ops
