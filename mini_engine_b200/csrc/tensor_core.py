@@ -13,7 +13,7 @@ from functools import lru_cache
 
 import torch
 
-from mini_engine_b200.csrc import ops
+from mini_engine_b200.csrc import build, ops
 from mini_engine_b200.csrc.build import load_library
 
 NUM_SMS = 148
@@ -241,16 +241,17 @@ def gemm_swiglu(
 # ------------------------------------------------------------------------------ float32
 
 # Tokens per CTA (with 16 two CTAs share an SM, else one), the us of a k block and of a round of CTAs beside its blocks.  Two CTAs on an SM have
-# SPLIT_SHARED for a block; 64 and 128 tokens have their pieces made by a launch more, SPLIT_PIECES; a cluster's exchange costs SPLIT_EXCHANGE
-# for each segment of 128 tokens.  Clusters of 1 to 8 CTAs that are resident at a time with one CTA to an SM (cudaOccupancyMaxActiveClusters
-# on a B200; with two to an SM twice as many and a few more).  Fitted to 478 shapes (1 to 2,048 tokens, 64 to 32,768 outputs of 64 to
-# 12,288 inputs) in all their forms: for 11 of them another form is more than 5 % faster (27 % at most).  us of 16, 16 side by side | 64, 64 side by side, 128: 17 tokens x
-# 2,048 x 2,048 34, 16 | 38, 30, 32; x 64 x 64 9 | 14, 15; 64 x 1,024 x 1,024 21, 13 | 28, 20, 22; x 2,048 x 512 14, 13 | 22, 20, 22; x 6,144 x
-# 2,048 47, 50 | 38, 40, 50; 128 x 160 x 2,048 34, 15 | 38, 20, 22; 256 x 12,288 x 1,024 116 | 62, 58; 512 x 2,048 x 512 31, 38 | 22, 32, 26 (all with the
-# 7 us of two events and a launch).  Without the 16-token form beyond 16 tokens, small products were up to 29 % behind what they took
-# before pieces were made ahead.
-SPLIT_TILES = {16: (0.80, 3.6), 64: (0.70, 5.8), 128: (1.15, 6.4)}
-SPLIT_SHARED, SPLIT_PIECES, SPLIT_EXCHANGE = 1.06, 3.4, 0.30
+# SPLIT_SHARED for a block; 64 and 128 tokens have their pieces made by a launch more, SPLIT_PIECES, of which nothing is left where launches overlap;
+# a cluster's exchange costs SPLIT_EXCHANGE for each segment of 128 tokens.  Clusters of 1 to 8 CTAs that are resident at a time with one CTA to an
+# SM (cudaOccupancyMaxActiveClusters on a B200; with two to an SM twice as many and two more).  The constants fit 478 shapes alone and 442 in chains
+# of products (1 to 2,048 tokens, 64 to 32,768 outputs of 64 to 12,288 inputs) in all their forms: for 13 of them another form is more than 5 %
+# faster.  us in a chain in plain stream order, 16 tokens to a CTA, 16 side by side | 64, 64 side by side, 128 side by side: 17 tokens x 2,048 x 2,048 29, 11 |
+# 30, 20, 24; 40 x 576 x 2,048 29, 8.3 | 31, 11.8, 13.5; 128 of these 28, 16 | 31, 12, 15; 40 x 4,096 x 2,048 30, 26 | 31, 25.6, 31; 256 of these 78, 111 |
+# 33, 62, 52; where launches overlap, 40 x 576 x 2,048 29, 8.3 | 28, 8.3, 10.5 and 40 x 4,096 x 2,048 34, 25 | 28, 22, 28.  With 64 and 128 alone, small
+# products in plain stream order were up to 29 % behind what they took before pieces were made ahead.
+SPLIT_TILES = {16: (0.84, 4.2), 64: (0.70, 5.8), 128: (1.15, 6.4)}
+SPLIT_SHARED, SPLIT_EXCHANGE = 1.12, 0.30
+SPLIT_PIECES = (3.4, 0.0)  # in plain stream order, and where a launch begins while the one before ends
 SPLIT_CLUSTERS = (NUM_SMS, 74, 45, 33, 26, 22, 15, 15)
 SPLIT_PIECES_MIN_TILE = 64  # tokens per CTA from which on their pieces are made ahead, by a kernel of their own
 # Bytes of pieces at a time: they come out of what the page pool leaves, so larger steps (from 7,281 tokens of 12,288 on) run in parts.  8,192 x 1,024 x
@@ -299,9 +300,10 @@ def split_segments(outs: int, inner: int) -> int:
 
 
 @lru_cache(maxsize=4096)
-def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | None = None) -> tuple[int, bool]:
+def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | None = None, overlapped: bool = False) -> tuple[int, bool]:
     """Tokens per CTA (or the given ``tile``), and whether a tile's segments run in the CTAs of a cluster or one after the other in a
-    CTA; the bits are the same in every form.  The form whose rounds of resident CTAs take least time."""
+    CTA; the bits are the same in every form.  The form whose rounds of resident CTAs take least time, in plain stream order or
+    (``overlapped``) as programmatic dependents."""
     blocks = -(-inner // BLOCK_K)
     per_segment = -(-blocks // segments)
     forms = []
@@ -309,13 +311,13 @@ def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | No
         if (rows != tile) if tile is not None else (rows > 16 and tokens <= 16):
             continue
         per_sm = 2 if rows == 16 else 1
-        pieces = SPLIT_PIECES if rows >= SPLIT_PIECES_MIN_TILE else 0.0
+        pieces = SPLIT_PIECES[overlapped] if rows >= SPLIT_PIECES_MIN_TILE else 0.0
         ctas = -(-outs // BLOCK_N) * -(-tokens // rows)
         cost = lambda resident: SPLIT_SHARED if rows == 16 and resident > NUM_SMS else block  # noqa: B023, E731
         if rows < 128 or segments == 1:
             forms.append((-(-ctas // (per_sm * NUM_SMS)) * (blocks * cost(ctas) + start) + pieces, rows, False))
         if segments > 1:
-            rounds = -(-ctas // (per_sm * SPLIT_CLUSTERS[segments - 1]))
+            rounds = -(-ctas // (per_sm * SPLIT_CLUSTERS[segments - 1] + 2 * (per_sm - 1)))
             forms.append((rounds * (per_segment * cost(ctas * segments) + start + SPLIT_EXCHANGE * segments * rows / 128) + pieces, rows, True))
     return min(forms)[1:]
 
@@ -369,7 +371,7 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
         raise RuntimeError(f"output {tuple(out.shape)} does not fit [{tokens}, {plan.rows}] float32")
     if tokens == 0:
         return
-    tile, side_by_side = split_form(tokens, plan.rows, plan.inner, plan.segments) if form is None else form
+    tile, side_by_side = form or split_form(tokens, plan.rows, plan.inner, plan.segments, None, build.programmatic_launch_enabled())
     _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, workspace)
 
 
@@ -424,7 +426,7 @@ def gemm_split_grouped(
     if pad not in SPLIT_TILES or rows % pad or group_of_block.dtype != torch.int32 or group_of_block.numel() < rows // pad:
         raise RuntimeError("the rows of a grouped product come in runs of a token tile with one int32 group each")
     if side_by_side is None:
-        side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad)[1]
+        side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad, build.programmatic_launch_enabled())[1]
     _launch_split(plan, x, out, outs, pad, side_by_side, group_of_block, workspace)
 
 

@@ -75,6 +75,14 @@ def test_the_form_that_was_measured_fastest_is_taken(tokens, outs, inner, form):
     assert tc.split_form(tokens, outs, inner, tc.split_segments(outs, inner)) == form
 
 
+def test_the_launch_that_makes_pieces_counts_in_plain_stream_order_only():
+    tc = tensor_core()
+    segments = tc.split_segments(2048, 2048)
+    assert tc.split_form(40, 2048, 2048, segments)[0] == 16  # 17.7 us, 21.1 with 64
+    segments = tc.split_segments(4096, 2048)
+    assert tc.split_form(40, 4096, 2048, segments, overlapped=True) == (64, True)  # 22.1 us, 25.4 with 16
+
+
 @pytest.mark.gpu
 def test_infinities_and_nan_come_out_as_in_one_chain():
     from mini_engine_b200.csrc import ops
