@@ -174,11 +174,6 @@ def set_programmatic_launch(enabled: bool) -> bool:
     return previous
 
 
-def programmatic_launch_enabled() -> bool:
-    """Whether launches are programmatic dependents of their predecessors at the moment."""
-    return _programmatic_launch
-
-
 def build_all(names: list[str] | None = None, verbose: bool = True) -> list[Path]:
     """Compile the named libraries (all by default), several at a time."""
     names = list(names or LIBRARIES)

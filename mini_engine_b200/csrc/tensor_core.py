@@ -371,7 +371,7 @@ def gemm_split(plan: SplitPlan, x: torch.Tensor, out: torch.Tensor, form: tuple[
         raise RuntimeError(f"output {tuple(out.shape)} does not fit [{tokens}, {plan.rows}] float32")
     if tokens == 0:
         return
-    tile, side_by_side = form or split_form(tokens, plan.rows, plan.inner, plan.segments, None, build.programmatic_launch_enabled())
+    tile, side_by_side = form or split_form(tokens, plan.rows, plan.inner, plan.segments, None, build._programmatic_launch)
     _launch_split(plan, x, out, plan.rows, tile, side_by_side, None, workspace)
 
 
@@ -380,32 +380,34 @@ def _launch_split(
     withheld: bool = False,
 ) -> None:  # fmt: skip
     rows, inner = x.shape
-    at_once, held = rows, None
-    if tile >= SPLIT_PIECES_MIN_TILE:
-        # as many rows at a time as their pieces have room, in parts of about the same size
+    pieces = None
+    if tile < SPLIT_PIECES_MIN_TILE:
+        x_map = _split_activation_map(x, tile)
+    else:
         width = 3 * (-(-inner // 8) * 8)
-        parts = -(-rows // max(tile, SPLIT_PIECES_BYTES // (2 * width) // tile * tile))
-        at_once = -(-rows // (parts * tile)) * tile
-        count = width * min(at_once, rows)
+        if 2 * width * rows > SPLIT_PIECES_BYTES:  # as many rows at a time as their pieces have room, in parts of about the same size
+            parts = -(-rows // max(tile, SPLIT_PIECES_BYTES // (2 * width) // tile * tile))
+            at_once = -(-rows // (parts * tile)) * tile
+            if at_once < rows:
+                for first in range(0, rows, at_once):
+                    part = slice(first, min(first + at_once, rows))
+                    _launch_split(
+                        plan, x[part], out[part], outs, tile, side_by_side, None if groups is None else groups[first // tile :], workspace, withheld
+                    )  # fmt: skip
+                return
         if workspace is None:
-            held = torch.empty(count, dtype=torch.bfloat16, device=x.device)
+            held = torch.empty(width * rows, dtype=torch.bfloat16, device=x.device)
         else:
-            held = workspace.growing("split.pieces", (count,), torch.bfloat16)
-    for first in range(0, rows, at_once):
-        some = min(at_once, rows - first)
-        if held is None:
-            pieces, x_map = None, _split_activation_map(x, tile)
-        else:
-            pieces, x_map = held.data_ptr(), _split_activation_map(held, tile, some, inner)
-            _count_launch()
-        code = _split_library().me_gemm_split(
-            plan.map, x_map, x.data_ptr() + 4 * first * inner, plan.weight.data_ptr(), out.data_ptr() + 4 * first * outs, some, outs, inner, tile,
-            pieces, plan.segments, 1 if side_by_side else 0, None if groups is None else groups.data_ptr() + 4 * (first // tile),
-            0 if groups is None else outs, 1 if withheld else 0, _ops_stream(),
-        )  # fmt: skip
+            held = workspace.growing("split.pieces", (width * rows,), torch.bfloat16)
+        pieces, x_map = held.data_ptr(), _split_activation_map(held, tile, rows, inner)
         _count_launch()
-        if code != 0:
-            raise RuntimeError(f"float32 tensor-core product failed to launch (code {code})")
+    code = _split_library().me_gemm_split(
+        plan.map, x_map, x.data_ptr(), plan.weight.data_ptr(), out.data_ptr(), rows, outs, inner, tile, pieces, plan.segments,
+        1 if side_by_side else 0, None if groups is None else groups.data_ptr(), 0 if groups is None else outs, 1 if withheld else 0, _ops_stream(),
+    )  # fmt: skip
+    _count_launch()
+    if code != 0:
+        raise RuntimeError(f"float32 tensor-core product failed to launch (code {code})")
 
 
 def gemm_split_grouped(
@@ -426,7 +428,7 @@ def gemm_split_grouped(
     if pad not in SPLIT_TILES or rows % pad or group_of_block.dtype != torch.int32 or group_of_block.numel() < rows // pad:
         raise RuntimeError("the rows of a grouped product come in runs of a token tile with one int32 group each")
     if side_by_side is None:
-        side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad, build.programmatic_launch_enabled())[1]
+        side_by_side = split_form(max(1, min(filled, rows // pad)) * pad, outs, plan.inner, plan.segments, pad, build._programmatic_launch)[1]
     _launch_split(plan, x, out, outs, pad, side_by_side, group_of_block, workspace)
 
 

@@ -31,6 +31,7 @@ class Workspace:
 
     def _view(self, name: str, dtype: torch.dtype, shape: tuple[int, ...], elements: int) -> torch.Tensor:
         """``shape`` at the start of the named buffer, which holds at least ``elements``."""
+        shape = tuple(shape)
         flat = self._flat(name, elements, dtype)
         views = self._views.setdefault((name, dtype), {})
         if len(views) >= 64:  # steps of many token counts
@@ -40,7 +41,10 @@ class Workspace:
 
     def _held_view(self, name: str, dtype: torch.dtype, shape: tuple[int, ...]) -> torch.Tensor | None:
         views = self._views.get((name, dtype))
-        return None if views is None else views.get(shape)
+        try:
+            return None if views is None else views.get(shape)
+        except TypeError:  # a list; looking first would cost a step of some hundred buffers more than the exception ever does
+            return views.get(tuple(shape))
 
     def _flat(self, name: str, elements: int, dtype: torch.dtype) -> torch.Tensor:
         key = (name, dtype)
@@ -58,7 +62,6 @@ class Workspace:
     def get(self, name: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """A contiguous view ``shape`` of the named buffer.  The first axis is a token count;
         the buffer is sized for ``max_tokens`` of them."""
-        shape = tuple(shape)
         held = self._held_view(name, dtype, shape)
         if held is not None:
             return held
@@ -77,7 +80,6 @@ class Workspace:
         token capacity (logits: ``[rows, vocab]`` is large and ``rows`` is usually small).  It grows
         by half at least, so that steps of ever longer prompts do not leave one buffer behind for
         every length: all that it has ever replaced is less than twice what it holds."""
-        shape = tuple(shape)
         view = self._held_view(name, dtype, shape)
         if view is not None:
             return view
