@@ -185,3 +185,11 @@ def test_plain_rotated_values_depend_on_the_distance_alone():
     assert torch.allclose(here, later, atol=1e-9)
     unturned = torch.softmax((q[6, 0] @ k[3:, 0].T) * 0.5, -1) @ v[3:, 0]
     assert not torch.allclose(here[6, 0], unturned, atol=1e-2)
+
+
+def test_expected_runs_of_sorted_rows():
+    """Few rows fill a run of every unit that is chosen; many fill whole runs and half of a last one each."""
+    from mini_engine_b200.parts.moe import expected_runs
+
+    assert [expected_runs(n, 8, 16) for n in (1, 2, 16, 32, 256)] == [1, 2, 8, 8, 20]
+    assert expected_runs(1024, 8, 64) == 20 and expected_runs(64, 64, 16) == 41 and expected_runs(5, 1, 16) == 1
