@@ -252,6 +252,9 @@ def gemm_swiglu(
 SPLIT_TILES = {16: (0.84, 4.2), 64: (0.70, 5.8), 128: (1.15, 6.4)}
 SPLIT_SHARED, SPLIT_EXCHANGE = 1.12, 0.30
 SPLIT_PIECES = (3.4, 0.0)  # in plain stream order, and where a launch begins while the one before ends
+# The same for runs of sorted rows, whose weights are each read once only, so that a CTA's block waits for memory more: one decoded token of Molotar's
+# sizes 668 us with these constants and 684 with those above, 48 tokens 1,263 and 1,281.
+SPLIT_GROUPED = {16: (1.0, 5.0), 64: (0.70, 5.0), 128: (1.25, 5.0)}
 SPLIT_CLUSTERS = (NUM_SMS, 74, 45, 33, 26, 22, 15, 15)
 SPLIT_PIECES_MIN_TILE = 64  # tokens per CTA from which on their pieces are made ahead, by a kernel of their own
 # Bytes of pieces at a time: they come out of what the page pool leaves, so larger steps (from 7,281 tokens of 12,288 on) run in parts.  8,192 x 1,024 x
@@ -302,22 +305,22 @@ def split_segments(outs: int, inner: int) -> int:
 @lru_cache(maxsize=4096)
 def split_form(tokens: int, outs: int, inner: int, segments: int, tile: int | None = None, overlapped: bool = False) -> tuple[int, bool]:
     """Tokens per CTA (or the given ``tile``), and whether a tile's segments run in the CTAs of a cluster or one after the other in a
-    CTA; the bits are the same in every form.  The form whose rounds of resident CTAs take least time, in plain stream order or
+    CTA; the bits are the same in every form.  ``tile``: of a grouped product.  The form whose rounds of resident CTAs take least time, in plain stream order or
     (``overlapped``) as programmatic dependents."""
     blocks = -(-inner // BLOCK_K)
     per_segment = -(-blocks // segments)
     forms = []
-    for rows, (block, start) in SPLIT_TILES.items():
+    for rows, (block, start) in (SPLIT_TILES if tile is None else SPLIT_GROUPED).items():
         if (rows != tile) if tile is not None else (rows > 16 and tokens <= 16):
             continue
         per_sm = 2 if rows == 16 else 1
         pieces = SPLIT_PIECES[overlapped] if rows >= SPLIT_PIECES_MIN_TILE else 0.0
         ctas = -(-outs // BLOCK_N) * -(-tokens // rows)
-        cost = lambda resident: SPLIT_SHARED if rows == 16 and resident > NUM_SMS else block  # noqa: B023, E731
+        cost = lambda resident: SPLIT_SHARED if tile is None and rows == 16 and resident > NUM_SMS else block  # noqa: B023, E731
         if rows < 128 or segments == 1:
             forms.append((-(-ctas // (per_sm * NUM_SMS)) * (blocks * cost(ctas) + start) + pieces, rows, False))
         if segments > 1:
-            rounds = -(-ctas // (per_sm * SPLIT_CLUSTERS[segments - 1] + 2 * (per_sm - 1)))
+            rounds = -(-ctas // (per_sm * SPLIT_CLUSTERS[segments - 1] + (2 * (per_sm - 1) if tile is None else 0)))
             forms.append((rounds * (per_segment * cost(ctas * segments) + start + SPLIT_EXCHANGE * segments * rows / 128) + pieces, rows, True))
     return min(forms)[1:]
 
