@@ -32,8 +32,8 @@
 // the narrow B operand.  Warp 0 loads raw float32 tiles with TMA, warp 1 issues the MMAs, converter warps make the pieces of the
 // weights (a thread's row goes to tensor memory, where A is read from), taker warps add the sums of a block up while the MMAs of the
 // next run.  The tokens' pieces are three stacked bfloat16 tiles in shared memory, so that one MMA multiplies a piece of the weights
-// by several pieces of the tokens.  Up to 16 tokens the converters make them too; for more, a kernel before this one makes them once
-// for all feature tiles (split_rows_kernel) and they arrive by TMA.
+// by several pieces of the tokens.  With 16 tokens to a CTA the converters make them too; with 64 and 128 a kernel before this one makes
+// them once for all feature tiles (split_rows_kernel) and they arrive by TMA.  Which form a product takes is the caller's choice.
 //
 // What bounds it: the issuing thread.  Alone, the MMAs of a k block take 768 cycles with 64 tokens and 1,536 with 128.  A look at a barrier takes
 // the thread 198 cycles, also when the barrier has long completed, and only the MMAs issued before run meanwhile (`kernel_bench mma-rate`, an
@@ -57,7 +57,7 @@ __device__ int g_split_error = 0;  // 0 ok; else (role << 8) | detail of the fir
 
 // NT: tokens per CTA.  The tiles pass through the roles in units, whole k blocks or (128 tokens, for which tensor memory has
 // no room otherwise) halves of 32 k; the weights' pieces have two buffers, so that the converters write one while the MMAs read the other.
-// PRE: the tokens' pieces were made by split_rows_kernel and arrive by TMA, a block at a time; up to 16 tokens the raw tokens arrive with
+// PRE: the tokens' pieces were made by split_rows_kernel and arrive by TMA, a block at a time; with 16 tokens the raw tokens arrive with
 // the raw weights and the converters make their pieces too.
 template <int NT>
 struct SplitConfig {
